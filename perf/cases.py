@@ -333,3 +333,164 @@ def tolerance(case):
     if kind == "tiles":
         return {"rel": 1e-6, "max": 1e-5}
     return {"rel": 2e-3, "max": 4e-2} if case["tf32"] else {"rel": 6e-5, "max": 1.5e-3}
+
+
+# ---------------------------------------------------------------------------------------------------------------
+# The same results in 64 bits
+# ---------------------------------------------------------------------------------------------------------------
+
+
+def _lse(dots, scale, bias, axis):
+    """log sum exp(scale * dots + bias) along an axis, the bias running along that axis, by blocks of rows."""
+    if axis == 1:
+        return torch.cat([torch.logsumexp(scale * r + bias, dim=1) for r in dots.split(2048)])
+    return torch.cat([torch.logsumexp(scale * c + bias[:, None], dim=0) for c in dots.split(2048, dim=1)])
+
+
+def _solve(case, x, y, a, b, eps_list, extra=0.0):
+    """Potentials (f, g) and those before the last extrapolation, by the textbook iteration. `extra` is added to the
+    products x.y (the label table)."""
+    cs = 0.5 if case.get("half_cost") else 1.0
+    rx = case.get("reach_x", case.get("reach"))
+    rx, ry = (None if r is None else r * r for r in (rx, case.get("reach")))
+    al, be, la, lb = cs * (x * x).sum(1), cs * (y * y).sum(1), a.log(), b.log()
+    dots = x @ y.T + extra
+    f, g = -al, -be
+
+    def half(axis, pot, logw, eps, rho):
+        damp = 1.0 if rho is None else 1.0 / (1.0 + eps / rho)
+        return -eps * damp * _lse(dots, 2.0 * cs / eps, pot / eps + logw, axis), damp
+
+    if case.get("backend") == "alternating":
+        for eps in eps_list:
+            f, _ = half(1, g, lb, eps, rx)
+            g, _ = half(0, f, la, eps, ry)
+        return f + al, g + be, f + al, g + be
+
+    def step(f, g, eps, w):
+        (nf, df), (ng, dg) = half(1, g, lb, eps, rx), half(0, f, la, eps, ry)
+        return ((1 - w) * f + w * (nf - al * (1 - df)), (1 - w) * g + w * (ng - be * (1 - dg)))
+
+    f, g = step(f, g, eps_list[0], 1.0)
+    seen = None
+    for i, eps in enumerate(eps_list):
+        f, g = step(f, g, eps, 0.5)
+        if case.get("threshold") is not None and (i + 1) % 10 == 0:
+            if seen is not None and max((f - seen[0]).abs().max(), (g - seen[1]).abs().max()) < case["threshold"]:
+                break
+            seen = (f, g)
+    last = step(f, g, eps_list[-1], 1.0)
+    return last[0] + al, last[1] + be, f + al, g + be
+
+
+def _barycentres(x, y, pot, logw, eps, cs, extra=0.0):
+    """Rows of the plan's normalised weights times y."""
+    scores = (2.0 * cs / eps) * (x @ y.T + extra) + ((pot - cs * (y * y).sum(1)) / eps + logw)
+    return torch.softmax(scores, dim=1) @ y
+
+
+def _schedule(case, x, y):
+    if not case.get("anneal"):
+        return [case["eps"]] * case["iters"]
+    both = torch.cat([x, y])
+    diam = float((both.max(0).values - both.min(0).values).norm())
+    out, lg = [diam**2], 2.0 * math.log(diam)
+    while lg > 2.0 * math.log(case["blur"]):
+        out.append(math.exp(lg))
+        lg += 2.0 * math.log(0.5)
+    return out + [case["blur"] ** 2]
+
+
+def _term(case, x, y, a, b, same, extra=0.0):
+    """OT value and its gradients to x and y (of a self term: the whole one, and nothing)."""
+    cs = 0.5 if case.get("half_cost") else 1.0
+    eps_list = _schedule(case, x, y)
+    f, g, fg, gg = _solve(case, x, y, a, b, eps_list, extra)
+    eps, turned = eps_list[-1], extra.T if torch.is_tensor(extra) else extra
+    if case.get("reach") is not None and case.get("backend", "symmetric") == "symmetric":
+        rho = case["reach"] ** 2
+        val = (rho + eps / 2) * ((a * (1 - (-f / rho).exp())).sum() + (b * (1 - (-g / rho).exp())).sum())
+    else:
+        val = (a * f).sum() + (b * g).sum()
+    gx = 2.0 * cs * a[:, None] * (x - _barycentres(x, y, gg, b.log(), eps, cs, extra))
+    gy = 2.0 * cs * b[:, None] * (y - _barycentres(y, x, fg, a.log(), eps, cs, turned))
+    return (val, gx + gy, None) if same else (val, gx, gy)
+
+
+def _divergence(case, x, y, a, b, table=None, lx=None, ly=None):
+    def extra(p, q):
+        return 0.0 if table is None else -0.5 * case["lambda_y"] * table[p][:, q]
+
+    val, gx, gy = _term(case, x, y, a, b, False, extra(lx, ly))
+    if case["debias"]:
+        vx, gxx, _ = _term(case, x, x, a, a, True, extra(lx, lx))
+        vy, _, _ = _term(case, y, y, b, b, True, extra(ly, ly))
+        val, gx = val - 0.5 * (vx + vy), gx - 0.5 * gxx
+    return val, gx, gy
+
+
+def _hessian_product(case, x, y, v):
+    """Loss, gradient and Hessian-vector product with uniform weights and the plan as a matrix; the Schur system is
+    solved by conjugate gradients under the module's defaults."""
+    n, m, eps = x.shape[0], y.shape[0], case["eps"]
+    a, b = x.new_full((n,), 1.0 / n), y.new_full((m,), 1.0 / m)
+    f, g, fg, gg = _solve(case, x, y, a, b, [eps] * case["iters"])
+    grad = 2.0 * a[:, None] * (x - _barycentres(x, y, gg, b.log(), eps, 1.0))
+    plan = (2.0 / eps) * (x @ y.T) + ((fg - (x * x).sum(1)) / eps + a.log())[:, None]
+    plan = (plan + (gg - (y * y).sum(1)) / eps + b.log()).exp_()
+    pa, pb = plan.sum(1), plan.sum(0)
+    xv, py = (x * v).sum(1), plan @ y
+    rx, ry = 2.0 * (pa * xv - (v * py).sum(1)), 2.0 * (plan.T @ xv - (y * (plan.T @ v)).sum(1))
+    z, r = torch.zeros_like(pb), ry - plan.T @ (rx / pa)
+    p, tol = r.clone(), max(1e-6, 1e-6 * float(r.norm()))
+    for _ in range(case["cg"]):
+        ap = (pb + eps * 1e-5) * p - plan.T @ ((plan @ p) / pa)
+        rr = r @ r
+        step = rr / (p @ ap)
+        z, r = z + step * p, r - step * ap
+        if float(r.norm()) <= tol:
+            break
+        p = r + (r @ r) / rr * p
+    pz = plan @ z
+    z1 = (rx - pz) / pa
+    hv = (2.0 / eps) * (x * (pa * z1 + pz)[:, None] - py * z1[:, None] - plan @ (y * z[:, None]))
+    k = 4.0 / eps
+    hv += 2.0 * pa[:, None] * v + k * (x * ((py * v).sum(1) - xv * pa)[:, None] + py * xv[:, None])
+    hv -= k * ((plan * (v @ y.T)) @ y)
+    return dict(loss=(a * f).sum() + (b * g).sum(), grad=grad, hvp=hv)
+
+
+def exact(case, seed):
+    """What run() returns for these inputs in 64 bits, by dense formulas; None where that would take too long."""
+    n, m, kind = case["n"], case["m"], case["kind"]
+    passes = {"plan": 2, "ctrans": 1, "tiles": 100, "batch": case.get("batch", 1) * 6 * case.get("iters", 1)}.get(
+        kind, 6 * case.get("iters", 12))
+    if float(max(n, m)) ** 2 * passes > 2.0e11 or max(n, m) > 50000 or kind == "tiles":
+        return None
+    s = prepare(case, seed)
+    x, y = s["x"].detach().double(), s["y"].detach().double()
+    if kind == "loss":
+        table = s["loss"].label_cost_matrix
+        val, gx, gy = _divergence(case, x, y, s["a"].double(), s["b"].double(),
+                                  None if table is None else table.double(), s.get("label_x"), s.get("label_y"))
+        return dict(loss=val, grads=(gx, gy) if case.get("grad_y") else (gx,))
+    if kind == "batch":
+        a, b = x.new_full((n,), 1.0 / n), x.new_full((m,), 1.0 / m)
+        out = [_divergence(case, p, q, a, b) for p, q in zip(x, y)]
+        return dict(loss=torch.stack([o[0] for o in out]), grads=(torch.stack([o[1] for o in out]),))
+    if kind == "hvp":
+        return _hessian_product(case, x, y, s["v"].double())
+    if kind == "plan":
+        # f and g are the shifted potentials
+        f, g, eps = s["f"].double(), s["g"].double(), case["eps"]
+        left, right = f / eps + s["la"].double(), g / eps + s["lb"].double()
+        mat, vec = s["mat"].double(), s["vec"].double()
+        moved, mass = [], 0.0
+        for r, l, v in zip(x.split(2048), left.split(2048), vec.split(2048)):
+            p = ((2.0 / eps) * (r @ y.T) + l[:, None] + right).exp_()
+            moved.append(p @ mat)
+            mass = mass + p.T @ v
+        return dict(moved=torch.cat(moved), mass=mass)
+    price = (y * y).sum(1) - s["psi"].double()
+    best = [torch.min((r * r).sum(1)[:, None] - 2.0 * (r @ y.T) + price, dim=1) for r in x.split(2048)]
+    return dict(values=torch.cat([v for v, _ in best]), index=torch.cat([i for _, i in best]))
