@@ -4,6 +4,7 @@
 #include "../../include/flash_sinkhorn_b200.h"
 #include "fs_common.cuh"
 #include "fs_tc.cuh"
+#include "fs_sym.cuh"
 
 #include <atomic>
 #include <cmath>
@@ -366,6 +367,106 @@ inline bool label_cost_from_abi(const fs_label_cost* in, float cost_scale, Label
   return true;
 }
 
+inline double dampening(double eps, double rho);
+
+// ---------------------------------------------------------------------------
+// Symmetric solves with one exponential per entry for both potentials (fs_sym.cu). Taken at every feature dimension
+// when the scratch of the per-tile sums stays within its budget (n*m up to about 3e10) and the workspace was sized
+// for it; the reasons are in fs_sym.cu. The rest steps side by side through Problem::lse below.
+// ---------------------------------------------------------------------------
+size_t sym_workspace(int n, int m, int d, int prec, int nlab) {
+  if (prec == FS_PREC_SIMT || !sym::supported(n, m, d, prec, nlab)) return 0;
+  return sym::bytes(n, m, d, prec, nlab) + 512 + ((size_t)n + m + 128) * sizeof(float);  // + early-stop snapshot
+}
+
+struct SymSolve {
+  sym::Problem p;
+  std::vector<double> eps;  // eps of every step
+  float* pre[2] = {nullptr, nullptr};
+  float* out[2] = {nullptr, nullptr};
+  float* snap[2] = {nullptr, nullptr};
+};
+
+int sym_prepare(SymSolve& s, const float* x, const float* y, int n, int m, int d, const float* log_a,
+                const float* log_b, const float* f_init, const float* g_init, bool self, float cs_dot, float cs_sq,
+                const LabelCost& lab, int prec, void* wsp) {
+  sym::Problem& p = s.p;
+  p.src[0] = x; p.src[1] = y; p.logw[0] = log_a; p.logw[1] = log_b; p.init[0] = f_init; p.init[1] = g_init;
+  p.n[0] = n; p.n[1] = m; p.d = d; p.prec = prec; p.self = self; p.cs_dot = cs_dot; p.cs_sq = cs_sq; p.lab = lab;
+  char* base = (char*)(((uintptr_t)wsp + 255) & ~(uintptr_t)255);
+  cudaError_t e = sym::layout(p, base);
+  if (e != cudaSuccess) return fail(FS_ERR_CUDA, "symmetric solve layout failed: %s", cudaGetErrorString(e));
+  s.snap[0] = (float*)(base + sym::bytes(n, m, d, prec, 3 * lab.V));
+  s.snap[1] = s.snap[0] + ((n + 63) & ~63);
+  return FS_OK;
+}
+
+void sym_schedule(SymSolve& s, const double* eps_list, int n_eps, int last_extrapolation) {
+  s.eps.assign(1, eps_list[0]);
+  s.eps.insert(s.eps.end(), eps_list, eps_list + n_eps);
+  if (last_extrapolation) s.eps.push_back(eps_list[n_eps - 1]);
+}
+
+// Lockstep: step t of every problem that still has one. threshold < 0: no early stopping (one problem otherwise).
+int sym_run(SymSolve* s, int cnt, int last_extrapolation, double rho_x, double rho_y, double threshold,
+            int check_every, cudaStream_t st) {
+  sym::Problem* probs[sym::kMaxProblems];
+  double eps0[sym::kMaxProblems];
+  size_t steps = 0;
+  for (int i = 0; i < cnt; ++i) {
+    probs[i] = &s[i].p;
+    eps0[i] = s[i].eps[0];
+    steps = s[i].eps.size() > steps ? s[i].eps.size() : steps;
+  }
+  FS_CUDA(sym::stage(probs, eps0, cnt, st));
+  const bool early = threshold >= 0.0;
+  for (size_t t = 0; t < steps; ++t) {
+    sym::Step batch[sym::kMaxProblems];
+    sym::Problem* last[sym::kMaxProblems];
+    float* pre[sym::kMaxProblems][2];
+    int k = 0, n_last = 0;
+    for (int i = 0; i < cnt; ++i) {
+      const size_t total = s[i].eps.size();
+      if (t >= total) continue;
+      const bool is_last = last_extrapolation && t + 1 == total;
+      if (is_last && (s[i].pre[0] || s[i].pre[1])) {
+        last[n_last] = &s[i].p;
+        pre[n_last][0] = s[i].pre[0];
+        pre[n_last++][1] = s[i].pre[1];
+      }
+      sym::Step& b = batch[k++];
+      b.p = &s[i].p;
+      b.eps = s[i].eps[t];
+      b.eps_prev = t ? s[i].eps[t - 1] : b.eps;
+      b.eps_next = t + 1 < total ? s[i].eps[t + 1] : b.eps;
+      b.w = (t == 0 || is_last) ? 1.0f : 0.5f;
+      b.damp[0] = (float)dampening(b.eps, rho_x);
+      b.damp[1] = (float)dampening(b.eps, rho_y);
+      b.early = early && t > 0 && !is_last;
+    }
+    if (n_last) FS_CUDA(sym::emit(last, pre, n_last, st));
+    FS_CUDA(sym::step(batch, k, (int)t, st));
+    const sym::Problem& p = s[0].p;
+    if (early && batch[0].early && t % (size_t)check_every == 0) {
+      const int n = p.n[0], m = p.n[1];
+      delta_kernel<<<g1(n + m), 256, 0, st>>>(p.pot[0], s[0].snap[0], n, p.pot[1], s[0].snap[1], m, p.ctrl);
+      decide_kernel<<<1, 1, 0, st>>>(p.ctrl, threshold);
+      snapshot_kernel<<<g1(n + m), 256, 0, st>>>(p.pot[0], s[0].snap[0], n, p.pot[1], s[0].snap[1], m, p.ctrl);
+    }
+  }
+  float* out[sym::kMaxProblems][2];
+  for (int i = 0; i < cnt; ++i)
+    for (int c = 0; c < 2; ++c) out[i][c] = s[i].out[c];
+  FS_CUDA(sym::emit(probs, out, cnt, st));
+  if (!last_extrapolation) {
+    for (int i = 0; i < cnt; ++i)
+      for (int c = 0; c < 2; ++c) out[i][c] = s[i].pre[c];
+    FS_CUDA(sym::emit(probs, out, cnt, st));
+  }
+  FS_CUDA(cudaGetLastError());
+  return FS_OK;
+}
+
 inline double dampening(double eps, double rho) {
   if (!(rho >= 0.0)) return 1.0;  // negative or NaN: balanced
   return 1.0 / (1.0 + eps / rho);
@@ -389,9 +490,15 @@ int fs_version(void) { return 200; }  // 0.2.0
 
 long long fs_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
 
-int fs_device_error(void) { return tc::read_error_flag(); }
+int fs_device_error(void) {
+  const int a = tc::read_error_flag(), b = sym::read_error_flag();
+  return a < 0 || b < 0 ? -1 : (a | b);
+}
 
-int fs_clear_device_error(void) { return tc::clear_error_flag(); }
+int fs_clear_device_error(void) {
+  const int a = tc::clear_error_flag(), b = sym::clear_error_flag();
+  return a ? a : b;
+}
 
 size_t fs_apply_mat_plan_bytes(int n, int m, int d, int dv, int prec) {
   if (n <= 0 || m <= 0 || d <= 0 || dv <= 0) return 0;
@@ -415,6 +522,8 @@ int fs_engine(int n, int m, int d, int prec) {
   if (prec == FS_PREC_SIMT || !tc::supported(n, m, d, prec, 0)) return 0;
   return tc::k_streamed(d, prec, 0) ? 2 : 1;
 }
+
+int fs_two_sided(int n, int m, int d, int prec) { return sym_workspace(n, m, d, prec, 0) > 0 ? 1 : 0; }
 
 int fs_plan_pv_split(int rows, int cols, int prec, int sms, int* slots) {
   return tc::plan_pv_split(rows, cols, prec, sms, slots);
@@ -461,6 +570,8 @@ size_t fs_workspace_bytes_labels(int op, int n, int m, int d, int prec, int n_cl
     case FS_OP_SOLVE_ALTERNATING: {
       SolveBufs b;
       carve_solve(ws, b, n, m);
+      const size_t two_sided = op == FS_OP_SOLVE_SYMMETRIC ? sym_workspace(n, m, d, prec, p.nlab) : 0;
+      if (two_sided > ws.off) ws.off = two_sided;
       break;
     }
     case FS_OP_APPLY_VEC:
@@ -565,6 +676,22 @@ int fs_solve_symmetric(const float* x, const float* y, int n, int m, int d, cons
   LabelCost lc;
   float cs_kernel;
   if (!label_cost_from_abi(labels, cost_scale, lc, cs_kernel)) return fail(FS_ERR_BAD_ARG, "invalid label cost descriptor");
+  // Self-transport problem (the debiasing terms OT(a,a), OT(b,b)): same cloud, weights, penalties and
+  // initial potentials on both sides. Both Jacobi updates then read identical inputs, so g equals f after every
+  // step and one of them is enough.
+  const bool self_problem = x == y && n == m && log_a == log_b && f_init == g_init && rho_x == rho_y &&
+                            lc.V == 0;  // a label table need not be symmetric: keep both sides then
+  const size_t two_sided = sym_workspace(n, m, d, prec, 3 * lc.V);
+  if (two_sided > 0 && two_sided <= ws_bytes) {
+    SymSolve s;
+    FS_TRY(sym_prepare(s, x, y, n, m, d, log_a, log_b, f_init, g_init, self_problem, cs_kernel, cost_scale, lc, prec, wsp));
+    sym_schedule(s, eps_list, n_eps, last_extrapolation);
+    s.pre[0] = f_pre; s.pre[1] = g_pre; s.out[0] = f; s.out[1] = g;
+    FS_TRY(sym_run(&s, 1, last_extrapolation, rho_x, rho_y, threshold, check_every, st));
+    if (iters_used) copy_int_kernel<<<1, 1, 0, st>>>(&s.p.ctrl->iters_used, iters_used);
+    FS_CUDA(cudaGetLastError());
+    return FS_OK;
+  }
   // lambda_x scales the dot term only; the shifts alpha, beta below keep the plain cost scale (as the reference does)
   FS_TRY(make_problem(p, ws, x, y, n, m, d, cs_kernel, prec, st, false, 0, true, &lc));
   SolveBufs b;
@@ -578,12 +705,6 @@ int fs_solve_symmetric(const float* x, const float* y, int n, int m, int d, cons
   axpby_kernel<<<g1(n), 256, 0, st>>>(n, 1.f, f_init, -1.f, b.alpha, b.fh[0]);
   axpby_kernel<<<g1(m), 256, 0, st>>>(m, 1.f, g_init, -1.f, b.beta, b.gh[0]);
   FS_CUDA(cudaGetLastError());
-
-  // Self-transport problem (the debiasing terms OT(a,a), OT(b,b)): same cloud, weights, penalties and
-  // initial potentials on both sides. Both Jacobi updates then read identical inputs through the same
-  // kernel, so g equals f bit for bit after every step: run one soft-min per step and copy its result.
-  const bool self_problem = x == y && n == m && log_a == log_b && f_init == g_init && rho_x == rho_y &&
-                            lc.V == 0;  // a label table need not be symmetric: keep both sides then
 
   int cur = 0;
   auto step = [&](double eps, float w, bool in_loop) -> int {
@@ -991,6 +1112,17 @@ extern "C" int fs_symmetric_step_multi(const fs_step_item* items, int n_items, i
   return FS_OK;
 }
 
+namespace {
+int check_batch_item(const fs_batch_item& in, int i, int d, float cost_scale, int prec) {
+  if (!in.eps_list_host || in.n_eps <= 0) return fail(FS_ERR_BAD_ARG, "item %d: eps_list must be non-empty", i);
+  FS_TRY(check_common(in.x, in.y, in.n, in.m, d, (float)in.eps_list_host[0], cost_scale, prec));
+  for (int k = 0; k < in.n_eps; ++k)
+    if (!(in.eps_list_host[k] > 0.0)) return fail(FS_ERR_BAD_ARG, "item %d: eps_list[%d] must be > 0", i, k);
+  if (!in.log_a || !in.log_b || !in.f || !in.g) return fail(FS_ERR_BAD_ARG, "item %d: log_a, log_b, f, g must be non-null", i);
+  return FS_OK;
+}
+}  // namespace
+
 // Several symmetric solves in lockstep (batched inputs, or the three problems of a debiased loss): every step of
 // all problems that still have one goes out as fused multi-pass launches, so B small problems cost about one
 // solve's worth of launches instead of B. Schedules may differ in length; a finished problem drops out.
@@ -1001,6 +1133,28 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
     return fail(FS_ERR_BAD_ARG, "fs_solve_symmetric_batched takes 1..%d items", kMaxBatch);
   FS_TRY(check_device());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  bool two_sided = true;
+  for (int i = 0; i < n_items && two_sided; ++i) {
+    const size_t need = items[i].n > 0 && items[i].m > 0 ? sym_workspace(items[i].n, items[i].m, d, prec, 0) : 0;
+    two_sided = need > 0 && need <= items[i].ws_bytes && items[i].ws;
+  }
+  if (two_sided) {
+    for (int i = 0; i < n_items; ++i) FS_TRY(check_batch_item(items[i], i, d, cost_scale, prec));
+    for (int i0 = 0; i0 < n_items; i0 += sym::kMaxProblems) {
+      const int cnt = n_items - i0 < sym::kMaxProblems ? n_items - i0 : sym::kMaxProblems;
+      std::vector<SymSolve> ss(cnt);
+      for (int k = 0; k < cnt; ++k) {
+        const fs_batch_item& in = items[i0 + k];
+        const bool self = in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y;
+        FS_TRY(sym_prepare(ss[k], in.x, in.y, in.n, in.m, d, in.log_a, in.log_b, nullptr, nullptr, self, cost_scale,
+                           cost_scale, LabelCost(), prec, in.ws));
+        sym_schedule(ss[k], in.eps_list_host, in.n_eps, last_extrapolation);
+        ss[k].pre[0] = in.f_pre; ss[k].pre[1] = in.g_pre; ss[k].out[0] = in.f; ss[k].out[1] = in.g;
+      }
+      FS_TRY(sym_run(ss.data(), cnt, last_extrapolation, rho_x, rho_y, -1.0, 1, st));
+    }
+    return FS_OK;
+  }
   struct Item {
     Problem p;
     SolveBufs b;
@@ -1011,11 +1165,7 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
   int max_steps = 0;
   for (int i = 0; i < n_items; ++i) {
     const fs_batch_item& in = items[i];
-    if (!in.eps_list_host || in.n_eps <= 0) return fail(FS_ERR_BAD_ARG, "item %d: eps_list must be non-empty", i);
-    FS_TRY(check_common(in.x, in.y, in.n, in.m, d, (float)in.eps_list_host[0], cost_scale, prec));
-    for (int k = 0; k < in.n_eps; ++k)
-      if (!(in.eps_list_host[k] > 0.0)) return fail(FS_ERR_BAD_ARG, "item %d: eps_list[%d] must be > 0", i, k);
-    if (!in.log_a || !in.log_b || !in.f || !in.g) return fail(FS_ERR_BAD_ARG, "item %d: log_a, log_b, f, g must be non-null", i);
+    FS_TRY(check_batch_item(in, i, d, cost_scale, prec));
     Item& it = its[i];
     Ws ws(in.ws, in.ws_bytes);
     FS_TRY(make_problem(it.p, ws, in.x, in.y, in.n, in.m, d, cost_scale, prec, st, false));

@@ -1273,6 +1273,13 @@ void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const f
                                                        ctrl, pot_shard, pot_stride);
 }
 
+int free_ctas() {
+  int g = sm_count() - g_reserved_sms.load(std::memory_order_relaxed);
+  const int limit = g_cta_limit.load(std::memory_order_relaxed);
+  if (limit >= 1 && limit < g) g = limit;
+  return g < 1 ? 1 : g;
+}
+
 int pick_ctas(int nblk, int ntiles) {
   return pick_ctas_for(nblk, ntiles, sm_count(), g_reserved_sms.load(std::memory_order_relaxed),
                        g_cta_limit.load(std::memory_order_relaxed));

@@ -125,6 +125,8 @@ bool encode_map(CUtensorMap* map, const float* base, long long rows, long long k
                 CUtensorMapSwizzle swz, long long row_pitch = 0);
 int pick_ctas(int nblk, int ntiles);
 int sm_count();
+// SMs a single-wave launch may take: all of them minus the reserved ones, within the CTA limit.
+int free_ctas();
 // Writes the column bias of a pass (divided by the logit scale, split into three TF32 pieces) into the bias
 // columns of the column operand.
 void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,

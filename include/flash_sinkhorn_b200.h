@@ -133,6 +133,10 @@ int fs_set_pv_split(int split);
  * with the row operand resident in shared memory, 2 = tcgen05 with both operands streamed in K chunks. */
 int fs_engine(int n, int m, int d, int prec);
 
+/* 1 when symmetric solves of these sizes evaluate each score entry once for both potentials and share the launches
+ * of a lockstep solve (fs_solve_symmetric_batched), 0 when they step side by side. */
+int fs_two_sided(int n, int m, int d, int prec);
+
 /* Host arithmetic only (no reference counterpart): the CTA count a streaming pass over n_row_blocks x
  * n_col_tiles work items gets on a device with `sms` SMs when `reserved` of them are left free and the CTA
  * limit is `limit` (0 = none). At most 16 CTAs ever share a row block. Returns 0 on non-positive sizes. */

@@ -1,0 +1,106 @@
+"""Symmetric solves that take one exponential per score entry for both potentials: edges of the tiles, the kernels
+for every contraction length, self-transport triangles, and inputs that force the one-sided steps."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import dev, host, rel
+from oracle import dense_sinkhorn as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def cta_limit():
+    """Few CTAs: small problems then share tiles and column runs the way large ones do on all SMs."""
+    from flash_sinkhorn_b200 import _lib
+    lib = _lib.load()
+    previous = lib.fs_set_cta_limit(0)
+    yield lib.fs_set_cta_limit
+    lib.fs_set_cta_limit(previous)
+
+
+def _clouds(n, m, d, seed=0, zeros=False):
+    r = np.random.default_rng(seed)
+    x, y = r.normal(size=(n, d)), 0.3 + r.normal(size=(m, d))
+    a, b = r.uniform(0.1, 1.1, n), r.uniform(0.1, 1.1, m)
+    if zeros:
+        a[::3] = 0.0
+    x, y, a, b = (np.float32(v).astype(np.float64) for v in (x, y, a / a.sum(), b / b.sum()))
+    return x, y, a, b
+
+
+def _solve(x, y, a, b, prec, **kw):
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric
+    xd, ad = dev(x), dev(a)
+    yd, bd = (xd, ad) if y is x else (dev(y), dev(b))
+    return sinkhorn_flashstyle_symmetric(xd, yd, ad, bd, allow_tf32=prec == "tf32", return_prelast=True,
+                                         use_epsilon_scaling=False, **kw)
+
+
+# (n, m, d): single points, one less and one more than a tile, runs that end inside a column tile; contractions that
+# stay in shared memory (3 to 64), K-streamed (200, 330) and long (1100)
+SHAPES = [(1, 1, 3), (1, 300, 7), (257, 1, 40), (128, 256, 64), (129, 257, 64), (511, 769, 3), (900, 640, 64),
+          (300, 515, 200), (513, 300, 330), (260, 520, 1100)]
+
+
+@pytest.mark.parametrize("limit", [1, 3, 0])
+@pytest.mark.parametrize("prec", ["fp32", "tf32"])
+@pytest.mark.parametrize("n,m,d", SHAPES)
+def test_potentials_against_the_oracle(cta_limit, n, m, d, prec, limit):
+    """eps small enough for one-sided first steps, then two-sided ones. Tolerances: fp32 potentials of size |x|^2
+    carry 2^-24 of it per step, which 14 averaged steps do not amplify (1e-5 allows 100 ulp); TF32 coordinates
+    move each squared distance by up to 2^-11 of |x||y|, 2e-3 of the largest potential."""
+    cta_limit(limit)
+    x, y, a, b = _clouds(n, m, d)
+    eps = 0.02 * d
+    want = O.solve_symmetric(x, y, a, b, [eps] * 14)
+    got = _solve(x, y, a, b, prec, eps=eps, n_iters=14)
+    tol = 1e-5 if prec == "fp32" else 2e-3
+    size = max(np.abs(want["f"]).max(), (x * x).sum(1).max())
+    for g, k in zip(got, ("f", "g", "f_pre", "g_pre")):
+        assert np.abs(host(g) - want[k]).max() < tol * size
+
+
+@pytest.mark.parametrize("limit", [2, 0])
+@pytest.mark.parametrize("n,d", [(1, 5), (130, 64), (385, 16), (640, 64), (300, 200), (515, 1100)])
+def test_self_transport_triangle(cta_limit, n, d, limit):
+    """One cloud against itself: only one side of the diagonal is evaluated."""
+    cta_limit(limit)
+    x, _, a, _ = _clouds(n, n, d, seed=1)
+    eps = 0.02 * d
+    want = O.solve_symmetric(x, x, a, a, [eps] * 10, rho_x=4.0, rho_y=4.0)
+    got = _solve(x, x, a, a, "fp32", eps=eps, n_iters=10, reach=2.0)
+    size = max(np.abs(want["f"]).max(), (x * x).sum(1).max())
+    assert torch.equal(got[0], got[1])
+    assert np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size
+
+
+@pytest.mark.parametrize("limit", [2, 0])
+def test_zero_weights_schedules_and_early_stop(cta_limit, limit):
+    """Zero weights and a rising eps have no bound on the next step's range: one-sided throughout, same results."""
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric
+    cta_limit(limit)
+    x, y, a, b = _clouds(400, 300, 32, seed=2, zeros=True)
+    sched = [4.0, 1.0, 0.5, 2.0, 0.25, 0.25]
+    want = O.solve_symmetric(x, y, a, b, sched)
+    got = sinkhorn_flashstyle_symmetric(dev(x), dev(y), dev(a), dev(b), eps_list=sched, allow_tf32=False)
+    size = (x * x).sum(1).max()
+    assert np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size
+    assert np.abs(host(got[1]) - want["g"]).max() < 1e-5 * size
+    x, y, a, b = _clouds(400, 300, 32, seed=3)
+    want = O.solve_symmetric(x, y, a, b, [8.0] * 60, threshold=1e-3, check_every=4)
+    got = sinkhorn_flashstyle_symmetric(dev(x), dev(y), dev(a), dev(b), eps=8.0, n_iters=60, use_epsilon_scaling=False,
+                                        threshold=1e-3, check_every=4, allow_tf32=False, return_n_iters=True)
+    assert got[2] == want["n_iters"] and np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size
+
+
+def test_not_a_number_stays_with_its_point(cta_limit):
+    """No bound on the range can be given: one-sided steps to the end, and no wait runs out."""
+    from flash_sinkhorn_b200 import _lib
+    cta_limit(2)
+    x, y, a, b = _clouds(300, 300, 64, seed=4)
+    x[17, 3] = np.nan
+    f = _solve(x, y, a, b, "tf32", eps=1.0, n_iters=5)[0]
+    torch.cuda.synchronize()
+    assert torch.isnan(f[17]) and _lib.load().fs_device_error() == 0
