@@ -3,6 +3,7 @@
 // internal to the including file.
 #pragma once
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -219,6 +220,75 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, u
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// kind::f16 with fp16 operands and an fp32 accumulator: K = 16 per instruction over the same 32 bytes of an operand
+// row that hold 8 TF32 values, at the same clocks - twice the products per instruction and per byte.
+__host__ __device__ constexpr uint32_t make_idesc_f16(int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+}
+// One 32-byte K step of an operand row: 16 scaled fp16 coordinates (half) or 8 TF32 columns.
+__device__ __forceinline__ void umma_step(bool half, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc_tf32,
+                                          uint32_t idesc_f16, uint32_t accumulate) {
+  if (half) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc_f16), "r"(accumulate)
+        : "memory");
+  } else {
+    umma_tf32(d_tmem, adesc, bdesc, idesc_tf32, accumulate);
+  }
+}
+
+// Power of two that brings a cloud whose largest |coordinate| has these float bits to [2^14, 2^15): there an fp16
+// carries the 11 significant bits of a TF32 value over 28 octaves and an absolute 2^-39 of the largest below that,
+// far under the fp32 rounding of the contraction. All-zero and non-finite clouds are left as they are; the limits
+// keep the product of two scales well inside the exponent range of the bias columns it multiplies (coordinates
+// beyond 2^64 overflow fp32 when squared anyway).
+__device__ __forceinline__ float cloud_scale(unsigned amax_bits) {
+  const int e = (int)(amax_bits >> 23);
+  if (amax_bits == 0u || e >= 255) return 1.f;
+  int k = 14 - (e - 127);
+  k = k > 30 ? 30 : (k < -50 ? -50 : k);
+  return __uint_as_float((unsigned)(k + 127) << 23);
+}
+// Product of the two clouds' scales (amax[0], amax[1]); 1 where the operands are not scaled (null).
+__device__ __forceinline__ float pair_scale(const unsigned* amax) {
+  return amax ? cloud_scale(amax[0]) * cloud_scale(amax[1]) : 1.f;
+}
+// Coordinate column k (32-bit word) of a staged operand row, row role (va) and column role (vb). parts = 1: the
+// coordinates to 11 significant bits; parts = 3: [hi | hi | lo] against [hi | lo | hi], 22 bits and a product that
+// drops only lo.lo. hs > 0: hs K steps of 16 scaled fp16 values, two per word, every part padded to whole steps;
+// hs == 0: TF32 values, one per word.
+__device__ __forceinline__ void stage_coord(const float* row, int k, int d, int parts, int hs, float scale, float& va,
+                                            float& vb) {
+  if (hs > 0) {
+    const int words = hs * 8 / parts, part = k / words, c = 2 * (k - part * words);
+    // rounded as TF32 values first (ties away from zero): the conversions of the scaled pieces are then exact
+    const float x0 = c < d ? row[c] : 0.f, x1 = c + 1 < d ? row[c + 1] : 0.f, h0 = to_tf32(x0), h1 = to_tf32(x1);
+    const __half2 hi = __floats2half2_rn(h0 * scale, h1 * scale);
+    const __half2 lo = __floats2half2_rn(to_tf32(x0 - h0) * scale, to_tf32(x1 - h1) * scale);
+    const __half2 a = part == 2 ? lo : hi, b = part == 1 ? lo : hi;
+    va = __uint_as_float(*reinterpret_cast<const unsigned*>(&a));
+    vb = __uint_as_float(*reinterpret_cast<const unsigned*>(&b));
+  } else {
+    const int part = k / d;
+    const float x = row[k - part * d], hi = to_tf32(x), lo = to_tf32(x - hi);
+    va = part == 2 ? lo : hi;
+    vb = part == 1 ? lo : hi;
+  }
+}
+// Largest |value| of an array as float bits (NaN and inf come out above every finite value). *out starts at zero.
+__device__ __forceinline__ void block_amax(const float* v, size_t count, size_t first, size_t stride, unsigned* out) {
+  unsigned m = 0u;
+  for (size_t i = first; i < count; i += stride) {
+    const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
+    m = b > m ? b : m;
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
 // Round-to-nearest (ties away) onto the 10-bit TF32 mantissa with two integer operations; the conversion

@@ -8,7 +8,8 @@
 // exact to 2^-33): the row operand carries (x | 1 1 1 | f pieces), the column operand (y | g pieces | 1 1 1), and
 // the drained accumulator times the logit scale is the finished exponent - no running maximum, no rescaling.
 // A self-transport problem (x = y, a = b) has a symmetric E: only the tiles on one side of the diagonal are
-// evaluated, their column sums standing in for the mirrored rows.
+// evaluated, their column sums standing in for the mirrored rows. (Coordinates are staged as scaled fp16 where that
+// takes fewer K steps, see Layout; the scales are powers of two and are taken out of the logit scale again.)
 //
 // Which steps. Without a running maximum the sums must stay inside the fp32 exponent range. After every step the
 // finalising kernel knows, per row, L_i = log2 sum_j b_j 2^{z_ij} (z = the exponent without the weights) and the
@@ -28,7 +29,7 @@
 // registers over a whole run of tiles: a column costs one FADD per entry and one cross-lane reduction per run.
 // The row sum of a tile is one value per thread; warp 2 adds the four warpgroups' parts and stores one value per
 // row and 256 columns (n*m/64 bytes in all, L2-resident at 50k x 50k), which the finalising kernel adds up.
-//   warp 0 TMA producer, warp 1 tcgen05.mma issuer (M = 128, N = 256, kind::tf32) and TMEM owner, warp 2 row-sum
+//   warp 0 TMA producer, warp 1 tcgen05.mma issuer (M = 128, N = 256) and TMEM owner, warp 2 row-sum
 //   collector, warps 4..19 four soft-max warpgroups, one per 64 columns.
 // What bounds it: the ex2 pipe (16 per clock and SM): 2048 clocks per tile against 128 per K step of tensor pipe;
 // operand traffic is one 128-row tile per 2048 clocks (18 bytes per clock and SM at d = 64).
@@ -66,6 +67,7 @@ struct Sub {
 template <int NS>
 struct Launch {
   int nsub, nfull, ntail, nstage, slot;
+  int hs;      // leading K steps that hold fp16 coordinates
   int two_ok;  // 0: every problem of this launch runs one-sided
   Sub sub[NS];
 };
@@ -145,6 +147,9 @@ __device__ bool two_sided(const Geo& g, int slot) {
   const float col_hi = r * (ug + df_max) + (r - 1.f) * wa, col_lo = r * (lg + df_min) - (r - 1.f) * mass_a;
   return row_hi + la <= 120.f && row_lo - wa >= -90.f && col_hi + lb <= 120.f && col_lo - wb >= -90.f;
 }
+
+// What a score is multiplied by in the contraction: the product of the two clouds' scales.
+__device__ __forceinline__ float unit_of(const Geo& g) { return g.scaled ? pair_scale(g.st->amax) : 1.f; }
 
 // Items of a launch: problem after problem; two-sided: column tile after column tile, all its row tiles (from the
 // diagonal on for a self problem); one-sided: side 0 that way, then side 1.
@@ -388,7 +393,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
     }
   } else if (warp == 1) {
     // ===================== MMA issuer (all lanes in the loop, one elected lane issues) =====================
-    constexpr uint32_t idesc = make_idesc(kBN);
+    constexpr uint32_t idesc = make_idesc(kBN), idesc_h = make_idesc_f16(kBN);
     auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
     bool ok = true;
     int jt = 0, seg = 0;
@@ -410,7 +415,8 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
             const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
 #pragma unroll 1
             for (int ks = 0; ks < steps; ++ks)
-              umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, (kc | ks) != 0);
+              umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                        idesc, idesc_h, (kc | ks) != 0);
             umma_commit(bar(A_EMPTY + st));
             if (kc + 1 == P.nfull) umma_commit(bar(S_FULL + buf));
           }
@@ -435,21 +441,24 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
         tc_fence_after();
         if (elect_one()) {
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
+          int left = P.hs;  // fp16 K steps to go
           uint32_t al = desc_lo(smem_u32(a_smem + st * a_bytes)), bl = desc_lo(smem_u32(b_smem));
           uint32_t acc = 0;
 #pragma unroll 1
           for (int kb = 0; kb < P.nfull; ++kb) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-              umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, acc);
+              umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc,
+                        idesc_h, acc);
               acc = 1;
             }
+            left -= 4;
             al += (128 * 128) >> 4;
             bl += (kBN * 128) >> 4;
           }
 #pragma unroll 1
           for (int k = 0; k < P.ntail; ++k) {
-            umma_tf32(d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, acc);
+            umma_step(left > k, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
             acc = 1;
             al += (128 * 32) >> 4;
             bl += (kBN * 32) >> 4;
@@ -549,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
 #pragma unroll 1
     for (int w = w_begin; w < w_end;) {
       const Seg s = locate(P, *plan, w, w_end);
-      const float scale = P.sub[s.sub].scale2;
+      const float scale = P.sub[s.sub].scale2 / unit_of(P.sub[s.sub].geo);  // exact: a power of two
       if (s.two) {
         const Geo& g = P.sub[s.sub].geo;
         const u64 sc = pk(scale, scale);
@@ -762,7 +771,7 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
     }
   } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
     const int h = warp == 1 ? 0 : 1;
-    constexpr uint32_t idesc = make_idesc(BN);
+    constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
     auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
     bool ok = true;
     int s = 0, jt = 0;
@@ -783,7 +792,8 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks)
           if (ks < steps && elect_one())
-            umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, (kc | ks) != 0);
+            umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                      idesc, idesc_h, (kc | ks) != 0);
         if (elect_one()) umma_commit(bar(EMPTY + s));
         __syncwarp();
         if (++s == P.nstage) { s = 0; ph ^= 1; }
@@ -800,7 +810,7 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
   } else if (warp >= 4) {
     const int wg = (warp - 4) >> 2, h = wg / PARTS, part = wg % PARTS, q = warp & 3;
     const int trow = h * 128 + q * 32 + lane, et = tid - 128;  // row inside the tile, epilogue thread
-    const float scale = u.scale2;
+    const float scale = u.scale2 / unit_of(g);  // exact: a power of two
     bool ok = true;
     int jt = 0;
 #pragma unroll 1
@@ -1014,8 +1024,9 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
     const float now = (float)v;
     u.pot[c][i] = now;
     const size_t at = (size_t)i * P.kp + P.kc;
-    write_bias(u.opA[c] + at + 3, ((double)now + own * u.eps_next) * u.inv2cs);
-    write_bias(u.opB[c] + at, ((double)now + lw * u.eps_next) * u.inv2cs);
+    const double to_unit = u.inv2cs * (double)unit_of(g);
+    write_bias(u.opA[c] + at + 3, ((double)now + own * u.eps_next) * to_unit);
+    write_bias(u.opB[c] + at, ((double)now + lw * u.eps_next) * to_unit);
     const float big_l = (float)((double)l2 - own * 1.4426950408889634);
     const float dlt = (float)(((double)now - old) * 1.4426950408889634 / u.eps);
     st_u = big_l + dlt;
@@ -1060,7 +1071,7 @@ struct StageSub {
 };
 template <int NS>
 struct StageLaunch {
-  int nsub, d, kc, kp, prec, cloud;
+  int nsub, d, kcoord, kc, kp, hs, prec, cloud;
   StageSub sub[NS];
 };
 
@@ -1074,11 +1085,20 @@ __global__ void sym_reset_kernel(const __grid_constant__ StageLaunch<NS> P) {
     st->slot[1][k] = st->slot[2][k] = 0u;
   }
   for (int k = 0; k < 4; ++k) st->cst[k] = 0u;
+  st->amax[0] = st->amax[1] = 0u;
   Ctrl* c = P.sub[i].ctrl;
   c->delta_bits = 0u; c->converged = 0; c->have_prev = 0; c->iters_used = 0;
 }
 
-// One warp per point of cloud P.cloud: both operand rows (TF32 rounding or hi/lo split, label columns), the squared
+template <int NS>
+__global__ void __launch_bounds__(256) sym_amax_kernel(const __grid_constant__ StageLaunch<NS> P) {
+  const StageSub& u = P.sub[blockIdx.y];
+  const int c = blockIdx.z;  // a self problem reads its cloud twice: both words are its own
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  block_amax(u.src[c], (size_t)u.n[c] * P.d, first, stride, &u.st->amax[c]);
+}
+
+// One warp per point of cloud P.cloud: both operand rows (stage_coord, label columns), the squared
 // norm, the initial shifted potential and the biases of the first step; column layout as in the header comment with
 // kc = coordinate and label columns.
 template <int NS>
@@ -1092,7 +1112,8 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
   __syncthreads();
   const int r = (int)blockIdx.x * 8 + warp;
   const bool real = r < u.n[c];
-  const int d = P.d, kc = P.kc, kp = P.kp, kcoord = P.prec == 0 ? d : 3 * d;
+  const int d = P.d, kc = P.kc, kp = P.kp, kcoord = P.kcoord;
+  const float own = P.hs ? cloud_scale(u.st->amax[c]) : 1.f, unit = P.hs ? pair_scale(u.st->amax) : 1.f;
   const float* src = u.src[c] + (size_t)r * d;
   float* rowA = u.opA[c] + (size_t)r * kp;
   float* rowB = u.opB[c] + (size_t)r * kp;
@@ -1106,20 +1127,12 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
     if (k >= kc && k < kc + 6) continue;
     float va = 0.f, vb = 0.f;
     if (k < kcoord && real) {
-      const int part = k / d;
-      const float x = src[k - part * d];
-      const float hi = to_tf32(x);
-      va = vb = hi;
-      if (P.prec != 0) {
-        const float lo = to_tf32(x - hi);
-        va = part == 2 ? lo : hi;
-        vb = part == 1 ? lo : hi;
-      }
+      stage_coord(src, k, d, P.prec == 0 ? 1 : 3, P.hs, own, va, vb);
     } else if (k < kc && real) {
       const int v = (k - kcoord) / 3, piece = (k - kcoord) % 3;
       va = lab == v ? 1.f : 0.f;
       // column role: the table entry between every class v of the other cloud and this point's label
-      const float w = u.w_coef * u.W[c == 0 ? lab * u.V + v : v * u.V + lab];
+      const float w = unit * u.w_coef * u.W[c == 0 ? lab * u.V + v : v * u.V + lab];
       const float h = to_tf32(w), mid = to_tf32(w - h), low = to_tf32(w - h - mid);
       vb = piece == 0 ? h : (piece == 1 ? mid : low);
     }
@@ -1137,8 +1150,8 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
       const float lw = u.logw[c][r];
       u.sq[c][r] = sq;
       u.pot[c][r] = pot;
-      write_bias(rowA + kc + 3, ((double)pot + own_logw(lw) * u.eps) * u.inv2cs);
-      write_bias(rowB + kc, ((double)pot + (double)lw * u.eps) * u.inv2cs);
+      write_bias(rowA + kc + 3, ((double)pot + own_logw(lw) * u.eps) * u.inv2cs * (double)unit);
+      write_bias(rowB + kc, ((double)pot + (double)lw * u.eps) * u.inv2cs * (double)unit);
       float l2 = lw * kLog2e;
       if (!(fabsf(l2) < 1e30f)) l2 = -1e30f;  // such a weight keeps every step one-sided
       atomicMax(&wmax[0], enc(-l2));
@@ -1173,7 +1186,7 @@ __global__ void sym_emit_kernel(const __grid_constant__ EmitJobs P) {
 enum Kind { RESIDENT = 0, STREAMED = 1, WIDE = 2, SMALL = 3 };
 struct Shape {
   int kind, bm, bn;
-  int kc, kp, nfull, ntail, nstage;  // K-streamed kinds: nfull chunks of 32 words, the last one with ntail K steps
+  int hs, kc, kp, nfull, ntail, nstage;  // K-streamed kinds: nfull chunks of 32 words, the last one with ntail K steps
   size_t smem;
 };
 
@@ -1181,8 +1194,10 @@ inline int tiles(int n, int t) { return (n + t - 1) / t; }
 
 Shape plan_shape(int n, int m, int d, int prec, int nlab) {
   Shape s{};
-  s.kc = (prec == 0 ? d : 3 * d) + nlab;
-  s.kp = (s.kc + kAug + 7) & ~7;
+  const tc::Layout l = tc::operand_layout(d, prec, nlab, kAug);
+  s.kc = l.kc;
+  s.kp = l.kp;
+  s.hs = l.hs;
   const size_t row = (size_t)s.kp * 4, budget = kSmemMax - kOverhead;
   s.bm = 128;
   s.bn = kBN;
@@ -1252,6 +1267,7 @@ size_t carve(Problem& p, char* buf) {
   g.bm = sh.bm;
   g.bn = sh.bn;
   g.by_tile = sh.kind >= WIDE ? 1 : 0;
+  g.scaled = sh.hs > 0 ? 1 : 0;
   for (int k = 0; k < 2; ++k) {
     g.n[k] = p.n[k];
     g.pad[k] = tc::detail::pad256(p.n[k]);
@@ -1301,6 +1317,7 @@ cudaError_t step_n(const Step* s, int cnt, int t, cudaStream_t st) {
   FinLaunch<NS> fp;
   lp.nsub = fp.nsub = cnt;
   lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage;
+  lp.hs = sh.hs;
   lp.slot = fp.slot = t % 3;
   fp.kc = sh.kc; fp.kp = sh.kp;
   long long most = 0;
@@ -1358,7 +1375,9 @@ cudaError_t step_n(const Step* s, int cnt, int t, cudaStream_t st) {
 template <int NS>
 cudaError_t stage_n(Problem* const* p, const double* eps0, int cnt, cudaStream_t st) {
   StageLaunch<NS> lp;
-  lp.nsub = cnt; lp.d = p[0]->d; lp.kc = p[0]->kc; lp.kp = p[0]->kp; lp.prec = p[0]->prec;
+  lp.nsub = cnt; lp.d = p[0]->d; lp.prec = p[0]->prec;
+  const tc::Layout lay = tc::operand_layout(lp.d, lp.prec, 3 * p[0]->lab.V, kAug);
+  lp.kcoord = lay.kcoord; lp.kc = lay.kc; lp.kp = lay.kp; lp.hs = lay.hs;
   int blocks[2] = {0, 0};  // one launch per cloud; problems of one cloud only have no second one
   for (int i = 0; i < cnt; ++i) {
     const Problem& q = *p[i];
@@ -1376,6 +1395,11 @@ cudaError_t stage_n(Problem* const* p, const double* eps0, int cnt, cudaStream_t
   }
   sym_reset_kernel<NS><<<1, 32, 0, st>>>(lp);
   count_launches(1);
+  if (lp.hs) {  // both scales are known before anything is staged
+    const int most = blocks[0] > blocks[1] ? blocks[0] : blocks[1];
+    sym_amax_kernel<NS><<<dim3(most < 296 ? most : 296, cnt, 2), 256, 0, st>>>(lp);
+    count_launches(1);
+  }
   for (lp.cloud = 0; lp.cloud < 2; ++lp.cloud)
     if (blocks[lp.cloud]) {
       sym_stage_kernel<NS><<<dim3(blocks[lp.cloud], cnt), 256, 0, st>>>(lp);

@@ -48,7 +48,8 @@ struct SubPass {
   int ntiles;        // column tiles of BN
   int nblk;          // row blocks of BM rows
   int item0;         // index of this pass's first (row block, column tile) item in the launch's item list
-  float scale2;      // 2*cs*log2e/eps: logit = scale2 * S
+  float scale2;      // 2*cs*log2e/eps: logit = scale2 * S / (product of the clouds' scales)
+  const unsigned* amax;  // where those scales come from (null: 1)
   float eps;
   LseEpilogue ep;
   // Partial (scale2*max, sum) pairs of row blocks that several CTAs share, and one arrival counter per row
@@ -73,7 +74,8 @@ struct SubPass {
 template <int NSUB>
 struct Launch {
   int nsub;
-  int nfull, ntail;  // K blocks: nfull of 32 floats (128B swizzle) + ntail of 8 floats (32B swizzle)
+  int nfull, ntail;  // K blocks: nfull of 32 words (128B swizzle) + ntail of 8 words (32B swizzle)
+  int hs;            // leading 32-byte K steps that hold fp16 coordinates
   int nstage;
   long long total;   // items of all passes (dense passes: sum of nblk * ntiles)
   SubPass sub[NSUB];
@@ -281,7 +283,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     auto pick = [&]() { return kWarpIssue ? elect_one() : true; };
     if (kWarpIssue || lane == 0) {
       const int h = (warp == 1) ? 0 : 1;
-      constexpr uint32_t idesc = make_idesc(BN);
+      constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
       const uint32_t a_lo0 = desc_lo(smem_u32(a_smem + h * a_half_bytes));
       bool ok = true;
       int jt = 0, seg = 0;  // column tiles processed so far by this CTA (ring / buffer position), segment count
@@ -313,21 +315,24 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
           constexpr bool kTileElect = (NHALF == 2);
           if (kTileElect ? pick() : true) {
             uint32_t acc = 0;
+            int left = P.hs;  // fp16 K steps to go
 #pragma unroll 1
             for (int kb = 0; kb < P.nfull; ++kb) {
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks) {
                 if (kTileElect || pick())
-                  umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, acc);
+                  umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                            idesc, idesc_h, acc);
                 acc = 1;
               }
+              left -= 4;
               al += (128 * 128) >> 4;
               bl += (BN * 128) >> 4;
             }
 #pragma unroll 1
             for (int t = 0; t < P.ntail; ++t) {
               if (kTileElect || pick())
-                umma_tf32(d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, acc);
+                umma_step(left > t, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
               acc = 1;
               al += (128 * 32) >> 4;
               bl += (BN * 32) >> 4;
@@ -360,7 +365,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     // (the soft-max warps set `sub` with blk_of(w_begin) below, before the first chunk is consumed)
     if (has_work) blk_of(w_begin);
-    float scale = SP().scale2;  // logit scale of the current segment's pass
+    auto pass_scale = [&]() { return SP().scale2 / pair_scale(SP().amax); };  // exact: a power of two
+    float scale = pass_scale();  // logit scale of the current segment's pass
     // off_run is the fp32 exponent offset all terms of s_run are relative to: sum = s_run * 2^off_run.
     // It is carried as the ROUNDED value scale*max (not recomputed from the max), so that rescaling by
     // 2^(off_old - off_new) and the final off_run + log2(s_run) are exact identities in fp32.
@@ -524,7 +530,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       }
       if (AM) {
         if (finish && live && part == 0 && r < SP().nr && !*abort_flag) {
-          SP().ep.out[r] = SP().scale2 * m_run;  // scale2 = -2*cost_scale turns the maximal score into the minimal cost
+          SP().ep.out[r] = scale * m_run;  // scale2 = -2*cost_scale turns the maximal score into the minimal cost
           SP().out_idx[r] = idx_run;
         }
       } else if (finish && live && part == 0 && r < SP().nr && !*abort_flag) {
@@ -545,7 +551,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       if (seg_w < w_end) {
         seg_blk = next_blk(seg_blk, seg_w);
         if (NSUB > 1) {  // the next segment may belong to another pass, with its own logit scale
-          scale = SP().scale2;
+          scale = pass_scale();
           off_run = __fmul_rn(scale, kRunInit);
         }
       }
@@ -612,6 +618,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
 // One CTA = 128 rows; TMEM columns: [0, 3*WCOLS) three S/W buffers, then DV_PAD columns of O.
 struct PvKernelParams {
   int nr, nc, ntiles, nfull, ntail;
+  int hs;                // leading 32-byte K steps that hold fp16 coordinates
+  const unsigned* amax;  // the clouds' scales (null: 1)
   int nb, nv;            // ring depths: column-operand tiles (freed after the score GEMM) and V tiles
   int row_begin;         // rows [row_begin, nr) are produced
   int dv, dv_pad, dv0;   // real width, padded slice width (multiple of 32, <= 128), first column of this slice
@@ -759,7 +767,7 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
     // instructions of a tile would otherwise queue behind each other. All 32 lanes run the loop (uniform
     // descriptor arithmetic), one elected lane issues.
     {
-      constexpr uint32_t idesc1 = make_idesc(BN);
+      constexpr uint32_t idesc1 = make_idesc(BN), idesc1_h = make_idesc_f16(BN);
       // every exit decision is a warp vote: elect.sync needs all 32 lanes at the same instruction
       const bool ok = __all_sync(0xffffffffu, mbar_wait(bar(A_FULL), 0, abort_flag, 2000));
       tc_fence_after();
@@ -774,19 +782,22 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
         uint32_t al = a_lo0, bl = desc_lo(smem_u32(b_smem + s * b_bytes));
         if (elect_one()) {  // one election per tile
           uint32_t acc = 0;
+          int left = p.hs;  // fp16 K steps to go
 #pragma unroll 1
           for (int kb = 0; kb < p.nfull; ++kb) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
-              umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc1, acc);
+              umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc1,
+                        idesc1_h, acc);
               acc = 1;
             }
+            left -= 4;
             al += (128 * 128) >> 4;
             bl += (BN * 128) >> 4;
           }
 #pragma unroll 1
           for (int t = 0; t < p.ntail; ++t) {
-            umma_tf32(d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc1, acc);
+            umma_step(left > t, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc1, idesc1_h, acc);
             acc = 1;
             al += (128 * 32) >> 4;
             bl += (BN * 32) >> 4;
@@ -853,7 +864,7 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int r_in = q * 32 + lane;  // row within the block
     const int r = row0 + r_in;
-    const float scale = p.scale2;
+    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
     const float negR = (r < p.nr) ? -p.R[r] : 0.f;
     bool ok = true;
     constexpr int CH = BN / 32 / kParts;
@@ -1026,41 +1037,43 @@ __global__ void stage_vt_kernel(const float* __restrict__ V, int nc, int dv, con
 }
 
 // ------------------------------------------------------------------ staging kernels
-// opA/opB for one cloud. Column layout (kp floats per row):
-//   TF32 mode : [ x (d) | aug (3) | 0 ... ]                       A-role aug = 1,1,1 ; B-role aug = bias split
-//   FP32 mode : A-role [ xh (d) | xh (d) | xl (d) | aug | 0 ...]   B-role [ yh | yl | yh | aug | 0 ... ]
-// so that sum_k A_k B_k = xh.yh + xh.yl + xl.yh + bias  (the dropped xl.yl term is ~2^-22 relative).
+// opA/opB for one cloud. Column layout (kp words per row, see Layout and stage_coord):
+//   TF32 mode : [ x | aug (3) | 0 ... ]                       A-role aug = 1,1,1 ; B-role aug = bias split
+//   FP32 mode : A-role [ xh | xh | xl | aug | 0 ...]   B-role [ yh | yl | yh | aug | 0 ... ]
+// so that sum_k A_k B_k = xh.yh + xh.yl + xl.yh + bias  (the dropped xl.yl term is ~2^-22 relative). With fp16
+// coordinates every product carries the two clouds' scales; label and bias columns are multiplied by them too.
 // Label cost: the coordinate columns are followed by 3V label columns per point, so that the table lookup
 // becomes part of the same contraction: in the row role a point of label l carries (1,1,1) in the three
 // columns of class l and zeros elsewhere; in the column role it carries, for every class v, the three-piece
 // TF32 split of w_coef * W[.,.] between v and its own label (exact in fp32, so the block is staged once in
 // either precision mode).
-__global__ void stage_kernel(const float* __restrict__ src, int rows, int rows_pad, int d, int kc, int kp, int prec,
+__global__ void amax_kernel(const float* x, size_t nx, const float* y, size_t ny, unsigned* amax) {
+  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
+  if (blockIdx.y == 0) block_amax(x, nx, first, stride, amax);
+  else block_amax(y, ny, first, stride, amax + 1);
+}
+
+__global__ void stage_kernel(const float* __restrict__ src, int rows, int rows_pad, int d, Layout lay, int prec,
+                             const unsigned* __restrict__ amax,
                              float* __restrict__ opA, float* __restrict__ opB,
                              const int* __restrict__ labels, const float* __restrict__ W, int V, int cloud,
                              float w_coef) {
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int kc = lay.kc, kp = lay.kp, kcoord = lay.kcoord;  // [kcoord, kc) is the label block
   size_t total = (size_t)rows_pad * kp;
   if (idx >= total) return;
   int r = (int)(idx / kp), k = (int)(idx % kp);
-  const int kcoord = (prec == 0) ? d : 3 * d;  // coordinate columns; [kcoord, kc) is the label block
   float va = 0.f, vb = 0.f;
   if (k < kcoord) {
-    if (r < rows) {
-      int part = k / d, c = k % d;
-      float x = src[(size_t)r * d + c];
-      float hi = to_tf32(x);
-      float lo = to_tf32(x - hi);
-      if (prec == 0) { va = hi; vb = hi; }
-      else { va = (part == 2) ? lo : hi; vb = (part == 1) ? lo : hi; }
-    }
+    if (r < rows)
+      stage_coord(src + (size_t)r * d, k, d, prec == 0 ? 1 : 3, lay.hs, amax ? cloud_scale(amax[cloud]) : 1.f, va, vb);
   } else if (k < kc) {
     if (r < rows) {
       const int v = (k - kcoord) / 3, piece = (k - kcoord) % 3;
       const int l = labels[r];
       va = (l == v) ? 1.f : 0.f;
       // cloud 0 (x) as column: rows are y points of label v -> W[l, v]; cloud 1 (y) as column: W[v, l]
-      const float w = w_coef * W[cloud == 0 ? l * V + v : v * V + l];
+      const float w = pair_scale(amax) * w_coef * W[cloud == 0 ? l * V + v : v * V + l];
       const float h = to_tf32(w), mid = to_tf32(w - h), low = to_tf32(w - h - mid);
       vb = piece == 0 ? h : (piece == 1 ? mid : low);
     }
@@ -1075,14 +1088,14 @@ __global__ void stage_kernel(const float* __restrict__ src, int rows, int rows_p
 // Writes the bias of a pass, divided by the logit scale and split into 3 TF32 pieces, into opB's aug columns.
 __global__ void bias_kernel(float* __restrict__ opB, int rows, int kc, int kp, const float* __restrict__ pot,
                             const float* __restrict__ logw, float inv_eps, float inv_scale2, const Ctrl* ctrl,
-                            int pot_shard = 0, int pot_stride = 0) {
+                            const unsigned* __restrict__ amax, int pot_shard = 0, int pot_stride = 0) {
   if (ctrl && ctrl->converged) return;
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   const float pr = pot_shard > 0 ? pot[(size_t)(r / pot_shard) * pot_stride + r % pot_shard] : pot[r];
   // bias in log2 units, same association as the reference kernels, then / scale2
   float b2 = logw ? (pr * (inv_eps * kLog2e) + logw[r] * kLog2e) : pr * kLog2e;
-  float b = b2 * inv_scale2;
+  float b = b2 * inv_scale2 * pair_scale(amax);
   float hi = to_tf32(b);
   float r1 = b - hi;
   float mid = to_tf32(r1);
@@ -1111,6 +1124,7 @@ bool encode_map(CUtensorMap* map, const float* base, int rows, int kp, int box_k
 }
 
 struct Shape {
+  Layout lay;
   int kc, kp, nfull, ntail, nhalf, bn, nstage;
   size_t smem;
   bool ok;
@@ -1120,8 +1134,9 @@ struct Shape {
 // nlab = label-table columns (3 per class), staged once in either precision mode: their values are exact in TF32.
 Shape plan_shape(int d, int prec, int nlab = 0) {
   Shape s{};
-  s.kc = ((prec == 0) ? d : 3 * d) + nlab;
-  s.kp = (s.kc + 3 + 7) & ~7;  // + 3 bias columns, padded to whole K steps of 8
+  s.lay = operand_layout(d, prec, nlab, 3);  // three bias columns
+  s.kc = s.lay.kc;
+  s.kp = s.lay.kp;
   s.nfull = s.kp / 32;
   s.ntail = (s.kp % 32) / 8;
   const size_t row_bytes = (size_t)s.kp * 4;
@@ -1130,7 +1145,8 @@ Shape plan_shape(int d, int prec, int nlab = 0) {
   const int cand[3][2] = {{2, 128}, {1, 128}, {1, 64}};
   for (auto& c : cand) {
     size_t a = (size_t)c[0] * 128 * row_bytes, b = (size_t)c[1] * row_bytes;
-    if (a + 2 * b > budget) continue;
+    // 64-column tiles issue half-efficient MMAs; only unscaled operands (few coordinates, many classes) use them
+    if (a + 2 * b > budget || (c[1] == 64 && s.lay.hs > 0)) continue;
     int ns = (int)((budget - a) / b);
     if (ns > 4) ns = 4;
     s.nhalf = c[0]; s.bn = c[1]; s.nstage = ns;
@@ -1179,6 +1195,7 @@ struct BiasJobs {
     const float* pot;
     const float* logw;
     float inv_eps, inv_scale2;
+    const unsigned* amax;
     int pot_shard, pot_stride;  // packed potential (see StreamArgs), 0 = contiguous
   } job[kMaxSub];
 };
@@ -1189,7 +1206,7 @@ __global__ void bias_multi_kernel(const BiasJobs jobs) {
   if (r >= j.rows) return;
   const float pr = j.pot_shard > 0 ? j.pot[(size_t)(r / j.pot_shard) * j.pot_stride + r % j.pot_shard] : j.pot[r];
   const float b2 = j.logw ? (pr * (j.inv_eps * kLog2e) + j.logw[r] * kLog2e) : pr * kLog2e;
-  const float b = b2 * j.inv_scale2;
+  const float b = b2 * j.inv_scale2 * pair_scale(j.amax);
   const float hi = to_tf32(b);
   const float r1 = b - hi;
   const float mid = to_tf32(r1);
@@ -1268,9 +1285,10 @@ int pick_ctas_for(int nblk, int ntiles, int sms, int reserved, int limit) {
 }
 
 void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,
-                 float inv_scale2, const Ctrl* ctrl, cudaStream_t st, int pot_shard, int pot_stride) {
+                 float inv_scale2, const Ctrl* ctrl, const unsigned* amax, cudaStream_t st, int pot_shard,
+                 int pot_stride) {
   bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, kc, kp, pot, logw, inv_eps, inv_scale2,
-                                                       ctrl, pot_shard, pot_stride);
+                                                       ctrl, amax, pot_shard, pot_stride);
 }
 
 int free_ctas() {
@@ -1350,6 +1368,7 @@ size_t staged_bytes(int n, int m, int d, int prec, int nlab) {
   b += 2 * (((size_t)pad256(m) * per_row + 1023) & ~size_t(1023));
   b += 2 * 2 * (size_t)kMaxChunks * pad256(n > m ? n : m) * sizeof(float);  // column-split partials, per side
   b += 2 * (size_t)(pad256(n > m ? n : m) / 128) * sizeof(int);             // row-block tickets, per side
+  b += 2 * sizeof(unsigned);                                                // largest coordinates
   return b + 1024;
 }
 
@@ -1358,7 +1377,7 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
   const int V = (lab && lab->V > 0) ? lab->V : 0;
   Shape sh = plan_shape(d, prec, 3 * V);  // the label table rides along as 3V extra columns (see stage_kernel)
   if (!sh.ok) return cudaErrorNotSupported;
-  s.d = d; s.nlab = 3 * V; s.kc = sh.kc; s.kp = sh.kp; s.prec = prec;
+  s.d = d; s.nlab = 3 * V; s.kc = sh.kc; s.kp = sh.kp; s.prec = prec; s.hs = sh.lay.hs;
   char* p = (char*)(((uintptr_t)buf + 1023) & ~(uintptr_t)1023);
   const float* src[2] = {x, y};
   const int rows[2] = {n, m};
@@ -1369,11 +1388,6 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
     size_t bytes = (((size_t)o.rows_pad * sh.kp * sizeof(float)) + 1023) & ~size_t(1023);
     o.opA = reinterpret_cast<float*>(p); p += bytes;
     o.opB = reinterpret_cast<float*>(p); p += bytes;
-    size_t total = (size_t)o.rows_pad * sh.kp;
-    if (run_kernels)
-      stage_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(src[c], o.rows, o.rows_pad, d, sh.kc, sh.kp, prec,
-                                                                    o.opA, o.opB, V ? lab->lab[c] : nullptr,
-                                                                    V ? lab->W : nullptr, V, c, w_coef);
   }
   s.part_stride = pad256(n > m ? n : m);
   // Each side has its own partial slots and tickets: the two passes of a Jacobi step may share one launch.
@@ -1386,9 +1400,23 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
   int* tk = reinterpret_cast<int*>(fp + 4 * slots);
   s.tickets[0] = tk;
   s.tickets[1] = tk + s.part_stride / 128;
+  unsigned* amax = reinterpret_cast<unsigned*>(tk + 2 * (size_t)(s.part_stride / 128));
+  s.amax = s.hs ? amax : nullptr;
   if (run_kernels) {
-    cudaError_t e = cudaMemsetAsync(tk, 0, 2 * (size_t)(s.part_stride / 128) * sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(tk, 0, 2 * (size_t)(s.part_stride / 128) * sizeof(int) + 2 * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
+    if (s.hs) {
+      const size_t most = (size_t)(n > m ? n : m) * d;
+      const int blocks = most / 256 + 1 < 592 ? (int)(most / 256 + 1) : 592;
+      amax_kernel<<<dim3(blocks, 2), 256, 0, st>>>(x, (size_t)n * d, y, (size_t)m * d, amax);
+    }
+    for (int c = 0; c < 2; ++c) {
+      CloudOps& o = s.cloud[c];
+      const size_t total = (size_t)o.rows_pad * sh.kp;
+      stage_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(src[c], o.rows, o.rows_pad, d, sh.lay, prec, s.amax,
+                                                                    o.opA, o.opB, V ? lab->lab[c] : nullptr,
+                                                                    V ? lab->W : nullptr, V, c, w_coef);
+    }
   }
   return cudaGetLastError();
 }
@@ -1413,7 +1441,7 @@ bool fill_subpass(SubPass& kp, const Staged& s, int side, const StreamArgs& a, c
   const int bm = 128 * sh.nhalf;
   kp.nblk = (a.nr - a.row_begin + bm - 1) / bm;
   kp.item0 = 0;
-  kp.scale2 = scale2; kp.eps = a.eps; kp.ep = e;
+  kp.scale2 = scale2; kp.amax = s.amax; kp.eps = a.eps; kp.ep = e;
   kp.part_m = s.part_m[side]; kp.part_s = s.part_s[side]; kp.part_stride = s.part_stride; kp.tickets = s.tickets[side];
   kp.out_idx = nullptr; kp.csr_rp = nullptr; kp.csr_ci = nullptr;
   return ok;
@@ -1439,13 +1467,14 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   const float scale2 = am ? -2.0f * a.cost_scale : (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (am)
     bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, nullptr, 1.0f,
-                                                         1.0f / (scale2 * kLog2e), nullptr);
+                                                         1.0f / (scale2 * kLog2e), nullptr, s.amax);
   else
     bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
-                                                         1.0f / a.eps, 1.0f / scale2, e.ctrl, a.pot_shard, a.pot_stride);
+                                                         1.0f / a.eps, 1.0f / scale2, e.ctrl, s.amax, a.pot_shard,
+                                                         a.pot_stride);
   Launch<1> lp{};
   lp.nsub = 1;
-  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage;
+  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
   SubPass& kp = lp.sub[0];
   if (!fill_subpass(kp, s, side, a, e, sh, scale2)) return cudaErrorInvalidValue;
   if (kp.nblk <= 0) return cudaSuccess;
@@ -1480,7 +1509,7 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
   if (!sh.ok || sh.streamed) return cudaErrorNotSupported;
   Launch<kMaxSub> lp{};
   BiasJobs jobs{};
-  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage;
+  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
   int used = 0, max_cols = 0;
   long long total = 0;
   for (int i = 0; i < n; ++i) {
@@ -1499,6 +1528,7 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
     BiasJobs::Job& j = jobs.job[used];
     j.opB = colc.opB; j.rows = colc.rows; j.kc = sh.kc; j.kp = sh.kp;
     j.pot = mp.a.pot; j.logw = mp.a.logw; j.inv_eps = 1.0f / mp.a.eps; j.inv_scale2 = 1.0f / scale2;
+    j.amax = s.amax;
     j.pot_shard = mp.a.pot_shard; j.pot_stride = mp.a.pot_stride;
     if (colc.rows > max_cols) max_cols = colc.rows;
     // Two passes of one launch must not write the bias columns of the same operand (nor merge in the same
@@ -1655,7 +1685,7 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
-                                                       1.0f / a.eps, 1.0f / scale2, nullptr);
+                                                       1.0f / a.eps, 1.0f / scale2, nullptr, s.amax);
   // V^T (hi / lo), [nslices*dv_pad, cols_pad]
   const int vrows = ps.nslices * ps.dv_pad, vcols = colc.rows_pad;
   char* p = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
@@ -1679,6 +1709,7 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   PvKernelParams kp;
   kp.nr = a.nr; kp.nc = a.nc; kp.row_begin = a.row_begin;
   kp.ntiles = (a.nc + ps.bn - 1) / ps.bn;
+  kp.hs = sh.lay.hs; kp.amax = s.amax;
   kp.nfull = sh.nfull; kp.ntail = sh.ntail; kp.nb = ps.nb; kp.nv = ps.nv;
   kp.dv = pa.dv; kp.dv_pad = ps.dv_pad; kp.ld_out = pa.dv;
   kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;

@@ -14,6 +14,24 @@
 namespace fs {
 namespace tc {
 
+// Columns (32-bit words) of a staged operand row: coordinates, label table, bias columns, padding to whole 32-byte
+// K steps. The coordinates are fp16, scaled by a power of two per cloud, where that takes fewer K steps than TF32
+// (every d above 8 to 13; d = 64: 5 against 9, and 13 against 25 in the 3-product mode): half the tensor time and
+// operand bytes at the same significand. hs = leading K steps that hold fp16.
+struct Layout {
+  int hs, kcoord, kc, kp;  // kcoord: coordinate words; kc: first bias column; kp: row pitch
+};
+inline Layout operand_layout(int d, int prec, int nlab, int aug) {
+  Layout l{};
+  const int parts = prec == 0 ? 1 : 3, rest = nlab + aug;
+  const int half = parts * ((d + 15) / 16) + (rest + 7) / 8, full = (parts * d + rest + 7) / 8;
+  l.hs = half < full ? parts * ((d + 15) / 16) : 0;
+  l.kcoord = l.hs ? l.hs * 8 : parts * d;
+  l.kc = l.kcoord + nlab;
+  l.kp = (l.kc + aug + 7) & ~7;
+  return l;
+}
+
 struct CloudOps {
   float* opA = nullptr;  // [rows_pad, kp] row-operand form (ones in the bias columns)
   float* opB = nullptr;  // [rows_pad, kp] column-operand form (bias columns rewritten per pass)
@@ -23,6 +41,8 @@ struct CloudOps {
 struct Staged {
   CloudOps cloud[2];  // 0 = x, 1 = y
   int d = 0, nlab = 0, kc = 0, kp = 0, prec = 0;  // nlab: label-table columns staged after the coordinates
+  int hs = 0;                      // leading K steps that hold fp16 coordinates
+  const unsigned* amax = nullptr;  // largest |coordinate| of either cloud as float bits (null: operands not scaled)
   // Per side (0: rows of x, 1: rows of y): [pieces, part_stride] partial scaled maxima and sums of row blocks
   // shared by several CTAs, and [rows_pad / 128] arrival counters of those CTAs (zero at rest).
   float* part_m[2] = {nullptr, nullptr};
@@ -130,7 +150,8 @@ int free_ctas();
 // Writes the column bias of a pass (divided by the logit scale, split into three TF32 pieces) into the bias
 // columns of the column operand.
 void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,
-                 float inv_scale2, const Ctrl* ctrl, cudaStream_t st, int pot_shard = 0, int pot_stride = 0);
+                 float inv_scale2, const Ctrl* ctrl, const unsigned* amax, cudaStream_t st, int pot_shard = 0,
+                 int pot_stride = 0);
 inline int pad256(int r) { return (r + 255) & ~255; }
 }  // namespace detail
 

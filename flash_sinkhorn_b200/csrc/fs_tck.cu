@@ -44,7 +44,9 @@ struct KParams {
   int nr, nc;       // end of the row range (rows >= nr are padding) / valid columns
   int row_begin;    // first row of the range; row blocks are counted from here
   int ntiles, nblk;
-  int nk;           // K chunks of 32 floats
+  int hs;           // leading 32-byte K steps that hold fp16 coordinates (0 for the second GEMM of a matrix pass)
+  const unsigned* amax;  // the clouds' scales (null: 1)
+  int nk;           // K chunks of 32 words
   int klast;        // K steps of 8 in the last chunk (1..4)
   int nstage;
   float scale2, eps;
@@ -165,7 +167,7 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     // decision is a warp vote, since elect.sync needs all lanes at the same instruction.
     {
       const int h = (warp == 1) ? 0 : 1;
-      constexpr uint32_t idesc = make_idesc(BN);
+      constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
       bool ok = true;
       int s = 0;
       uint32_t ph = 0;
@@ -191,14 +193,16 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
               if (elect_one())
-                umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, acc);
+                umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                          idesc, idesc_h, acc);
               acc = 1;
             }
           } else {
 #pragma unroll 1
             for (int ks = 0; ks < p.klast; ++ks) {
               if (elect_one())
-                umma_tf32(d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc, acc);
+                umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                          idesc, idesc_h, acc);
               acc = 1;
             }
           }
@@ -224,7 +228,7 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     const int q = warp & 3;         // TMEM lane quarter this warp may read
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int trow = h * 128 + q * 32 + lane;  // this thread's row inside a row block
-    const float scale = p.scale2;
+    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
     constexpr int CH = BN / 32 / kPartsK;  // 32-column chunks of a tile owned by this warpgroup
     const int total = (w_end - w_begin) * CH;
     const int c_base = part * CH;
@@ -499,6 +503,10 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 // One CTA = 128 rows, column tiles of 64. TMEM: NSW buffers of [S -> Wh | Wl (split) | E (MAT5)], then O.
 struct KPvParams {
   int nr, nc, ntiles, row_begin;
+  int hs;                      // leading K steps that hold fp16 coordinates
+  const unsigned* amax;        // the clouds' scales (null: 1)
+  const unsigned* amax2;       // MAT5: largest |entry| of the second row operand, and of the column cloud
+  const unsigned* amax_col;
   int nk, klast, nstage, nv;   // K chunks, K steps of the last one, ring depths (K chunks / V tiles)
   int dv, dv_pad, dv0, ld_out;
   float scale2, eps;
@@ -620,7 +628,7 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
   } else if (warp == 1) {
     {  // score GEMM(s) of tile j into buffer j % NSW, accumulated over the K chunks. All 32 lanes run the loop
        // (warp-uniform descriptor arithmetic), one elected lane issues; exits are warp votes.
-      constexpr uint32_t idesc1 = make_idesc(BN);
+      constexpr uint32_t idesc1 = make_idesc(BN), idesc1_h = make_idesc_f16(BN);
       bool ok = true;
       int s = 0;
       uint32_t ph = 0;
@@ -642,10 +650,12 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
 #pragma unroll 1
           for (int ks = 0; ks < nks; ++ks) {
             if (elect_one()) {
-              umma_tf32(s_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc1, acc);
+              const bool half = kc * 4 + ks < p.hs;
+              umma_step(half, s_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc1,
+                        idesc1_h, acc);
               if (MAT5)
-                umma_tf32(s_tmem + WCOLS, pack_desc(a2l + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                          idesc1, acc);
+                umma_step(half, s_tmem + WCOLS, pack_desc(a2l + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                          idesc1, idesc1_h, acc);
             }
             acc = 1;
           }
@@ -709,7 +719,8 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int r = row0 + q * 32 + lane;
-    const float scale = p.scale2;
+    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
+    const float unit2 = MAT5 && p.amax2 ? 1.f / (cloud_scale(*p.amax2) * cloud_scale(*p.amax_col)) : 1.f;
     const float negR = (r < p.nr) ? -p.R[r] : 0.f;
     bool ok = true;
     constexpr int CH = BN / 32 / kPartsK;
@@ -737,7 +748,7 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           float w = ex2(fmaf(__uint_as_float(rg[i]), scale, negR));
-          if (MAT5) w *= e[i];
+          if (MAT5) w *= e[i] * unit2;
           const float hi = round_tf32_pos(w);
           lo[i] = round_tf32_pos(w - hi);
           v[i] = hi;
@@ -747,7 +758,7 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
           float w = ex2(fmaf(__uint_as_float(rg[i]), scale, negR));
-          if (MAT5) w *= e[i];
+          if (MAT5) w *= e[i] * unit2;
           v[i] = round_tf32_pos(w);
         }
       }
@@ -825,8 +836,10 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
 // [Wh | Wl | Wh] in three blocks of cols_pad columns, which the GEMM pairs with [Vh | Vh | Vl]. Columns beyond
 // nc get zero weight without looking at the stored value.
 __global__ void wexp_kernel(float* __restrict__ W, long long ld, int rows, int row0, int nc, int cols_pad,
-                            const float* __restrict__ R, float scale2, int split, const int* skip) {
+                            const float* __restrict__ R, float scale2, const unsigned* __restrict__ amax, int split,
+                            const int* skip) {
   if (skip && *skip) return;
+  scale2 /= pair_scale(amax);
   const int quads = cols_pad >> 2;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)rows * quads) return;
@@ -957,10 +970,11 @@ cudaError_t kstream_lse(const Staged& s, int side, const StreamArgs& a, const Ls
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, st, a.pot_shard,
-                      a.pot_stride);
+  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, s.amax, st,
+                      a.pot_shard, a.pot_stride);
   KParams kp{};
   set_chunks(kp, s.kp);
+  kp.hs = s.hs; kp.amax = s.amax;
   const KPlan k = plan_k(kp.nk, a.nc);
   CUtensorMap ma, mb;
   if (!make_maps(&ma, &mb, rowc.opA, rowc.rows_pad, colc.opB, colc.rows_pad, s.kp, k.bn)) return cudaErrorInvalidValue;
@@ -982,11 +996,12 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st);
+  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
   pad_vec_kernel<<<(colc.rows_pad + 255) / 256, 256, 0, st>>>(pa.V, a.nc, colc.rows_pad, vpad, pa.skip);
   KParams kp{};
   set_chunks(kp, s.kp);
+  kp.hs = s.hs; kp.amax = s.amax;
   const KPlan k = plan_k(kp.nk, a.nc);
   CUtensorMap ma, mb;
   if (!make_maps(&ma, &mb, rowc.opA, rowc.rows_pad, colc.opB, colc.rows_pad, s.kp, k.bn)) return cudaErrorInvalidValue;
@@ -1005,20 +1020,21 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
 // ---- narrow plan-times-matrix pass (second GEMM from TMEM) -------------------------------------------
 namespace {
 
+__global__ void rows2_amax_kernel(const float* A, size_t count, unsigned* out) {
+  block_amax(A, count, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, out);
+}
+
 // Second row operand of the Mat5 term in the row-role layout of the staged clouds: [Ah | Ah | Al | 0 ...] in the
-// split mode, [Ah | 0 ...] in TF32 mode, so that its contraction with the staged column operand is A_i . y_j
+// split mode, [Ah | 0 ...] in TF32 mode (fp16 scaled by its own power of two where the clouds are), so that its contraction with the staged column operand is A_i . y_j
 // (the bias and label columns of the column operand meet zeros).
-__global__ void stage_rows2_kernel(const float* __restrict__ A, int rows, int rows_pad, int d, int kp, int split,
-                                   float* __restrict__ out) {
+__global__ void stage_rows2_kernel(const float* __restrict__ A, int rows, int rows_pad, int d, int kp, int kcoord,
+                                   int hs, int split, const unsigned* __restrict__ amax, float* __restrict__ out) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)rows_pad * kp) return;
   const int r = (int)(idx / kp), k = (int)(idx % kp);
-  float v = 0.f;
-  if (r < rows && k < (split ? 3 * d : d)) {
-    const float a = A[(size_t)r * d + k % d];
-    const float hi = to_tf32(a);
-    v = (split && k / d == 2) ? to_tf32(a - hi) : hi;
-  }
+  float v = 0.f, unused;
+  if (r < rows && k < kcoord)
+    stage_coord(A + (size_t)r * d, k, d, split ? 3 : 1, hs, amax ? cloud_scale(*amax) : 1.f, v, unused);
   out[idx] = v;
 }
 
@@ -1040,7 +1056,7 @@ KPvPlan plan_kpv(int nr, int nc, int kp, int dv, int prec, bool mat5) {
   k.parts = split ? 3 : 1;
   k.ld_v = (long long)k.cols_pad * k.parts;
   k.vt_bytes = (((size_t)k.vrows * k.ld_v * sizeof(float)) + 1023) & ~size_t(1023);
-  k.a2_bytes = mat5 ? ((((size_t)detail::pad256(nr) * kp * sizeof(float)) + 1023) & ~size_t(1023)) : 0;
+  k.a2_bytes = mat5 ? ((((size_t)detail::pad256(nr) * kp * sizeof(float)) + 2047) & ~size_t(1023)) : 0;
   const size_t stage = (size_t)(mat5 ? 2 : 1) * 128 * 128 + 64 * 128;
   const size_t v_stage = (size_t)(split ? 2 : 1) * 2 * k.dv_pad * 128;
   const size_t budget = kSmemMax - 2048;
@@ -1080,19 +1096,27 @@ cudaError_t kstream_pv(const Staged& s, int side, const StreamArgs& a, const PvA
   if (!k.ok) return cudaErrorNotSupported;
   if (k.vt_bytes + k.a2_bytes + 2048 > scratch_bytes) return cudaErrorInvalidValue;
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st, a.pot_shard,
-                      a.pot_stride);
+  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st,
+                      a.pot_shard, a.pot_stride);
   char* p0 = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
   float* vt = reinterpret_cast<float*>(p0);
   float* a2 = mat5 ? reinterpret_cast<float*>(p0 + k.vt_bytes) : nullptr;
+  // the last kilobyte of the second operand's part holds its largest entry
+  unsigned* amax2 = mat5 && s.hs ? reinterpret_cast<unsigned*>(p0 + k.vt_bytes + k.a2_bytes - 1024) : nullptr;
   {
     dim3 grid((k.cols_pad + 31) / 32, (k.vrows + 31) / 32), block(32, 8);
     stage_vt_cat_kernel<<<grid, block, 0, st>>>(pa.V, a.nc, pa.dv, pa.colscale, k.vrows, k.cols_pad, split, vt);
   }
   if (mat5) {
+    if (amax2) {
+      const size_t count = (size_t)rowc.rows * s.d;
+      cudaError_t e = cudaMemsetAsync(amax2, 0, sizeof(unsigned), st);
+      if (e != cudaSuccess) return e;
+      rows2_amax_kernel<<<count / 256 + 1 < 592 ? (int)(count / 256 + 1) : 592, 256, 0, st>>>(pa.rows2, count, amax2);
+    }
     const size_t total = (size_t)rowc.rows_pad * s.kp;
-    stage_rows2_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(pa.rows2, rowc.rows, rowc.rows_pad, s.d, s.kp,
-                                                                        split, a2);
+    stage_rows2_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
+        pa.rows2, rowc.rows, rowc.rows_pad, s.d, s.kp, operand_layout(s.d, s.prec, s.nlab, 3).kcoord, s.hs, split, amax2, a2);
   }
   CUtensorMap maps[5];
   bool ok = true;
@@ -1108,6 +1132,7 @@ cudaError_t kstream_pv(const Staged& s, int side, const StreamArgs& a, const PvA
   kp.ntiles = (a.nc + 63) / 64;
   KParams chunks{};
   set_chunks(chunks, s.kp);
+  kp.hs = s.hs; kp.amax = s.amax; kp.amax2 = amax2; kp.amax_col = s.amax ? s.amax + (side == 0 ? 1 : 0) : nullptr;
   kp.nk = chunks.nk; kp.klast = chunks.klast; kp.nstage = k.nstage; kp.nv = k.nv;
   kp.dv = pa.dv; kp.dv_pad = k.dv_pad; kp.ld_out = pa.dv;
   kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;
@@ -1190,7 +1215,7 @@ cudaError_t kstream_mat(const Staged& s, int side, const StreamArgs& a, const Pv
     // 2. scores -> TF32 weights in place
     const long long quads = (long long)(r1 - r0) * (m.cols_pad / 4);
     wexp_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, st>>>(W, m.k2, r1 - r0, r0, a.nc, m.cols_pad, R_out, scale2,
-                                                                 m.parts == 3, pa.skip);
+                                                                 s.amax, m.parts == 3, pa.skip);
     // 3. out[r0:r1] = epilogue(W x Vt^T)
     g2.nr = r1 - r0; g2.nc = pa.dv; g2.row_begin = 0;
     g2.ntiles = (pa.dv + k2.bn - 1) / k2.bn;

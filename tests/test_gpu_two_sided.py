@@ -104,3 +104,42 @@ def test_not_a_number_stays_with_its_point(cta_limit):
     f = _solve(x, y, a, b, "tf32", eps=1.0, n_iters=5)[0]
     torch.cuda.synchronize()
     assert torch.isnan(f[17]) and _lib.load().fs_device_error() == 0
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1e-4, 1.0, 3e4, 1e9])
+def test_operand_scale_follows_the_clouds(scale):
+    """Coordinates ride as fp16 scaled by a power of two per cloud: any size of the clouds, also very different ones
+    and with one far larger coordinate, gives the soft-min the precision of the 3-product mode (22 bits of every
+    product against a largest potential of the size of the logits: 2e-6)."""
+    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse
+    r = np.random.default_rng(5)
+    x, y = np.float32(scale * r.normal(size=(300, 48))), np.float32(0.1 / scale * r.normal(size=(260, 48)))
+    x[0, 0] *= 1000.0
+    bias = np.float32(r.normal(size=260))
+    got = flashsinkhorn_lse(dev(x), dev(y), dev(bias), eps=0.05, allow_tf32=False)
+    want = O.lse_update(x.astype(np.float64), y.astype(np.float64), bias.astype(np.float64), 0.05)
+    assert rel(host(got), want) < 2e-6
+
+
+@pytest.mark.parametrize("d", [1, 8, 13, 14, 16, 17, 63, 80, 81])
+@pytest.mark.parametrize("prec", ["fp32", "tf32"])
+def test_every_operand_layout(prec, d):
+    """Feature dimensions around the change from TF32 to fp16 columns and the ends of 16-coordinate steps: soft-min,
+    nearest target, gradient and plan application against fp64 (the operand rounding is the only TF32 error: 2^-11 of
+    |x||y| in the exponent of a weight)."""
+    from flash_sinkhorn_b200.c_transform import c_transform_fwd
+    from flash_sinkhorn_b200.kernels.apply_flash import apply_plan_mat_flashstyle
+    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse
+    x, y, a, b = _clouds(200, 333, d, seed=7)
+    tf32, eps = prec == "tf32", 0.5 * d
+    r = np.random.default_rng(8)
+    bias, mat = np.float32(r.normal(size=333)), np.float32(r.normal(size=(333, d)))
+    got = flashsinkhorn_lse(dev(x), dev(y), dev(bias), eps=eps, allow_tf32=tf32)
+    assert rel(host(got), O.lse_update(x, y, bias.astype(np.float64), eps)) < (3e-3 if tf32 else 2e-6)
+    val, _ = c_transform_fwd(dev(x), dev(y), dev(bias), allow_tf32=tf32)
+    assert rel(host(val), O.c_transform(x, y, bias.astype(np.float64))[0]) < (3e-3 if tf32 else 2e-6)
+    fh, gh = -(x * x).sum(1), -(y * y).sum(1)
+    args = [dev(v) for v in (x, y, fh, gh, np.log(a), np.log(b), mat)]
+    got = apply_plan_mat_flashstyle(*args, eps=eps, axis=1, allow_tf32=tf32)
+    want = O.apply_mat(x, y, fh, gh, np.log(a), np.log(b), mat.astype(np.float64), eps, 1)
+    assert rel(host(got), want) < (5e-3 if tf32 else 3e-5)
