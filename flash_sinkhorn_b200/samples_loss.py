@@ -17,6 +17,7 @@ from typing import Optional, Sequence, Tuple, Union
 
 import torch
 
+from flash_sinkhorn_b200 import _lib
 from flash_sinkhorn_b200._autograd import _SinkhornConfig, _SinkhornCostFn
 from flash_sinkhorn_b200.kernels._common import epsilon_schedule, max_diameter
 from flash_sinkhorn_b200.sinkhorn_solvers import (
@@ -289,26 +290,53 @@ class SamplesLoss(torch.nn.Module):
             threshold=self.threshold, check_every=self.inner_iterations, process_group=self.process_group,
         )
 
+    def _lockstep(self, x: torch.Tensor, y: torch.Tensor, labels_on: bool) -> bool:
+        """Whether the three solves of the divergence go to the library as one lockstep call. Early stopping, the
+        label cost and schedules fixed in the constructor keep the one-at-a-time solves."""
+        if (self.backend == "alternating" or self.threshold is not None or labels_on or self.eps_list is not None
+                or self.diameter is not None):
+            return False
+        prec = _lib.precision_id(self.allow_tf32)
+        (n, d), m = x.shape, y.shape[0]
+        return all(_lib.load().fs_two_sided(r, c, d, prec) for r, c in ((n, m), (n, n), (m, m)))
+
+    def _divergence_schedules(self, x: torch.Tensor, y: torch.Tensor):
+        """Schedules of OT(x,y), OT(x,x) and OT(y,y); with annealing the three diameters cost one host read."""
+        if not self.use_epsilon_scaling:
+            return [self._eps_list_for_inputs(x, y)] * 3
+        (lx, hx), (ly, hy) = ((t.float().amin(dim=0), t.float().amax(dim=0)) for t in (x, y))
+        diams = torch.stack([(torch.maximum(hx, hy) - torch.minimum(lx, ly)).norm(), (hx - lx).norm(),
+                             (hy - ly).norm()]).tolist()
+        out = [list(epsilon_schedule(diam, self.blur, self.scaling, p=2.0)) for diam in diams]
+        if self.n_iters is not None:
+            out = [sched[: int(self.n_iters)] for sched in out]
+        if not all(out):
+            raise ValueError("eps_list is empty after applying n_iters.")
+        return out
+
     def forward(self, *args, label_x: Optional[torch.Tensor] = None, label_y: Optional[torch.Tensor] = None):
         parsed = _process_args(*args, normalize=self.normalize)
         if not parsed.x.is_cuda or not parsed.y.is_cuda:
             raise ValueError("flash_sinkhorn.SamplesLoss requires CUDA tensors.")
         config = self._make_config()
 
-        def ot(xs, ys, ws_a, ws_b, lx, ly, presolved=None):
-            sched = tuple(self._eps_list_for_inputs(xs, ys))
+        def ot(xs, ys, ws_a, ws_b, lx, ly, presolved=None, sched=None):
+            sched = tuple(self._eps_list_for_inputs(xs, ys)) if sched is None else tuple(sched)
             return _SinkhornCostFn.apply(xs, ys, ws_a, ws_b, sched, config, lx, ly, self.label_cost_matrix,
                                          presolved)
 
         multi_gpu = (self.process_group is not None and self.backend != "alternating"
                      and torch.distributed.get_world_size(self.process_group) > 1)
 
+        labels_on = (self.label_cost_matrix is not None and label_x is not None and label_y is not None
+                     and self.lambda_y != 0.0)
+
         def divergence(xs, ys, ws_a, ws_b):
             if not self.debias:
                 return ot(xs, ys, ws_a, ws_b, label_x, label_y)
             terms = [(xs, ys, ws_a, ws_b, label_x, label_y), (xs, xs, ws_a, ws_a, label_x, label_x),
                      (ys, ys, ws_b, ws_b, label_y, label_y)]
-            pre = [None, None, None]
+            pre, scheds = [None, None, None], [None, None, None]
             if multi_gpu and self.label_cost_matrix is not None and label_x is not None and self.lambda_y != 0.0:
                 raise NotImplementedError("The label cost is not available in the multi-GPU sharded solver.")
             if multi_gpu:
@@ -323,15 +351,23 @@ class SamplesLoss(torch.nn.Module):
                         rho_y=self.rho_y, last_extrapolation=self.last_extrapolation,
                         threshold=self.threshold, check_every=self.inner_iterations)
                 pre = [(f, g, f, g) if fp is None else (f, g, fp, gp) for (f, g, fp, gp, _) in sols]
-            cross, self_x, self_y = (ot(*t, presolved=p) for t, p in zip(terms, pre))
+            elif self._lockstep(xs, ys, labels_on):
+                # One library call for the three solves: their steps share launches.
+                with torch.no_grad():
+                    scheds = self._divergence_schedules(xs.detach(), ys.detach())
+                    sols = sinkhorn_flashstyle_symmetric_batched(
+                        [tuple(u.detach() for u in t[:4]) for t in terms], schedules=scheds, blur=self.blur,
+                        scaling=self.scaling, use_epsilon_scaling=self.use_epsilon_scaling, eps=self.eps,
+                        n_iters=self.n_iters, allow_tf32=self.allow_tf32, cost_scale=self.cost_scale,
+                        rho_x=self.rho_x, rho_y=self.rho_y, last_extrapolation=self.last_extrapolation)
+                pre = [sol[:4] for sol in sols]
+            cross, self_x, self_y = (ot(*t, presolved=p, sched=e) for t, p, e in zip(terms, pre, scheds))
             return cross - 0.5 * self_x - 0.5 * self_y
 
         # Batched inputs: the reference loops over the items (samples_loss.py:515-552). Here all symmetric solves of
         # the batch - three per item for the debiased loss - go to the library in ONE call and advance in lockstep,
         # several soft-min passes per launch; the cost / gradient nodes then receive the finished potentials. Early
         # stopping, the label cost, the alternating backend and sharded runs keep the per-item loop.
-        labels_on = (self.label_cost_matrix is not None and label_x is not None and label_y is not None
-                     and self.lambda_y != 0.0)
         if (parsed.batched and self.backend != "alternating" and self.threshold is None and not labels_on
                 and not multi_gpu):
             items = list(zip(parsed.x, parsed.y, parsed.a, parsed.b))

@@ -315,6 +315,7 @@ def sinkhorn_flashstyle_symmetric(
 def sinkhorn_flashstyle_symmetric_batched(
     problems,
     *,
+    schedules=None,
     blur: float = 0.05,
     scaling: float = 0.5,
     use_epsilon_scaling: bool = True,
@@ -339,7 +340,8 @@ def sinkhorn_flashstyle_symmetric_batched(
     No early stopping, warm start or label cost. Returns one ``(f, g, f_prelast, g_prelast, n_steps)`` per problem
     (the pre-extrapolation pair equals ``(f, g)`` without ``last_extrapolation``); results equal the one-at-a-time
     solves up to the merge order of partial sums (rounding level). A problem given as ``(x, x, a, a)`` - the same
-    tensors twice - is solved as a self-transport problem with one soft-min per step.
+    tensors twice - is solved as a self-transport problem with one soft-min per step. ``schedules`` gives the eps
+    lists of the problems outright (``n_iters`` still cuts them).
     """
     rho_x, rho_y = resolve_marginal_penalties(rho, reach, rho_x, rho_y, reach_x, reach_y)
     problems = list(problems)
@@ -350,7 +352,7 @@ def sinkhorn_flashstyle_symmetric_batched(
     arr = (_lib.BatchItem * len(problems))()
     keep, outs = [], []
     dev = None
-    for slot, (x, y, a, b) in zip(arr, problems):
+    for slot, (x, y, a, b), given in zip(arr, problems, schedules or [None] * len(problems)):
         if x.shape[1] != d or y.shape[1] != d:
             raise ValueError("all problems of a batched solve must share the feature dimension")
         pdev = _lib.require_cuda(x=x, y=y, a=a, b=b)
@@ -359,7 +361,9 @@ def sinkhorn_flashstyle_symmetric_batched(
         elif pdev != dev:
             raise ValueError("all problems of a batched solve must be on the same device")
         n, m = x.shape[0], y.shape[0]
-        if use_epsilon_scaling:
+        if given is not None:
+            sched = given
+        elif use_epsilon_scaling:
             sched = epsilon_schedule(max_diameter(x, y), blur, scaling, p=2.0)
         else:
             if eps is None or n_iters is None:

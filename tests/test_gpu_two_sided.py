@@ -143,3 +143,18 @@ def test_every_operand_layout(prec, d):
     got = apply_plan_mat_flashstyle(*args, eps=eps, axis=1, allow_tf32=tf32)
     want = O.apply_mat(x, y, fh, gh, np.log(a), np.log(b), mat.astype(np.float64), eps, 1)
     assert rel(host(got), want) < (5e-3 if tf32 else 3e-5)
+
+
+def test_divergence_solves_share_their_launches(cta_limit):
+    """The three solves of a debiased loss go out as one lockstep call; values and gradients equal the dense ones."""
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = _clouds(700, 450, 24, seed=6)
+    want = O.samples_loss(x, y, a, b, [0.5] * 20, debias=True, want_grad_x=True)
+    for limit in (5, 0):
+        cta_limit(limit)
+        xs = dev(x).requires_grad_(True)
+        val = SamplesLoss("sinkhorn", use_epsilon_scaling=False, eps=0.5, n_iters=20, blur=0.5**0.5, debias=True,
+                          allow_tf32=False)(dev(a), xs, dev(b), dev(y))
+        (gx,) = torch.autograd.grad(val, xs)
+        assert abs(float(val) - want["loss"]) < 2e-5 * abs(want["loss"])
+        assert rel(host(gx), want["grad_x"]) < 3e-4
