@@ -82,9 +82,15 @@ struct Launch {
 };
 constexpr int kMaxSub = 4;  // passes per multi-pass launch (keeps the kernel parameters under 4 KB)
 
-// Soft-max warpgroups per 128-row half: each takes half of every tile's 32-column chunks (more warps per
-// scheduler to hide the fixed latencies around the chunk max / rescale); their partials merge at the end.
+// Soft-max warpgroups per 128-row half of the plan-times-matrix kernel: each takes half of every tile's 32-column
+// chunks (more warps per scheduler to hide fixed latencies).
 constexpr int kParts = 2;
+// The same for the soft-min kernel, whose partials merge at the end of a segment: sixteen soft-max warps per CTA
+// with one 128-row half as with two (tile lists: one chunk per warp and tile).
+__host__ __device__ constexpr int lse_parts(int nhalf, int bn) { return nhalf == 1 && bn == 128 ? 4 : 2; }
+// Every kFmaShare-th pair of exponentials of the soft-min kernel goes to the FMA pipe (exp2_fma): the ex2 pipe binds
+// these passes and the packed arithmetic around it leaves half of the issue slots free.
+constexpr int kFmaShare = 4;
 
 // AM = false: online log-sum-exp of the scaled scores (potential update). AM = true: running maximum of the
 // raw scores and the smallest column attaining it (hard c-transform); no exponentials at all.
@@ -92,8 +98,9 @@ constexpr int kParts = 2;
 // of all nblk x ntiles pairs; everything else - contiguous ranges per CTA, segments, ticketed merge - is the same.
 // NSUB > 1: several dense passes in one launch (no arg-max, no tile list, no device-side early-stop flag).
 template <int NHALF, int BN, bool AM, bool CSR = false, int NSUB = 1>
-__global__ void __launch_bounds__(128 + 128 * NHALF * kParts, 1)
+__global__ void __launch_bounds__(128 + 128 * NHALF * lse_parts(NHALF, BN), 1)
 tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
+  constexpr int PARTS = lse_parts(NHALF, BN);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int BM = 128 * NHALF;
@@ -175,8 +182,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   uint32_t* tmem_slot = (uint32_t*)(bars + NBARS);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* last_flag = (volatile int*)(tmem_slot + 2);  // this CTA took the last ticket of its row block
-  float* merge_off = (float*)(tmem_slot + 4);        // [NHALF*128] partials of the second column part
-  float* merge_sum = merge_off + NHALF * 128;
+  float* merge_off = (float*)(tmem_slot + 4);        // [PARTS - 1][NHALF*128] partials of the other column parts
+  float* merge_sum = merge_off + (PARTS - 1) * NHALF * 128;
   auto bar = [&](int i) { return smem_u32(bars + i); };
 
   constexpr uint32_t kTmemCols = (2 * NHALF * BN) < 32 ? 32 : (2 * NHALF * BN);
@@ -188,7 +195,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     }
     for (int i = 0; i < 2 * NHALF; ++i) {
       mbar_init(bar(S_FULL + i), 1);
-      mbar_init(bar(S_EMPTY + i), 4 * kParts);  // one arrive per soft-max warp reading the buffer
+      mbar_init(bar(S_EMPTY + i), 4 * PARTS);  // one arrive per soft-max warp reading the buffer
     }
     mbar_init(bar(A_FULL), 1);
     mbar_init(bar(A_EMPTY), NHALF);
@@ -359,8 +366,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   } else if (warp >= 4) {
     // ===================== soft-max warpgroups =====================
     const int wg = (warp - 4) >> 2;      // warpgroup index
-    const int h = wg / kParts;           // 128-row half
-    const int part = wg % kParts;        // which half of each tile's chunks
+    const int h = wg / PARTS;           // 128-row half
+    const int part = wg % PARTS;        // which half of each tile's chunks
     const int q = warp & 3;              // TMEM lane quarter this warp may read
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     // (the soft-max warps set `sub` with blk_of(w_begin) below, before the first chunk is consumed)
@@ -374,7 +381,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     int idx_run = 0;   // AM: column of the running maximum m_run
     int col_tile = CSR ? 0 : w_begin % p.ntiles;  // AM: column tile of the chunk being consumed
     bool ok = true;
-    constexpr int CH = BN / 32 / kParts;  // 32-column chunks of a tile owned by this warpgroup
+    constexpr int CH = BN / 32 / PARTS;  // 32-column chunks of a tile owned by this warpgroup
     const int total = (w_end - w_begin) * CH;  // chunks of all segments; g / CH counts the CTA's tiles
     const int c_base = part * CH;
     // One online-softmax update with the 32 scores of a chunk (this thread's row).
@@ -407,16 +414,25 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       const float nms = -off_new;
       // After the first tiles the running max rarely moves; when it moved for no row of the warp the
       // rescale factor is exactly 2^0 and its ex2 (one slot of the saturated pipe in 33) is skipped.
-      float s0 = s_run, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      if (__any_sync(0xffffffffu, off_new != off_run)) s0 *= ex2(off_run - off_new);
+      u64 s0 = pk(s_run, 0.f), s1 = 0ull;
+      if (__any_sync(0xffffffffu, off_new != off_run)) s0 = pk(s_run * ex2(off_run - off_new), 0.f);
+      const u64 sc2 = pk(scale, scale), off2 = pk(nms, nms);
 #pragma unroll
-      for (int i = 0; i < 32; i += 4) {
-        s0 += ex2(fmaf(v[i], scale, nms));
-        s1 += ex2(fmaf(v[i + 1], scale, nms));
-        s2 += ex2(fmaf(v[i + 2], scale, nms));
-        s3 += ex2(fmaf(v[i + 3], scale, nms));
+      for (int i = 0; i < 16; ++i) {
+        const u64 z = fma2(pk(v[2 * i], v[2 * i + 1]), sc2, off2);
+        u64 e;
+        if (i % kFmaShare == 1) {
+          e = exp2_fma(z);
+        } else {
+          float z0, z1;
+          upk(z, z0, z1);
+          e = pk(ex2(z0), ex2(z1));
+        }
+        if (i & 1) s1 = add2(s1, e); else s0 = add2(s0, e);
       }
-      s_run = (s0 + s1) + (s2 + s3);
+      float a0, a1;
+      upk(add2(s0, s1), a0, a1);
+      s_run = a0 + a1;
       m_run = m_new;
       off_run = off_new;
     };
@@ -474,19 +490,23 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       const int r = SP().row_begin + blk * BM + h * 128 + q * 32 + lane;
       // AM: a partial is (maximum, column); the larger maximum wins, equal maxima keep the smaller column.
       auto better = [](float va, int ia, float vb, int ib) { return vb > va || (vb == va && ib < ia); };
-      if (part == 1) {  // second column part parks its partial in shared memory
-        merge_off[h * 128 + q * 32 + lane] = live ? (AM ? m_run : off_run) : kRunInit;
-        merge_sum[h * 128 + q * 32 + lane] = AM ? __int_as_float(idx_run) : (live ? s_run : 0.f);
+      const int slot = h * 128 + q * 32 + lane;
+      if (part > 0) {  // the other column parts park their partials in shared memory
+        merge_off[(part - 1) * NHALF * 128 + slot] = live ? (AM ? m_run : off_run) : kRunInit;
+        merge_sum[(part - 1) * NHALF * 128 + slot] = AM ? __int_as_float(idx_run) : (live ? s_run : 0.f);
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * kParts) : "memory");  // soft-max warps only
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");  // soft-max warps only
       if (part == 0) {
-        const float o2 = merge_off[h * 128 + q * 32 + lane], s2 = merge_sum[h * 128 + q * 32 + lane];
-        if (AM) {
-          if (better(m_run, idx_run, o2, __float_as_int(s2))) { m_run = o2; idx_run = __float_as_int(s2); }
-        } else {
-          const float on = fmaxf(off_run, o2);
-          s_run = s_run * ex2(off_run - on) + s2 * ex2(o2 - on);
-          off_run = on;
+#pragma unroll
+        for (int i = 0; i < PARTS - 1; ++i) {
+          const float o2 = merge_off[i * NHALF * 128 + slot], s2 = merge_sum[i * NHALF * 128 + slot];
+          if (AM) {
+            if (better(m_run, idx_run, o2, __float_as_int(s2))) { m_run = o2; idx_run = __float_as_int(s2); }
+          } else {
+            const float on = fmaxf(off_run, o2);
+            s_run = s_run * ex2(off_run - on) + s2 * ex2(o2 - on);
+            off_run = on;
+          }
         }
       }
       const int c_lo = cta_of(row_start(blk)), c_hi = cta_of(row_end(blk) - 1);
@@ -498,9 +518,9 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
           SP().part_s[(size_t)piece * SP().part_stride + r] = AM ? __int_as_float(idx_run) : s_run;
         }
         __threadfence();  // the pairs must be visible device-wide before the ticket is taken
-        asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * kParts) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");
         if (warp == 4 && lane == 0) *last_flag = (atomicAdd(SP().tickets + blk, 1) == pieces - 1) ? 1 : 0;
-        asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * kParts) : "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");
         finish = *last_flag != 0;
         if (finish) {
           __threadfence();
@@ -537,7 +557,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         store_lse(r, off_run + log2f(fmaxf(s_run, 1e-40f)));
       }
       // merge_off / merge_sum / last_flag are re-used by the next segment
-      asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * kParts) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");
       m_run = kRunInit;
       off_run = __fmul_rn(scale, kRunInit);
       s_run = 0.f;
@@ -1123,6 +1143,8 @@ bool encode_map(CUtensorMap* map, const float* base, int rows, int kp, int box_k
   return detail::encode_map(map, base, rows, kp, box_k, box_rows, swz);
 }
 
+constexpr size_t kLseSlack = 5120;  // barriers, merge buffers, alignment of the soft-min kernel
+
 struct Shape {
   Layout lay;
   int kc, kp, nfull, ntail, nhalf, bn, nstage;
@@ -1140,7 +1162,7 @@ Shape plan_shape(int d, int prec, int nlab = 0) {
   s.nfull = s.kp / 32;
   s.ntail = (s.kp % 32) / 8;
   const size_t row_bytes = (size_t)s.kp * 4;
-  const size_t budget = kSmemMax - 4096;  // barriers, merge buffers, alignment slack
+  const size_t budget = kSmemMax - kLseSlack;
   s.ok = false;
   const int cand[3][2] = {{2, 128}, {1, 128}, {1, 64}};
   for (auto& c : cand) {
@@ -1150,7 +1172,7 @@ Shape plan_shape(int d, int prec, int nlab = 0) {
     int ns = (int)((budget - a) / b);
     if (ns > 4) ns = 4;
     s.nhalf = c[0]; s.bn = c[1]; s.nstage = ns;
-    s.smem = a + ns * b + 4096;
+    s.smem = a + ns * b + kLseSlack;
     if (s.smem < (size_t)kSmemMin) s.smem = kSmemMin;
     s.ok = true;
     break;
@@ -1166,13 +1188,13 @@ Shape plan_shape(int d, int prec, int nlab = 0) {
 Shape plan_shape_csr(int d, int prec, int nlab) {
   Shape s = plan_shape(d, prec, nlab);
   if (!s.ok || s.streamed) { s.ok = false; return s; }
-  const size_t row_bytes = (size_t)s.kp * 4, budget = kSmemMax - 4096;
+  const size_t row_bytes = (size_t)s.kp * 4, budget = kSmemMax - kLseSlack;
   const size_t a = 128 * row_bytes, b = 128 * row_bytes;
   if (a + 2 * b > budget) { s.ok = false; return s; }
   int ns = (int)((budget - a) / b);
   if (ns > 4) ns = 4;
   s.nhalf = 1; s.bn = 128; s.nstage = ns;
-  s.smem = a + ns * b + 4096;
+  s.smem = a + ns * b + kLseSlack;
   if (s.smem < (size_t)kSmemMin) s.smem = kSmemMin;
   return s;
 }
@@ -1183,7 +1205,7 @@ cudaError_t launch(const Launch<NSUB>& lp, dim3 grid, size_t smem, cudaStream_t 
   // Per device (context) attribute; cheap enough to set on every launch.
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   if (e != cudaSuccess) return e;
-  kern<<<grid, 128 + 128 * NHALF * kParts, smem, st>>>(lp);
+  kern<<<grid, 128 + 128 * NHALF * lse_parts(NHALF, BN), smem, st>>>(lp);
   return cudaGetLastError();
 }
 
