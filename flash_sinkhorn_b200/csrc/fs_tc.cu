@@ -58,6 +58,14 @@ struct SubPass {
   float* part_s;
   int part_stride;
   int* tickets;
+  // VEC kernels: known log2 normaliser per row, the vector padded with zeros to whole tiles, the row's own term
+  // (potential and log-weight) and where the result goes; a non-zero device flag makes the launch a no-op.
+  const float* R;
+  const float* vpad;
+  const float* rowpot;
+  const float* rowlogw;
+  float* vout;
+  const int* skip;
   int* out_idx;  // AM kernels: arg-max column per row (values go to ep.out, multiplied by scale2)
   // CSR kernels: block-sparse list of kept (128-row block, 128-column tile) pairs. csr_rp points at the entry
   // of the first row block of this launch's row range (nblk + 1 entries are read), csr_ci is the whole
@@ -92,21 +100,26 @@ __host__ __device__ constexpr int lse_parts(int nhalf, int bn) { return nhalf ==
 // these passes and the packed arithmetic around it leaves half of the issue slots free.
 constexpr int kFmaShare = 4;
 
-// AM = false: online log-sum-exp of the scaled scores (potential update). AM = true: running maximum of the
-// raw scores and the smallest column attaining it (hard c-transform); no exponentials at all.
+// MODE_LSE: online log-sum-exp of the scaled scores (potential update). MODE_MAX: running maximum of the raw scores
+// and the smallest column attaining it (hard c-transform); no exponentials at all. MODE_VEC: weighted sum
+// sum_j 2^(t_ij - R_i) v_j in fp32 with the known normaliser R (plan times vector): no running maximum. It is bound
+// by the ex2 pipe like the soft-min and replaces a plan-times-matrix pass with one column, whose second GEMM costs as
+// much as one with 32.
 // CSR = true: the item list is the list of kept tiles (row block after row block, NHALF = 1, BN = 128) instead
 // of all nblk x ntiles pairs; everything else - contiguous ranges per CTA, segments, ticketed merge - is the same.
 // NSUB > 1: several dense passes in one launch (no arg-max, no tile list, no device-side early-stop flag).
-template <int NHALF, int BN, bool AM, bool CSR = false, int NSUB = 1>
+enum { MODE_LSE = 0, MODE_MAX = 1, MODE_VEC = 2 };
+template <int NHALF, int BN, int MODE, bool CSR = false, int NSUB = 1>
 __global__ void __launch_bounds__(128 + 128 * NHALF * lse_parts(NHALF, BN), 1)
 tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   constexpr int PARTS = lse_parts(NHALF, BN);
+  constexpr bool AM = MODE == MODE_MAX, VEC = MODE == MODE_VEC;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int BM = 128 * NHALF;
   // This CTA's items [w_begin, w_end) of the flattened (row block, column tile) list.
-  static_assert(!CSR || (NHALF == 1 && BN == 128 && !AM), "tile lists are over 128 x 128 tiles");
-  static_assert(NSUB == 1 || (!CSR && !AM), "multi-pass launches are dense soft-min passes");
+  static_assert(!CSR || (NHALF == 1 && BN == 128 && MODE == MODE_LSE), "tile lists are over 128 x 128 tiles");
+  static_assert(NSUB == 1 || (!CSR && MODE == MODE_LSE), "multi-pass launches are dense soft-min passes");
   int sub = 0;  // pass of the segment this thread's role is working on (always 0 when NSUB == 1)
   auto SP = [&]() -> const SubPass& { return P.sub[NSUB == 1 ? 0 : sub]; };
   const SubPass& p = P.sub[0];  // single-pass code paths (CSR, arg-max, early-stop flag) read pass 0
@@ -168,6 +181,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         SP().ep.out[r] = SP().ep.old[r];
     return;
   }
+
+  if (VEC && p.skip && *p.skip) return;  // uniform across the grid
 
   // ---- shared memory carve-up (all operand blocks 1024-byte aligned) ----
   uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -377,18 +392,43 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     // off_run is the fp32 exponent offset all terms of s_run are relative to: sum = s_run * 2^off_run.
     // It is carried as the ROUNDED value scale*max (not recomputed from the max), so that rescaling by
     // 2^(off_old - off_new) and the final off_run + log2(s_run) are exact identities in fp32.
-    float m_run = kRunInit, off_run = __fmul_rn(scale, kRunInit), s_run = 0.f;
+    float m_run = kRunInit, off_run = VEC ? 0.f : __fmul_rn(scale, kRunInit), s_run = 0.f;
+    float negR = 0.f;  // VEC: minus the row's normaliser
     int idx_run = 0;   // AM: column of the running maximum m_run
-    int col_tile = CSR ? 0 : w_begin % p.ntiles;  // AM: column tile of the chunk being consumed
+    int col_tile = CSR ? 0 : w_begin % p.ntiles;  // AM, VEC: column tile of the chunk being consumed
     bool ok = true;
     constexpr int CH = BN / 32 / PARTS;  // 32-column chunks of a tile owned by this warpgroup
     const int total = (w_end - w_begin) * CH;  // chunks of all segments; g / CH counts the CTA's tiles
     const int c_base = part * CH;
+    auto row_of = [&](int blk) { return SP().row_begin + blk * BM + h * 128 + q * 32 + lane; };
+    auto load_row = [&](int blk) {
+      if (VEC) negR = row_of(blk) < SP().nr ? -__ldg(SP().R + row_of(blk)) : 0.f;
+    };
     // One online-softmax update with the 32 scores of a chunk (this thread's row).
     auto consume = [&](const uint32_t (&r)[32], int chunk_in_tile) {
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
+      if (VEC) {
+        // the 32 entries of the vector: the same addresses for the whole warp
+        const float4* vv = reinterpret_cast<const float4*>(SP().vpad + col_tile * BN + (c_base + chunk_in_tile) * 32);
+        const u64 sc2 = pk(scale, scale), off2 = pk(negR, negR);
+        u64 s0 = pk(s_run, 0.f), s1 = 0ull;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 w = __ldg(vv + i);
+          const u64 za = fma2(pk(v[4 * i], v[4 * i + 1]), sc2, off2), zb = fma2(pk(v[4 * i + 2], v[4 * i + 3]), sc2, off2);
+          float z0, z1, z2, z3;
+          upk(za, z0, z1);
+          upk(zb, z2, z3);
+          s0 = fma2(pk(ex2(z0), ex2(z1)), pk(w.x, w.y), s0);
+          s1 = fma2((i & 1) ? exp2_fma(zb) : pk(ex2(z2), ex2(z3)), pk(w.z, w.w), s1);
+        }
+        float a0, a1;
+        upk(add2(s0, s1), a0, a1);
+        s_run = a0 + a1;
+        return;
+      }
       float t[11];
 #pragma unroll
       for (int i = 0; i < 10; ++i) t[i] = max3(v[3 * i], v[3 * i + 1], v[3 * i + 2]);
@@ -553,13 +593,18 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
           SP().ep.out[r] = scale * m_run;  // scale2 = -2*cost_scale turns the maximal score into the minimal cost
           SP().out_idx[r] = idx_run;
         }
+      } else if (VEC) {
+        if (finish && live && part == 0 && r < SP().nr && !*abort_flag) {
+          const float rt = (__ldg(SP().rowpot + r) * (1.0f / SP().eps) + (SP().rowlogw ? __ldg(SP().rowlogw + r) : 0.f)) * kLog2e;
+          SP().vout[r] = ex2(rt + __ldg(SP().R + r)) * s_run;
+        }
       } else if (finish && live && part == 0 && r < SP().nr && !*abort_flag) {
         store_lse(r, off_run + log2f(fmaxf(s_run, 1e-40f)));
       }
       // merge_off / merge_sum / last_flag are re-used by the next segment
       asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");
       m_run = kRunInit;
-      off_run = __fmul_rn(scale, kRunInit);
+      off_run = VEC ? 0.f : __fmul_rn(scale, kRunInit);
       s_run = 0.f;
       idx_run = 0;
     };
@@ -570,6 +615,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       seg_w += seg_len();
       if (seg_w < w_end) {
         seg_blk = next_blk(seg_blk, seg_w);
+        load_row(seg_blk);
         if (NSUB > 1) {  // the next segment may belong to another pass, with its own logit scale
           scale = pass_scale();
           off_run = __fmul_rn(scale, kRunInit);
@@ -577,13 +623,14 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       }
     };
     int seg_end_g = has_work ? seg_len() * CH : 0;
+    if (has_work) load_row(seg_blk);
     auto consumed = [&](int g) {  // chunk g has been folded in: close the segment if it was its last chunk
-      if (AM && g % CH == CH - 1) ++col_tile;
+      if ((AM || VEC) && g % CH == CH - 1) ++col_tile;
       if (g + 1 == seg_end_g) {
         finalize(seg_blk, true);
         next_seg();
         if (seg_w < w_end) seg_end_g += seg_len() * CH;
-        if (AM) col_tile = 0;  // every later segment starts a new row block at column 0
+        if (AM || VEC) col_tile = 0;  // every later segment starts a new row block at column 0
       }
     };
     // Software pipeline, two register buffers: the load of chunk g+1 is in flight while chunk g is consumed
@@ -1199,9 +1246,9 @@ Shape plan_shape_csr(int d, int prec, int nlab) {
   return s;
 }
 
-template <int NHALF, int BN, bool AM, bool CSR = false, int NSUB = 1>
+template <int NHALF, int BN, int MODE, bool CSR = false, int NSUB = 1>
 cudaError_t launch(const Launch<NSUB>& lp, dim3 grid, size_t smem, cudaStream_t st) {
-  auto kern = tc_lse_kernel<NHALF, BN, AM, CSR, NSUB>;
+  auto kern = tc_lse_kernel<NHALF, BN, MODE, CSR, NSUB>;
   // Per device (context) attribute; cheap enough to set on every launch.
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   if (e != cudaSuccess) return e;
@@ -1505,15 +1552,15 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   kp.csr_rp = csr ? a.tile_row_ptr + a.row_begin / 128 : nullptr;
   kp.csr_ci = a.tile_col_idx;
   dim3 grid(pick_ctas(kp.nblk, kp.ntiles));
-  if (csr) return launch<1, 128, false, true>(lp, grid, sh.smem, st);
+  if (csr) return launch<1, 128, MODE_LSE, true>(lp, grid, sh.smem, st);
   if (am) {
-    if (sh.nhalf == 2) return launch<2, 128, true>(lp, grid, sh.smem, st);
-    if (sh.bn == 128) return launch<1, 128, true>(lp, grid, sh.smem, st);
-    return launch<1, 64, true>(lp, grid, sh.smem, st);
+    if (sh.nhalf == 2) return launch<2, 128, MODE_MAX>(lp, grid, sh.smem, st);
+    if (sh.bn == 128) return launch<1, 128, MODE_MAX>(lp, grid, sh.smem, st);
+    return launch<1, 64, MODE_MAX>(lp, grid, sh.smem, st);
   }
-  if (sh.nhalf == 2) return launch<2, 128, false>(lp, grid, sh.smem, st);
-  if (sh.bn == 128) return launch<1, 128, false>(lp, grid, sh.smem, st);
-  return launch<1, 64, false>(lp, grid, sh.smem, st);
+  if (sh.nhalf == 2) return launch<2, 128, MODE_LSE>(lp, grid, sh.smem, st);
+  if (sh.bn == 128) return launch<1, 128, MODE_LSE>(lp, grid, sh.smem, st);
+  return launch<1, 64, MODE_LSE>(lp, grid, sh.smem, st);
 }
 }  // namespace
 
@@ -1574,9 +1621,9 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
   for (int k = 0; k < used; ++k) max_tiles = lp.sub[k].ntiles > max_tiles ? lp.sub[k].ntiles : max_tiles;
   while (g > 1 && (long long)max_tiles * g / total + 2 > kMaxChunks) --g;
   dim3 grid((unsigned)g);
-  if (sh.nhalf == 2) return launch<2, 128, false, false, kMaxSub>(lp, grid, sh.smem, st);
-  if (sh.bn == 128) return launch<1, 128, false, false, kMaxSub>(lp, grid, sh.smem, st);
-  return launch<1, 64, false, false, kMaxSub>(lp, grid, sh.smem, st);
+  if (sh.nhalf == 2) return launch<2, 128, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
+  if (sh.bn == 128) return launch<1, 128, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
+  return launch<1, 64, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
 }
 
 cudaError_t argmax(const Staged& s, int side, const StreamArgs& a, float* out_val, int* out_idx, cudaStream_t st) {
@@ -1690,8 +1737,35 @@ size_t pv_scratch_bytes(int nc, int d, int prec, int dv, int nlab) {
          (size_t)pv_share_slots(nc, s.bn) * 128 * s.dv_pad * sizeof(float);
 }
 
+namespace {
+// Plan times vector with the row operand resident (MODE_VEC). scratch: the padded vector.
+cudaError_t vec_pass(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa, char* scratch, const Shape& sh,
+                     cudaStream_t st) {
+  if (!scratch || !pa.R || !pa.V || !pa.out) return cudaErrorInvalidValue;
+  const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
+  const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
+  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
+  float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
+  detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
+  Launch<1> lp{};
+  lp.nsub = 1;
+  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
+  SubPass& kp = lp.sub[0];
+  if (!fill_subpass(kp, s, side, a, LseEpilogue(), sh, scale2)) return cudaErrorInvalidValue;
+  if (kp.nblk <= 0) return cudaSuccess;
+  lp.total = (long long)kp.nblk * kp.ntiles;
+  kp.R = pa.R; kp.vpad = vpad; kp.rowpot = pa.rowpot; kp.rowlogw = pa.rowlogw; kp.vout = pa.out; kp.skip = pa.skip;
+  dim3 grid(pick_ctas(kp.nblk, kp.ntiles));
+  return sh.nhalf == 2 ? launch<2, 128, MODE_VEC>(lp, grid, sh.smem, st) : launch<1, 128, MODE_VEC>(lp, grid, sh.smem, st);
+}
+}  // namespace
+
 cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa, char* scratch, cudaStream_t st) {
   Shape sh = plan_shape(s.d, s.prec, s.nlab);
+  // Plan times vector proper: a one-column gradient (d = 1) or a scaled matrix of one column is a matrix pass.
+  if (sh.ok && !sh.streamed && sh.bn == 128 && pa.dv == 1 && !pa.rows2 && pa.epilogue == PV_APPLY && !pa.colscale &&
+      pa.coef == 1.f && pa.rowpot)
+    return vec_pass(s, side, a, pa, scratch, sh, st);
   if (sh.ok && pa.dv == 1 && !pa.rows2 && sh.bn == 64 && !sh.streamed && g_prefer_streamed.load(std::memory_order_relaxed))
     return kstream_vec(s, side, a, pa, scratch, st);
   if (sh.ok && (sh.streamed || pa.rows2)) {

@@ -152,6 +152,8 @@ int free_ctas();
 void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,
                  float inv_scale2, const Ctrl* ctrl, const unsigned* amax, cudaStream_t st, int pot_shard = 0,
                  int pot_stride = 0);
+// Copies v to out and fills up to cols_pad with zeros (a no-op when *skip is set).
+void launch_pad_vec(const float* v, int nc, int cols_pad, float* out, const int* skip, cudaStream_t st);
 inline int pad256(int r) { return (r + 255) & ~255; }
 }  // namespace detail
 

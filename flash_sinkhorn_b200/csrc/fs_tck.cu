@@ -965,6 +965,12 @@ int set_wide_tile_min_chunks(int k) {
   return g_wide_min_chunks.exchange(k, std::memory_order_relaxed);
 }
 
+namespace detail {
+void launch_pad_vec(const float* v, int nc, int cols_pad, float* out, const int* skip, cudaStream_t st) {
+  pad_vec_kernel<<<(cols_pad + 255) / 256, 256, 0, st>>>(v, nc, cols_pad, out, skip);
+}
+}  // namespace detail
+
 cudaError_t kstream_lse(const Staged& s, int side, const StreamArgs& a, const LseEpilogue& e, float* s_out,
                         long long ld_s, cudaStream_t st) {
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
@@ -998,7 +1004,7 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
-  pad_vec_kernel<<<(colc.rows_pad + 255) / 256, 256, 0, st>>>(pa.V, a.nc, colc.rows_pad, vpad, pa.skip);
+  detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
   KParams kp{};
   set_chunks(kp, s.kp);
   kp.hs = s.hs; kp.amax = s.amax;
