@@ -67,6 +67,7 @@ struct Sub {
 template <int NS>
 struct Launch {
   int nsub, nfull, ntail, nstage, slot;
+  int nb;      // column tiles in shared memory: with two, the next run's is loaded ahead
   int hs;      // leading K steps that hold fp16 coordinates
   int two_ok;  // 0: every problem of this launch runs one-sided
   Sub sub[NS];
@@ -78,7 +79,7 @@ struct FinSub {
   const float* sq[2];
   float* opA[2];
   float* opB[2];
-  double eps, eps_next, inv2cs;
+  double eps, eps_next, inv2cs, log2e_eps;
   float w, damp[2], shiftcoef[2];
 };
 template <int NS>
@@ -98,19 +99,15 @@ __device__ __forceinline__ float dec(unsigned u) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
+__device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
 }
-__device__ __forceinline__ void tmem_ld16_wait(uint32_t (&r)[16]) {
+__device__ __forceinline__ void tmem_ld8_wait(uint32_t (&r)[8]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
                :
                : "memory");
 }
@@ -142,13 +139,21 @@ struct Plan {
   int ctas;      // CTAs that take part (no more than items)
 };
 __device__ __forceinline__ int diag_tiles(const Geo& g) { return g.bn / g.bm; }  // row tiles on the diagonal: 1 or 2
-__device__ __forceinline__ int self_offset(const Geo& g, int ct) {  // items of the column tiles before ct
-  return ct * g.nrt[0] - diag_tiles(g) * (ct * (ct - 1) / 2);
+// Row tiles of column tile ct of a self problem, and the items before it: column tiles go in pairs (p, last - p), whose
+// lengths add up to the same number for every pair, so that short and long runs spread evenly over the CTAs.
+__device__ __forceinline__ int self_len(const Geo& g, int ct) { return g.nrt[0] - diag_tiles(g) * ct; }
+__device__ __forceinline__ int self_offset(const Geo& g, int ct) {
+  const int last = g.nct[0] - 1, pair = self_len(g, 0) + self_len(g, last);
+  return 2 * ct <= last ? ct * pair : (last - ct) * pair + self_len(g, last - ct);
+}
+__device__ __forceinline__ int self_items(const Geo& g) {
+  const int last = g.nct[0] - 1, pair = self_len(g, 0) + self_len(g, last);
+  return (g.nct[0] / 2) * pair + ((g.nct[0] & 1) ? self_len(g, last / 2) : 0);
 }
 __device__ int item_count(const Geo& g, bool two) {
   if (g.early && g.ctrl->converged) return 0;
   const int one = g.nct[1] * g.nrt[0];
-  if (two) return g.self ? self_offset(g, g.nct[0]) : one;
+  if (two) return g.self ? self_items(g) : one;
   return g.self ? one : one + g.nct[0] * g.nrt[1];
 }
 // By one whole warp.
@@ -175,9 +180,14 @@ __device__ void make_plan(const L& P, int slot, int max_ctas, Plan* pl, int lane
     pl->ctas = total < max_ctas ? total : max_ctas;
   }
 }
-__device__ __forceinline__ int cta_first(int total, int ctas, int c) { return (int)(((long long)total * c) / ctas); }
+// (a * b) / c for a * b of up to 63 bits; one 32-bit division where the product fits.
+__device__ __forceinline__ int mul_div(int a, int b, int c) {
+  const unsigned long long p = (unsigned long long)(unsigned)a * (unsigned)b;
+  return p >> 32 ? (int)(p / (unsigned)c) : (int)((unsigned)p / (unsigned)c);
+}
+__device__ __forceinline__ int cta_first(int total, int ctas, int c) { return mul_div(total, c, ctas); }
 __device__ __forceinline__ int cta_of(int total, int ctas, int t) {
-  int c = (int)(((long long)t * ctas) / total);
+  int c = mul_div(t, ctas, total);
   while (c + 1 < ctas && cta_first(total, ctas, c + 1) <= t) ++c;
   while (c > 0 && cta_first(total, ctas, c) > t) --c;
   return c;
@@ -201,15 +211,15 @@ __device__ Seg locate(const L& P, const Plan& pl, int w, int w_end) {
   s.strip0 = pl.item0[s.sub];
   const int r0 = g.nrt[0];
   if (s.two && g.self) {
-    int lo = 0, hi = g.nct[0] - 1;  // largest ct with self_offset(ct) <= k
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (self_offset(g, mid) <= k) lo = mid; else hi = mid - 1;
+    const int last = g.nct[0] - 1, pair = self_len(g, 0) + self_len(g, last), p = k / pair;
+    k -= p * pair;
+    s.ct = p;
+    if (k >= self_len(g, p)) {
+      k -= self_len(g, p);
+      s.ct = last - p;
     }
-    s.ct = lo;
-    s.strip0 += self_offset(g, lo);
-    k -= self_offset(g, lo);
-    s.rt = diag_tiles(g) * lo + k;
+    s.strip0 += self_offset(g, s.ct);
+    s.rt = diag_tiles(g) * s.ct + k;
     left = r0 - s.rt;
   } else {
     int rows = r0;
@@ -224,6 +234,22 @@ __device__ Seg locate(const L& P, const Plan& pl, int w, int w_end) {
     s.strip0 += s.ct * rows;
     left = rows - s.rt;
   }
+  s.len = left < w_end - w ? left : w_end - w;
+  return s;
+}
+
+// The run after s, which starts at item w, without the divisions of locate() while the problem and side stay the same.
+template <class L>
+__device__ __forceinline__ Seg next_run(const L& P, const Plan& pl, Seg s, int w, int w_end) {
+  const Geo& g = P.sub[s.sub].geo;
+  const bool fold = s.two && g.self;
+  const int last = g.nct[1 - s.side] - 1;
+  const int ct = !fold ? s.ct + 1 : (2 * s.ct < last ? last - s.ct : last - s.ct + 1);
+  if (w >= pl.item0[s.sub + 1] || ct > last || (fold && 2 * s.ct == last)) return locate(P, pl, w, w_end);
+  s.strip0 = w;
+  s.ct = ct;
+  s.rt = fold ? diag_tiles(g) * ct : 0;
+  const int left = g.nrt[s.side] - s.rt;
   s.len = left < w_end - w ? left : w_end - w;
   return s;
 }
@@ -252,11 +278,10 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   const uint32_t b_bytes = KS ? 0 : P.nfull * (kBN * 128) + P.ntail * (kBN * 32);
   const uint32_t a_bytes = KS ? kChunk : P.nfull * (128 * 128) + P.ntail * (128 * 32);
   uint8_t* b_smem = base;
-  uint8_t* a_smem = b_smem + b_bytes;
+  uint8_t* a_smem = b_smem + P.nb * b_bytes;
   float* part = (float*)(a_smem + P.nstage * a_bytes);  // [2 slots][offset | sum][kWG][128]
-  float* colred = part + 2 * 2 * kWG * 128;             // [kWG][4 warps][64]
-  uint64_t* bars = (uint64_t*)(colred + kWG * 4 * 64);
-  const int A_FULL = 0, A_EMPTY = P.nstage, B_FULL = 2 * P.nstage, B_EMPTY = B_FULL + 1, S_FULL = B_EMPTY + 1,
+  uint64_t* bars = (uint64_t*)(part + 2 * 2 * kWG * 128);
+  const int A_FULL = 0, A_EMPTY = P.nstage, B_FULL = 2 * P.nstage, B_EMPTY = B_FULL + 2, S_FULL = B_EMPTY + 2,
             S_EMPTY = S_FULL + 2, R_FULL = S_EMPTY + 2, R_EMPTY = R_FULL + 2, DRAIN = R_EMPTY + 2, NBARS = DRAIN + 1;
   uint32_t* tmem_slot = (uint32_t*)(bars + NBARS);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
@@ -268,9 +293,9 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
       mbar_init(bar(A_FULL + s), 1);
       mbar_init(bar(A_EMPTY + s), 1);
     }
-    mbar_init(bar(B_FULL), 1);
-    mbar_init(bar(B_EMPTY), 1);
     for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(B_FULL + i), 1);
+      mbar_init(bar(B_EMPTY + i), 1);
       mbar_init(bar(S_FULL + i), 1);
       mbar_init(bar(S_EMPTY + i), 4 * kWG);  // one arrive per soft-max warp
       mbar_init(bar(R_FULL + i), 4 * kWG);
@@ -342,34 +367,44 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
         ++issued;
         return true;
       };
-      Seg s = locate(P, *plan, w_begin, w_end);
-#pragma unroll 1
-      for (int w = w_begin; ok && w < w_end; ++seg) {
-        // the previous column tile must have been read by its last MMA
-        if (!mbar_wait(bar(B_EMPTY), (seg & 1) ^ 1, abort_flag, 2000)) break;
-        mbar_expect_tx(bar(B_FULL), b_bytes);
+      auto load_b = [&](const Seg& s) -> bool {  // column tile of run `seg`
+        const int sl = seg % P.nb;
+        // the column tile that was there must have been read by its last MMA
+        if (!mbar_wait(bar(B_EMPTY + sl), ((seg / P.nb) & 1) ^ 1, abort_flag, 2000)) return false;
+        mbar_expect_tx(bar(B_FULL + sl), b_bytes);
         const Sub& u = P.sub[s.sub];
-        const uint32_t dst = smem_u32(b_smem);
+        const uint32_t dst = smem_u32(b_smem + sl * b_bytes);
         for (int kb = 0; kb < P.nfull; ++kb)
-          tma_load_2d(dst + kb * (kBN * 128), &u.b_full[s.side], kb * 32, s.ct * kBN, bar(B_FULL));
+          tma_load_2d(dst + kb * (kBN * 128), &u.b_full[s.side], kb * 32, s.ct * kBN, bar(B_FULL + sl));
         for (int k = 0; k < P.ntail; ++k)
           tma_load_2d(dst + P.nfull * (kBN * 128) + k * (kBN * 32), &u.b_tail[s.side], P.nfull * 32 + k * 8, s.ct * kBN,
-                      bar(B_FULL));
+                      bar(B_FULL + sl));
+        ++seg;
+        return true;
+      };
+      Seg s = locate(P, *plan, w_begin, w_end);
+      ok = load_b(s);
+#pragma unroll 1
+      for (int w = w_begin; ok;) {
 #pragma unroll 1
         for (int t = pre; ok && t < s.len; ++t) ok = load_a(s, t);
         w += s.len;
-        // The first row tiles of the next run do not need its column tile: they fill ring slots meanwhile (every
-        // slot waited for holds a tile that the MMA warp consumes without that column tile).
+        if (!ok || w >= w_end) break;
+        s = next_run(P, *plan, s, w, w_end);
         pre = 0;
-        if (ok && w < w_end) {
-          s = locate(P, *plan, w, w_end);
+        if (P.nb > 1) {
+          ok = load_b(s);
+        } else {
+          // The first row tiles of the next run do not need its column tile: they fill ring slots meanwhile (every
+          // slot waited for holds a tile that the MMA warp consumes without that column tile).
           const int npre = s.len < P.nstage ? s.len : P.nstage;
 #pragma unroll 1
           for (; ok && pre < npre; ++pre) ok = load_a(s, pre);
+          if (ok) ok = load_b(s);
         }
       }
       if (*abort_flag) {  // let every copy issued land before the CTA goes away
-        if (seg > 0) mbar_wait_quiet(bar(B_FULL), (seg - 1) & 1);
+        for (int j = (seg > P.nb ? seg - P.nb : 0); j < seg; ++j) mbar_wait_quiet(bar(B_FULL + j % P.nb), (j / P.nb) & 1);
         for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
           mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
       }
@@ -409,9 +444,13 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
       }
     }
 #pragma unroll 1
+    Seg s;
+    if (!KS && has_work) s = locate(P, *plan, w_begin, w_end);
+#pragma unroll 1
     for (int w = w_begin; !KS && ok && w < w_end; ++seg) {
-      const Seg s = locate(P, *plan, w, w_end);
-      if (!vote(mbar_wait(bar(B_FULL), seg & 1, abort_flag, 2000))) break;
+      if (w > w_begin) s = next_run(P, *plan, s, w, w_end);
+      const int sl = seg % P.nb;
+      if (!vote(mbar_wait(bar(B_FULL + sl), (seg / P.nb) & 1, abort_flag, 2000))) break;
       tc_fence_after();
 #pragma unroll 1
       for (int i = 0; i < s.len; ++i, ++jt) {
@@ -425,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
         if (elect_one()) {
           const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
           int left = P.hs;  // fp16 K steps to go
-          uint32_t al = desc_lo(smem_u32(a_smem + st * a_bytes)), bl = desc_lo(smem_u32(b_smem));
+          uint32_t al = desc_lo(smem_u32(a_smem + st * a_bytes)), bl = desc_lo(smem_u32(b_smem + sl * b_bytes));
           uint32_t acc = 0;
 #pragma unroll 1
           for (int kb = 0; kb < P.nfull; ++kb) {
@@ -451,7 +490,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
         }
         __syncwarp();
       }
-      if (elect_one()) umma_commit(bar(B_EMPTY));  // the column tile may be replaced once these MMAs retired
+      if (elect_one()) umma_commit(bar(B_EMPTY + sl));  // the column tile may be replaced once these MMAs retired
       __syncwarp();
       w += s.len;
     }
@@ -464,9 +503,11 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
     // ===================== row-sum collector: adds the warpgroups' parts, one value per row =====================
     int jt = 0;
     bool ok = true;
+    Seg s;
+    if (has_work) s = locate(P, *plan, w_begin, w_end);
 #pragma unroll 1
     for (int w = w_begin; ok && w < w_end;) {
-      const Seg s = locate(P, *plan, w, w_end);
+      if (w > w_begin) s = next_run(P, *plan, s, w, w_end);
       const Geo& g = P.sub[s.sub].geo;
       const size_t at = (size_t)s.ct * g.pad[s.side] + (size_t)s.rt * 128 + lane * 4;
 #pragma unroll 1
@@ -517,8 +558,8 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
     const int trow = q * 32 + lane;
     bool ok = true;
     int jt = 0;
-    auto wait_tile = [&]() -> bool {
-      if (!mbar_wait(bar(S_FULL + (jt & 1)), (jt >> 1) & 1, abort_flag)) return false;
+    auto wait_tile = [&](int j) -> bool {
+      if (!mbar_wait(bar(S_FULL + (j & 1)), (j >> 1) & 1, abort_flag)) return false;
       __syncwarp();
       tc_fence_after();
       return true;
@@ -538,9 +579,11 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
       if (lane == 0) mbar_arrive(bar(R_FULL + slot));
       return true;
     };
+    Seg s;
+    if (has_work) s = locate(P, *plan, w_begin, w_end);
 #pragma unroll 1
     for (int w = w_begin; w < w_end;) {
-      const Seg s = locate(P, *plan, w, w_end);
+      if (w > w_begin) s = next_run(P, *plan, s, w, w_end);
       const float scale = P.sub[s.sub].scale2 / unit_of(P.sub[s.sub].geo);  // exact: a power of two
       if (s.two) {
         const Geo& g = P.sub[s.sub].geo;
@@ -550,64 +593,66 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
         u64 acc[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) acc[i] = 0ull;
+        uint32_t ra[8], rb[8];
+        // the first scores of a tile load while the last ones of the tile before are worked on
+        if (ok && (ok = wait_tile(jt))) tmem_ld8_nowait(lane_addr + (uint32_t)((jt & 1) * kBN), ra);
 #pragma unroll 1
         for (int i = 0; ok && i < s.len; ++i, ++jt) {
-          if (!(ok = wait_tile())) break;
           const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
           u64 rs0 = 0ull, rs1 = 0ull;
-          uint32_t ra[16], rb[16];
-          tmem_ld16_nowait(src, ra);
-          auto eat = [&](const uint32_t (&r)[16], int c) {
+          auto eat = [&](const uint32_t (&r)[8], int c) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
+            for (int k = 0; k < 4; ++k) {
               float z0, z1;
               upk(mul2(pk(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1])), sc), z0, z1);
               const u64 e = pk(ex2(z0), ex2(z1));
-              acc[c * 8 + k] = add2(acc[c * 8 + k], e);
+              acc[c * 4 + k] = add2(acc[c * 4 + k], e);
               if (k & 1) rs1 = add2(rs1, e); else rs0 = add2(rs0, e);
             }
           };
-          tmem_ld16_wait(ra);
-          tmem_ld16_nowait(src + 16, rb);
-          eat(ra, 0);
-          tmem_ld16_wait(rb);
-          tmem_ld16_nowait(src + 32, ra);
-          eat(rb, 1);
-          tmem_ld16_wait(ra);
-          tmem_ld16_nowait(src + 48, rb);
-          eat(ra, 2);
-          tmem_ld16_wait(rb);
+#pragma unroll
+          for (int c = 0; c < 6; c += 2) {
+            tmem_ld8_wait(ra);
+            tmem_ld8_nowait(src + (c + 1) * 8, rb);
+            eat(ra, c);
+            tmem_ld8_wait(rb);
+            tmem_ld8_nowait(src + (c + 2) * 8, ra);
+            eat(rb, c + 1);
+          }
+          tmem_ld8_wait(ra);
+          tmem_ld8_nowait(src + 56, rb);
+          eat(ra, 6);
+          tmem_ld8_wait(rb);
           release_tile();
-          eat(rb, 3);
+          bool more = i + 1 < s.len;
+          if (more && !wait_tile(jt + 1)) more = ok = false;
+          if (more) tmem_ld8_nowait(lane_addr + (uint32_t)(((jt + 1) & 1) * kBN), ra);
+          eat(rb, 7);
           float a0, a1, a2, a3;
           upk(rs0, a0, a1);
           upk(rs1, a2, a3);
-          if (!(ok = post(0.f, (a0 + a1) + (a2 + a3)))) break;
+          if (!post(0.f, (a0 + a1) + (a2 + a3))) ok = false;
+          if (!ok) break;
           if (diag > 0) {
             --diag;
 #pragma unroll
             for (int k = 0; k < 32; ++k) acc[k] = 0ull;
           }
         }
-        // End of the run: one sum per column. Every warp goes through the barriers, also after an abort.
+        // End of the run: one sum per column and warp.
         float v[64];
 #pragma unroll
         for (int k = 0; k < 32; ++k) upk(acc[k], v[2 * k], v[2 * k + 1]);
         warp_columns(v, lane);
-        float* cr = colred + (wg * 4 + q) * 64;
-        cr[2 * lane] = v[0];
-        cr[2 * lane + 1] = v[1];
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
-        if (trow < 64 && ok) {
-          const float* c0 = colred + wg * 4 * 64 + trow;
-          const int piece = (int)blockIdx.x - cta_of(total, ctas, s.strip0);
-          g.cp[(size_t)piece * g.pad[1] + s.ct * kBN + wg * 64 + trow] = (c0[0] + c0[64]) + (c0[128] + c0[192]);
+        if (ok) {  // one row of partials per warp (32 rows of each tile): no barrier at the end of a run
+          const int piece = s.strip0 >= w_begin ? 0 : (int)blockIdx.x - cta_of(total, ctas, s.strip0);
+          float* to = g.cp + (size_t)(piece * 4 + q) * g.pad[1] + s.ct * kBN + wg * 64 + 2 * lane;
+          *reinterpret_cast<float2*>(to) = make_float2(v[0], v[1]);
         }
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + wg) : "memory");
       } else {
 #pragma unroll 1
         for (int i = 0; ok && i < s.len; ++i, ++jt) {
-          if (!(ok = wait_tile())) break;
+          if (!(ok = wait_tile(jt))) break;
           const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
           uint32_t r[32];
           float m_run = kRunInit, off = __fmul_rn(scale, kRunInit), sum = 0.f;
@@ -936,10 +981,19 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
   }
   const int nb0 = (g.n[0] + 31) / 32, nb1 = g.self ? 0 : (g.n[1] + 31) / 32;
   if ((int)blockIdx.x >= nb0 + nb1) return;
-  if (warp == 0) make_plan(P, P.slot, P.ctas, &plan, lane);
-  __syncthreads();
   const int c = (int)blockIdx.x < nb0 ? 0 : 1;
   const int i0 = ((int)blockIdx.x - (c ? nb0 : 0)) * 32, i = i0 + lane;
+  // what the last warp standing needs is fetched together with the words of the plan
+  float pot_i = 0.f, logw_i = 0.f, sq_i = 0.f;
+  if (warp == 0) {
+    if (i < g.n[c]) {
+      pot_i = __ldcg(u.pot[c] + i);
+      logw_i = __ldg(u.logw[c] + i);
+      if (u.shiftcoef[c] != 0.f) sq_i = __ldcg(u.sq[c] + i);
+    }
+    make_plan(P, P.slot, P.ctas, &plan, lane);
+  }
+  __syncthreads();
   const bool two = (plan.two >> blockIdx.y) & 1u;
   const int pad = g.pad[c];
 
@@ -954,30 +1008,32 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
         k_cols = g.nrt[0] - (int)col0;
       } else {
         const int total = plan.item0[P.nsub];
-        const int len = g.self ? g.nrt[0] - diag_tiles(g) * ct : g.nrt[0];
+        const int len = g.self ? self_len(g, ct) : g.nrt[0];
         const int first = plan.item0[blockIdx.y] + (g.self ? self_offset(g, ct) : ct * g.nrt[0]);
-        k_cols = cta_of(total, plan.ctas, first + len - 1) - cta_of(total, plan.ctas, first) + 1;
+        k_cols = 4 * (cta_of(total, plan.ctas, first + len - 1) - cta_of(total, plan.ctas, first) + 1);
       }
     }
     const int pad1 = g.pad[1];
-    float s0 = 0.f, s1 = 0.f;
-    const float* rows = g.rp_s[0] + i;
-    for (int k = warp; k < k_rows; k += 16) {
-      s0 += __ldcg(rows + (size_t)k * g.pad[0]);
-      if (k + 8 < k_rows) s1 += __ldcg(rows + (size_t)(k + 8) * g.pad[0]);
-    }
-    const float* cols = g.cp + col0 * pad1 + i;
-    for (int k = warp; k < k_cols; k += 16) {
-      s0 += __ldcg(cols + (size_t)k * pad1);
-      if (k + 8 < k_cols) s1 += __ldcg(cols + (size_t)(k + 8) * pad1);
-    }
+    // eight independent loads in flight per thread: at 50,000 points a side there are 200 partials per row, and the
+    // kernel is bound by their latency (100 us of a 1.56 ms step with two at a time)
+    auto gather = [&](const float* from, int count, size_t pitch) {
+      float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int k = warp; k < count; k += 64) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+          if (k + 8 * e < count) t[e] += __ldcg(from + (size_t)(k + 8 * e) * pitch);
+      }
+      return ((t[0] + t[1]) + (t[2] + t[3])) + ((t[4] + t[5]) + (t[6] + t[7]));
+    };
     red_m[warp][lane] = 0.f;
-    red_s[warp][lane] = s0 + s1;
+    red_s[warp][lane] = gather(g.rp_s[0] + i, k_rows, g.pad[0]) + gather(g.cp + col0 * pad1 + i, k_cols, pad1);
   } else {
     const int parts = g.nct[g.self ? 0 : 1 - c];
     float m = -INFINITY, s = 0.f;
     const float *pm = g.rp_m[c] + i, *ps = g.rp_s[c] + i;
+#pragma unroll 8
     for (int k = warp; k < parts; k += 8) m = fmaxf(m, __ldcg(pm + (size_t)k * pad));
+#pragma unroll 4
     for (int k = warp; k < parts; k += 8) s += __ldcg(ps + (size_t)k * pad) * ex2(__ldcg(pm + (size_t)k * pad) - m);
     red_m[warp][lane] = m;
     red_s[warp][lane] = s;
@@ -1000,10 +1056,10 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
   if (i < g.n[c]) {
     // log2 of the weighted sum with the point's own bias inside; the candidate takes that bias out again
     const float l2 = m + log2f(fmaxf(s, 1e-40f));
-    const double old = (double)u.pot[c][i], lw = (double)u.logw[c][i], own = own_logw(lw);
+    const double old = (double)pot_i, lw = (double)logw_i, own = own_logw(lw);
     const double cand = (double)u.damp[c] * (old + u.eps * (own - (double)l2 * 0.69314718055994530942));
     double v = (1.0 - (double)u.w) * old + (double)u.w * cand;
-    if (u.shiftcoef[c] != 0.f) v -= (double)u.shiftcoef[c] * (double)u.sq[c][i];
+    if (u.shiftcoef[c] != 0.f) v -= (double)u.shiftcoef[c] * (double)sq_i;
     const float now = (float)v;
     u.pot[c][i] = now;
     const size_t at = (size_t)i * P.kp + P.kc;
@@ -1011,7 +1067,7 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
     write_bias(u.opA[c] + at + 3, ((double)now + own * u.eps_next) * to_unit);
     write_bias(u.opB[c] + at, ((double)now + lw * u.eps_next) * to_unit);
     const float big_l = (float)((double)l2 - own * 1.4426950408889634);
-    const float dlt = (float)(((double)now - old) * 1.4426950408889634 / u.eps);
+    const float dlt = (float)(((double)now - old) * u.log2e_eps);
     st_u = big_l + dlt;
     st_l = -st_u;
     st_dx = dlt;
@@ -1169,7 +1225,7 @@ __global__ void sym_emit_kernel(const __grid_constant__ EmitJobs P) {
 enum Kind { RESIDENT = 0, STREAMED = 1, WIDE = 2, SMALL = 3 };
 struct Shape {
   int kind, bm, bn;
-  int hs, kc, kp, nfull, ntail, nstage;  // K-streamed kinds: nfull chunks of 32 words, the last one with ntail K steps
+  int nb, hs, kc, kp, nfull, ntail, nstage;  // K-streamed kinds: nfull chunks of 32 words, the last one with ntail K steps
   size_t smem;
 };
 
@@ -1188,9 +1244,10 @@ Shape plan_shape(int n, int m, int d, int prec, int nlab) {
     s.kind = RESIDENT;
     s.nfull = s.kp / 32;
     s.ntail = (s.kp % 32) / 8;
-    s.nstage = (int)((budget - kBN * row) / (128 * row));
+    s.nb = (2 * kBN + 3 * 128) * row <= budget ? 2 : 1;
+    s.nstage = (int)((budget - s.nb * kBN * row) / (128 * row));
     if (s.nstage > 4) s.nstage = 4;
-    s.smem = kBN * row + s.nstage * 128 * row + kOverhead;
+    s.smem = s.nb * kBN * row + s.nstage * 128 * row + kOverhead;
     if (s.smem < (size_t)kSmemMin) s.smem = kSmemMin;
     return s;
   }
@@ -1273,7 +1330,7 @@ size_t carve(Problem& p, char* buf) {
     g.rp_m[k] = c.take<float>((size_t)g.nct[1 - k] * g.pad[k]);
     g.rp_s[k] = c.take<float>((size_t)g.nct[1 - k] * g.pad[k]);
   }
-  g.cp = c.take<float>((size_t)(g.by_tile ? g.nrt[0] : max_pieces(p.n[0], p.n[1])) * g.pad[1]);
+  g.cp = c.take<float>((size_t)(g.by_tile ? g.nrt[0] : 4 * max_pieces(p.n[0], p.n[1])) * g.pad[1]);
   return c.off;
 }
 
@@ -1301,6 +1358,7 @@ cudaError_t step_n(const Step* s, int cnt, int t, cudaStream_t st) {
   lp.nsub = fp.nsub = cnt;
   lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage;
   lp.hs = sh.hs;
+  lp.nb = sh.nb;
   lp.slot = fp.slot = t % 3;
   fp.kc = sh.kc; fp.kp = sh.kp;
   long long most = 0;
@@ -1327,6 +1385,7 @@ cudaError_t step_n(const Step* s, int cnt, int t, cudaStream_t st) {
     f.eps = (float)s[i].eps;
     f.eps_next = (float)s[i].eps_next;
     f.inv2cs = 0.5 / (double)p.cs_dot;
+    f.log2e_eps = 1.4426950408889634 / f.eps;
     f.w = s[i].w;
     most += (long long)g.nct[1] * g.nrt[0] + (p.self ? 0 : (long long)g.nct[0] * g.nrt[1]);
     const int nb = tiles(p.n[0], 32) + (p.self ? 0 : tiles(p.n[1], 32));
