@@ -32,7 +32,11 @@
 //   warp 0 TMA producer, warp 1 tcgen05.mma issuer (M = 128, N = 256) and TMEM owner, warp 2 row-sum
 //   collector, warps 4..19 four soft-max warpgroups, one per 64 columns.
 // What bounds it: the ex2 pipe (16 per clock and SM): 2048 clocks per tile against 128 per K step of tensor pipe;
-// operand traffic is one 128-row tile per 2048 clocks (18 bytes per clock and SM at d = 64).
+// operand traffic is one 128-row tile per 2048 clocks (10 bytes per clock and SM at d = 64 in fp16).
+// Measured on one B200 (debiased loss and gradient, d = 64, 100 steps, TF32 mode), against two soft-mins per step:
+// 50,000 x 50,000 307 -> 172 ms (a two-sided step of the three problems 1.45 ms, 12 exponentials per clock and SM, the
+// ex2 pipe 78 % busy), 4,096 x 4,096 10.8 -> 3.8 ms (36 us a step, 9 of them exponentials: the chain of the two
+// launches binds). 16,384 x 16,384 x 2,048, 50 steps: 201 -> 58 ms.
 //
 // Every mbarrier wait is bounded; on expiry the CTA raises an abort flag, lets its copies and MMAs land, frees its
 // TMEM and returns, and a device-global error word records the event.
