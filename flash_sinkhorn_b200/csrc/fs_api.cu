@@ -216,7 +216,7 @@ struct Problem {
     if (vec_on_tc() && R) {
       PvArgs pa;
       pa.R = R; pa.V = v.v; pa.dv = 1; pa.epilogue = PV_APPLY;
-      pa.rowpot = v.rowpot; pa.rowlogw = v.rowlogw; pa.out = v.out; pa.skip = v.skip;
+      pa.rowpot = v.rowpot; pa.rowlogw = v.rowlogw; pa.out = v.out; pa.skip = v.skip; pa.bias_ready = v.bias_ready;
       return tc::pv(staged, side, s, pa, pv_scratch, st);
     }
     return simt_vec(s, v, st);
@@ -248,6 +248,7 @@ struct Problem {
     ep.lse2 = R;
     cudaError_t e = lse(side, pot, logw, eps, ep);
     if (e != cudaSuccess) return e;
+    pa.bias_ready = true;
     return pv(side, pot, logw, eps, pa);
   }
   char* pv_scratch = nullptr;  // transposed copy of V for the tensor-core matrix pass
@@ -857,6 +858,7 @@ int fs_apply_vec(const float* x, const float* y, int n, int m, int d, const floa
     ep.lse2 = R;
     FS_CUDA(p.lse(side, cpot, clw, eps, ep));
     Rp = R;
+    v.bias_ready = true;
   }
   FS_CUDA(p.vec(side, cpot, clw, eps, v, Rp));
   return FS_OK;
@@ -1555,11 +1557,11 @@ extern "C" int fs_schur_cg(const float* x, const float* y, int n, int m, int d, 
   cg_init_kernel<<<1, 1024, 0, st>>>(m, rhs, z, r, pv, s, rtol, atol);
   for (int it = 0; it < max_iter; ++it) {
     VecArgs v1;
-    v1.v = pv; v1.rowpot = f_hat; v1.rowlogw = log_a; v1.out = t; v1.skip = &s->done;
+    v1.v = pv; v1.rowpot = f_hat; v1.rowlogw = log_a; v1.out = t; v1.skip = &s->done; v1.bias_ready = on_tc;
     FS_CUDA(p.vec(0, g_hat, log_b, eps, v1, on_tc ? R_row : nullptr));
     cg_div_kernel<<<g1(n), 256, 0, st>>>(n, t, diag_x, t, s);
     VecArgs v0;
-    v0.v = t; v0.rowpot = g_hat; v0.rowlogw = log_b; v0.out = q; v0.skip = &s->done;
+    v0.v = t; v0.rowpot = g_hat; v0.rowlogw = log_b; v0.out = q; v0.skip = &s->done; v0.bias_ready = on_tc;
     FS_CUDA(p.vec(1, f_hat, log_a, eps, v0, on_tc ? R_col : nullptr));
     cg_update_kernel<<<1, 1024, 0, st>>>(m, denom, q, z, r, pv, s, it);
   }
@@ -1595,10 +1597,11 @@ extern "C" int fs_plan_session_cg(const float* x, const float* y, int n, int m, 
   for (int it = 0; it < max_iter; ++it) {
     VecArgs v1;
     v1.v = pv; v1.rowpot = f_hat; v1.rowlogw = log_a; v1.out = t; v1.skip = &s->done;
+    v1.bias_ready = it > 0;  // staged by the first iteration; nothing else of this loop writes it
     FS_CUDA(p.vec(0, g_hat, log_b, eps, v1, on_tc ? se.R[0] : nullptr));
     cg_div_kernel<<<g1(n), 256, 0, st>>>(n, t, diag_x, t, s);
     VecArgs v0;
-    v0.v = t; v0.rowpot = g_hat; v0.rowlogw = log_b; v0.out = q; v0.skip = &s->done;
+    v0.v = t; v0.rowpot = g_hat; v0.rowlogw = log_b; v0.out = q; v0.skip = &s->done; v0.bias_ready = it > 0;
     FS_CUDA(p.vec(1, f_hat, log_a, eps, v0, on_tc ? se.R[1] : nullptr));
     cg_update_kernel<<<1, 1024, 0, st>>>(m, denom, q, z, r, pv, s, it);
   }

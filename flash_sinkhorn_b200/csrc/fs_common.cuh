@@ -85,6 +85,7 @@ struct VecArgs {
   const float* rowlogw = nullptr;  // [nr]
   float* out = nullptr;            // [nr]
   const int* skip = nullptr;       // device flag: non-zero => the pass is a no-op (finished CG)
+  bool bias_ready = false;         // an earlier pass of the same call staged this side's bias from the same potential
 };
 
 enum PvEpilogue { PV_APPLY = 0, PV_GRAD = 1, PV_MAT5 = 2 };
@@ -108,6 +109,7 @@ struct PvArgs {
   float coef = 1.f;
   float* out = nullptr;            // [nr, dv]
   const int* skip = nullptr;       // device flag: non-zero => the pass is a no-op (finished CG)
+  bool bias_ready = false;         // an earlier pass of the same call staged this side's bias from the same potential
 };
 
 // --- CUDA-core engine (fs_simt.cu) ---

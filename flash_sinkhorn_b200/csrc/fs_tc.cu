@@ -413,7 +413,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         // the 32 entries of the vector: the same addresses for the whole warp
         const float4* vv = reinterpret_cast<const float4*>(SP().vpad + col_tile * BN + (c_base + chunk_in_tile) * 32);
         const u64 sc2 = pk(scale, scale), off2 = pk(negR, negR);
-        u64 s0 = pk(s_run, 0.f), s1 = 0ull;
+        u64 s0 = 0ull, s1 = 0ull;  // the chunk's own sum first: one rounding of the running sum per chunk
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const float4 w = __ldg(vv + i);
@@ -426,7 +426,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         }
         float a0, a1;
         upk(add2(s0, s1), a0, a1);
-        s_run = a0 + a1;
+        s_run += a0 + a1;
         return;
       }
       float t[11];
@@ -454,8 +454,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       const float nms = -off_new;
       // After the first tiles the running max rarely moves; when it moved for no row of the warp the
       // rescale factor is exactly 2^0 and its ex2 (one slot of the saturated pipe in 33) is skipped.
-      u64 s0 = pk(s_run, 0.f), s1 = 0ull;
-      if (__any_sync(0xffffffffu, off_new != off_run)) s0 = pk(s_run * ex2(off_run - off_new), 0.f);
+      u64 s0 = 0ull, s1 = 0ull;  // the chunk's own sum first: one rounding of the running sum per chunk
+      if (__any_sync(0xffffffffu, off_new != off_run)) s_run *= ex2(off_run - off_new);
       const u64 sc2 = pk(scale, scale), off2 = pk(nms, nms);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
@@ -472,7 +472,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       }
       float a0, a1;
       upk(add2(s0, s1), a0, a1);
-      s_run = a0 + a1;
+      s_run += a0 + a1;
       m_run = m_new;
       off_run = off_new;
     };
@@ -1120,11 +1120,21 @@ __global__ void amax_kernel(const float* x, size_t nx, const float* y, size_t ny
   else block_amax(y, ny, first, stride, amax + 1);
 }
 
-__global__ void stage_kernel(const float* __restrict__ src, int rows, int rows_pad, int d, Layout lay, int prec,
-                             const unsigned* __restrict__ amax,
-                             float* __restrict__ opA, float* __restrict__ opB,
-                             const int* __restrict__ labels, const float* __restrict__ W, int V, int cloud,
-                             float w_coef) {
+struct StageCloud {
+  const float* src;
+  int rows, rows_pad;
+  float *opA, *opB;
+  const int* labels;
+};
+__global__ void stage_kernel(const StageCloud cx, const StageCloud cy, int d, Layout lay, int prec,
+                             const unsigned* __restrict__ amax, const float* __restrict__ W, int V, float w_coef) {
+  const int cloud = blockIdx.y;
+  const StageCloud& c = cloud ? cy : cx;
+  const float* __restrict__ src = c.src;
+  const int rows = c.rows, rows_pad = c.rows_pad;
+  float* __restrict__ opA = c.opA;
+  float* __restrict__ opB = c.opB;
+  const int* __restrict__ labels = c.labels;
   size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int kc = lay.kc, kp = lay.kp, kcoord = lay.kcoord;  // [kcoord, kc) is the label block
   size_t total = (size_t)rows_pad * kp;
@@ -1479,13 +1489,16 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
       const int blocks = most / 256 + 1 < 592 ? (int)(most / 256 + 1) : 592;
       amax_kernel<<<dim3(blocks, 2), 256, 0, st>>>(x, (size_t)n * d, y, (size_t)m * d, amax);
     }
+    StageCloud sc[2];
+    size_t total = 0;
     for (int c = 0; c < 2; ++c) {
-      CloudOps& o = s.cloud[c];
-      const size_t total = (size_t)o.rows_pad * sh.kp;
-      stage_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(src[c], o.rows, o.rows_pad, d, sh.lay, prec, s.amax,
-                                                                    o.opA, o.opB, V ? lab->lab[c] : nullptr,
-                                                                    V ? lab->W : nullptr, V, c, w_coef);
+      const CloudOps& o = s.cloud[c];
+      sc[c] = StageCloud{src[c], o.rows, o.rows_pad, o.opA, o.opB, V ? lab->lab[c] : nullptr};
+      const size_t words = (size_t)o.rows_pad * sh.kp;
+      total = words > total ? words : total;
     }
+    stage_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(sc[0], sc[1], d, sh.lay, prec, s.amax,
+                                                                          V ? lab->W : nullptr, V, w_coef);
   }
   return cudaGetLastError();
 }
@@ -1744,7 +1757,8 @@ cudaError_t vec_pass(const Staged& s, int side, const StreamArgs& a, const PvArg
   if (!scratch || !pa.R || !pa.V || !pa.out) return cudaErrorInvalidValue;
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
+  if (!pa.bias_ready)
+    detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
   detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
   Launch<1> lp{};
@@ -1780,8 +1794,9 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
-                                                       1.0f / a.eps, 1.0f / scale2, nullptr, s.amax);
+  if (!pa.bias_ready)
+    bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
+                                                         1.0f / a.eps, 1.0f / scale2, nullptr, s.amax);
   // V^T (hi / lo), [nslices*dv_pad, cols_pad]
   const int vrows = ps.nslices * ps.dv_pad, vcols = colc.rows_pad;
   char* p = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);

@@ -1002,7 +1002,8 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
+  if (!pa.bias_ready)
+    detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
   detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
   KParams kp{};
