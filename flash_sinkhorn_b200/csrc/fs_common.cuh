@@ -78,6 +78,18 @@ struct LseEpilogue {
   const Ctrl* ctrl = nullptr;
 };
 
+// How the staged fp16 coordinates of a pair of clouds (0 = x, 1 = y) are scaled (fs_ptx.cuh, wide_range).
+constexpr int kRangeWords = 6;  // float bits of the largest |coordinate| of x, of y, complements of their smallest non-zero
+                                // row maximum; 1 when the range is wide; counter of the blocks that looked
+struct OperandScales {
+  const unsigned* range = nullptr;           // kRangeWords of them (null: not scaled)
+  const float* inv[2] = {nullptr, nullptr};  // 1 / scale of every point (padded rows: 1), used when the range is wide
+};
+// Octaves below a cloud's largest coordinate over which the other points' largest ones may spread. From 2^14 down, an
+// fp16 keeps 11 significant bits to its smallest normal number 2^-14 (28 octaves, two in reserve). A pair of pieces keeps
+// 22 as long as the second one, 22 bits below, is above the smallest subnormal 2^-24.
+__host__ __device__ inline int scale_octaves(int prec) { return prec == 0 ? 26 : 15; }
+
 // Weighted pass: out_i = 2^(rowterm2_i) * sum_j 2^(t_ij) * v_j, rowterm2_i = (rowpot_i/eps + rowlogw_i)*log2e
 struct VecArgs {
   const float* v = nullptr;        // [nc]

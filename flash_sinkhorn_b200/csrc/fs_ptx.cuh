@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fs_common.cuh"
+
 namespace fs {
 namespace tc {
 namespace {
@@ -287,21 +289,54 @@ __device__ __forceinline__ void umma_step(bool half, uint32_t d_tmem, uint64_t a
   }
 }
 
-// Power of two that brings a cloud whose largest |coordinate| has these float bits to [2^14, 2^15): there an fp16
-// carries the 11 significant bits of a TF32 value over 28 octaves and an absolute 2^-39 of the largest below that,
-// far under the fp32 rounding of the contraction. All-zero and non-finite clouds are left as they are; the limits
-// keep the product of two scales well inside the exponent range of the bias columns it multiplies (coordinates
-// beyond 2^64 overflow fp32 when squared anyway).
-__device__ __forceinline__ float cloud_scale(unsigned amax_bits) {
-  const int e = (int)(amax_bits >> 23);
-  if (amax_bits == 0u || e >= 255) return 1.f;
-  int k = 14 - (e - 127);
-  k = k > 30 ? 30 : (k < -50 ? -50 : k);
-  return __uint_as_float((unsigned)(k + 127) << 23);
+// Scaled fp16 coordinates. Float bits of a magnitude -> k of the power of two that brings it to [2^14, 2^15): there an
+// fp16 carries the 11 significant bits of a TF32 value, and a pair of them 22, over some octaves below.
+__device__ __forceinline__ int scale_exponent(unsigned bits, int lo, int hi) {
+  const int e = (int)(bits >> 23);
+  if (bits == 0u || e >= 255) return 0;
+  const int k = 14 - (e - 127);
+  return k > hi ? hi : (k < lo ? lo : k);
 }
-// Product of the two clouds' scales (amax[0], amax[1]); 1 where the operands are not scaled (null).
-__device__ __forceinline__ float pair_scale(const unsigned* amax) {
-  return amax ? cloud_scale(amax[0]) * cloud_scale(amax[1]) : 1.f;
+__device__ __forceinline__ float power_of_two(int k) { return __uint_as_float((unsigned)(k + 127) << 23); }
+// ONE scale per cloud, from its largest |coordinate|: the product of two clouds' scales divides the logit scale. The
+// limits keep that product well inside the exponent range of the bias columns it multiplies.
+__device__ __forceinline__ float cloud_scale(unsigned amax_bits) { return power_of_two(scale_exponent(amax_bits, -50, 30)); }
+__device__ __forceinline__ float pair_scale(const unsigned* range) {
+  return range ? cloud_scale(range[0]) * cloud_scale(range[1]) : 1.f;
+}
+// A scale of its own for a point. The upper limit leaves bias columns of up to 2^30 against two tiny points.
+__device__ __forceinline__ int point_exponent(unsigned max_bits) { return scale_exponent(max_bits, -113, 48); }
+
+// Whether one scale per cloud is enough: it has to carry the largest coordinate without overflow and the largest
+// coordinate of EVERY point (other than zeros) within `octaves` below it, the range over which the point keeps the
+// significant bits of TF32 pieces. A point far from the rest, an infinity or a NaN would take them from all others.
+__device__ __forceinline__ bool narrow_cloud(unsigned top, unsigned low_complement, int octaves) {
+  const int k = scale_exponent(top, -50, 30) - 127;
+  return top == 0u || (top < 0x7f800000u && (int)(top >> 23) + k <= 14 && (int)(~low_complement >> 23) + k >= 14 - octaves);
+}
+// Where it is not enough for either cloud, every point has its own scale in both roles, ones, bias and label columns carry
+// it along, and each score is divided by the two points' scales where it leaves the accumulator.
+__device__ __forceinline__ bool wide_range(const OperandScales& s) { return s.range && s.range[4] != 0u; }
+// What the coordinates of point r of a cloud are multiplied by; its column of ones; its bias and label columns.
+__device__ __forceinline__ float coord_factor(const OperandScales& s, bool wide, int cloud, int r) {
+  return !s.range ? 1.f : (wide ? 1.f / s.inv[cloud][r] : cloud_scale(s.range[cloud]));
+}
+__device__ __forceinline__ float ones_factor(const OperandScales& s, bool wide, int cloud, int r) {
+  return wide ? 1.f / s.inv[cloud][r] : 1.f;
+}
+__device__ __forceinline__ float bias_factor(const OperandScales& s, bool wide, int cloud, int r) {
+  return wide ? 1.f / s.inv[cloud][r] : pair_scale(s.range);
+}
+// 32 scores against consecutive columns whose 1 / scale are at inv (the same addresses for the whole warp).
+__device__ __forceinline__ void unscale_columns(uint32_t (&r)[32], const float* inv) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 f = __ldg(reinterpret_cast<const float4*>(inv) + i);
+    r[4 * i] = __float_as_uint(__uint_as_float(r[4 * i]) * f.x);
+    r[4 * i + 1] = __float_as_uint(__uint_as_float(r[4 * i + 1]) * f.y);
+    r[4 * i + 2] = __float_as_uint(__uint_as_float(r[4 * i + 2]) * f.z);
+    r[4 * i + 3] = __float_as_uint(__uint_as_float(r[4 * i + 3]) * f.w);
+  }
 }
 // Coordinate column k (32-bit word) of a staged operand row, row role (va) and column role (vb). parts = 1: the
 // coordinates to 11 significant bits; parts = 3: [hi | hi | lo] against [hi | lo | hi], 22 bits and a product that
@@ -325,15 +360,71 @@ __device__ __forceinline__ void stage_coord(const float* row, int k, int d, int 
     vb = part == 1 ? lo : hi;
   }
 }
-// Largest |value| of an array as float bits (NaN and inf come out above every finite value). *out starts at zero.
-__device__ __forceinline__ void block_amax(const float* v, size_t count, size_t first, size_t stride, unsigned* out) {
-  unsigned m = 0u;
-  for (size_t i = first; i < count; i += stride) {
-    const unsigned b = __float_as_uint(v[i]) & 0x7fffffffu;
-    m = b > m ? b : m;
+// Largest |coordinate| of every row of x [rows, d]: 1 / point scale to inv [pad] (1 for padded rows; null: not wanted) and,
+// unless range is null, the range over all rows into its words `cloud` and 2 + cloud, as float bits (NaN and inf come out
+// above every finite value). range starts at zero; the last of `looking` blocks, over both clouds, decides whether it is
+// wide. By whole blocks, `block` of `blocks`. Bound by the read of the cloud: 256 KB and more in flight per SM.
+__device__ __forceinline__ void row_ranges(const float* x, int rows, int pad, int d, int block, int blocks, float* inv,
+                                           unsigned* range, int cloud, int looking, int octaves) {
+  const int lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5, warp = (int)threadIdx.x >> 5;
+  unsigned hi = 0u, lo = 0u;
+  auto bits = [&](long long r, int k) { return __float_as_uint(__ldg(x + (size_t)r * d + k)) & 0x7fffffffu; };
+  auto put = [&](unsigned m) {
+    hi = m > hi ? m : hi;
+    lo = m && ~m > lo ? ~m : lo;
+  };
+  if (d <= 64) {  // eight short rows at a time
+    for (long long r0 = (long long)(block * warps + warp) * 8; r0 < pad; r0 += (long long)blocks * warps * 8) {
+      unsigned m[8], mine = 0u;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const bool in = r0 + u < rows;
+        const unsigned a = in && lane < d ? bits(r0 + u, lane) : 0u, b = in && lane + 32 < d ? bits(r0 + u, lane + 32) : 0u;
+        m[u] = a > b ? a : b;
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        m[u] = __reduce_max_sync(0xffffffffu, m[u]);
+        put(m[u]);
+        mine = lane == u ? m[u] : mine;
+      }
+      if (inv && lane < 8 && r0 + lane < pad) inv[r0 + lane] = power_of_two(-point_exponent(mine));
+    }
+  } else {
+    for (long long r = block * warps + warp; r < pad; r += (long long)blocks * warps) {
+      unsigned m = 0u;
+      if (r < rows) {
+#pragma unroll 8
+        for (int k = lane; k < d; k += 32) {
+          const unsigned b = bits(r, k);
+          m = b > m ? b : m;
+        }
+      }
+      m = __reduce_max_sync(0xffffffffu, m);
+      put(m);
+      if (inv && lane == 0) inv[r] = power_of_two(-point_exponent(m));
+    }
   }
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+  if (!range) return;
+  __shared__ unsigned red[2][32];
+  if (lane == 0) {
+    red[0][warp] = hi;
+    red[1][warp] = lo;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    hi = __reduce_max_sync(0xffffffffu, lane < warps ? red[0][lane] : 0u);
+    lo = __reduce_max_sync(0xffffffffu, lane < warps ? red[1][lane] : 0u);
+    if (lane == 0) {
+      if (hi) atomicMax(range + cloud, hi);
+      if (lo) atomicMax(range + 2 + cloud, lo);
+      __threadfence();
+      if (atomicAdd(range + 5, 1u) == (unsigned)looking - 1u) {
+        const volatile unsigned* w = range;
+        range[4] = narrow_cloud(w[0], w[2], octaves) && narrow_cloud(w[1], w[3], octaves) ? 0u : 1u;
+      }
+    }
+  }
 }
 
 // Round-to-nearest (ties away) onto the 10-bit TF32 mantissa with two integer operations; the conversion

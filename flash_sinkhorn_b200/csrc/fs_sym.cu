@@ -18,8 +18,8 @@
 //                                                 >= r (L_i + dlt_i + min dlt_j) - (r - 1) max(0, log2 sum b)
 // (upper: b_j 2^{z_ij} <= 2^{L_i}; lower: Jensen). A step is "two-sided" when these bounds keep every weighted row
 // and column sum inside [2^-90, 2^120]; otherwise - the first steps of a solve from zero potentials at small eps,
-// weights of zero, any NaN - the same kernel runs it "one-sided": rows of x, then rows of y, per-tile maxima, as
-// (offset, sum) pairs. The decision is taken on the device from the same words by every CTA; the host enqueues the
+// weights of zero, any NaN, points with scales of their own (wide_range) - the same kernel runs it "one-sided": rows of
+// x, then rows of y, per-tile maxima, as (offset, sum) pairs. The decision is taken on the device from the same words by every CTA; the host enqueues the
 // same launches either way. Simulated over eps from 0.0002 d to annealed schedules: two-sided from the second to
 // the seventh step on, the row sums then within 2^+-30 of their weights.
 //
@@ -131,9 +131,6 @@ __device__ bool two_sided(const Geo& g, int slot) {
   const float col_hi = r * (ug + df_max) + (r - 1.f) * wa, col_lo = r * (lg + df_min) - (r - 1.f) * mass_a;
   return row_hi + la <= 120.f && row_lo - wa >= -90.f && col_hi + lb <= 120.f && col_lo - wb >= -90.f;
 }
-
-// What a score is multiplied by in the contraction: the product of the two clouds' scales.
-__device__ __forceinline__ float unit_of(const Geo& g) { return g.scaled ? pair_scale(g.st->amax) : 1.f; }
 
 // Items of a launch: problem after problem; two-sided: column tile after column tile, all its row tiles (from the
 // diagonal on for a self problem); one-sided: side 0 that way, then side 1.
@@ -588,9 +585,10 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
 #pragma unroll 1
     for (int w = w_begin; w < w_end;) {
       if (w > w_begin) s = next_run(P, *plan, s, w, w_end);
-      const float scale = P.sub[s.sub].scale2 / unit_of(P.sub[s.sub].geo);  // exact: a power of two
+      const Geo& g = P.sub[s.sub].geo;
+      const float pair = P.sub[s.sub].scale2 / pair_scale(g.scales.range);  // exact: a power of two
       if (s.two) {
-        const Geo& g = P.sub[s.sub].geo;
+        const float scale = pair;
         const u64 sc = pk(scale, scale);
         // row tiles that lie on the diagonal of a self problem: row sums only (both halves of each pair are there)
         int diag = g.self ? 2 * s.ct + 2 - s.rt : 0;
@@ -654,16 +652,19 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
           *reinterpret_cast<float2*>(to) = make_float2(v[0], v[1]);
         }
       } else {
+        const bool wide = wide_range(g.scales);
 #pragma unroll 1
         for (int i = 0; ok && i < s.len; ++i, ++jt) {
           if (!(ok = wait_tile(jt))) break;
           const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
+          const float scale = wide ? P.sub[s.sub].scale2 * g.scales.inv[s.side][(s.rt + i) * 128 + trow] : pair;
           uint32_t r[32];
           float m_run = kRunInit, off = __fmul_rn(scale, kRunInit), sum = 0.f;
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
             tmem_ld32_nowait(src + c * 32, r);
             tmem_ld_wait(r);
+            if (wide) unscale_columns(r, g.scales.inv[1 - s.side] + s.ct * kBN + wg * 64 + c * 32);
             float cm = __uint_as_float(r[0]);
 #pragma unroll
             for (int k = 1; k < 31; k += 2) cm = max3(cm, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
@@ -842,7 +843,8 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
   } else if (warp >= 4) {
     const int wg = (warp - 4) >> 2, h = wg / PARTS, part = wg % PARTS, q = warp & 3;
     const int trow = h * 128 + q * 32 + lane, et = tid - 128;  // row inside the tile, epilogue thread
-    const float scale = u.scale2 / unit_of(g);  // exact: a power of two
+    const float pair = u.scale2 / pair_scale(g.scales.range);  // exact: a power of two
+    const bool wide = wide_range(g.scales);
     bool ok = true;
     int jt = 0;
 #pragma unroll 1
@@ -852,6 +854,7 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
       const int buf = h * NBUF + jt % NBUF, sl = jt & 1;
       if (ok) ok = mbar_wait(bar(S_FULL + buf), (jt / NBUF) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok) != 0;
+      const float scale = wide ? u.scale2 * g.scales.inv[side][rt * BM + trow] : pair;
       float off = two ? 0.f : __fmul_rn(scale, kRunInit), m_run = kRunInit, sum = 0.f;
       if (ok) {
         tc_fence_after();
@@ -866,6 +869,7 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(S_EMPTY + buf));
           }
+          if (wide) unscale_columns(r, g.scales.inv[1 - side] + ct * BN + (part * CH + c) * 32);
           float v[32], s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
           if (two) {
 #pragma unroll
@@ -988,9 +992,10 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
   const int c = (int)blockIdx.x < nb0 ? 0 : 1;
   const int i0 = ((int)blockIdx.x - (c ? nb0 : 0)) * 32, i = i0 + lane;
   // what the last warp standing needs is fetched together with the words of the plan
-  float pot_i = 0.f, logw_i = 0.f, sq_i = 0.f;
+  float pot_i = 0.f, logw_i = 0.f, sq_i = 0.f, unit_i = 1.f;
   if (warp == 0) {
     if (i < g.n[c]) {
+      unit_i = bias_factor(g.scales, wide_range(g.scales), c, i);
       pot_i = __ldcg(u.pot[c] + i);
       logw_i = __ldg(u.logw[c] + i);
       if (u.shiftcoef[c] != 0.f) sq_i = __ldcg(u.sq[c] + i);
@@ -1067,7 +1072,7 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
     const float now = (float)v;
     u.pot[c][i] = now;
     const size_t at = (size_t)i * P.kp + P.kc;
-    const double to_unit = u.inv2cs * (double)unit_of(g);
+    const double to_unit = u.inv2cs * (double)unit_i;
     write_bias(u.opA[c] + at + 3, ((double)now + own * u.eps_next) * to_unit);
     write_bias(u.opB[c] + at, ((double)now + lw * u.eps_next) * to_unit);
     const float big_l = (float)((double)l2 - own * 1.4426950408889634);
@@ -1109,6 +1114,8 @@ struct StageSub {
   float* opB[2];
   float* pot[2];
   float* sq[2];
+  float* inv[2];
+  OperandScales scales;
   State* st;
   Ctrl* ctrl;
 };
@@ -1128,17 +1135,17 @@ __global__ void sym_reset_kernel(const __grid_constant__ StageLaunch<NS> P) {
     st->slot[1][k] = st->slot[2][k] = 0u;
   }
   for (int k = 0; k < 4; ++k) st->cst[k] = 0u;
-  st->amax[0] = st->amax[1] = 0u;
+  for (int k = 0; k < kRangeWords; ++k) st->range[k] = 0u;
   Ctrl* c = P.sub[i].ctrl;
   c->delta_bits = 0u; c->converged = 0; c->have_prev = 0; c->iters_used = 0;
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) sym_amax_kernel(const __grid_constant__ StageLaunch<NS> P) {
+__global__ void __launch_bounds__(256) sym_range_kernel(const __grid_constant__ StageLaunch<NS> P) {
   const StageSub& u = P.sub[blockIdx.y];
-  const int c = blockIdx.z;  // a self problem reads its cloud twice: both words are its own
-  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
-  block_amax(u.src[c], (size_t)u.n[c] * P.d, first, stride, &u.st->amax[c]);
+  const int c = blockIdx.z;  // a self problem reads its cloud twice: both ranges are its own
+  row_ranges(u.src[c], u.n[c], u.pad[c], P.d, blockIdx.x, gridDim.x, c == 1 && u.self ? nullptr : u.inv[c], u.st->range, c,
+             2 * gridDim.x, scale_octaves(P.prec));
 }
 
 // One warp per point of cloud P.cloud: both operand rows (stage_coord, label columns), the squared
@@ -1156,7 +1163,9 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
   const int r = (int)blockIdx.x * 8 + warp;
   const bool real = r < u.n[c];
   const int d = P.d, kc = P.kc, kp = P.kp, kcoord = P.kcoord;
-  const float own = P.hs ? cloud_scale(u.st->amax[c]) : 1.f, unit = P.hs ? pair_scale(u.st->amax) : 1.f;
+  const bool wide = wide_range(u.scales);
+  const float own = coord_factor(u.scales, wide, c, r), ones = ones_factor(u.scales, wide, c, r),
+              unit = bias_factor(u.scales, wide, c, r);
   const float* src = u.src[c] + (size_t)r * d;
   float* rowA = u.opA[c] + (size_t)r * kp;
   float* rowB = u.opB[c] + (size_t)r * kp;
@@ -1173,7 +1182,7 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
       stage_coord(src, k, d, P.prec == 0 ? 1 : 3, P.hs, own, va, vb);
     } else if (k < kc && real) {
       const int v = (k - kcoord) / 3, piece = (k - kcoord) % 3;
-      va = lab == v ? 1.f : 0.f;
+      va = lab == v ? ones : 0.f;
       // column role: the table entry between every class v of the other cloud and this point's label
       const float w = unit * u.w_coef * u.W[c == 0 ? lab * u.V + v : v * u.V + lab];
       const float h = to_tf32(w), mid = to_tf32(w - h), low = to_tf32(w - h - mid);
@@ -1183,8 +1192,8 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
     rowB[k] = vb;
   }
   if (lane < 3) {
-    rowA[kc + lane] = 1.f;
-    rowB[kc + 3 + lane] = 1.f;
+    rowA[kc + lane] = ones;
+    rowB[kc + 3 + lane] = ones;
   }
   if (lane == 0) {
     if (real) {
@@ -1196,7 +1205,7 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
       write_bias(rowA + kc + 3, ((double)pot + own_logw(lw) * u.eps) * u.inv2cs * (double)unit);
       write_bias(rowB + kc, ((double)pot + (double)lw * u.eps) * u.inv2cs * (double)unit);
       float l2 = lw * kLog2e;
-      if (!(fabsf(l2) < 1e30f)) l2 = -1e30f;  // such a weight keeps every step one-sided
+      if (!(fabsf(l2) < 1e30f) || wide) l2 = -1e30f;  // such a weight keeps every step one-sided, as a wide range does
       atomicMax(&wmax[0], enc(-l2));
       atomicMax(&wmax[1], enc(l2));
     } else {  // padded points contribute 2^(-2^100 * scale) = 0 in either role
@@ -1311,7 +1320,6 @@ size_t carve(Problem& p, char* buf) {
   g.bm = sh.bm;
   g.bn = sh.bn;
   g.by_tile = sh.kind >= WIDE ? 1 : 0;
-  g.scaled = sh.hs > 0 ? 1 : 0;
   for (int k = 0; k < 2; ++k) {
     g.n[k] = p.n[k];
     g.pad[k] = tc::detail::pad256(p.n[k]);
@@ -1321,6 +1329,13 @@ size_t carve(Problem& p, char* buf) {
   p.ctrl = c.take<Ctrl>(1);
   g.ctrl = p.ctrl;
   g.st = c.take<State>(1);
+  float* inv[2];
+  inv[0] = c.take<float>(g.pad[0]);
+  inv[1] = p.self ? inv[0] : c.take<float>(g.pad[1]);
+  if (sh.hs && g.st) {
+    g.scales.range = g.st->range;
+    for (int k = 0; k < 2; ++k) g.scales.inv[k] = inv[k];
+  }
   for (int k = 0; k < 2; ++k) {
     if (k == 1 && p.self) {
       p.opA[1] = p.opA[0]; p.opB[1] = p.opB[0]; p.pot[1] = p.pot[0]; p.sq[1] = p.sq[0];
@@ -1432,7 +1447,9 @@ cudaError_t stage_n(Problem* const* p, const double* eps0, int cnt, cudaStream_t
       u.src[k] = q.src[k]; u.logw[k] = q.logw[k]; u.init[k] = q.init[k]; u.label[k] = q.lab.lab[k];
       u.n[k] = q.n[k]; u.pad[k] = q.geo.pad[k];
       u.opA[k] = q.opA[k]; u.opB[k] = q.opB[k]; u.pot[k] = q.pot[k]; u.sq[k] = q.sq[k];
+      u.inv[k] = const_cast<float*>(q.geo.scales.inv[k]);
     }
+    u.scales = q.geo.scales;
     u.W = q.lab.W; u.V = q.lab.V; u.w_coef = -q.lab.lam_w / (2.0f * q.cs_dot);
     u.cs_sq = q.cs_sq; u.eps = (float)eps0[i]; u.inv2cs = 0.5 / (double)q.cs_dot;
     u.self = q.self ? 1 : 0; u.st = q.geo.st; u.ctrl = q.ctrl;
@@ -1442,8 +1459,8 @@ cudaError_t stage_n(Problem* const* p, const double* eps0, int cnt, cudaStream_t
   sym_reset_kernel<NS><<<1, 32, 0, st>>>(lp);
   count_launches(1);
   if (lp.hs) {  // both scales are known before anything is staged
-    const int most = blocks[0] > blocks[1] ? blocks[0] : blocks[1];
-    sym_amax_kernel<NS><<<dim3(most < 296 ? most : 296, cnt, 2), 256, 0, st>>>(lp);
+    const int pad = 8 * (blocks[0] > blocks[1] ? blocks[0] : blocks[1]);
+    sym_range_kernel<NS><<<dim3(tc::detail::range_blocks(pad, lp.d), cnt, 2), 256, 0, st>>>(lp);
     count_launches(1);
   }
   for (lp.cloud = 0; lp.cloud < 2; ++lp.cloud)

@@ -15,7 +15,7 @@ constexpr int kMaxProblems = 24;  // problems that advance in one launch (kernel
 struct State {
   unsigned slot[3][8];  // per step modulo 3: {max u, -min u, max dlt, -min dlt} of the rows, then of the columns
   unsigned cst[4];      // max(-log2 a), max(log2 a), max(-log2 b), max(log2 b)
-  unsigned amax[2];     // largest |coordinate| of either cloud as float bits
+  unsigned range[kRangeWords];  // of the coordinates (OperandScales)
 };
 
 // What every kernel of a step needs to know about a problem. Cloud 0 = x, cloud 1 = y.
@@ -25,8 +25,8 @@ struct Geo {
   int self;                          // one cloud against itself: only the tiles on one side of the diagonal
   int early;                         // 1: leave everything alone once ctrl->converged is set
   int by_tile;                       // column partials are one per row tile (not one per CTA and column tile)
-  int scaled;                        // the staged coordinates are multiplied by the clouds' scales
   float ratio;                       // eps of the previous step / eps of this step
+  OperandScales scales;              // of the fp16 coordinates
   State* st;
   Ctrl* ctrl;
   float* rp_m[2];  // one-sided steps: [column tile][row] offsets (log2 units) of the row sums of side c

@@ -32,6 +32,7 @@
 #include <cstdlib>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 namespace fs {
 namespace tc {
@@ -48,8 +49,9 @@ struct SubPass {
   int ntiles;        // column tiles of BN
   int nblk;          // row blocks of BM rows
   int item0;         // index of this pass's first (row block, column tile) item in the launch's item list
-  float scale2;      // 2*cs*log2e/eps: logit = scale2 * S / (product of the clouds' scales)
-  const unsigned* amax;  // where those scales come from (null: 1)
+  float scale2;      // 2*cs*log2e/eps: logit = scale2 * S / (product of the two points' scales)
+  OperandScales scales;
+  int side;          // cloud of the rows
   float eps;
   LseEpilogue ep;
   // Partial (scale2*max, sum) pairs of row blocks that several CTAs share, and one arrival counter per row
@@ -380,6 +382,9 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     }
   } else if (warp >= 4) {
     // ===================== soft-max warpgroups =====================
+    // Twice the same code: points with scales of their own (wide_range) take registers that the ordinary form needs.
+    auto soft_max = [&](auto wide_form) {
+    constexpr bool WIDE = decltype(wide_form)::value;
     const int wg = (warp - 4) >> 2;      // warpgroup index
     const int h = wg / PARTS;           // 128-row half
     const int part = wg % PARTS;        // which half of each tile's chunks
@@ -387,8 +392,14 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     // (the soft-max warps set `sub` with blk_of(w_begin) below, before the first chunk is consumed)
     if (has_work) blk_of(w_begin);
-    auto pass_scale = [&]() { return SP().scale2 / pair_scale(SP().amax); };  // exact: a power of two
-    float scale = pass_scale();  // logit scale of the current segment's pass
+    auto row_of = [&](int blk) { return SP().row_begin + blk * BM + h * 128 + q * 32 + lane; };
+    bool wide = false;
+    float scale = 1.f;  // logit scale of the current segment's pass (of this thread's row when the range is wide)
+    auto load_pass = [&]() {
+      wide = WIDE && wide_range(SP().scales);
+      scale = SP().scale2 / pair_scale(SP().scales.range);  // exact: a power of two
+    };
+    load_pass();
     // off_run is the fp32 exponent offset all terms of s_run are relative to: sum = s_run * 2^off_run.
     // It is carried as the ROUNDED value scale*max (not recomputed from the max), so that rescaling by
     // 2^(off_old - off_new) and the final off_run + log2(s_run) are exact identities in fp32.
@@ -400,12 +411,17 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     constexpr int CH = BN / 32 / PARTS;  // 32-column chunks of a tile owned by this warpgroup
     const int total = (w_end - w_begin) * CH;  // chunks of all segments; g / CH counts the CTA's tiles
     const int c_base = part * CH;
-    auto row_of = [&](int blk) { return SP().row_begin + blk * BM + h * 128 + q * 32 + lane; };
     auto load_row = [&](int blk) {
       if (VEC) negR = row_of(blk) < SP().nr ? -__ldg(SP().R + row_of(blk)) : 0.f;
+      if (wide) scale = row_of(blk) < SP().nr ? SP().scale2 * __ldg(SP().scales.inv[SP().side] + row_of(blk)) : SP().scale2;
     };
-    // One online-softmax update with the 32 scores of a chunk (this thread's row).
-    auto consume = [&](const uint32_t (&r)[32], int chunk_in_tile) {
+    // One online-softmax update with the 32 scores of chunk g (this thread's row).
+    auto consume = [&](uint32_t (&r)[32], int g) {
+      const int chunk_in_tile = g % CH;
+      if (wide) {
+        const int w = w_begin + g / CH, tile = CSR ? p.csr_ci[rp0 + w] : (w - SP().item0) % SP().ntiles;
+        unscale_columns(r, SP().scales.inv[1 - SP().side] + tile * BN + (c_base + chunk_in_tile) * 32);
+      }
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
@@ -615,15 +631,14 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       seg_w += seg_len();
       if (seg_w < w_end) {
         seg_blk = next_blk(seg_blk, seg_w);
+        if (NSUB > 1) load_pass();  // the next segment may belong to another pass, with its own logit scale
         load_row(seg_blk);
-        if (NSUB > 1) {  // the next segment may belong to another pass, with its own logit scale
-          scale = pass_scale();
-          off_run = __fmul_rn(scale, kRunInit);
-        }
+        if (!VEC) off_run = __fmul_rn(scale, kRunInit);
       }
     };
     int seg_end_g = has_work ? seg_len() * CH : 0;
     if (has_work) load_row(seg_blk);
+    if (!VEC) off_run = __fmul_rn(scale, kRunInit);
     auto consumed = [&](int g) {  // chunk g has been folded in: close the segment if it was its last chunk
       if ((AM || VEC) && g % CH == CH - 1) ++col_tile;
       if (g + 1 == seg_end_g) {
@@ -644,7 +659,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         ok = issue(g + 1, rb);
         if (!ok) break;
       }
-      consume(ra, g % CH);
+      consume(ra, g);
       if (CH == 1) consumed(g);  // with two chunks per tile a segment can only end on the odd chunk
       if (g + 1 >= total) break;
       landed(g + 1, rb);
@@ -652,7 +667,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         ok = issue(g + 2, ra);
         if (!ok) break;
       }
-      consume(rb, (g + 1) % CH);
+      consume(rb, g + 1);
       consumed(g + 1);
     }
     // After an abort: keep the barrier sequence of the remaining segments (no data is written).
@@ -660,6 +675,15 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     while (seg_w < w_end) {
       finalize(seg_blk, false);
       next_seg();
+    }
+    };
+    bool any_wide = false;
+#pragma unroll
+    for (int i = 0; i < NSUB; ++i) any_wide |= i < P.nsub && wide_range(P.sub[i].scales);
+    if constexpr (BN == 128) {  // operands of the narrow tiles are not scaled (plan_shape)
+      if (any_wide) soft_max(std::true_type{}); else soft_max(std::false_type{});
+    } else {
+      soft_max(std::false_type{});
     }
   }
 
@@ -686,7 +710,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
 struct PvKernelParams {
   int nr, nc, ntiles, nfull, ntail;
   int hs;                // leading 32-byte K steps that hold fp16 coordinates
-  const unsigned* amax;  // the clouds' scales (null: 1)
+  OperandScales scales;
+  int side;              // cloud of the rows
   int nb, nv;            // ring depths: column-operand tiles (freed after the score GEMM) and V tiles
   int row_begin;         // rows [row_begin, nr) are produced
   int dv, dv_pad, dv0;   // real width, padded slice width (multiple of 32, <= 128), first column of this slice
@@ -931,7 +956,9 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int r_in = q * 32 + lane;  // row within the block
     const int r = row0 + r_in;
-    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
+    const bool wide = wide_range(p.scales);
+    // exact: powers of two
+    const float scale = wide ? p.scale2 * (r < p.nr ? p.scales.inv[p.side][r] : 1.f) : p.scale2 / pair_scale(p.scales.range);
     const float negR = (r < p.nr) ? -p.R[r] : 0.f;
     bool ok = true;
     constexpr int CH = BN / 32 / kParts;
@@ -951,6 +978,7 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
     auto weigh = [&](int g, uint32_t (&rg)[32]) {
       const int j = g / CH, c = g % CH, buf = j % kNSW;
       const uint32_t taddr = lane_addr + buf * WCOLS + (c_base + c) * 32;
+      if (wide) unscale_columns(rg, p.scales.inv[1 - p.side] + (j0 + j) * BN + (c_base + c) * 32);
       float v[32];
       if (SPLIT) {
         float lo[32];
@@ -1108,16 +1136,18 @@ __global__ void stage_vt_kernel(const float* __restrict__ V, int nc, int dv, con
 //   TF32 mode : [ x | aug (3) | 0 ... ]                       A-role aug = 1,1,1 ; B-role aug = bias split
 //   FP32 mode : A-role [ xh | xh | xl | aug | 0 ...]   B-role [ yh | yl | yh | aug | 0 ... ]
 // so that sum_k A_k B_k = xh.yh + xh.yl + xl.yh + bias  (the dropped xl.yl term is ~2^-22 relative). With fp16
-// coordinates every product carries the two clouds' scales; label and bias columns are multiplied by them too.
+// coordinates every product carries the scales of its two clouds, or points (wide_range); ones, label and bias columns
+// are multiplied so that the whole sum does.
 // Label cost: the coordinate columns are followed by 3V label columns per point, so that the table lookup
 // becomes part of the same contraction: in the row role a point of label l carries (1,1,1) in the three
 // columns of class l and zeros elsewhere; in the column role it carries, for every class v, the three-piece
 // TF32 split of w_coef * W[.,.] between v and its own label (exact in fp32, so the block is staged once in
 // either precision mode).
-__global__ void amax_kernel(const float* x, size_t nx, const float* y, size_t ny, unsigned* amax) {
-  const size_t first = (size_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (size_t)gridDim.x * blockDim.x;
-  if (blockIdx.y == 0) block_amax(x, nx, first, stride, amax);
-  else block_amax(y, ny, first, stride, amax + 1);
+__global__ void __launch_bounds__(256) range_kernel(const float* x, int n, int pad_n, const float* y, int m, int pad_m, int d,
+                                                    unsigned* range, int octaves, float* inv_x, float* inv_y) {
+  const bool c = blockIdx.y != 0;
+  row_ranges(c ? y : x, c ? m : n, c ? pad_m : pad_n, d, blockIdx.x, gridDim.x, c ? inv_y : inv_x, range, c, 2 * gridDim.x,
+             octaves);
 }
 
 struct StageCloud {
@@ -1127,7 +1157,7 @@ struct StageCloud {
   const int* labels;
 };
 __global__ void stage_kernel(const StageCloud cx, const StageCloud cy, int d, Layout lay, int prec,
-                             const unsigned* __restrict__ amax, const float* __restrict__ W, int V, float w_coef) {
+                             const OperandScales sc, const float* __restrict__ W, int V, float w_coef) {
   const int cloud = blockIdx.y;
   const StageCloud& c = cloud ? cy : cx;
   const float* __restrict__ src = c.src;
@@ -1141,21 +1171,22 @@ __global__ void stage_kernel(const StageCloud cx, const StageCloud cy, int d, La
   if (idx >= total) return;
   int r = (int)(idx / kp), k = (int)(idx % kp);
   float va = 0.f, vb = 0.f;
+  const bool wide = wide_range(sc);
   if (k < kcoord) {
     if (r < rows)
-      stage_coord(src + (size_t)r * d, k, d, prec == 0 ? 1 : 3, lay.hs, amax ? cloud_scale(amax[cloud]) : 1.f, va, vb);
+      stage_coord(src + (size_t)r * d, k, d, prec == 0 ? 1 : 3, lay.hs, coord_factor(sc, wide, cloud, r), va, vb);
   } else if (k < kc) {
     if (r < rows) {
       const int v = (k - kcoord) / 3, piece = (k - kcoord) % 3;
       const int l = labels[r];
-      va = (l == v) ? 1.f : 0.f;
+      va = (l == v) ? ones_factor(sc, wide, cloud, r) : 0.f;
       // cloud 0 (x) as column: rows are y points of label v -> W[l, v]; cloud 1 (y) as column: W[v, l]
-      const float w = pair_scale(amax) * w_coef * W[cloud == 0 ? l * V + v : v * V + l];
+      const float w = bias_factor(sc, wide, cloud, r) * w_coef * W[cloud == 0 ? l * V + v : v * V + l];
       const float h = to_tf32(w), mid = to_tf32(w - h), low = to_tf32(w - h - mid);
       vb = piece == 0 ? h : (piece == 1 ? mid : low);
     }
   } else if (k < kc + 3) {
-    va = 1.f;
+    va = ones_factor(sc, wide, cloud, r);
     vb = (k == kc && r >= rows) ? kMaskBias : 0.f;  // padded rows are masked for good
   }
   opA[idx] = va;
@@ -1165,14 +1196,14 @@ __global__ void stage_kernel(const StageCloud cx, const StageCloud cy, int d, La
 // Writes the bias of a pass, divided by the logit scale and split into 3 TF32 pieces, into opB's aug columns.
 __global__ void bias_kernel(float* __restrict__ opB, int rows, int kc, int kp, const float* __restrict__ pot,
                             const float* __restrict__ logw, float inv_eps, float inv_scale2, const Ctrl* ctrl,
-                            const unsigned* __restrict__ amax, int pot_shard = 0, int pot_stride = 0) {
+                            const OperandScales sc, int cloud, int pot_shard = 0, int pot_stride = 0) {
   if (ctrl && ctrl->converged) return;
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   const float pr = pot_shard > 0 ? pot[(size_t)(r / pot_shard) * pot_stride + r % pot_shard] : pot[r];
   // bias in log2 units, same association as the reference kernels, then / scale2
   float b2 = logw ? (pr * (inv_eps * kLog2e) + logw[r] * kLog2e) : pr * kLog2e;
-  float b = b2 * inv_scale2 * pair_scale(amax);
+  float b = b2 * inv_scale2 * bias_factor(sc, wide_range(sc), cloud, r);
   float hi = to_tf32(b);
   float r1 = b - hi;
   float mid = to_tf32(r1);
@@ -1274,7 +1305,8 @@ struct BiasJobs {
     const float* pot;
     const float* logw;
     float inv_eps, inv_scale2;
-    const unsigned* amax;
+    OperandScales scales;
+    int cloud;
     int pot_shard, pot_stride;  // packed potential (see StreamArgs), 0 = contiguous
   } job[kMaxSub];
 };
@@ -1285,7 +1317,7 @@ __global__ void bias_multi_kernel(const BiasJobs jobs) {
   if (r >= j.rows) return;
   const float pr = j.pot_shard > 0 ? j.pot[(size_t)(r / j.pot_shard) * j.pot_stride + r % j.pot_shard] : j.pot[r];
   const float b2 = j.logw ? (pr * (j.inv_eps * kLog2e) + j.logw[r] * kLog2e) : pr * kLog2e;
-  const float b = b2 * j.inv_scale2 * pair_scale(j.amax);
+  const float b = b2 * j.inv_scale2 * bias_factor(j.scales, wide_range(j.scales), j.cloud, r);
   const float hi = to_tf32(b);
   const float r1 = b - hi;
   const float mid = to_tf32(r1);
@@ -1363,11 +1395,11 @@ int pick_ctas_for(int nblk, int ntiles, int sms, int reserved, int limit) {
   return (int)g;
 }
 
-void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,
-                 float inv_scale2, const Ctrl* ctrl, const unsigned* amax, cudaStream_t st, int pot_shard,
-                 int pot_stride) {
-  bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, kc, kp, pot, logw, inv_eps, inv_scale2,
-                                                       ctrl, amax, pot_shard, pot_stride);
+void launch_bias(const Staged& s, int cloud, const float* pot, const float* logw, float inv_eps, float inv_scale2,
+                 const Ctrl* ctrl, cudaStream_t st, int pot_shard, int pot_stride) {
+  const CloudOps& o = s.cloud[cloud];
+  bias_kernel<<<(o.rows + 255) / 256, 256, 0, st>>>(o.opB, o.rows, s.kc, s.kp, pot, logw, inv_eps, inv_scale2, ctrl,
+                                                    s.scales, cloud, pot_shard, pot_stride);
 }
 
 int free_ctas() {
@@ -1447,7 +1479,8 @@ size_t staged_bytes(int n, int m, int d, int prec, int nlab) {
   b += 2 * (((size_t)pad256(m) * per_row + 1023) & ~size_t(1023));
   b += 2 * 2 * (size_t)kMaxChunks * pad256(n > m ? n : m) * sizeof(float);  // column-split partials, per side
   b += 2 * (size_t)(pad256(n > m ? n : m) / 128) * sizeof(int);             // row-block tickets, per side
-  b += 2 * sizeof(unsigned);                                                // largest coordinates
+  b += kRangeWords * sizeof(unsigned) + 256;                                         // ranges of the coordinates
+  b += ((size_t)pad256(n) + pad256(m)) * sizeof(float);                     // 1 / scale of every point
   return b + 1024;
 }
 
@@ -1479,15 +1512,22 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
   int* tk = reinterpret_cast<int*>(fp + 4 * slots);
   s.tickets[0] = tk;
   s.tickets[1] = tk + s.part_stride / 128;
-  unsigned* amax = reinterpret_cast<unsigned*>(tk + 2 * (size_t)(s.part_stride / 128));
-  s.amax = s.hs ? amax : nullptr;
+  unsigned* range = reinterpret_cast<unsigned*>(tk + 2 * (size_t)(s.part_stride / 128));
+  float* inv[2];
+  inv[0] = reinterpret_cast<float*>(((uintptr_t)(range + kRangeWords) + 255) & ~(uintptr_t)255);
+  inv[1] = inv[0] + s.cloud[0].rows_pad;
+  s.scales = OperandScales();
+  if (s.hs) {
+    s.scales.range = range;
+    s.scales.inv[0] = inv[0];
+    s.scales.inv[1] = inv[1];
+  }
   if (run_kernels) {
-    cudaError_t e = cudaMemsetAsync(tk, 0, 2 * (size_t)(s.part_stride / 128) * sizeof(int) + 2 * sizeof(unsigned), st);
+    cudaError_t e = cudaMemsetAsync(tk, 0, 2 * (size_t)(s.part_stride / 128) * sizeof(int) + kRangeWords * sizeof(unsigned), st);
     if (e != cudaSuccess) return e;
     if (s.hs) {
-      const size_t most = (size_t)(n > m ? n : m) * d;
-      const int blocks = most / 256 + 1 < 592 ? (int)(most / 256 + 1) : 592;
-      amax_kernel<<<dim3(blocks, 2), 256, 0, st>>>(x, (size_t)n * d, y, (size_t)m * d, amax);
+      range_kernel<<<dim3(detail::range_blocks(s.part_stride, d), 2), 256, 0, st>>>(
+          x, n, s.cloud[0].rows_pad, y, m, s.cloud[1].rows_pad, d, range, scale_octaves(prec), inv[0], inv[1]);
     }
     StageCloud sc[2];
     size_t total = 0;
@@ -1497,7 +1537,7 @@ cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, i
       const size_t words = (size_t)o.rows_pad * sh.kp;
       total = words > total ? words : total;
     }
-    stage_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(sc[0], sc[1], d, sh.lay, prec, s.amax,
+    stage_kernel<<<dim3((unsigned)((total + 255) / 256), 2), 256, 0, st>>>(sc[0], sc[1], d, sh.lay, prec, s.scales,
                                                                           V ? lab->W : nullptr, V, w_coef);
   }
   return cudaGetLastError();
@@ -1523,7 +1563,7 @@ bool fill_subpass(SubPass& kp, const Staged& s, int side, const StreamArgs& a, c
   const int bm = 128 * sh.nhalf;
   kp.nblk = (a.nr - a.row_begin + bm - 1) / bm;
   kp.item0 = 0;
-  kp.scale2 = scale2; kp.amax = s.amax; kp.eps = a.eps; kp.ep = e;
+  kp.scale2 = scale2; kp.scales = s.scales; kp.side = side; kp.eps = a.eps; kp.ep = e;
   kp.part_m = s.part_m[side]; kp.part_s = s.part_s[side]; kp.part_stride = s.part_stride; kp.tickets = s.tickets[side];
   kp.out_idx = nullptr; kp.csr_rp = nullptr; kp.csr_ci = nullptr;
   return ok;
@@ -1542,18 +1582,13 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   // with its 256 x 128 tiles is faster there (d = 64 in the exact mode: K = 195), unless a knob says otherwise.
   if (sh.bn == 64 && !am && !csr && g_prefer_streamed.load(std::memory_order_relaxed))
     return kstream_lse(s, side, a, e, nullptr, 0, st);
-  const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
-  const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   // LSE: logit = scale2 * (x.y + bias/scale2). Arg-max: cost = -2cs * (x.y - bias/(2cs)), so the column
   // "bias" staged next to y is -bias/(2cs) (a.pot holds the raw bias, no log-weights) and scale2 = -2cs.
   const float scale2 = am ? -2.0f * a.cost_scale : (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (am)
-    bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, nullptr, 1.0f,
-                                                         1.0f / (scale2 * kLog2e), nullptr, s.amax);
+    detail::launch_bias(s, 1 - side, a.pot, nullptr, 1.0f, 1.0f / (scale2 * kLog2e), nullptr, st);
   else
-    bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
-                                                         1.0f / a.eps, 1.0f / scale2, e.ctrl, s.amax, a.pot_shard,
-                                                         a.pot_stride);
+    detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, st, a.pot_shard, a.pot_stride);
   Launch<1> lp{};
   lp.nsub = 1;
   lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
@@ -1610,7 +1645,7 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
     BiasJobs::Job& j = jobs.job[used];
     j.opB = colc.opB; j.rows = colc.rows; j.kc = sh.kc; j.kp = sh.kp;
     j.pot = mp.a.pot; j.logw = mp.a.logw; j.inv_eps = 1.0f / mp.a.eps; j.inv_scale2 = 1.0f / scale2;
-    j.amax = s.amax;
+    j.scales = s.scales; j.cloud = 1 - mp.side;
     j.pot_shard = mp.a.pot_shard; j.pot_stride = mp.a.pot_stride;
     if (colc.rows > max_cols) max_cols = colc.rows;
     // Two passes of one launch must not write the bias columns of the same operand (nor merge in the same
@@ -1758,7 +1793,7 @@ cudaError_t vec_pass(const Staged& s, int side, const StreamArgs& a, const PvArg
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (!pa.bias_ready)
-    detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
+    detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
   detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
   Launch<1> lp{};
@@ -1795,8 +1830,7 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (!pa.bias_ready)
-    bias_kernel<<<(colc.rows + 255) / 256, 256, 0, st>>>(colc.opB, colc.rows, sh.kc, sh.kp, a.pot, a.logw,
-                                                         1.0f / a.eps, 1.0f / scale2, nullptr, s.amax);
+    detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st);
   // V^T (hi / lo), [nslices*dv_pad, cols_pad]
   const int vrows = ps.nslices * ps.dv_pad, vcols = colc.rows_pad;
   char* p = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
@@ -1820,7 +1854,7 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   PvKernelParams kp;
   kp.nr = a.nr; kp.nc = a.nc; kp.row_begin = a.row_begin;
   kp.ntiles = (a.nc + ps.bn - 1) / ps.bn;
-  kp.hs = sh.lay.hs; kp.amax = s.amax;
+  kp.hs = sh.lay.hs; kp.scales = s.scales; kp.side = side;
   kp.nfull = sh.nfull; kp.ntail = sh.ntail; kp.nb = ps.nb; kp.nv = ps.nv;
   kp.dv = pa.dv; kp.dv_pad = ps.dv_pad; kp.ld_out = pa.dv;
   kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;

@@ -42,7 +42,7 @@ struct Staged {
   CloudOps cloud[2];  // 0 = x, 1 = y
   int d = 0, nlab = 0, kc = 0, kp = 0, prec = 0;  // nlab: label-table columns staged after the coordinates
   int hs = 0;                      // leading K steps that hold fp16 coordinates
-  const unsigned* amax = nullptr;  // largest |coordinate| of either cloud as float bits (null: operands not scaled)
+  OperandScales scales;            // of the fp16 coordinates
   // Per side (0: rows of x, 1: rows of y): [pieces, part_stride] partial scaled maxima and sums of row blocks
   // shared by several CTAs, and [rows_pad / 128] arrival counters of those CTAs (zero at rest).
   float* part_m[2] = {nullptr, nullptr};
@@ -149,11 +149,15 @@ int sm_count();
 int free_ctas();
 // Writes the column bias of a pass (divided by the logit scale, split into three TF32 pieces) into the bias
 // columns of the column operand.
-void launch_bias(const CloudOps& colc, int kc, int kp, const float* pot, const float* logw, float inv_eps,
-                 float inv_scale2, const Ctrl* ctrl, const unsigned* amax, cudaStream_t st, int pot_shard = 0,
-                 int pot_stride = 0);
+void launch_bias(const Staged& s, int cloud, const float* pot, const float* logw, float inv_eps, float inv_scale2,
+                 const Ctrl* ctrl, cudaStream_t st, int pot_shard = 0, int pot_stride = 0);
 // Copies v to out and fills up to cols_pad with zeros (a no-op when *skip is set).
 void launch_pad_vec(const float* v, int nc, int cols_pad, float* out, const int* skip, cudaStream_t st);
+// Blocks of eight warps that look for the range of a cloud (row_ranges): eight short rows or one long one per warp.
+inline int range_blocks(int rows_pad, int d) {
+  const int most = rows_pad / (d <= 64 ? 64 : 8);
+  return most < 592 ? most : 592;
+}
 inline int pad256(int r) { return (r + 255) & ~255; }
 }  // namespace detail
 

@@ -27,6 +27,7 @@
 #include "fs_ptx.cuh"
 
 #include <cudaTypedefs.h>
+#include <type_traits>
 
 #include <atomic>
 
@@ -45,7 +46,8 @@ struct KParams {
   int row_begin;    // first row of the range; row blocks are counted from here
   int ntiles, nblk;
   int hs;           // leading 32-byte K steps that hold fp16 coordinates (0 for the second GEMM of a matrix pass)
-  const unsigned* amax;  // the clouds' scales (null: 1)
+  OperandScales scales;
+  int side;         // cloud of the rows
   int nk;           // K chunks of 32 words
   int klast;        // K steps of 8 in the last chunk (1..4)
   int nstage;
@@ -222,25 +224,34 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     }
   } else if (warp >= 4) {
     // ===================== epilogue warpgroups =====================
+    // Twice the same code: points with scales of their own (wide_range) take registers that the ordinary form needs.
+    auto epilogue = [&](auto wide_form) {
+    constexpr bool wide = decltype(wide_form)::value;
     const int wg = (warp - 4) >> 2;
     const int h = wg / kPartsK;     // 128-row half
     const int part = wg % kPartsK;  // which half of each tile's chunks
     const int q = warp & 3;         // TMEM lane quarter this warp may read
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int trow = h * 128 + q * 32 + lane;  // this thread's row inside a row block
-    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
+    float scale = p.scale2 / pair_scale(p.scales.range);  // exact: a power of two (wide: of this thread's row)
     constexpr int CH = BN / 32 / kPartsK;  // 32-column chunks of a tile owned by this warpgroup
     const int total = (w_end - w_begin) * CH;
     const int c_base = part * CH;
     // Running state of the current segment (the part of one row block this CTA covers). LSE: sum =
     // s_run * 2^off_run with off_run the rounded value scale*max. VEC: off_run stays 0 and s_run is the signed
     // weighted sum, so the same merge formulas (2^0 = 1 exactly) serve both.
-    const float off_init = (EPI == EPI_LSE) ? __fmul_rn(scale, kRunInit) : 0.f;
+    float off_init = (EPI == EPI_LSE) ? __fmul_rn(scale, kRunInit) : 0.f;
     float m_run = kRunInit, off_run = off_init, s_run = 0.f;
     int cur_blk = w_begin / p.ntiles, cur_jt = w_begin - cur_blk * p.ntiles;  // item of the chunk being consumed
     bool row_fresh = true;  // per-row constants (negR, fac) belong to another row block
     float negR = 0.f, fac = 0.f;
     bool ok = true;
+    auto wide_row = [&](int blk) {  // the row of this thread in a row block has a scale of its own
+      const int r = p.row_begin + blk * BM + trow;
+      scale = r < p.nr ? p.scale2 * __ldg(p.scales.inv[p.side] + r) : p.scale2;
+      if (EPI == EPI_LSE) off_run = off_init = __fmul_rn(scale, kRunInit);
+    };
+    if (wide) wide_row(cur_blk);
 
     auto load_row_consts = [&]() {
       row_fresh = false;
@@ -262,11 +273,12 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
       }
     };
 
-    auto consume = [&](const uint32_t (&r)[32], int chunk_in_tile) {
+    auto consume = [&](uint32_t (&r)[32], int chunk_in_tile) {
+      const int col0 = cur_jt * BN + (c_base + chunk_in_tile) * 32;
+      if (wide) unscale_columns(r, p.scales.inv[1 - p.side] + col0);
       float v[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-      const int col0 = cur_jt * BN + (c_base + chunk_in_tile) * 32;
       if (EPI == EPI_LSE) {
         if (p.s_out) {
           const int lr = cur_blk * BM + trow;
@@ -446,7 +458,10 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
       if (g + 1 == seg_end_g) {
         if (EPI != EPI_OUT) finalize(seg_w / p.ntiles, true);
         seg_w += seg_len(seg_w);
-        if (seg_w < w_end) seg_end_g += seg_len(seg_w) * CH;
+        if (seg_w < w_end) {
+          seg_end_g += seg_len(seg_w) * CH;
+          if (wide) wide_row(seg_w / p.ntiles);
+        }
       }
     };
     // Software pipeline, two register buffers: the load of chunk g+1 is in flight while chunk g is consumed.
@@ -478,6 +493,8 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         seg_w += seg_len(seg_w);
       }
     }
+    };
+    if (EPI != EPI_OUT && wide_range(p.scales)) epilogue(std::true_type{}); else epilogue(std::false_type{});
   }
 
   tc_fence_before();
@@ -504,9 +521,9 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 struct KPvParams {
   int nr, nc, ntiles, row_begin;
   int hs;                      // leading K steps that hold fp16 coordinates
-  const unsigned* amax;        // the clouds' scales (null: 1)
-  const unsigned* amax2;       // MAT5: largest |entry| of the second row operand, and of the column cloud
-  const unsigned* amax_col;
+  OperandScales scales;
+  int side;                    // cloud of the rows
+  const float* inv2;           // MAT5: 1 / scale of every row of the second row operand (null: not scaled)
   int nk, klast, nstage, nv;   // K chunks, K steps of the last one, ring depths (K chunks / V tiles)
   int dv, dv_pad, dv0, ld_out;
   float scale2, eps;
@@ -719,8 +736,11 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
     const int q = warp & 3;
     const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
     const int r = row0 + q * 32 + lane;
-    const float scale = p.scale2 / pair_scale(p.amax);  // exact: a power of two
-    const float unit2 = MAT5 && p.amax2 ? 1.f / (cloud_scale(*p.amax2) * cloud_scale(*p.amax_col)) : 1.f;
+    const bool wide = wide_range(p.scales);
+    // exact: powers of two
+    const float scale = wide ? p.scale2 * (r < p.nr ? p.scales.inv[p.side][r] : 1.f) : p.scale2 / pair_scale(p.scales.range);
+    float unit2 = 1.f;
+    if (MAT5 && p.inv2 && r < p.nr) unit2 = p.inv2[r] * (wide ? 1.f : 1.f / cloud_scale(p.scales.range[1 - p.side]));
     const float negR = (r < p.nr) ? -p.R[r] : 0.f;
     bool ok = true;
     constexpr int CH = BN / 32 / kPartsK;
@@ -740,8 +760,16 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
     auto weigh = [&](int g, uint32_t (&rg)[32]) {
       const int j = g / CH, c = g % CH, buf = j % NSW;
       const uint32_t taddr = lane_addr + buf * BUFCOLS + (c_base + c) * 32;
+      const float* inv_col = wide ? p.scales.inv[1 - p.side] + j * BN + (c_base + c) * 32 : nullptr;
+      if (wide) unscale_columns(rg, inv_col);
       float e[32];
-      if (MAT5) tmem_ld32(taddr + WCOLS, e);  // E = rows2 . cols of the same entries
+      if (MAT5) {
+        tmem_ld32(taddr + WCOLS, e);  // E = rows2 . cols of the same entries
+        if (wide) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) e[i] *= __ldg(inv_col + i);
+        }
+      }
       float v[32];
       if (SPLIT) {
         float lo[32];
@@ -836,16 +864,17 @@ tck_pv_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ 
 // [Wh | Wl | Wh] in three blocks of cols_pad columns, which the GEMM pairs with [Vh | Vh | Vl]. Columns beyond
 // nc get zero weight without looking at the stored value.
 __global__ void wexp_kernel(float* __restrict__ W, long long ld, int rows, int row0, int nc, int cols_pad,
-                            const float* __restrict__ R, float scale2, const unsigned* __restrict__ amax, int split,
+                            const float* __restrict__ R, float scale2, const OperandScales sc, int side, int split,
                             const int* skip) {
   if (skip && *skip) return;
-  scale2 /= pair_scale(amax);
+  const bool wide = wide_range(sc);
   const int quads = cols_pad >> 2;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (long long)rows * quads) return;
   const int r = (int)(idx / quads), j4 = (int)(idx - (long long)r * quads);
   float* row = W + (size_t)r * ld;
   const float negR = -__ldg(R + row0 + r);
+  scale2 = wide ? scale2 * sc.inv[side][row0 + r] : scale2 / pair_scale(sc.range);  // the scores have lost their columns'
   const float4 s = *reinterpret_cast<const float4*>(row + 4 * j4);
   const float sv[4] = {s.x, s.y, s.z, s.w};
   float hi[4], lo[4];
@@ -976,11 +1005,10 @@ cudaError_t kstream_lse(const Staged& s, int side, const StreamArgs& a, const Ls
   const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, s.amax, st,
-                      a.pot_shard, a.pot_stride);
+  detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, st, a.pot_shard, a.pot_stride);
   KParams kp{};
   set_chunks(kp, s.kp);
-  kp.hs = s.hs; kp.amax = s.amax;
+  kp.hs = s.hs; kp.scales = s.scales; kp.side = side;
   const KPlan k = plan_k(kp.nk, a.nc);
   CUtensorMap ma, mb;
   if (!make_maps(&ma, &mb, rowc.opA, rowc.rows_pad, colc.opB, colc.rows_pad, s.kp, k.bn)) return cudaErrorInvalidValue;
@@ -1003,12 +1031,12 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
   const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (!pa.bias_ready)
-    detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st);
+    detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st);
   float* vpad = reinterpret_cast<float*>(((uintptr_t)scratch + 255) & ~(uintptr_t)255);
   detail::launch_pad_vec(pa.V, a.nc, colc.rows_pad, vpad, pa.skip, st);
   KParams kp{};
   set_chunks(kp, s.kp);
-  kp.hs = s.hs; kp.amax = s.amax;
+  kp.hs = s.hs; kp.scales = s.scales; kp.side = side;
   const KPlan k = plan_k(kp.nk, a.nc);
   CUtensorMap ma, mb;
   if (!make_maps(&ma, &mb, rowc.opA, rowc.rows_pad, colc.opB, colc.rows_pad, s.kp, k.bn)) return cudaErrorInvalidValue;
@@ -1027,21 +1055,21 @@ cudaError_t kstream_vec(const Staged& s, int side, const StreamArgs& a, const Pv
 // ---- narrow plan-times-matrix pass (second GEMM from TMEM) -------------------------------------------
 namespace {
 
-__global__ void rows2_amax_kernel(const float* A, size_t count, unsigned* out) {
-  block_amax(A, count, (size_t)blockIdx.x * blockDim.x + threadIdx.x, (size_t)gridDim.x * blockDim.x, out);
+__global__ void __launch_bounds__(256) rows2_range_kernel(const float* A, int rows, int rows_pad, int d, float* inv) {
+  row_ranges(A, rows, rows_pad, d, blockIdx.x, gridDim.x, inv, nullptr, 0, 0, 0);
 }
 
 // Second row operand of the Mat5 term in the row-role layout of the staged clouds: [Ah | Ah | Al | 0 ...] in the
-// split mode, [Ah | 0 ...] in TF32 mode (fp16 scaled by its own power of two where the clouds are), so that its contraction with the staged column operand is A_i . y_j
-// (the bias and label columns of the column operand meet zeros).
+// split mode, [Ah | 0 ...] in TF32 mode, so that its contraction with the staged column operand is A_i . y_j (the bias
+// and label columns of the column operand meet zeros). Where the clouds are scaled fp16, every row has its own scale: it
+// leaves with the row's factor of the epilogue.
 __global__ void stage_rows2_kernel(const float* __restrict__ A, int rows, int rows_pad, int d, int kp, int kcoord,
-                                   int hs, int split, const unsigned* __restrict__ amax, float* __restrict__ out) {
+                                   int hs, int split, const float* __restrict__ inv, float* __restrict__ out) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)rows_pad * kp) return;
   const int r = (int)(idx / kp), k = (int)(idx % kp);
   float v = 0.f, unused;
-  if (r < rows && k < kcoord)
-    stage_coord(A + (size_t)r * d, k, d, split ? 3 : 1, hs, amax ? cloud_scale(*amax) : 1.f, v, unused);
+  if (r < rows && k < kcoord) stage_coord(A + (size_t)r * d, k, d, split ? 3 : 1, hs, inv ? 1.f / inv[r] : 1.f, v, unused);
   out[idx] = v;
 }
 
@@ -1063,7 +1091,7 @@ KPvPlan plan_kpv(int nr, int nc, int kp, int dv, int prec, bool mat5) {
   k.parts = split ? 3 : 1;
   k.ld_v = (long long)k.cols_pad * k.parts;
   k.vt_bytes = (((size_t)k.vrows * k.ld_v * sizeof(float)) + 1023) & ~size_t(1023);
-  k.a2_bytes = mat5 ? ((((size_t)detail::pad256(nr) * kp * sizeof(float)) + 2047) & ~size_t(1023)) : 0;
+  k.a2_bytes = mat5 ? ((((size_t)detail::pad256(nr) * (kp + 1) * sizeof(float)) + 2047) & ~size_t(1023)) : 0;
   const size_t stage = (size_t)(mat5 ? 2 : 1) * 128 * 128 + 64 * 128;
   const size_t v_stage = (size_t)(split ? 2 : 1) * 2 * k.dv_pad * 128;
   const size_t budget = kSmemMax - 2048;
@@ -1103,27 +1131,22 @@ cudaError_t kstream_pv(const Staged& s, int side, const StreamArgs& a, const PvA
   if (!k.ok) return cudaErrorNotSupported;
   if (k.vt_bytes + k.a2_bytes + 2048 > scratch_bytes) return cudaErrorInvalidValue;
   const float scale2 = (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
-  detail::launch_bias(colc, s.kc, s.kp, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, s.amax, st,
-                      a.pot_shard, a.pot_stride);
+  detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, nullptr, st, a.pot_shard, a.pot_stride);
   char* p0 = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
   float* vt = reinterpret_cast<float*>(p0);
   float* a2 = mat5 ? reinterpret_cast<float*>(p0 + k.vt_bytes) : nullptr;
-  // the last kilobyte of the second operand's part holds its largest entry
-  unsigned* amax2 = mat5 && s.hs ? reinterpret_cast<unsigned*>(p0 + k.vt_bytes + k.a2_bytes - 1024) : nullptr;
+  // behind the second operand: 1 / scale of its rows
+  float* inv2 = mat5 && s.hs ? a2 + (size_t)rowc.rows_pad * s.kp : nullptr;
   {
     dim3 grid((k.cols_pad + 31) / 32, (k.vrows + 31) / 32), block(32, 8);
     stage_vt_cat_kernel<<<grid, block, 0, st>>>(pa.V, a.nc, pa.dv, pa.colscale, k.vrows, k.cols_pad, split, vt);
   }
   if (mat5) {
-    if (amax2) {
-      const size_t count = (size_t)rowc.rows * s.d;
-      cudaError_t e = cudaMemsetAsync(amax2, 0, sizeof(unsigned), st);
-      if (e != cudaSuccess) return e;
-      rows2_amax_kernel<<<count / 256 + 1 < 592 ? (int)(count / 256 + 1) : 592, 256, 0, st>>>(pa.rows2, count, amax2);
-    }
+    if (inv2)
+      rows2_range_kernel<<<detail::range_blocks(rowc.rows_pad, s.d), 256, 0, st>>>(pa.rows2, rowc.rows, rowc.rows_pad, s.d, inv2);
     const size_t total = (size_t)rowc.rows_pad * s.kp;
     stage_rows2_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(
-        pa.rows2, rowc.rows, rowc.rows_pad, s.d, s.kp, operand_layout(s.d, s.prec, s.nlab, 3).kcoord, s.hs, split, amax2, a2);
+        pa.rows2, rowc.rows, rowc.rows_pad, s.d, s.kp, operand_layout(s.d, s.prec, s.nlab, 3).kcoord, s.hs, split, inv2, a2);
   }
   CUtensorMap maps[5];
   bool ok = true;
@@ -1139,7 +1162,7 @@ cudaError_t kstream_pv(const Staged& s, int side, const StreamArgs& a, const PvA
   kp.ntiles = (a.nc + 63) / 64;
   KParams chunks{};
   set_chunks(chunks, s.kp);
-  kp.hs = s.hs; kp.amax = s.amax; kp.amax2 = amax2; kp.amax_col = s.amax ? s.amax + (side == 0 ? 1 : 0) : nullptr;
+  kp.hs = s.hs; kp.scales = s.scales; kp.side = side; kp.inv2 = inv2;
   kp.nk = chunks.nk; kp.klast = chunks.klast; kp.nstage = k.nstage; kp.nv = k.nv;
   kp.dv = pa.dv; kp.dv_pad = k.dv_pad; kp.ld_out = pa.dv;
   kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;
@@ -1222,7 +1245,7 @@ cudaError_t kstream_mat(const Staged& s, int side, const StreamArgs& a, const Pv
     // 2. scores -> TF32 weights in place
     const long long quads = (long long)(r1 - r0) * (m.cols_pad / 4);
     wexp_kernel<<<(unsigned)((quads + 255) / 256), 256, 0, st>>>(W, m.k2, r1 - r0, r0, a.nc, m.cols_pad, R_out, scale2,
-                                                                 s.amax, m.parts == 3, pa.skip);
+                                                                 s.scales, side, m.parts == 3, pa.skip);
     // 3. out[r0:r1] = epilogue(W x Vt^T)
     g2.nr = r1 - r0; g2.nc = pa.dv; g2.row_begin = 0;
     g2.ntiles = (pa.dv + k2.bn - 1) / k2.bn;
