@@ -966,9 +966,15 @@ __device__ __forceinline__ void write_bias(float* at, double bd) {
   at[1] = mid;
   at[2] = to_tf32((float)(bd - (double)hi - (double)mid));
 }
-// The log-weight of a point in its row role. A weight of zero (log = -1e5) rules out two-sided steps; leaving it out
-// of the row's own bias then keeps the finished sum small, where fp32 is fine-grained.
+// What a point brings into its own sum: its potential and log-weight. Both stay out of it when they would only take bits
+// from the finished sum, whose exponent the candidate subtracts again: a potential far above the eps of the step (the first
+// steps of a point far from the rest: |x|^2 / eps, while its scores are |x||y| / eps), where an exponent of 2^31 rounds
+// to more than fp32's range. Up to 2^20 its rounding is below 2^-4, that of potentials which fp32 holds anyway. A weight
+// of zero (log = -1e5) stays out by itself. Two-sided steps need both inside: they run one-sided otherwise.
 __device__ __forceinline__ double own_logw(double lw) { return lw < -700.0 ? 0.0 : lw; }
+__device__ __forceinline__ bool own_inside(double pot, double own, double eps) {
+  return fabs(pot / eps + own) * 1.4426950408889634 <= 1048576.0;
+}
 
 // Adds the partial sums of a step, updates the potentials in place (rounded once from fp64), stages the biases of
 // the next step and records the ranges that decide how it runs. One block per 32 points, eight warps share the
@@ -1066,14 +1072,17 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
     // log2 of the weighted sum with the point's own bias inside; the candidate takes that bias out again
     const float l2 = m + log2f(fmaxf(s, 1e-40f));
     const double old = (double)pot_i, lw = (double)logw_i, own = own_logw(lw);
-    const double cand = (double)u.damp[c] * (old + u.eps * (own - (double)l2 * 0.69314718055994530942));
+    const bool inside = own_inside(old, own, u.eps);
+    const double cand =
+        (double)u.damp[c] * ((inside ? old : 0.0) + u.eps * ((inside ? own : 0.0) - (double)l2 * 0.69314718055994530942));
     double v = (1.0 - (double)u.w) * old + (double)u.w * cand;
     if (u.shiftcoef[c] != 0.f) v -= (double)u.shiftcoef[c] * (double)sq_i;
     const float now = (float)v;
     u.pot[c][i] = now;
     const size_t at = (size_t)i * P.kp + P.kc;
     const double to_unit = u.inv2cs * (double)unit_i;
-    write_bias(u.opA[c] + at + 3, ((double)now + own * u.eps_next) * to_unit);
+    const bool inside_next = own_inside((double)now, own, u.eps_next);
+    write_bias(u.opA[c] + at + 3, inside_next ? ((double)now + own * u.eps_next) * to_unit : 0.0);
     write_bias(u.opB[c] + at, ((double)now + lw * u.eps_next) * to_unit);
     const float big_l = (float)((double)l2 - own * 1.4426950408889634);
     const float dlt = (float)(((double)now - old) * u.log2e_eps);
@@ -1081,7 +1090,8 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
     st_l = -st_u;
     st_dx = dlt;
     st_dn = -dlt;
-    if (!(fabsf(st_u) < 1e30f) || !(fabsf(dlt) < 1e30f)) st_u = INFINITY;  // no bound: the next step runs one-sided
+    // no bound: the next step runs one-sided
+    if (!(fabsf(st_u) < 1e30f) || !(fabsf(dlt) < 1e30f) || !inside || !inside_next) st_u = INFINITY;
   }
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -1202,7 +1212,8 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
       const float lw = u.logw[c][r];
       u.sq[c][r] = sq;
       u.pot[c][r] = pot;
-      write_bias(rowA + kc + 3, ((double)pot + own_logw(lw) * u.eps) * u.inv2cs * (double)unit);
+      const double in = own_logw(lw);
+      write_bias(rowA + kc + 3, own_inside((double)pot, in, u.eps) ? ((double)pot + in * u.eps) * u.inv2cs * (double)unit : 0.0);
       write_bias(rowB + kc, ((double)pot + (double)lw * u.eps) * u.inv2cs * (double)unit);
       float l2 = lw * kLog2e;
       if (!(fabsf(l2) < 1e30f) || wide) l2 = -1e30f;  // such a weight keeps every step one-sided, as a wide range does

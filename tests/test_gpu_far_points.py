@@ -121,6 +121,77 @@ def test_plan_applications_and_gradient(prec, d, far, where):
     assert (np.abs(got - want) < tol * scale).all()
 
 
+@pytest.mark.parametrize("prec", ["fp32", "tf32"])
+@pytest.mark.parametrize("n,m,d", [(400, 300, 16), (400, 300, 64), (400, 300, 200), (2100, 1950, 200), (4100, 3900, 512)])
+@pytest.mark.parametrize("weight", [0.0, 1.0])
+def test_symmetric_and_alternating_solves(prec, n, m, d, weight):
+    """Every kernel of the solvers: a far point without weight in a balanced problem, two with weight in a relaxed one (two
+    without would meet in a product of 1e16 that their potentials, in fp32, cannot cancel). The far point's potential starts
+    at 1e16 d and must not enter its own sums either. Tolerances as for ordinary clouds: 1e-5 and 2e-3 of the largest near
+    potential."""
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_alternating, sinkhorn_flashstyle_symmetric
+    tf32, eps, iters = prec == "tf32", 0.5 * d, 3
+    where = "xy" if weight else "x"
+    x, y = _points(d, 1e8, where, seed=5, n=n, m=m)
+    kx, ky = _near(n, where, "x"), _near(m, where, "y")
+    r = np.random.default_rng(6)
+    a, b = r.uniform(0.5, 1.5, n), r.uniform(0.5, 1.5, m)
+    a[5] *= weight
+    a, b = (np.float32(w / w.sum()).astype(np.float64) for w in (a, b))
+    rho = None if weight == 0.0 else 4.0
+    want = O.solve_symmetric(x, y, a, b, [eps] * iters, rho_x=rho, rho_y=rho)
+    reach = None if rho is None else 2.0
+    size = max(np.abs(want["f"][kx]).max(), (_norm(x[kx])**2).max(), (_norm(y[ky])**2).max())
+    tol = (2e-3 if tf32 else 1e-5) * size
+    args = [dev(v) for v in (x, y, a, b)]
+    got = sinkhorn_flashstyle_symmetric(*args, eps=eps, n_iters=iters, use_epsilon_scaling=False, reach=reach, allow_tf32=tf32)
+    assert np.abs(host(got[0]) - want["f"])[kx].max() < tol
+    assert np.abs(host(got[1]) - want["g"])[ky].max() < tol
+    if n * m < 1e6 and rho is None:
+        want = O.solve_alternating(x, y, a, b, [eps], iters)
+        got = sinkhorn_flashstyle_alternating(*args, eps_list=[eps], iters_per_eps=iters, allow_tf32=tf32)
+        assert np.abs(host(got[0]) - want["f"])[kx].max() < tol
+        assert np.abs(host(got[1]) - want["g"])[ky].max() < tol
+
+
+def test_lockstep_labels_and_tile_lists_with_a_far_point():
+    """One far problem among ordinary ones of a lockstep launch, the label table, and a list of kept tiles."""
+    from flash_sinkhorn_b200.sinkhorn_solvers import (sinkhorn_flashstyle_alternating, sinkhorn_flashstyle_symmetric,
+                                                      sinkhorn_flashstyle_symmetric_batched)
+    d, eps = 24, 12.0
+    r = np.random.default_rng(7)
+    probs, wants = [], []
+    for far in (1.0, 1e9, 1.0):
+        x, y = _points(d, far, "x", seed=8)
+        a, b = r.uniform(0.5, 1.5, N), r.uniform(0.5, 1.5, M)
+        a[5] = 0.0
+        a, b = (np.float32(w / w.sum()).astype(np.float64) for w in (a, b))
+        wants.append(O.solve_symmetric(x, y, a, b, [eps] * 4))
+        probs.append(tuple(dev(v) for v in (x, y, a, b)))
+    got = sinkhorn_flashstyle_symmetric_batched(probs, use_epsilon_scaling=False, eps=eps, n_iters=4, allow_tf32=False)
+    kx = _near(N, "x", "x")
+    tol = 1e-5 * max((_norm(x[kx])**2).max(), (_norm(y)**2).max())
+    for out, want in zip(got, wants):
+        assert np.abs(host(out[0]) - want["f"])[kx].max() < tol and np.abs(host(out[1]) - want["g"]).max() < tol
+
+    x, y = _points(d, 1e9, "x", seed=8)
+    lx, ly = r.integers(0, 4, N), r.integers(0, 4, M)
+    table = r.uniform(0.0, 5.0, (4, 4))
+    table = np.float32(table + table.T).astype(np.float64)
+    want = O.label_solve_symmetric(x, y, a, b, [eps] * 4, lx, ly, table)
+    out = sinkhorn_flashstyle_symmetric(
+        *(dev(v) for v in (x, y, a, b)), eps=eps, n_iters=4, use_epsilon_scaling=False, allow_tf32=False,
+        label_x=torch.as_tensor(lx).cuda(), label_y=torch.as_tensor(ly).cuda(), label_cost_matrix=dev(table), lambda_y=1.0)
+    assert np.abs(host(out[0]) - want["f"])[kx].max() < tol and np.abs(host(out[1]) - want["g"]).max() < tol
+
+    mask = np.ones((4, 3), bool)
+    mask[1, 2] = mask[3, 0] = False
+    want = O.solve_alternating(x, y, a, b, [eps], 4, tile_mask=mask)
+    out = sinkhorn_flashstyle_alternating(*(dev(v) for v in (x, y, a, b)), eps_list=[eps], iters_per_eps=4,
+                                          tile_mask=torch.as_tensor(mask), allow_tf32=False)
+    assert np.abs(host(out[0]) - want["f"])[kx].max() < tol and np.abs(host(out[1]) - want["g"]).max() < tol
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 @pytest.mark.parametrize("d", [64, 520])
 def test_a_non_finite_point_leaves_the_rows_of_its_own_cloud_alone(bad, d):
