@@ -446,6 +446,12 @@ int sym_run(SymSolve* s, int cnt, int last_extrapolation, double rho_x, double r
       b.early = early && t > 0 && !is_last;
     }
     if (n_last) FS_CUDA(sym::emit(last, pre, n_last, st));
+    if (early && last_extrapolation && t + 1 == steps) {
+      // where the schedule varies, a solve that stopped early holds the biases of the step after its last one
+      bool varies = false;
+      for (double e : s[0].eps) varies = varies || e != s[0].eps[t];
+      if (varies) FS_CUDA(sym::rebias(s[0].p, s[0].eps[t], st));
+    }
     FS_CUDA(sym::step(batch, k, (int)t, st));
     const sym::Problem& p = s[0].p;
     if (early && batch[0].early && t % (size_t)check_every == 0) {

@@ -1231,6 +1231,19 @@ __global__ void __launch_bounds__(256) sym_stage_kernel(const __grid_constant__ 
   }
 }
 
+// Stages the biases again for a step at eps (FinSub::eps_next), from the potentials as they are. One thread per point.
+__global__ void sym_rebias_kernel(const __grid_constant__ FinLaunch<1> P) {
+  const FinSub& u = P.sub[0];
+  const Geo& g = u.geo;
+  const int c = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.n[c]) return;
+  const double pot = (double)u.pot[c][i], lw = (double)u.logw[c][i], own = own_logw(lw);
+  const double to_unit = u.inv2cs * (double)bias_factor(g.scales, wide_range(g.scales), c, i);
+  const size_t at = (size_t)i * P.kp + P.kc;
+  write_bias(u.opA[c] + at + 3, own_inside(pot, own, u.eps_next) ? (pot + own * u.eps_next) * to_unit : 0.0);
+  write_bias(u.opB[c] + at, (pot + lw * u.eps_next) * to_unit);
+}
+
 struct EmitJobs {
   struct Job {
     const float *pot[2], *sq[2];
@@ -1535,6 +1548,22 @@ cudaError_t step(const Step* s, int cnt, int t, cudaStream_t st) {
   if (cnt == 1) return step_n<1>(s, cnt, t, st);
   if (cnt <= 3) return step_n<3>(s, cnt, t, st);
   return step_n<kMaxProblems>(s, cnt, t, st);
+}
+
+cudaError_t rebias(const Problem& p, double eps, cudaStream_t st) {
+  FinLaunch<1> fp;
+  fp.kc = p.kc; fp.kp = p.kp;
+  FinSub& f = fp.sub[0];
+  f.geo = p.geo;
+  for (int k = 0; k < 2; ++k) {
+    f.pot[k] = p.pot[k]; f.logw[k] = p.logw[k]; f.opA[k] = p.opA[k]; f.opB[k] = p.opB[k];
+  }
+  f.eps_next = (float)eps;
+  f.inv2cs = 0.5 / (double)p.cs_dot;
+  const int rows = p.n[0] > p.n[1] ? p.n[0] : p.n[1];
+  sym_rebias_kernel<<<dim3((rows + 255) / 256, p.self ? 1 : 2), 256, 0, st>>>(fp);
+  count_launches(1);
+  return cudaGetLastError();
 }
 
 cudaError_t emit(Problem* const* p, float* const (*out)[2], int cnt, cudaStream_t st) {

@@ -71,6 +71,8 @@ cudaError_t layout(Problem& p, char* buf);
 cudaError_t stage(Problem* const* p, const double* eps0, int cnt, cudaStream_t st);
 // One step of cnt <= kMaxProblems problems of one feature dimension; t counts the steps since stage().
 cudaError_t step(const Step* s, int cnt, int t, cudaStream_t st);
+// Stages the biases again for a step at eps: steps that an early stop skipped have left those of their own.
+cudaError_t rebias(const Problem& p, double eps, cudaStream_t st);
 // out[c] = potential + squared-norm shift for both clouds (null pointers are skipped).
 cudaError_t emit(Problem* const* p, float* const (*out)[2], int cnt, cudaStream_t st);
 

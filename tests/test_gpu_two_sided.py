@@ -95,6 +95,24 @@ def test_zero_weights_schedules_and_early_stop(cta_limit, limit):
     assert got[2] == want["n_iters"] and np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size
 
 
+@pytest.mark.parametrize("limit", [2, 0])
+@pytest.mark.parametrize("extrapolate", [True, False])
+@pytest.mark.parametrize("zeros", [True, False])
+def test_early_stop_inside_a_varying_schedule(cta_limit, limit, extrapolate, zeros):
+    """The steps that are skipped have other eps than the last one, which runs all the same, at its own eps."""
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric
+    cta_limit(limit)
+    x, y, a, b = _clouds(400, 300, 32, seed=9, zeros=zeros)
+    sched = [16.0] * 30 + [8.0, 4.0, 2.0, 1.0]
+    want = O.solve_symmetric(x, y, a, b, sched, threshold=1e-2, check_every=4, last_extrapolation=extrapolate)
+    assert want["n_iters"] < 25
+    got = sinkhorn_flashstyle_symmetric(dev(x), dev(y), dev(a), dev(b), eps_list=sched, threshold=1e-2, check_every=4,
+                                        last_extrapolation=extrapolate, allow_tf32=False, return_n_iters=True)
+    size = (x * x).sum(1).max()
+    assert got[2] == want["n_iters"]
+    assert np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size and np.abs(host(got[1]) - want["g"]).max() < 1e-5 * size
+
+
 def test_not_a_number_stays_with_its_point(cta_limit):
     """No bound on the range can be given: one-sided steps to the end, and no wait runs out."""
     from flash_sinkhorn_b200 import _lib
