@@ -215,28 +215,6 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-// 2^z for two exponents on the FMA pipe: z = n + f with n the nearest integer (the 1.5 * 2^23 shift leaves it in the
-// low bits of the sum), 2^f by the degree-6 polynomial with the smallest relative error on [-1/2, 1/2] (1.9e-9, found
-// by Lawson's iteration; 7.9e-8 once evaluated in fp32), n added to the exponent field. Exponents below -125 count
-// as -125: no sum that such a term could change leaves the range of a two-sided step.
-__device__ __forceinline__ u64 exp2_fma(u64 z) {
-  float z0, z1, p0, p1, t0, t1;
-  upk(z, z0, z1);
-  z = pk(fmaxf(z0, -125.f), fmaxf(z1, -125.f));
-  const u64 t = add2(z, pk(12582912.f, 12582912.f)), n = add2(t, pk(-12582912.f, -12582912.f));
-  const u64 f = fma2(n, pk(-1.f, -1.f), z);
-  u64 p = fma2(f, pk(1.534581243e-4f, 1.534581243e-4f), pk(1.339993090e-3f, 1.339993090e-3f));
-  p = fma2(f, p, pk(9.618489072e-3f, 9.618489072e-3f));
-  p = fma2(f, p, pk(5.550328642e-2f, 5.550328642e-2f));
-  p = fma2(f, p, pk(2.402264625e-1f, 2.402264625e-1f));
-  p = fma2(f, p, pk(6.931471825e-1f, 6.931471825e-1f));
-  p = fma2(f, p, pk(1.f, 1.f));
-  upk(p, p0, p1);
-  upk(t, t0, t1);
-  return pk(__uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23)),
-            __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23)));
-}
-
 // Shared-memory matrix descriptor, K-major operand (PTX "tcgen05 matrix descriptor"):
 //   [0,14) start address >> 4, [16,30) leading byte offset >> 4 (unused for swizzled K-major: 1),
 //   [32,46) stride byte offset >> 4 (distance between 8-row groups), [46,48) version = 1,

@@ -98,15 +98,13 @@ constexpr int kParts = 2;
 // The same for the soft-min kernel, whose partials merge at the end of a segment: sixteen soft-max warps per CTA
 // with one 128-row half as with two (tile lists: one chunk per warp and tile).
 __host__ __device__ constexpr int lse_parts(int nhalf, int bn) { return nhalf == 1 && bn == 128 ? 4 : 2; }
-// Every kFmaShare-th pair of exponentials of the soft-min kernel goes to the FMA pipe (exp2_fma): the ex2 pipe binds
-// these passes and the packed arithmetic around it leaves half of the issue slots free.
-constexpr int kFmaShare = 4;
-
 // MODE_LSE: online log-sum-exp of the scaled scores (potential update). MODE_MAX: running maximum of the raw scores
 // and the smallest column attaining it (hard c-transform); no exponentials at all. MODE_VEC: weighted sum
 // sum_j 2^(t_ij - R_i) v_j in fp32 with the known normaliser R (plan times vector): no running maximum. It is bound
 // by the ex2 pipe like the soft-min and replaces a plan-times-matrix pass with one column, whose second GEMM costs as
-// much as one with 32.
+// much as one with 32. Every exponential is an ex2: a quarter of them as a polynomial on the FMA pipe made each form
+// slower (50,000 x 50,000 x 64: soft-min 0.751 -> 0.764 ms, with plan times vector 1.59 -> 1.73; d = 3 0.69 -> 0.70;
+// tile lists of 200,000 points 57.7 -> 60.3; one 128-row half in the exact mode 0.93 both).
 // CSR = true: the item list is the list of kept tiles (row block after row block, NHALF = 1, BN = 128) instead
 // of all nblk x ntiles pairs; everything else - contiguous ranges per CTA, segments, ticketed merge - is the same.
 // NSUB > 1: several dense passes in one launch (no arg-max, no tile list, no device-side early-stop flag).
@@ -438,7 +436,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
           upk(za, z0, z1);
           upk(zb, z2, z3);
           s0 = fma2(pk(ex2(z0), ex2(z1)), pk(w.x, w.y), s0);
-          s1 = fma2((i & 1) ? exp2_fma(zb) : pk(ex2(z2), ex2(z3)), pk(w.z, w.w), s1);
+          s1 = fma2(pk(ex2(z2), ex2(z3)), pk(w.z, w.w), s1);
         }
         float a0, a1;
         upk(add2(s0, s1), a0, a1);
@@ -475,15 +473,9 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       const u64 sc2 = pk(scale, scale), off2 = pk(nms, nms);
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
-        const u64 z = fma2(pk(v[2 * i], v[2 * i + 1]), sc2, off2);
-        u64 e;
-        if (i % kFmaShare == 1) {
-          e = exp2_fma(z);
-        } else {
-          float z0, z1;
-          upk(z, z0, z1);
-          e = pk(ex2(z0), ex2(z1));
-        }
+        float z0, z1;
+        upk(fma2(pk(v[2 * i], v[2 * i + 1]), sc2, off2), z0, z1);
+        const u64 e = pk(ex2(z0), ex2(z1));
         if (i & 1) s1 = add2(s1, e); else s0 = add2(s0, e);
       }
       float a0, a1;

@@ -209,6 +209,25 @@ def test_a_non_finite_point_leaves_the_rows_of_its_own_cloud_alone(bad, d):
     assert (np.abs(got - want) < tol)[keep].all()
 
 
+@pytest.mark.parametrize("column", range(40, 48))
+@pytest.mark.parametrize("d,tf32", [(64, True), (64, False), (520, True)])
+def test_a_target_that_is_not_a_number_counts_wherever_it_stands(column, d, tf32):
+    """The soft-min of every source then has its sum at the floor of the logarithm (1e-40 of the largest other term) and the
+    weighted sum is not a number, for every place of the target in a chunk of columns."""
+    from flash_sinkhorn_b200.kernels.apply_flash import apply_plan_vec_flashstyle
+    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse
+    x, y = _points(d, 1.0, "", seed=13)
+    bias = np.float32(np.random.default_rng(14).normal(size=M)).astype(np.float64)
+    eps = 0.5 * d
+    top = np.delete(2.0 / eps * x @ y.T + bias, column, axis=1).max(1)
+    y[column, 3] = np.nan
+    got = host(flashsinkhorn_lse(dev(x), dev(y), dev(bias), eps=eps, allow_tf32=tf32))
+    assert np.allclose(got / -eps, top + np.log(1e-40), rtol=0, atol=0.05)
+    r = [dev(v) for v in (-(x * x).sum(1), np.zeros(M), np.full(N, -np.log(N)), np.full(M, -np.log(M)))]
+    out = apply_plan_vec_flashstyle(dev(x), dev(y), *r, dev(np.ones(M)), eps=eps, axis=1, allow_tf32=tf32)
+    assert torch.isnan(out).all()
+
+
 @pytest.mark.parametrize("size", [1e-14, 1e-12, 1e-9])
 def test_clouds_near_the_origin_keep_their_bits(size):
     """Tiny coordinates against a large cloud: the products are of order one and carry 22 bits."""
