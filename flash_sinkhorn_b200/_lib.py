@@ -60,6 +60,7 @@ SIGNATURES = {
     "fs_two_sided": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_plan_ctas": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "fs_plan_pv_split": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)]),
+    "fs_symmetric_workspace_bytes": (c_size_t, [c_int] * 7),
     "fs_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int]),
     "fs_workspace_bytes_labels": (c_size_t, [c_int, c_int, c_int, c_int, c_int, c_int]),
     "fs_lse": (c_int, [_P, _P, c_int, c_int, c_int, _P, _P, _P, c_float, c_float, c_float, c_int, _P, c_size_t, _P]),
@@ -216,6 +217,13 @@ def workspace(op: int, n: int, m: int, d: int, prec: int, device: torch.device, 
     """Scratch tensor for one call of ``op``; ``n_classes`` = V of the label cost the call will pass (0 = none)."""
     nbytes = int(load().fs_workspace_bytes_labels(op, n, m, d, prec, int(n_classes)))
     return torch.empty(max(nbytes, 256), dtype=torch.uint8, device=device)
+
+
+def symmetric_bytes(n: int, m: int, d: int, prec: int, n_classes: int = 0, same: bool = False,
+                    two_sided: bool = True) -> int:
+    """Scratch of one symmetric solve; ``same``: a cloud against itself. ``two_sided=False``: of the solve that evaluates
+    the scores once per side, which takes no scratch that grows with ``n * m``."""
+    return max(int(load().fs_symmetric_workspace_bytes(n, m, d, prec, int(n_classes), int(same), int(two_sided))), 256)
 
 
 class LabelCostStruct(ctypes.Structure):

@@ -375,9 +375,9 @@ inline double dampening(double eps, double rho);
 // when the scratch of the per-tile sums stays within its budget (n*m up to about 3e10) and the workspace was sized
 // for it; the reasons are in fs_sym.cu. The rest steps side by side through Problem::lse below.
 // ---------------------------------------------------------------------------
-size_t sym_workspace(int n, int m, int d, int prec, int nlab) {
+size_t sym_workspace(int n, int m, int d, int prec, int nlab, bool self) {
   if (prec == FS_PREC_SIMT || !sym::supported(n, m, d, prec, nlab)) return 0;
-  return sym::bytes(n, m, d, prec, nlab) + 512 + ((size_t)n + m + 128) * sizeof(float);  // + early-stop snapshot
+  return sym::bytes(n, m, d, prec, nlab, self) + 512 + ((size_t)n + m + 128) * sizeof(float);  // + early-stop snapshot
 }
 
 struct SymSolve {
@@ -397,7 +397,7 @@ int sym_prepare(SymSolve& s, const float* x, const float* y, int n, int m, int d
   char* base = (char*)(((uintptr_t)wsp + 255) & ~(uintptr_t)255);
   cudaError_t e = sym::layout(p, base);
   if (e != cudaSuccess) return fail(FS_ERR_CUDA, "symmetric solve layout failed: %s", cudaGetErrorString(e));
-  s.snap[0] = (float*)(base + sym::bytes(n, m, d, prec, 3 * lab.V));
+  s.snap[0] = (float*)(base + sym::bytes(n, m, d, prec, 3 * lab.V, self));
   s.snap[1] = s.snap[0] + ((n + 63) & ~63);
   return FS_OK;
 }
@@ -530,7 +530,7 @@ int fs_engine(int n, int m, int d, int prec) {
   return tc::k_streamed(d, prec, 0) ? 2 : 1;
 }
 
-int fs_two_sided(int n, int m, int d, int prec) { return sym_workspace(n, m, d, prec, 0) > 0 ? 1 : 0; }
+int fs_two_sided(int n, int m, int d, int prec) { return sym_workspace(n, m, d, prec, 0, false) > 0 ? 1 : 0; }
 
 int fs_plan_pv_split(int rows, int cols, int prec, int sms, int* slots) {
   return tc::plan_pv_split(rows, cols, prec, sms, slots);
@@ -577,7 +577,7 @@ size_t fs_workspace_bytes_labels(int op, int n, int m, int d, int prec, int n_cl
     case FS_OP_SOLVE_ALTERNATING: {
       SolveBufs b;
       carve_solve(ws, b, n, m);
-      const size_t two_sided = op == FS_OP_SOLVE_SYMMETRIC ? sym_workspace(n, m, d, prec, p.nlab) : 0;
+      const size_t two_sided = op == FS_OP_SOLVE_SYMMETRIC ? sym_workspace(n, m, d, prec, p.nlab, false) : 0;
       if (two_sided > ws.off) ws.off = two_sided;
       break;
     }
@@ -605,6 +605,15 @@ size_t fs_workspace_bytes_labels(int op, int n, int m, int d, int prec, int n_cl
       return 0;
   }
   return ws.off + 256;
+}
+
+size_t fs_symmetric_workspace_bytes(int n, int m, int d, int prec, int n_classes, int self_problem, int two_sided) {
+  if (n <= 0 || m <= 0 || d <= 0) return 0;
+  const size_t plain = fs_workspace_bytes_labels(FS_OP_SOLVE_ALTERNATING, n, m, d, prec, n_classes);
+  if (!two_sided) return plain;
+  const int nlab = n_classes > 0 ? 3 * n_classes : 0;
+  const size_t need = sym_workspace(n, m, d, prec, nlab, self_problem != 0);
+  return need > 0 ? need + 256 : plain;
 }
 
 int fs_lse(const float* x, const float* y, int n, int m, int d, const float* pot, const float* logw, float* out,
@@ -688,7 +697,7 @@ int fs_solve_symmetric(const float* x, const float* y, int n, int m, int d, cons
   // step and one of them is enough.
   const bool self_problem = x == y && n == m && log_a == log_b && f_init == g_init && rho_x == rho_y &&
                             lc.V == 0;  // a label table need not be symmetric: keep both sides then
-  const size_t two_sided = sym_workspace(n, m, d, prec, 3 * lc.V);
+  const size_t two_sided = sym_workspace(n, m, d, prec, 3 * lc.V, self_problem);
   if (two_sided > 0 && two_sided <= ws_bytes) {
     SymSolve s;
     FS_TRY(sym_prepare(s, x, y, n, m, d, log_a, log_b, f_init, g_init, self_problem, cs_kernel, cost_scale, lc, prec, wsp));
@@ -1142,8 +1151,12 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
   FS_TRY(check_device());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   bool two_sided = true;
+  auto self_item = [&](const fs_batch_item& in) {
+    return in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y;
+  };
   for (int i = 0; i < n_items && two_sided; ++i) {
-    const size_t need = items[i].n > 0 && items[i].m > 0 ? sym_workspace(items[i].n, items[i].m, d, prec, 0) : 0;
+    const bool sizes = items[i].n > 0 && items[i].m > 0;
+    const size_t need = sizes ? sym_workspace(items[i].n, items[i].m, d, prec, 0, self_item(items[i])) : 0;
     two_sided = need > 0 && need <= items[i].ws_bytes && items[i].ws;
   }
   if (two_sided) {
@@ -1153,8 +1166,7 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
       std::vector<SymSolve> ss(cnt);
       for (int k = 0; k < cnt; ++k) {
         const fs_batch_item& in = items[i0 + k];
-        const bool self = in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y;
-        FS_TRY(sym_prepare(ss[k], in.x, in.y, in.n, in.m, d, in.log_a, in.log_b, nullptr, nullptr, self, cost_scale,
+        FS_TRY(sym_prepare(ss[k], in.x, in.y, in.n, in.m, d, in.log_a, in.log_b, nullptr, nullptr, self_item(in), cost_scale,
                            cost_scale, LabelCost(), prec, in.ws));
         sym_schedule(ss[k], in.eps_list_host, in.n_eps, last_extrapolation);
         ss[k].pre[0] = in.f_pre; ss[k].pre[1] = in.g_pre; ss[k].out[0] = in.f; ss[k].out[1] = in.g;

@@ -1505,8 +1505,9 @@ bool supported(int n, int m, int d, int prec, int nlab) {
   return 2 * rows * sizeof(float) <= kMaxPartialBytes;
 }
 
-size_t bytes(int n, int m, int d, int prec, int nlab) {
+size_t bytes(int n, int m, int d, int prec, int nlab, bool self) {
   Problem p;
+  p.self = self;
   p.n[0] = n; p.n[1] = m; p.d = d; p.prec = prec; p.lab.V = nlab / 3;
   return carve(p, nullptr) + 1024;
 }

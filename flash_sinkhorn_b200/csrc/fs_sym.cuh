@@ -64,7 +64,7 @@ struct Step {
 };
 
 bool supported(int n, int m, int d, int prec, int nlab);
-size_t bytes(int n, int m, int d, int prec, int nlab);
+size_t bytes(int n, int m, int d, int prec, int nlab, bool self);
 // Lays the problem out inside buf (bytes() of it) and encodes its tensor maps.
 cudaError_t layout(Problem& p, char* buf);
 // Operands, squared norms, initial potentials and the biases of a first step at eps0[i].

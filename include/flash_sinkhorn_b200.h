@@ -168,6 +168,11 @@ typedef struct fs_label_cost {
 size_t fs_workspace_bytes(int op, int n, int m, int d, int prec);
 /* The same for a call that passes an fs_label_cost with V = n_classes (0 = none). */
 size_t fs_workspace_bytes_labels(int op, int n, int m, int d, int prec, int n_classes);
+/* Scratch of fs_solve_symmetric (or of one item of fs_solve_symmetric_batched). two_sided != 0: of the solve that
+ * evaluates each score once for both potentials, about 16 n m / 256 bytes above the linear part (self_problem != 0, a
+ * cloud and its weights against themselves: half of that); two_sided == 0: of the solve that evaluates it once per
+ * side, linear in n + m, which the entry points run when the scratch they get is too small for the other. */
+size_t fs_symmetric_workspace_bytes(int n, int m, int d, int prec, int n_classes, int self_problem, int two_sided);
 
 /* Row log-sum-exp potential update.
  *   out_i = -eps*damping * log sum_j exp( (2cs/eps) x_i.y_j + bias_j )

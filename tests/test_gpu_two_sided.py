@@ -176,3 +176,79 @@ def test_divergence_solves_share_their_launches(cta_limit):
         (gx,) = torch.autograd.grad(val, xs)
         assert abs(float(val) - want["loss"]) < 2e-5 * abs(want["loss"])
         assert rel(host(gx), want["grad_x"]) < 3e-4
+
+
+def _problems(sizes, d=20):
+    out, wants = [], []
+    for k, (n, m) in enumerate(sizes):
+        x, y, a, b = _clouds(n, m, d, seed=20 + k)
+        if k % 3 == 2:
+            y, b = x, a
+        wants.append(O.solve_symmetric(x, y, a, b, [6.0] * 5))
+        xd, ad = dev(x), dev(a)
+        out.append((xd, xd, ad, ad) if y is x else (xd, dev(y), ad, dev(b)))
+    return out, wants
+
+
+def _check(got, wants):
+    for out, want in zip(got, wants):
+        size = np.abs(want["f"]).max() + 40.0
+        for t, k in zip(out, ("f", "g", "f_pre", "g_pre")):
+            assert np.abs(host(t) - want[k]).max() < 1e-5 * size
+
+
+@pytest.mark.parametrize("count", [1, 3, 24, 25, 60])
+def test_lockstep_calls_of_many_problems(count):
+    """More problems than one launch takes (24), of different sizes and kinds."""
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric_batched
+    r = np.random.default_rng(count)
+    probs, wants = _problems([(int(r.integers(1, 400)), int(r.integers(1, 400))) for _ in range(count)])
+    _check(sinkhorn_flashstyle_symmetric_batched(probs, use_epsilon_scaling=False, eps=6.0, n_iters=5, allow_tf32=False), wants)
+
+
+def test_lockstep_calls_split_where_their_sums_take_too_much(monkeypatch):
+    from flash_sinkhorn_b200 import _lib, sinkhorn_solvers as S
+    r = torch.Generator().manual_seed(3)
+    probs = []
+    for n in (6000, 6500, 7000, 8000):
+        x, y = torch.randn(n, 20, generator=r).cuda(), torch.randn(n - 100, 20, generator=r).cuda()
+        probs.append((x, y, torch.full((n,), 1.0 / n).cuda(), torch.full((n - 100,), 1.0 / (n - 100)).cuda()))
+    probs[2] = (probs[2][0], probs[2][0], probs[2][2], probs[2][2])
+    kw = dict(use_epsilon_scaling=False, eps=6.0, n_iters=5, allow_tf32=False)
+    want = [S.sinkhorn_flashstyle_symmetric(*p, return_prelast=True, **kw) for p in probs]
+    launches = []
+    for limit in (1 << 30, 3 << 20, 0):
+        monkeypatch.setattr(S, "LOCKSTEP_SCRATCH_BYTES", limit)
+        before = _lib.load().fs_launch_count()
+        got = S.sinkhorn_flashstyle_symmetric_batched(probs, **kw)
+        launches.append(_lib.load().fs_launch_count() - before)
+        for g, w in zip(got, want):  # another order of the partial sums: rounding of potentials below 100
+            assert max(float((p - q).abs().max()) for p, q in zip(g, w)) < 1e-4
+    assert launches[0] < launches[1] < launches[2]
+
+
+def test_scratch_too_small_for_two_sided_steps():
+    """Callers that bring the smaller scratch, and a device that has no room for the larger one, get the solve that evaluates
+    the scores once per side: same results, alone and in a lockstep call."""
+    from flash_sinkhorn_b200 import _lib, sinkhorn_solvers as S
+    x, y, a, b = _clouds(40000, 36000, 16, seed=30)
+    args = [dev(v) for v in (x, y, a, b)]
+    kw = dict(use_epsilon_scaling=False, eps=4.0, n_iters=3, allow_tf32=False)
+    full = S.sinkhorn_flashstyle_symmetric(*args, **kw)
+    own = S.sinkhorn_flashstyle_symmetric(args[0], args[0], args[2], args[2], **kw)
+    need = [_lib.symmetric_bytes(40000, 36000, 16, _lib.PREC_FP32, two_sided=t) for t in (True, False)]
+    assert need[0] - need[1] > 5e7
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    room = torch.cuda.memory_reserved(0) + need[1] + 4.5e7
+    torch.cuda.set_per_process_memory_fraction(room / total)
+    try:
+        small = S.sinkhorn_flashstyle_symmetric(*args, **kw)
+        torch.cuda.empty_cache()
+        both = S.sinkhorn_flashstyle_symmetric_batched([tuple(args), (args[0], args[0], args[2], args[2])], **kw)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    size = (x * x).sum(1).max()
+    for got, want in ((small, full), (both[0], full), (both[1], own)):
+        assert max(float((g - w).abs().max()) for g, w in zip(got[:2], want)) < 1e-5 * size

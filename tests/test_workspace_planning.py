@@ -95,3 +95,22 @@ def test_matrix_pass_column_shares_fit_the_scratch(sms):
             if -(-max(n, m) // bn) < 16:  # fewer than 16 column tiles: no shares
                 assert slots.value == 0 and s == 1
     assert lib.fs_plan_pv_split(0, 5, 0, sms, None) == 0
+
+
+@pytest.mark.parametrize("prec", [_lib.PREC_TF32, _lib.PREC_FP32, _lib.PREC_SIMT])
+def test_symmetric_scratch_by_kind_of_problem(prec):
+    """A cloud against itself needs the operands and sums of one side (its column sums have as many pieces as those of a pair: up
+    to a third of the whole where there are few column tiles); without two-sided steps nothing grows with n * m; the size that
+    serves any call covers both; above the budget of the sums and on the CUDA cores there is one size."""
+    for n, d in ((300, 3), (4096, 64), (50000, 64), (16384, 2048)):
+        cross, own = (_lib.symmetric_bytes(n, n, d, prec, same=s) for s in (False, True))
+        plain = _lib.symmetric_bytes(n, n, d, prec, two_sided=False)
+        assert max(cross, plain) <= _lib.load().fs_workspace_bytes(_lib.OP_SOLVE_SYMMETRIC, n, n, d, prec) + 256
+        if prec == _lib.PREC_SIMT:
+            assert cross == own == plain
+        else:
+            assert own < 0.7 * cross
+            assert n < 50000 or own < 0.55 * cross
+    at = [_lib.symmetric_bytes(n, n, 64, prec, two_sided=False) for n in (100000, 200000, 400000)]
+    assert at[2] - at[1] < 2.01 * (at[1] - at[0])
+    assert _lib.symmetric_bytes(400000, 400000, 64, prec) == at[2]
