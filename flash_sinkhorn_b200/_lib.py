@@ -58,6 +58,8 @@ SIGNATURES = {
     "fs_set_pv_split": (c_int, [c_int]),
     "fs_engine": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_two_sided": (c_int, [c_int, c_int, c_int, c_int]),
+    "fs_two_sided_kernel": (c_int, [c_int, c_int, c_int, c_int]),
+    "fs_two_sided_steps": (ctypes.c_longlong, []),
     "fs_plan_ctas": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "fs_plan_pv_split": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)]),
     "fs_symmetric_workspace_bytes": (c_size_t, [c_int] * 7),

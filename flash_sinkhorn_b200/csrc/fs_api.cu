@@ -530,6 +530,12 @@ int fs_engine(int n, int m, int d, int prec) {
   return tc::k_streamed(d, prec, 0) ? 2 : 1;
 }
 
+int fs_two_sided_kernel(int n, int m, int d, int prec) {
+  return sym_workspace(n, m, d, prec, 0, false) > 0 ? sym::kernel_of(n, m, d, prec, 0) : 0;
+}
+
+long long fs_two_sided_steps(void) { return sym::two_sided_steps(); }
+
 int fs_two_sided(int n, int m, int d, int prec) { return sym_workspace(n, m, d, prec, 0, false) > 0 ? 1 : 0; }
 
 int fs_plan_pv_split(int rows, int cols, int prec, int sms, int* slots) {

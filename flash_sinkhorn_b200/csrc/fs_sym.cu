@@ -52,6 +52,7 @@ namespace sym {
 using namespace fs::tc;  // PTX wrappers (internal linkage) and the tensor-map encoder
 
 __device__ int g_sym_error = 0;
+__device__ unsigned long long g_sym_two_sided = 0;  // steps of problems that ran two-sided
 
 namespace {
 
@@ -1106,6 +1107,7 @@ __global__ void __launch_bounds__(256) sym_finalize_kernel(const __grid_constant
   }
   if (blockIdx.x == 0) {
     if (lane == 31) g.ctrl->iters_used += 1;
+    if (lane == 30 && two) atomicAdd(&g_sym_two_sided, 1ull);
     if (lane >= 8 && lane < 16) g.st->slot[(P.slot + 2) % 3][lane - 8] = 0u;
   }
 }
@@ -1578,6 +1580,16 @@ cudaError_t emit(Problem* const* p, float* const (*out)[2], int cnt, cudaStream_
     }
   count_launches(1);
   return launch_pdl(sym_emit_kernel, dim3((rows + 255) / 256, cnt, 2), 256, 0, st, jobs);
+}
+
+int kernel_of(int n, int m, int d, int prec, int nlab) {
+  const int kind = plan_shape(n, m, d, prec, nlab).kind;
+  return kind == RESIDENT ? 1 : (kind == STREAMED ? 2 : (kind == WIDE ? 3 : 4));
+}
+
+long long two_sided_steps() {
+  unsigned long long v = 0;
+  return cudaMemcpyFromSymbol(&v, g_sym_two_sided, sizeof(v)) == cudaSuccess ? (long long)v : -1;
 }
 
 int read_error_flag() {

@@ -76,6 +76,11 @@ cudaError_t rebias(const Problem& p, double eps, cudaStream_t st);
 // out[c] = potential + squared-norm shift for both clouds (null pointers are skipped).
 cudaError_t emit(Problem* const* p, float* const (*out)[2], int cnt, cudaStream_t st);
 
+// Kernel of these sizes: 1 operands resident, 2 streamed in K chunks, 3 / 4 the same by tiles of 256 x 256 / 128 x 128.
+int kernel_of(int n, int m, int d, int prec, int nlab);
+// Two-sided steps that problems have taken on the current device (-1: error).
+long long two_sided_steps();
+
 int read_error_flag();
 int clear_error_flag();
 

@@ -136,6 +136,12 @@ int fs_engine(int n, int m, int d, int prec);
 /* 1 when symmetric solves of these sizes evaluate each score entry once for both potentials and share the launches
  * of a lockstep solve (fs_solve_symmetric_batched), 0 when they step side by side. */
 int fs_two_sided(int n, int m, int d, int prec);
+/* Kernel of those solves: 0 = side by side, 1 = operands resident in shared memory, 2 = streamed in K chunks, 3 / 4 = streamed,
+ * by tiles of 256 x 256 / 128 x 128. */
+int fs_two_sided_kernel(int n, int m, int d, int prec);
+/* Steps, counted per problem, that took one exponential for both potentials on the current device since the library was
+ * loaded (first steps and problems whose range has no bound do not); waits for the device. -1 on an error. */
+long long fs_two_sided_steps(void);
 
 /* Host arithmetic only (no reference counterpart): the CTA count a streaming pass over n_row_blocks x
  * n_col_tiles work items gets on a device with `sms` SMs when `reserved` of them are left free and the CTA

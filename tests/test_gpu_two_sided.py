@@ -1,5 +1,5 @@
-"""Symmetric solves that take one exponential per score entry for both potentials: edges of the tiles, the kernels
-for every contraction length, self-transport triangles, and inputs that force the one-sided steps."""
+"""Symmetric solves that take one exponential per score entry for both potentials: edges of the tiles, every kernel that
+serves them, self-transport triangles, and inputs that force the one-sided steps."""
 import numpy as np
 import pytest
 import torch
@@ -39,7 +39,8 @@ def _solve(x, y, a, b, prec, **kw):
 
 
 # (n, m, d): single points, one less and one more than a tile, runs that end inside a column tile; contractions that
-# stay in shared memory (3 to 64), K-streamed (200, 330) and long (1100)
+# stay in shared memory (3 to 64) and streamed ones on tiles of 128 x 128 (the other streamed kernels serve larger clouds:
+# test_every_kernel_of_the_two_sided_steps)
 SHAPES = [(1, 1, 3), (1, 300, 7), (257, 1, 40), (128, 256, 64), (129, 257, 64), (511, 769, 3), (900, 640, 64),
           (300, 515, 200), (513, 300, 330), (260, 520, 1100)]
 
@@ -60,6 +61,63 @@ def test_potentials_against_the_oracle(cta_limit, n, m, d, prec, limit):
     size = max(np.abs(want["f"]).max(), (x * x).sum(1).max())
     for g, k in zip(got, ("f", "g", "f_pre", "g_pre")):
         assert np.abs(host(g) - want[k]).max() < tol * size
+
+
+def _dense(x, y, a, b, eps, iters):
+    """The textbook iteration in fp64 on the device (the numpy oracle takes minutes at these sizes)."""
+    x, y, a, b = (torch.as_tensor(v).cuda() for v in (x, y, a, b))
+    cost = (x * x).sum(1)[:, None] + (y * y).sum(1)[None] - 2.0 * x @ y.T
+    f, g = torch.zeros_like(a), torch.zeros_like(b)
+    for w in [1.0] + [0.5] * iters + [1.0]:
+        pre = (f, g)
+        nf = -eps * torch.logsumexp((g[None] - cost) / eps + b.log()[None], dim=1)
+        ng = -eps * torch.logsumexp((f[:, None] - cost) / eps + a.log()[:, None], dim=0)
+        f, g = (1 - w) * f + w * nf, (1 - w) * g + w * ng
+    return f, g, pre[0], pre[1]
+
+
+@pytest.mark.parametrize("limit", [40, 0])
+@pytest.mark.parametrize("prec", ["fp32", "tf32"])
+@pytest.mark.parametrize("n,m,d,kernel", [(1900, 1430, 64, 1), (2100, 1950, 200, 2), (2200, 2050, 512, 3), (300, 515, 200, 4)])
+def test_every_kernel_of_the_two_sided_steps(cta_limit, n, m, d, kernel, prec, limit):
+    """Ragged clouds on each of the four kernels: against each other, against themselves, and the three problems of a
+    divergence in one call, with two-sided steps among theirs (all but the first ones; on all SMs the smallest have a CTA
+    for every one-sided tile and nothing to share). Tolerances as in test_potentials_against_the_oracle."""
+    from flash_sinkhorn_b200 import _lib
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric_batched
+    lib = _lib.load()
+    cta_limit(limit)
+    prec_id = _lib.PREC_TF32 if prec == "tf32" else _lib.PREC_FP32
+    sizes = ((n, m), (n, n), (m, m))
+    assert lib.fs_two_sided_kernel(n, m, d, prec_id) == kernel
+    x, y, a, b = _clouds(n, m, d, seed=40)
+    eps, iters = 0.02 * d, 10
+    wants = [_dense(*p, eps, iters) for p in ((x, y, a, b), (x, x, a, a), (y, y, b, b))]
+    tol = (1e-5 if prec == "fp32" else 2e-3) * max((x * x).sum(1).max(), (y * y).sum(1).max())
+
+    def check(out, want):
+        for t, w in zip(out, want):
+            assert float((t.double() - w).abs().max()) < tol
+
+    def tiles(k, t):
+        return (k + t - 1) // t
+
+    bm, bn = {1: (128, 256), 2: (128, 256), 3: (256, 256), 4: (128, 128)}[kernel]
+    shared = [tiles(p, bm) * tiles(q, bn) + (tiles(q, bm) * tiles(p, bn) if p != q else 0) > (limit or 148) for p, q in sizes]
+    before = lib.fs_two_sided_steps()
+    check(_solve(x, y, a, b, prec, eps=eps, n_iters=iters), wants[0])
+    crossed = lib.fs_two_sided_steps()
+    assert (crossed - before >= 4) == shared[0]
+    check(_solve(x, x, a, a, prec, eps=eps, n_iters=iters), wants[1])
+    assert (lib.fs_two_sided_steps() - crossed >= 4) == shared[1]
+    xd, yd, ad, bd = (dev(v) for v in (x, y, a, b))
+    before = lib.fs_two_sided_steps()
+    got = sinkhorn_flashstyle_symmetric_batched([(xd, yd, ad, bd), (xd, xd, ad, ad), (yd, yd, bd, bd)], eps=eps, n_iters=iters,
+                                                use_epsilon_scaling=False, allow_tf32=prec == "tf32")
+    assert lib.fs_two_sided_steps() - before >= 4 * sum(shared)
+    for out, want in zip(got, wants):
+        check(out, want)
+    assert lib.fs_device_error() == 0
 
 
 @pytest.mark.parametrize("limit", [2, 0])
