@@ -57,6 +57,7 @@ SIGNATURES = {
     "fs_set_prefer_streamed": (c_int, [c_int]),
     "fs_set_pv_split": (c_int, [c_int]),
     "fs_engine": (c_int, [c_int, c_int, c_int, c_int]),
+    "fs_engine_labels": (c_int, [c_int] * 5),
     "fs_two_sided": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_two_sided_kernel": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_two_sided_steps": (ctypes.c_longlong, []),

@@ -525,9 +525,12 @@ int fs_set_prefer_streamed(int on) { return tc::set_prefer_streamed(on); }
 
 int fs_set_pv_split(int split) { return tc::set_pv_split(split); }
 
-int fs_engine(int n, int m, int d, int prec) {
-  if (prec == FS_PREC_SIMT || !tc::supported(n, m, d, prec, 0)) return 0;
-  return tc::k_streamed(d, prec, 0) ? 2 : 1;
+int fs_engine(int n, int m, int d, int prec) { return fs_engine_labels(n, m, d, prec, 0); }
+
+int fs_engine_labels(int n, int m, int d, int prec, int n_classes) {
+  const int nlab = n_classes > 0 ? 3 * n_classes : 0;
+  if (prec == FS_PREC_SIMT || !tc::supported(n, m, d, prec, nlab)) return 0;
+  return tc::soft_min_streamed(d, prec, nlab) ? 2 : 1;
 }
 
 int fs_two_sided_kernel(int n, int m, int d, int prec) {

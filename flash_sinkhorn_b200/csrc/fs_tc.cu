@@ -1323,6 +1323,7 @@ constexpr int kMaxChunks = 16;
 std::atomic<int> g_reserved_sms{0};
 std::atomic<int> g_cta_limit{0};
 std::atomic<int> g_prefer_streamed{1};
+bool prefer_streamed() { return g_prefer_streamed.load(std::memory_order_relaxed) != 0; }
 std::atomic<int> g_pv_split{0};  // column shares per row block of the matrix pass. 0: chosen by SM fill, 1..8: forced
 
 }  // namespace
@@ -1436,6 +1437,11 @@ int plan_ctas(int nblk, int ntiles, int sms, int reserved, int limit) {
 }
 
 bool k_streamed(int d, int prec, int nlab) { return plan_shape(d, prec, nlab).streamed; }
+
+bool soft_min_streamed(int d, int prec, int nlab) {
+  const Shape s = plan_shape(d, prec, nlab);
+  return s.streamed || (s.bn == 64 && prefer_streamed());
+}
 
 size_t mat5_scratch_bytes(int nr, int nc, int d, int prec, int dv, int nlab) {
   const Shape sh = plan_shape(d, prec, nlab);
@@ -1568,12 +1574,13 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   Shape sh = csr ? plan_shape_csr(s.d, s.prec, s.nlab) : plan_shape(s.d, s.prec, s.nlab);
   if (!sh.ok) return cudaErrorNotSupported;
   const bool am = out_idx != nullptr;
+  if (am && sh.bn == 64) return cudaErrorNotSupported;  // label tables only, which no nearest target has
   if (csr && (am || !a.tile_col_idx || (a.row_begin & 127))) return cudaErrorNotSupported;
   if (sh.streamed) return am ? cudaErrorNotSupported : kstream_lse(s, side, a, e, nullptr, 0, st);
-  // A resident plan that only fits 64-column tiles issues half-efficient MMAs (N = 64); the K-streamed kernel
-  // with its 256 x 128 tiles is faster there (d = 64 in the exact mode: K = 195), unless a knob says otherwise.
-  if (sh.bn == 64 && !am && !csr && g_prefer_streamed.load(std::memory_order_relaxed))
-    return kstream_lse(s, side, a, e, nullptr, 0, st);
+  // A resident plan that only fits 64-column tiles (TF32 coordinates beside a label table of 46 to 70 classes) issues
+  // half-efficient MMAs (N = 64); the K-streamed kernel with its 256 x 128 tiles is faster there (0.68 of the time of a
+  // pass at K = 195), unless a knob says otherwise.
+  if (sh.bn == 64 && !csr && prefer_streamed()) return kstream_lse(s, side, a, e, nullptr, 0, st);
   // LSE: logit = scale2 * (x.y + bias/scale2). Arg-max: cost = -2cs * (x.y - bias/(2cs)), so the column
   // "bias" staged next to y is -bias/(2cs) (a.pot holds the raw bias, no log-weights) and scale2 = -2cs.
   const float scale2 = am ? -2.0f * a.cost_scale : (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
@@ -1595,8 +1602,7 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   if (csr) return launch<1, 128, MODE_LSE, true>(lp, grid, sh.smem, st);
   if (am) {
     if (sh.nhalf == 2) return launch<2, 128, MODE_MAX>(lp, grid, sh.smem, st);
-    if (sh.bn == 128) return launch<1, 128, MODE_MAX>(lp, grid, sh.smem, st);
-    return launch<1, 64, MODE_MAX>(lp, grid, sh.smem, st);
+    return launch<1, 128, MODE_MAX>(lp, grid, sh.smem, st);
   }
   if (sh.nhalf == 2) return launch<2, 128, MODE_LSE>(lp, grid, sh.smem, st);
   if (sh.bn == 128) return launch<1, 128, MODE_LSE>(lp, grid, sh.smem, st);
@@ -1615,7 +1621,7 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
   if (n > kMaxSub || !passes) return cudaErrorInvalidValue;
   const Staged& s0 = *passes[0].s;
   const Shape sh = plan_shape(s0.d, s0.prec, s0.nlab);
-  if (!sh.ok || sh.streamed) return cudaErrorNotSupported;
+  if (!sh.ok || sh.streamed || sh.bn == 64) return cudaErrorNotSupported;  // 64 columns: label tables only
   Launch<kMaxSub> lp{};
   BiasJobs jobs{};
   lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
@@ -1662,8 +1668,7 @@ cudaError_t lse_multi(const MultiPass* passes, int n, cudaStream_t st) {
   while (g > 1 && (long long)max_tiles * g / total + 2 > kMaxChunks) --g;
   dim3 grid((unsigned)g);
   if (sh.nhalf == 2) return launch<2, 128, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
-  if (sh.bn == 128) return launch<1, 128, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
-  return launch<1, 64, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
+  return launch<1, 128, MODE_LSE, false, kMaxSub>(lp, grid, sh.smem, st);
 }
 
 cudaError_t argmax(const Staged& s, int side, const StreamArgs& a, float* out_val, int* out_idx, cudaStream_t st) {
@@ -1807,7 +1812,7 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   if (sh.ok && !sh.streamed && sh.bn == 128 && pa.dv == 1 && !pa.rows2 && pa.epilogue == PV_APPLY && !pa.colscale &&
       pa.coef == 1.f && pa.rowpot)
     return vec_pass(s, side, a, pa, scratch, sh, st);
-  if (sh.ok && pa.dv == 1 && !pa.rows2 && sh.bn == 64 && !sh.streamed && g_prefer_streamed.load(std::memory_order_relaxed))
+  if (sh.ok && pa.dv == 1 && !pa.rows2 && sh.bn == 64 && !sh.streamed && prefer_streamed())
     return kstream_vec(s, side, a, pa, scratch, st);
   if (sh.ok && (sh.streamed || pa.rows2)) {
     if (pa.dv == 1 && !pa.rows2) return kstream_vec(s, side, a, pa, scratch, st);

@@ -112,6 +112,8 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& p, 
 // mode) both operands stream through shared memory in 32-float K chunks and the score tile accumulates in
 // TMEM over the chunks. lse() and pv() route there by themselves; the functions below are their back ends.
 bool k_streamed(int d, int prec, int nlab = 0);
+// True when the soft-min passes of these sizes do: also where the resident plan fits next to 64-column tiles only.
+bool soft_min_streamed(int d, int prec, int nlab);
 // Tuning knob of the K-streamed kernels: contractions of at least k 32-float chunks take 256 x 256 tiles with
 // one accumulator per half, shorter ones 256 x 128 tiles with two (returns the previous value).
 int set_wide_tile_min_chunks(int k);

@@ -117,7 +117,7 @@ int fs_set_cta_limit(int k);
 int fs_set_wide_tile_min_chunks(int k);
 
 /* Tuning knob (no reference counterpart): shapes whose row operand fits in shared memory only next to
- * 64-column score tiles (e.g. d = 64 in the exact mode) run their soft-min and plan-times-vector passes on the
+ * 64-column score tiles (a few coordinates beside 46 to 70 label classes) run their soft-min and plan-times-vector passes on the
  * K-streamed kernels (on != 0, the default: larger, MMA-efficient tiles) or on the resident-operand kernels
  * (on = 0). Returns the previous value. */
 int fs_set_prefer_streamed(int on);
@@ -132,6 +132,8 @@ int fs_set_pv_split(int split);
 /* Which engine serves a problem of these sizes (no reference counterpart): 0 = CUDA-core fp32 FMA, 1 = tcgen05
  * with the row operand resident in shared memory, 2 = tcgen05 with both operands streamed in K chunks. */
 int fs_engine(int n, int m, int d, int prec);
+/* The same for the passes of a label cost with n_classes classes (0 = none). */
+int fs_engine_labels(int n, int m, int d, int prec, int n_classes);
 
 /* 1 when symmetric solves of these sizes evaluate each score entry once for both potentials and share the launches
  * of a lockstep solve (fs_solve_symmetric_batched), 0 when they step side by side. */

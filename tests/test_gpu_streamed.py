@@ -340,9 +340,8 @@ def test_fused_sharded_debiased_solves_on_a_one_rank_group(monkeypatch):
 
 @pytest.mark.parametrize("d,tf32", [(64, False), (160, True), (100, True)])
 def test_resident_and_streamed_kernels_agree_on_shapes_both_can_serve(d, tf32):
-    """Shapes whose resident-operand plan only fits 64-column tiles run on the K-streamed kernels by default; the
-    resident kernels stay selectable (`fs_set_prefer_streamed(0)`) and are what multi-pass launches use. Both
-    contract the same staged operands in the same K order, so soft-mins and plan-times-vector agree to rounding."""
+    """The knob for shapes whose resident-operand plan only fits 64-column tiles leaves these, whose plan fits 128-column
+    ones, as they are (the shapes that it moves have a label table: the test below)."""
     from flash_sinkhorn_b200 import _lib
     from flash_sinkhorn_b200.kernels.apply_flash import apply_plan_vec_flashstyle
     from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse
@@ -370,6 +369,48 @@ def test_resident_and_streamed_kernels_agree_on_shapes_both_can_serve(d, tf32):
     # plan-times-vector: the resident kernel rounds weights and vector to TF32 for its second GEMM in TF32 mode,
     # the K-streamed one multiplies them in fp32
     assert _r(out[1][1], out[0][1]) < (2e-3 if tf32 else 2e-5)
+    assert lib.fs_device_error() == 0
+
+
+@pytest.mark.parametrize("tf32", [False, True])
+@pytest.mark.parametrize("n,m,d,classes", [(300, 260, 8, 47), (1900, 2300, 4, 60), (130, 513, 2, 69)])
+def test_narrow_tiles_of_many_label_classes_agree_with_the_streamed_kernels(n, m, d, classes, tf32):
+    """A few TF32 coordinates beside 46 to 70 classes: the resident plan fits next to 64-column tiles only, and the passes run
+    on the K-streamed kernels unless told otherwise. Both contract the same operands in the same K order: one step of both
+    potentials and the gradient agree to rounding, and with fp64 to the rounding of the operands (TF32: 2^-11 of either
+    factor of the products)."""
+    from flash_sinkhorn_b200 import _lib
+    from flash_sinkhorn_b200.kernels.grad_sqeuclid import sinkhorn_geomloss_online_grad_sqeuclid
+    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_symmetric_step
+    lib = _lib.load()
+    prec = _lib.PREC_TF32 if tf32 else _lib.PREC_FP32
+    g = torch.Generator().manual_seed(n)
+    x, y = torch.randn(n, d, generator=g).cuda(), torch.randn(m, d, generator=g).cuda()
+    a, b = torch.softmax(torch.randn(n, generator=g), 0).cuda(), torch.softmax(torch.randn(m, generator=g), 0).cuda()
+    lx, ly = (torch.randint(0, classes, (k,), generator=g).cuda() for k in (n, m))
+    table = (5.0 * torch.rand(classes, classes, generator=g)).cuda()
+    fh, gh = -(x**2).sum(1), -(y**2).sum(1)
+    lab = dict(label_x=lx, label_y=ly, label_cost_matrix=table, lambda_y=1.0)
+    out = {}
+    previous = lib.fs_set_prefer_streamed(1)
+    try:
+        for on in (1, 0):
+            lib.fs_set_prefer_streamed(on)
+            assert lib.fs_engine_labels(n, m, d, prec, classes) == (2 if on else 1)
+            step = flashsinkhorn_symmetric_step(x, y, fh, gh, a.log(), b.log(), 1.0, allow_tf32=tf32, **lab)
+            grad = sinkhorn_geomloss_online_grad_sqeuclid(x, y, a, b, fh, gh, eps=1.0, allow_tf32=tf32, **lab)
+            out[on] = (*step, *grad)
+    finally:
+        lib.fs_set_prefer_streamed(previous)
+    score = 2.0 * x.double() @ y.double().T - table.double()[lx][:, ly]
+    want = (0.5 * fh.double() - 0.5 * torch.logsumexp(score + (gh + b.log()).double(), 1),
+            0.5 * gh.double() - 0.5 * torch.logsumexp(score + (fh + a.log()).double()[:, None], 0))
+    for p, q in zip(out[1][:2], out[0][:2]):
+        assert _r(p, q) < 2e-6
+    for p, q in zip(out[0][:2], want):
+        assert _r(p, q) < (2e-3 if tf32 else 2e-6)
+    for p, q in zip(out[1][2:], out[0][2:]):  # the second GEMM is the same kernel for both, on their own soft-mins
+        assert _r(p, q) < (2e-3 if tf32 else 2e-5)
     assert lib.fs_device_error() == 0
 
 

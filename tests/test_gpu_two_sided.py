@@ -310,3 +310,22 @@ def test_scratch_too_small_for_two_sided_steps():
     size = (x * x).sum(1).max()
     for got, want in ((small, full), (both[0], full), (both[1], own)):
         assert max(float((g - w).abs().max()) for g, w in zip(got[:2], want)) < 1e-5 * size
+
+
+def test_lockstep_calls_that_step_side_by_side(monkeypatch):
+    """A lockstep call whose items bring the smaller scratch: several soft-min passes per launch, one per potential."""
+    from flash_sinkhorn_b200 import _lib, sinkhorn_solvers as S
+    r = torch.Generator().manual_seed(4)
+    probs = []
+    for n, m in ((6000, 5800), (7000, 6100), (6400, 6300)):
+        x, y = torch.randn(n, 20, generator=r).cuda(), 0.2 + torch.randn(m, 20, generator=r).cuda()
+        probs.append((x, y, torch.softmax(torch.randn(n, generator=r), 0).cuda(), torch.softmax(torch.randn(m, generator=r), 0).cuda()))
+    kw = dict(use_epsilon_scaling=False, eps=6.0, n_iters=5, allow_tf32=False)
+    want = S.sinkhorn_flashstyle_symmetric_batched(probs, **kw)
+    full = _lib.symmetric_bytes
+    monkeypatch.setattr(_lib, "symmetric_bytes", lambda n, m, d, prec, *a, **k: full(n, m, d, prec, two_sided=False))
+    before = _lib.load().fs_two_sided_steps()
+    got = S.sinkhorn_flashstyle_symmetric_batched(probs, **kw)
+    assert _lib.load().fs_two_sided_steps() == before
+    for g, w in zip(got, want):
+        assert max(float((p - q).abs().max()) for p, q in zip(g, w)) < 1e-4
