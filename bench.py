@@ -650,21 +650,33 @@ def main():
     ms_e2e = t0.elapsed_time(t1)
     clocks = sampler.stop()
 
-    # dominant kernel (one soft-min pass over all n x m entries), timed alone on the launching stream
-    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse_fused
-    gh = -(y_dev**2).sum(1)
-    lb = torch.full((m,), -float(torch.log(torch.tensor(float(m)))), device=dev)
-    for _ in range(3):
-        flashsinkhorn_lse_fused(x_dev, y_dev, gh, lb, eps, allow_tf32=not args.fp32)
-    reps = 10
+    # Dominant kernel: on one GPU the two-sided step of a symmetric solve (one exponential per entry for both potentials, its
+    # finalising kernel included), timed inside solves of two lengths; on several the soft-min pass of a row shard's
+    # engine over all n x m entries, timed alone.
     k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    torch.cuda.synchronize()
-    k0.record()
-    for _ in range(reps):
-        flashsinkhorn_lse_fused(x_dev, y_dev, gh, lb, eps, allow_tf32=not args.fp32)
-    k1.record()
-    torch.cuda.synchronize()
-    kernel_ms = k0.elapsed_time(k1) / reps
+    reps = 10
+    if world == 1:
+        from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric as _pass_solve
+        aw, bw = torch.full((n,), 1.0 / n, device=dev), torch.full((m,), 1.0 / m, device=dev)
+        kernel_ms = pass_ms_by_difference(
+            lambda k: _pass_solve(x_dev, y_dev, aw, bw, use_epsilon_scaling=False, eps=eps, n_iters=k,
+                                  last_extrapolation=False, allow_tf32=not args.fp32), 20, 40)
+        kernel_name = ("two-sided step of a symmetric solve (sym_kernel and sym_finalize_kernel), n*m exponentials; inside a "
+                       "solve: (T(40 iterations) - T(20 iterations)) / 20")
+    else:
+        from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse_fused
+        gh = -(y_dev**2).sum(1)
+        lb = torch.full((m,), -float(torch.log(torch.tensor(float(m)))), device=dev)
+        for _ in range(3):
+            flashsinkhorn_lse_fused(x_dev, y_dev, gh, lb, eps, allow_tf32=not args.fp32)
+        torch.cuda.synchronize()
+        k0.record()
+        for _ in range(reps):
+            flashsinkhorn_lse_fused(x_dev, y_dev, gh, lb, eps, allow_tf32=not args.fp32)
+        k1.record()
+        torch.cuda.synchronize()
+        kernel_ms = k0.elapsed_time(k1) / reps
+        kernel_name = "row soft-min pass (fs_lse), n*m exponentials per launch"
 
     # plan-times-matrix on a 50,000 x 64 N(0,1) matrix at the solved potentials (second item of the config)
     apply_ms = None
@@ -730,13 +742,13 @@ def main():
         sm_mhz = clocks.get("sm_mhz") or 1965.0
         # exp roofline: ex2 issue rate MEASURED on this GPU by the library's micro-benchmark (all SMs, 32
         # warps/SM, register data only); nominal 16 ex2/clk/SM x 148 SMs x sampled clock kept for context.
-        # tensor roofline: TF32 dense = half the measured bf16 rate, 2*d flops per entry (x3 in 3xTF32 mode)
+        # tensor roofline: the measured bf16 rate (fp16 operands have the same), 2*d flops per entry (x3 in the exact mode)
         exp_nominal = 16 * 148 * sm_mhz * 1e6
         exp_measured = float(lib.fs_micro_exp_rate(0, 32))
         softmax_loop_rate = float(lib.fs_micro_exp_rate(1, 16))
         exp_peak = exp_measured if exp_measured > 0 else exp_nominal
         bf16 = peaks.get("bf16_tflops_sustained", 1400.0) * 1e12
-        tc_peak = (bf16 / 2) / (2 * d * (3 if args.fp32 else 1))
+        tc_peak = bf16 / (2 * d * (3 if args.fp32 else 1))
         peak = min(exp_peak, tc_peak)
         achieved = n * m / (kernel_ms * 1e-3)
         total = per_step * args.steps  # strong scaling: the ranks share one problem
@@ -749,7 +761,7 @@ def main():
             "config": {"workload": workload, "entries_per_step": per_step, "parallelism": (f"rows sharded over {world} GPUs, all-gather per half-step" if world > 1 else "single GPU"),
                        "l2": "inputs 25.6 MB < L2; the pass is "
                        "compute-bound (one exp + 2d flops per entry), L2 is not flushed between steps",
-                       "self_terms": "OT(x,x), OT(y,y): one soft-min per step (f == g bit for bit)",
+                       "self_terms": "OT(x,x), OT(y,y): one soft-min per step (both potentials are equal)",
                        "ms_per_100iter_solve": ms_solve,
                        "ms_per_100iter_solve_note": "one OT(x,y) solve, debias off, last_extrapolation off "
                                                     f"({iters + 1} Jacobi steps), timed directly",
@@ -764,16 +776,13 @@ def main():
             "gpu_launches": int(launches),
             "clocks": clocks,
             "roofline": {"bound": "exp" if exp_peak <= tc_peak else "tensor", "achieved": achieved, "peak": peak,
-                         "unit": "entries/s", "frac": achieved / peak,
-                         # DRAM bytes per launch of this kernel at this size, from an
-                         # ncu capture of this kernel at this size (algorithmic: 29.2 MB of staged operands)
-                         "traffic": 28925952 if (n == 50000 and m == 50000 and d == 64 and not args.fp32) else None,
-                         "traffic_unit": "bytes per launch (dram read + write)",
-                         "kernel": "row soft-min pass (fs_lse), n*m entries per launch", "kernel_ms": kernel_ms,
+                         "unit": "exponentials/s (one per score entry and pass; a two-sided step serves two entries of "
+                                 "the metric with each)", "frac": achieved / peak,
+                         "traffic": None, "kernel": kernel_name, "kernel_ms": kernel_ms,
                          "exp_peak": exp_peak, "exp_peak_nominal": exp_nominal, "tensor_peak": tc_peak,
                          "softmax_loop_rate": softmax_loop_rate,
                          "peak_source": "of measured: ex2.approx rate from fs_micro_exp_rate(0,32) on this GPU; "
-                                        "tensor = measured bf16 (MEASURED_PEAKS.json, sustained)/2 for TF32; "
+                                        "tensor = measured bf16 (MEASURED_PEAKS.json, sustained), the rate of fp16; "
                                         "nominal = 16 ex2/clk/SM x 148 SM x sampled SM clock"},
             "loss": loss_val,
         }
