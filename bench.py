@@ -411,7 +411,7 @@ def bench_extra(args):
             roof = {"bound": "exp", "achieved": achieved, "peak": exp_peak, "unit": "entries/s", "frac": achieved / exp_peak}
         roof.update({"traffic": None, "kernel": kernel_name, "kernel_ms": kernel_ms, "kernel_timing": kernel_how,
                      "flop_per_entry": flop_per_entry * mult, "entries_per_s": achieved,
-                     "peak_source": "of measured: tensor = bf16 sustained (MEASURED_PEAKS.json) / 2 for TF32; exp = "
+                     "peak_source": "of measured: tensor = bf16 sustained (MEASURED_PEAKS.json), the rate of fp16; exp = "
                                     "ex2.approx rate from fs_micro_exp_rate(0,32) on this GPU"})
         total = per_step * args.steps
         h2d = sum(t.numel() * 4 for t in host_in)

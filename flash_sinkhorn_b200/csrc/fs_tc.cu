@@ -11,8 +11,8 @@
 //   warp 2      : idle
 //   warps 4..   : soft-max warpgroups, one per 128-row half and half of each tile's columns; thread t of a
 //                 warpgroup owns score row t (TMEM lane t), so row max / row sum need no shuffles.
-// Per column tile and half an MMA lane accumulates S = A_half x B_tile^T (M=128, N=BN, K=8 per instruction,
-// kind::tf32) into one of two TMEM buffers of that half, commits to an mbarrier, and the warpgroups drain the
+// Per column tile and half an MMA lane accumulates S = A_half x B_tile^T (M=128, N=BN, 32 bytes of K
+// per instruction: 16 fp16 or 8 TF32 columns) into one of two TMEM buffers of that half, commits to an mbarrier, and the warpgroups drain the
 // other buffer with tcgen05.ld meanwhile. Because the bias sits in the contraction, the drained value is
 // (logit / scale): max -> one FFMA + one ex2.approx + one FADD per entry. A row block shared by several CTAs
 // gets one partial per row from each; the CTA that takes the block's last ticket merges them in a fixed order.

@@ -1,8 +1,9 @@
 // tcgen05 / TMEM / TMA engine interface (implemented in fs_tc.cu).
 //
 // The score tile S = rows x cols^T is a dense contraction, so it runs on the 5th-gen
-// tensor cores: operands are staged once per call as K-padded, TF32-rounded copies
-// (3xTF32 hi/lo splits in exact-fp32 mode) whose last K columns carry the per-column
+// tensor cores: operands are staged once per call as K-padded copies rounded to TF32's
+// 11 bits (hi/lo splits and three products in exact-fp32 mode), held as scaled fp16 where
+// that takes fewer K steps (Layout), whose last K columns carry the per-column
 // bias, split into three TF32 pieces that multiply constant ones on the row side --
 // the bias add is done by the MMA itself and the soft-max warps only see finished
 // logits (up to a common positive scale).

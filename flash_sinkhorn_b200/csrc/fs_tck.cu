@@ -1,12 +1,12 @@
 // K-streamed tcgen05 passes for sm_100a: the score tile S = rows x cols^T accumulates in TMEM while BOTH
-// operands stream through shared memory in 32-float K chunks, so the feature dimension is unbounded
+// operands stream through shared memory in K chunks of 32 words, so the feature dimension is unbounded
 // (d = 2048, or d = 128 in the 3xTF32 mode whose contraction is three times as long).
 //
 // Work item = (row block of BM = 128*NHALF rows, column tile of BN columns). The items, row block after
 // row block, are cut into equal contiguous ranges, one per CTA, one CTA per SM. Per item and K chunk the
 // producer lane fills one ring stage with the chunk of the row block (NHALF x 128 rows x 128 bytes) and of
 // the column tile (BN rows x 128 bytes), both 128-byte swizzled by TMA; one MMA lane per 128-row half issues
-// four tcgen05.mma kind::tf32 (M = 128, N = BN, K = 8) per stage into that half's TMEM accumulator and
+// four tcgen05.mma (M = 128, N = BN, 16 fp16 or 8 TF32 columns) per stage into that half's TMEM accumulator and
 // commits the stage back to the producer; after the last chunk it commits the accumulator to the epilogue
 // warps. Large tiles matter here: a 256 x 256 tile needs 64 flop per operand byte, a 256 x 128 one 43.
 // Warp roles: warp 0 producer, warps 1 and 3 MMA issuers (warp 1 owns the TMEM allocation), warps 4.. are

@@ -356,7 +356,8 @@ def sinkhorn_flashstyle_symmetric_batched(
     Extension without a reference counterpart (the reference loops over batch items in Python,
     samples_loss.py:515-552). ``problems`` is a sequence of ``(x, y, a, b)`` with one feature dimension; every
     problem gets the schedule :func:`sinkhorn_flashstyle_symmetric` would give it (its own diameter with
-    ``use_epsilon_scaling``), and all of them advance in lockstep, up to four soft-min passes per kernel launch.
+    ``use_epsilon_scaling``), and all of them advance in lockstep, up to 24 problems per kernel launch (four soft-min
+    passes where they step side by side), in several calls where their scratch passes ``LOCKSTEP_SCRATCH_BYTES``.
     No early stopping, warm start or label cost. Returns one ``(f, g, f_prelast, g_prelast, n_steps)`` per problem
     (the pre-extrapolation pair equals ``(f, g)`` without ``last_extrapolation``); results equal the one-at-a-time
     solves up to the merge order of partial sums (rounding level). A problem given as ``(x, x, a, a)`` - the same

@@ -16,8 +16,8 @@
  *    nothing synchronises with the host unless stated.
  *  - Return value: FS_OK or an fs_status; fs_last_error() gives the message of
  *    the calling thread's last failure.
- *  - `prec`: FS_PREC_TF32 (one tcgen05 kind::tf32 pass), FS_PREC_FP32 (3xTF32
- *    split, fp32-equivalent products) or FS_PREC_SIMT (CUDA-core fp32 FMA).
+ *  - `prec`: FS_PREC_TF32 (coordinates rounded to TF32's 11 bits, one tcgen05 product), FS_PREC_FP32 (two pieces of
+ *    11 bits, three products: fp32-equivalent) or FS_PREC_SIMT (CUDA-core fp32 FMA).
  *  - rho < 0 (or NaN) means "balanced side" (no marginal relaxation).
  *  - Notation: cs = cost_scale, C_ij = cs*|x_i-y_j|^2, alpha_i = cs*|x_i|^2,
  *    beta_j = cs*|y_j|^2, shifted potentials f_hat = f-alpha, g_hat = g-beta.
