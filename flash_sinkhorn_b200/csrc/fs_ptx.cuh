@@ -19,6 +19,10 @@ constexpr long long kSpinLimit = 1ll << 28;  // ~0.14 s of SM cycles per wait (a
 constexpr int kSmemMin = 120 * 1024;         // force one CTA per SM (TMEM is allocated per CTA)
 constexpr int kSmemMax = 227 * 1024;
 
+// Initial running maximum of scores that `scale` > 0 turns into exponents: their product stays finite, so that a stretch of
+// padded columns (whose scores may reach -inf as exponents) adds nothing at an offset that compares and subtracts.
+__device__ __forceinline__ float run_init(float scale) { return fmaxf(kRunInit, -1.0e38f / scale); }
+
 // ------------------------------------------------------------------ PTX wrappers
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

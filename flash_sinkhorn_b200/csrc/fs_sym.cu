@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
           const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
           const float scale = wide ? P.sub[s.sub].scale2 * g.scales.inv[s.side][(s.rt + i) * 128 + trow] : pair;
           uint32_t r[32];
-          float m_run = kRunInit, off = __fmul_rn(scale, kRunInit), sum = 0.f;
+          float m_run = run_init(scale), off = __fmul_rn(scale, m_run), sum = 0.f;
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
             tmem_ld32_nowait(src + c * 32, r);
@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
       if (ok) ok = mbar_wait(bar(S_FULL + buf), (jt / NBUF) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok) != 0;
       const float scale = wide ? u.scale2 * g.scales.inv[side][rt * BM + trow] : pair;
-      float off = two ? 0.f : __fmul_rn(scale, kRunInit), m_run = kRunInit, sum = 0.f;
+      float m_run = run_init(scale), off = two ? 0.f : __fmul_rn(scale, m_run), sum = 0.f;
       if (ok) {
         tc_fence_after();
         const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN) + part * CH * 32;

@@ -401,7 +401,11 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     // off_run is the fp32 exponent offset all terms of s_run are relative to: sum = s_run * 2^off_run.
     // It is carried as the ROUNDED value scale*max (not recomputed from the max), so that rescaling by
     // 2^(off_old - off_new) and the final off_run + log2(s_run) are exact identities in fp32.
-    float m_run = kRunInit, off_run = VEC ? 0.f : __fmul_rn(scale, kRunInit), s_run = 0.f;
+    float m_run = kRunInit, off_run = 0.f, s_run = 0.f;
+    auto start_row = [&]() {  // (the arg-max has a negative scale and no use for the offset)
+      m_run = AM ? kRunInit : run_init(scale);
+      off_run = VEC || AM ? 0.f : __fmul_rn(scale, m_run);
+    };
     float negR = 0.f;  // VEC: minus the row's normaliser
     int idx_run = 0;   // AM: column of the running maximum m_run
     int col_tile = CSR ? 0 : w_begin % p.ntiles;  // AM, VEC: column tile of the chunk being consumed
@@ -611,8 +615,6 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
       }
       // merge_off / merge_sum / last_flag are re-used by the next segment
       asm volatile("bar.sync 1, %0;" ::"n"(128 * NHALF * PARTS) : "memory");
-      m_run = kRunInit;
-      off_run = VEC ? 0.f : __fmul_rn(scale, kRunInit);
       s_run = 0.f;
       idx_run = 0;
     };
@@ -625,12 +627,12 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         seg_blk = next_blk(seg_blk, seg_w);
         if (NSUB > 1) load_pass();  // the next segment may belong to another pass, with its own logit scale
         load_row(seg_blk);
-        if (!VEC) off_run = __fmul_rn(scale, kRunInit);
+        start_row();
       }
     };
     int seg_end_g = has_work ? seg_len() * CH : 0;
     if (has_work) load_row(seg_blk);
-    if (!VEC) off_run = __fmul_rn(scale, kRunInit);
+    start_row();
     auto consumed = [&](int g) {  // chunk g has been folded in: close the segment if it was its last chunk
       if ((AM || VEC) && g % CH == CH - 1) ++col_tile;
       if (g + 1 == seg_end_g) {

@@ -240,8 +240,8 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     // Running state of the current segment (the part of one row block this CTA covers). LSE: sum =
     // s_run * 2^off_run with off_run the rounded value scale*max. VEC: off_run stays 0 and s_run is the signed
     // weighted sum, so the same merge formulas (2^0 = 1 exactly) serve both.
-    float off_init = (EPI == EPI_LSE) ? __fmul_rn(scale, kRunInit) : 0.f;
-    float m_run = kRunInit, off_run = off_init, s_run = 0.f;
+    float m_init = run_init(scale), off_init = (EPI == EPI_LSE) ? __fmul_rn(scale, m_init) : 0.f;
+    float m_run = m_init, off_run = off_init, s_run = 0.f;
     int cur_blk = w_begin / p.ntiles, cur_jt = w_begin - cur_blk * p.ntiles;  // item of the chunk being consumed
     bool row_fresh = true;  // per-row constants (negR, fac) belong to another row block
     float negR = 0.f, fac = 0.f;
@@ -249,7 +249,10 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     auto wide_row = [&](int blk) {  // the row of this thread in a row block has a scale of its own
       const int r = p.row_begin + blk * BM + trow;
       scale = r < p.nr ? p.scale2 * __ldg(p.scales.inv[p.side] + r) : p.scale2;
-      if (EPI == EPI_LSE) off_run = off_init = __fmul_rn(scale, kRunInit);
+      if (EPI == EPI_LSE) {
+        m_run = m_init = run_init(scale);
+        off_run = off_init = __fmul_rn(scale, m_init);
+      }
     };
     if (wide) wide_row(cur_blk);
 
@@ -440,7 +443,7 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         }
       }
       asm volatile("bar.sync 1, %0;" ::"n"(NSYNC) : "memory");  // merge buffers are re-used by the next segment
-      m_run = kRunInit;
+      m_run = m_init;
       off_run = off_init;
       s_run = 0.f;
     };

@@ -182,6 +182,28 @@ def test_not_a_number_stays_with_its_point(cta_limit):
     assert torch.isnan(f[17]) and _lib.load().fs_device_error() == 0
 
 
+@pytest.mark.parametrize("zeros", [True, False])
+@pytest.mark.parametrize("n,m,d", [(300, 20, 3), (20, 300, 3), (295, 260, 8), (130, 70, 2)])
+def test_eps_at_which_the_mask_of_padded_points_leaves_fp32(n, m, d, zeros):
+    """Clouds in units of 1e-3 and eps = 1e-9: the exponent of a padded point is -inf, also where a stretch of columns holds
+    nothing else, in one-sided steps (weights of zero keep all of them so), soft-mins and alternating solves. Scores are 2e3
+    to 2e4 times eps: the tolerance of the other tests, 1e-5 of |x|^2."""
+    from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_alternating
+    x, y, a, b = _clouds(n, m, d, seed=11, zeros=zeros)
+    x, y = (np.float32(1e-3 * v).astype(np.float64) for v in (x, y))
+    eps, size = 1e-9, max((x * x).sum(1).max(), (y * y).sum(1).max())
+    bias = np.float32(np.random.default_rng(12).normal(size=m)).astype(np.float64)
+    got = flashsinkhorn_lse(dev(x), dev(y), dev(bias), eps=eps, allow_tf32=False)
+    assert np.abs(host(got) - O.lse_update(x, y, bias, eps)).max() < 1e-5 * size
+    want = O.solve_symmetric(x, y, a, b, [eps] * 6)
+    got = _solve(x, y, a, b, "fp32", eps=eps, n_iters=6)
+    assert np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size and np.abs(host(got[1]) - want["g"]).max() < 1e-5 * size
+    want = O.solve_alternating(x, y, a, b, [eps], 3)
+    got = sinkhorn_flashstyle_alternating(*(dev(v) for v in (x, y, a, b)), eps_list=[eps], iters_per_eps=3, allow_tf32=False)
+    assert np.abs(host(got[0]) - want["f"]).max() < 1e-5 * size and np.abs(host(got[1]) - want["g"]).max() < 1e-5 * size
+
+
 @pytest.mark.parametrize("scale", [1e-9, 1e-4, 1.0, 3e4, 1e9])
 def test_operand_scale_follows_the_clouds(scale):
     """Coordinates ride as fp16 scaled by a power of two per cloud: any size of the clouds, also very different ones
