@@ -138,7 +138,7 @@ def pass_ms_by_difference(run_solve, k1, k2, reps=3):
     """Device time of ONE pass over the score entries inside a symmetric solve: (T(k2 iterations) - T(k1 iterations))
     divided by the k2 - k1 steps the longer solve adds. A step passes over the entries once for both soft-mins; the
     first steps, which take them one after the other, are in both solves when k1 covers them. Staging, norms and
-    Python overhead drop out; the finalising kernel stays in (it is part of every step)."""
+    Python overhead drop out; the finish of a step stays in (it is part of every step)."""
     import torch
     times = []
     for k in (k1, k2):
@@ -651,7 +651,7 @@ def main():
     clocks = sampler.stop()
 
     # Dominant kernel: on one GPU the two-sided step of a symmetric solve (one exponential per entry for both potentials, its
-    # finalising kernel included), timed inside solves of two lengths; on several the soft-min pass of a row shard's
+    # the finish included), timed inside solves of two lengths; on several the soft-min pass of a row shard's
     # engine over all n x m entries, timed alone.
     k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     reps = 10
@@ -661,7 +661,7 @@ def main():
         kernel_ms = pass_ms_by_difference(
             lambda k: _pass_solve(x_dev, y_dev, aw, bw, use_epsilon_scaling=False, eps=eps, n_iters=k,
                                   last_extrapolation=False, allow_tf32=not args.fp32), 20, 40)
-        kernel_name = ("two-sided step of a symmetric solve (sym_kernel and sym_finalize_kernel), n*m exponentials; inside a "
+        kernel_name = ("two-sided step of a symmetric solve (sym_kernel), n*m exponentials; inside a "
                        "solve: (T(40 iterations) - T(20 iterations)) / 20")
     else:
         from flash_sinkhorn_b200.kernels.sinkhorn_flashstyle_sqeuclid import flashsinkhorn_lse_fused

@@ -408,67 +408,107 @@ void sym_schedule(SymSolve& s, const double* eps_list, int n_eps, int last_extra
   if (last_extrapolation) s.eps.push_back(eps_list[n_eps - 1]);
 }
 
-// Lockstep: step t of every problem that still has one. threshold < 0: no early stopping (one problem otherwise).
+// What step t of a solve does, as the kernels read it.
+sym::StepRec sym_record(const SymSolve& s, size_t t, int last_extrapolation, double rho_x, double rho_y, bool early,
+                        int check_every) {
+  const size_t total = s.eps.size();
+  const bool is_last = t + 1 == total, extrapolation = last_extrapolation && is_last;
+  sym::StepRec r;
+  const double eps = s.eps[t];
+  r.eps = (float)eps;
+  r.eps_next = (float)(is_last ? eps : s.eps[t + 1]);
+  r.ratio = t ? (float)(s.eps[t - 1] / eps) : 1.0f;
+  r.scale2 = (2.0f * s.p.cs_dot) * (1.0f / (float)eps) * kLog2e;
+  r.w = (t == 0 || extrapolation) ? 1.0f : 0.5f;
+  r.damp[0] = (float)dampening(eps, rho_x);
+  r.damp[1] = (float)dampening(eps, rho_y);
+  r.todo = 0;
+  if (!early) {  // results that an early stop may leave with an earlier step are written at the end (sym_run)
+    if (is_last) r.todo |= sym::kEmitOut | (last_extrapolation ? 0u : sym::kEmitPre);
+    if (last_extrapolation && t + 2 == total) r.todo |= sym::kEmitPre;
+  } else if (t > 0 && !extrapolation && t % (size_t)check_every == 0) {
+    r.todo |= sym::kCheck | (unsigned)(t / (size_t)check_every - 1) << 8;
+  }
+  return r;
+}
+
+// Lockstep: step t of every problem that still has one, as many steps per launch as the same problems take.
+// threshold < 0: no early stopping (one problem otherwise).
 int sym_run(SymSolve* s, int cnt, int last_extrapolation, double rho_x, double rho_y, double threshold,
             int check_every, cudaStream_t st) {
   sym::Problem* probs[sym::kMaxProblems];
-  double eps0[sym::kMaxProblems];
-  size_t steps = 0;
-  for (int i = 0; i < cnt; ++i) {
-    probs[i] = &s[i].p;
-    eps0[i] = s[i].eps[0];
-    steps = s[i].eps.size() > steps ? s[i].eps.size() : steps;
+  for (int i = 0; i < cnt; ++i) probs[i] = &s[i].p;
+  if (!sym::lockstep(probs, cnt)) {
+    for (int i = 0; i < cnt; ++i) FS_TRY(sym_run(s + i, 1, last_extrapolation, rho_x, rho_y, threshold, check_every, st));
+    return FS_OK;
   }
-  FS_CUDA(sym::stage(probs, eps0, cnt, st));
   const bool early = threshold >= 0.0;
-  for (size_t t = 0; t < steps; ++t) {
-    sym::Step batch[sym::kMaxProblems];
-    sym::Problem* last[sym::kMaxProblems];
-    float* pre[sym::kMaxProblems][2];
-    int k = 0, n_last = 0;
+  size_t steps = 0;
+  std::vector<std::vector<sym::StepRec>> recs(cnt);
+  for (int i = 0; i < cnt; ++i) {
+    const size_t total = s[i].eps.size();
+    steps = total > steps ? total : steps;
+    recs[i].resize(total);
+    for (size_t t = 0; t < total; ++t) recs[i][t] = sym_record(s[i], t, last_extrapolation, rho_x, rho_y, early, check_every);
+    for (int c = 0; c < 2; ++c) {
+      s[i].p.out[c] = s[i].out[c];
+      s[i].p.pre[c] = s[i].pre[c];
+      s[i].p.snap[c] = s[i].snap[c];
+    }
+  }
+  // records of steps [t0, t0 + kTableSteps) of all problems
+  const sym::StepRec* window[sym::kMaxProblems];
+  int count[sym::kMaxProblems];
+  auto fill = [&](size_t t0) {
+    for (int i = 0; i < cnt; ++i) {
+      const size_t total = s[i].eps.size(), from = t0 < total ? t0 : total;
+      window[i] = recs[i].data() + from;
+      count[i] = (int)(total - from < (size_t)sym::kTableSteps ? total - from : (size_t)sym::kTableSteps);
+    }
+  };
+  fill(0);
+  FS_CUDA(sym::stage(probs, window, count, cnt, st));
+  size_t table = 0;
+  for (size_t t = 0; t < steps;) {
+    if (t == table + sym::kTableSteps) {
+      table = t;
+      fill(t);
+      FS_CUDA(sym::upload(probs, window, count, cnt, st));
+    }
+    // up to the end of the table, or of the first problem that ends
+    size_t to = table + sym::kTableSteps;
+    sym::Problem* active[sym::kMaxProblems];
+    int k = 0;
     for (int i = 0; i < cnt; ++i) {
       const size_t total = s[i].eps.size();
       if (t >= total) continue;
-      const bool is_last = last_extrapolation && t + 1 == total;
-      if (is_last && (s[i].pre[0] || s[i].pre[1])) {
-        last[n_last] = &s[i].p;
-        pre[n_last][0] = s[i].pre[0];
-        pre[n_last++][1] = s[i].pre[1];
+      active[k++] = &s[i].p;
+      to = total < to ? total : to;
+    }
+    bool may_stop = early;
+    if (early && last_extrapolation) {
+      if (t + 1 == steps) {  // the step after the loop, whether or not the loop stopped early
+        may_stop = false;
+        float* pre[1][2] = {{s[0].pre[0], s[0].pre[1]}};
+        FS_CUDA(sym::emit(probs, pre, 1, st));
+        // where the schedule varies, a solve that stopped early holds the biases of the step after its last one
+        bool varies = false;
+        for (double e : s[0].eps) varies = varies || e != s[0].eps[t];
+        if (varies) FS_CUDA(sym::rebias(s[0].p, s[0].eps[t], st));
+      } else if (to == steps) {
+        to = steps - 1;
       }
-      sym::Step& b = batch[k++];
-      b.p = &s[i].p;
-      b.eps = s[i].eps[t];
-      b.eps_prev = t ? s[i].eps[t - 1] : b.eps;
-      b.eps_next = t + 1 < total ? s[i].eps[t + 1] : b.eps;
-      b.w = (t == 0 || is_last) ? 1.0f : 0.5f;
-      b.damp[0] = (float)dampening(b.eps, rho_x);
-      b.damp[1] = (float)dampening(b.eps, rho_y);
-      b.early = early && t > 0 && !is_last;
     }
-    if (n_last) FS_CUDA(sym::emit(last, pre, n_last, st));
-    if (early && last_extrapolation && t + 1 == steps) {
-      // where the schedule varies, a solve that stopped early holds the biases of the step after its last one
-      bool varies = false;
-      for (double e : s[0].eps) varies = varies || e != s[0].eps[t];
-      if (varies) FS_CUDA(sym::rebias(s[0].p, s[0].eps[t], st));
-    }
-    FS_CUDA(sym::step(batch, k, (int)t, st));
-    const sym::Problem& p = s[0].p;
-    if (early && batch[0].early && t % (size_t)check_every == 0) {
-      const int n = p.n[0], m = p.n[1];
-      delta_kernel<<<g1(n + m), 256, 0, st>>>(p.pot[0], s[0].snap[0], n, p.pot[1], s[0].snap[1], m, p.ctrl);
-      decide_kernel<<<1, 1, 0, st>>>(p.ctrl, threshold);
-      snapshot_kernel<<<g1(n + m), 256, 0, st>>>(p.pot[0], s[0].snap[0], n, p.pot[1], s[0].snap[1], m, p.ctrl);
-    }
+    FS_CUDA(sym::steps(active, k, (int)t, (int)to, (int)table, may_stop, threshold, st));
+    t = to;
   }
-  float* out[sym::kMaxProblems][2];
-  for (int i = 0; i < cnt; ++i)
-    for (int c = 0; c < 2; ++c) out[i][c] = s[i].out[c];
-  FS_CUDA(sym::emit(probs, out, cnt, st));
-  if (!last_extrapolation) {
-    for (int i = 0; i < cnt; ++i)
-      for (int c = 0; c < 2; ++c) out[i][c] = s[i].pre[c];
-    FS_CUDA(sym::emit(probs, out, cnt, st));
+  if (early) {
+    float* out[1][2] = {{s[0].out[0], s[0].out[1]}};
+    FS_CUDA(sym::emit(probs, out, 1, st));
+    if (!last_extrapolation) {
+      float* pre[1][2] = {{s[0].pre[0], s[0].pre[1]}};
+      FS_CUDA(sym::emit(probs, pre, 1, st));
+    }
   }
   FS_CUDA(cudaGetLastError());
   return FS_OK;

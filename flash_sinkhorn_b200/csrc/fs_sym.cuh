@@ -16,16 +16,26 @@ struct State {
   unsigned slot[3][8];  // per step modulo 3: {max u, -min u, max dlt, -min dlt} of the rows, then of the columns
   unsigned cst[4];      // max(-log2 a), max(log2 a), max(-log2 b), max(log2 b)
   unsigned range[kRangeWords];  // of the coordinates (OperandScales)
+  unsigned delta[2];    // early stop: largest move of a potential since the last check, checks taken in turn
+  unsigned bar_count, bar_leave;  // grid barrier of the launches that this problem is the first of
 };
+
+// One step of one problem, in the problem's table on the device.
+struct alignas(16) StepRec {
+  float eps, eps_next, ratio, scale2;  // eps_next: of the step after this one (staged into the biases); ratio: eps of the
+                                       // previous step / eps; scale2 = 2 cs log2e / eps
+  float w, damp[2];
+  unsigned todo;                       // kEmitPre | kEmitOut | kCheck | ordinal of the check << 8
+};
+constexpr unsigned kEmitPre = 1, kEmitOut = 2, kCheck = 4;  // write the potentials after this step to pre / out; early-stop test
+constexpr int kTableSteps = 256;                            // records that a problem's table holds
 
 // What every kernel of a step needs to know about a problem. Cloud 0 = x, cloud 1 = y.
 struct Geo {
   int n[2], nrt[2], nct[2], pad[2];  // points, row tiles of bm, column tiles of bn, padded points
   int bm, bn;
   int self;                          // one cloud against itself: only the tiles on one side of the diagonal
-  int early;                         // 1: leave everything alone once ctrl->converged is set
   int by_tile;                       // column partials are one per row tile (not one per CTA and column tile)
-  float ratio;                       // eps of the previous step / eps of this step
   OperandScales scales;              // of the fp16 coordinates
   State* st;
   Ctrl* ctrl;
@@ -50,27 +60,30 @@ struct Problem {
   float* opB[2];
   float* pot[2];  // shifted potentials, updated in place
   float* sq[2];   // cost scale * squared norms
+  float* out[2] = {nullptr, nullptr};   // results of the steps that ask for them (null: not wanted)
+  float* pre[2] = {nullptr, nullptr};
+  float* snap[2] = {nullptr, nullptr};  // early stop: potentials at the last check
   Ctrl* ctrl;
+  StepRec* table;        // of its own
+  const StepRec* sched;  // table in use: its own, or that of a problem with the same steps
   Geo geo;
   CUtensorMap map[8];  // per side: A-role full / tail, B-role full / tail
-};
-
-// Parameters of one step of one problem.
-struct Step {
-  Problem* p;
-  double eps, eps_prev, eps_next;  // eps_next: eps of the step after this one (staged into the biases)
-  float w, damp[2];
-  bool early;
 };
 
 bool supported(int n, int m, int d, int prec, int nlab);
 size_t bytes(int n, int m, int d, int prec, int nlab, bool self);
 // Lays the problem out inside buf (bytes() of it) and encodes its tensor maps.
 cudaError_t layout(Problem& p, char* buf);
-// Operands, squared norms, initial potentials and the biases of a first step at eps0[i].
-cudaError_t stage(Problem* const* p, const double* eps0, int cnt, cudaStream_t st);
-// One step of cnt <= kMaxProblems problems of one feature dimension; t counts the steps since stage().
-cudaError_t step(const Step* s, int cnt, int t, cudaStream_t st);
+// Operands, squared norms, initial potentials and the biases of the first step, at the eps of rec[i][0]; the first
+// records of every problem (count[i] of them, kTableSteps at most).
+cudaError_t stage(Problem* const* p, const StepRec* const* rec, const int* count, int cnt, cudaStream_t st);
+// Replaces the records.
+cudaError_t upload(Problem* const* p, const StepRec* const* rec, const int* count, int cnt, cudaStream_t st);
+// Steps [t0, t1) (counted since stage()) of cnt <= kMaxProblems problems of one kernel in lockstep, in one launch; the table's
+// first record is that of step t_table. early: nothing happens once the problem has converged.
+cudaError_t steps(Problem* const* p, int cnt, int t0, int t1, int t_table, bool early, double threshold, cudaStream_t st);
+// Whether problems can share a launch.
+bool lockstep(const Problem* const* p, int cnt);
 // Stages the biases again for a step at eps: steps that an early stop skipped have left those of their own.
 cudaError_t rebias(const Problem& p, double eps, cudaStream_t st);
 // out[c] = potential + squared-norm shift for both clouds (null pointers are skipped).
