@@ -18,6 +18,7 @@ from typing import Optional, Tuple
 
 import torch
 
+from flash_sinkhorn_b200 import _lib
 from flash_sinkhorn_b200.hvp import geomloss_to_ott_potentials, hvp_x_sqeuclid_from_potentials
 from flash_sinkhorn_b200.kernels.grad_sqeuclid import sinkhorn_geomloss_online_grad_sqeuclid
 from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_alternating, sinkhorn_flashstyle_symmetric
@@ -111,6 +112,140 @@ class _SinkhornGradFn(torch.autograd.Function):
                 )
                 out_x = hv * grad_scale
         return (out_x,) + (None,) * 13
+
+
+@dataclass(frozen=True)
+class _LossTerms:
+    """What the node of a batch of losses knows beside its tensors."""
+
+    eps: float
+    config: _SinkhornConfig
+    debias: bool
+    labels: Optional[list]  # label costs of the terms
+
+
+def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y):
+    """Gradients of ``sum_i scale_i loss_i`` to the clouds ``[B, n, d]``, ``[B, m, d]`` (or one item without the leading
+    axis); pots: ``f, g, f_pre, g_pre`` of every term."""
+    if x.dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        raise ValueError(f"Unsupported dtype for x/y: {x.dtype}")
+    cfg, dev = meta.config, x.device
+    n, m, d = x.shape[-2], y.shape[-2], x.shape[-1]
+    x32, y32, a32, b32, la, lb = map(_lib.f32c, (x, y, a, b, log_a, log_b))
+    pots = [_lib.f32c(p) for p in pots]
+    gs = _lib.f32c(scale.detach().reshape(-1))
+    prec = _lib.precision_id(cfg.allow_tf32)
+    X, Y = (x32, a32, la, n), (y32, b32, lb, m)
+
+    def term(k, u, v, scales, out_u, out_v):
+        (pu, wu, lu, r), (pv, wv, lv, c) = u, v
+        f_pre, g_pre = pots[4 * k + 2], pots[4 * k + 3]
+        label = meta.labels[k] if meta.labels else None
+        ws = _lib.workspace(_lib.OP_GRAD, r, c, d, prec, dev, label.V if label else 0)
+        tensors = (pu, pv, wu, wv, lu, lv, f_pre, g_pre, scales, out_u, out_v)
+        pitch = [4 * q for q in (r * d, c * d, r, c, r, c, r, c, 1, r * d, c * d)]
+        addr = [_lib.ptr(t) for t in tensors]
+        for i in range(gs.numel()):
+            at = [None if p is None else p + i * q for p, q in zip(addr, pitch)]
+            _lib.call("fs_grad", dev, at[0], at[1], r, c, d, *at[2:], meta.eps, float(cfg.cost_scale), prec, _lib.ptr(ws),
+                      ws.numel(), _lib.stream_ptr(dev), label.ref if label else None)
+
+    gx = torch.empty(x.shape, device=dev, dtype=torch.float32) if want_x else None
+    gy = torch.empty(y.shape, device=dev, dtype=torch.float32) if want_y else None
+    term(0, X, Y, gs, gx, gy)
+    for k, side, out in ((1, X, gx), (2, Y, gy)):
+        if not meta.debias or out is None:
+            continue
+        if pots[4 * k + 2].data_ptr() == pots[4 * k + 3].data_ptr():  # equal potentials: the two sides' gradients are equal
+            own = torch.empty_like(out)
+            term(k, side, side, -gs, own, None)
+            out += own
+        else:
+            own, other = torch.empty_like(out), torch.empty_like(out)
+            term(k, side, side, -0.5 * gs, own, other)
+            out += own + other
+    return gx, gy
+
+
+class _SinkhornLossGradFn(torch.autograd.Function):
+    """Gradients of a batch of losses; differentiable once more w.r.t. x where they are not debiased."""
+
+    @staticmethod
+    def forward(ctx, x, y, a, b, log_a, log_b, scale, meta, want_x, want_y, *pots):
+        ctx.save_for_backward(x, y, a, b, scale, *pots[2:4])
+        ctx.meta = meta
+        return _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
+
+    @staticmethod
+    def backward(ctx, v_x, v_y):
+        x, y, a, b, scale, f_pre, g_pre = ctx.saved_tensors
+        if v_y is not None or ctx.meta.debias:  # a self term has its cloud on both sides
+            raise NotImplementedError("Double backward w.r.t y is not implemented yet.")
+        out = None
+        if v_x is not None:
+            items = []
+            for i in range(x.shape[0]):
+                sub = _HvpContext((x[i], y[i], a[i], b[i], f_pre[i], g_pre[i], scale[i]), ctx.meta.eps, ctx.meta.config)
+                items.append(_SinkhornGradFn.backward(sub, v_x[i], None)[0])
+            out = torch.stack(items, dim=0)
+        return (out,) + (None,) * (9 + len(ctx.needs_input_grad) - 10)
+
+
+@dataclass
+class _HvpContext:
+    """The part of an autograd context that the Hessian-vector product of one item reads."""
+
+    saved_tensors: tuple
+    eps: float
+    config: _SinkhornConfig
+    use_label_cost: bool = False
+
+
+class _SinkhornLossFn(torch.autograd.Function):
+    """A batch of losses ``OT(x,y) - OT(x,x)/2 - OT(y,y)/2`` (or ``OT(x,y)`` alone) from finished potentials as ONE node:
+    the values of :class:`_SinkhornCostFn` for every term, combined, and their gradients in one pass over the terms. ``x``,
+    ``y``, ``a``, ``b`` have a leading batch axis or describe one item; ``pots`` are ``f, g, f_pre, g_pre`` of every term
+    (the last two those that gradients are taken at), shaped like the weights."""
+
+    @staticmethod
+    def forward(ctx, x, y, a, b, log_a, log_b, meta, *pots):
+        ctx.save_for_backward(x, y, a, b, log_a, log_b, *pots)
+        ctx.meta = meta
+        cfg = meta.config
+
+        def value(w, pot, rho):
+            if cfg.rho_x is None or cfg.rho_y is None:  # balanced or semi-unbalanced
+                return w * pot
+            return (rho + meta.eps / 2) * (w * (1 - (-pot / rho).exp()))
+
+        def side(k, w, rho, own, other):
+            # the potential of this side in OT(x,y), minus half of both potentials of the self term
+            if not meta.debias:
+                return value(w, pots[k], rho).sum(dim=-1)
+            if cfg.rho_x is None or cfg.rho_y is None:
+                return (w * (pots[k] - _half_sum(pots[own], pots[other]))).sum(dim=-1)
+            both = value(w, pots[own], cfg.rho_x) + value(w, pots[other], cfg.rho_y)
+            return (value(w, pots[k], rho) - 0.5 * both).sum(dim=-1)
+
+        return side(0, a, cfg.rho_x, 4, 5) + side(1, b, cfg.rho_y, 8, 9)
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        x, y, a, b, log_a, log_b, *pots = ctx.saved_tensors
+        gx = gy = ga = gb = None
+        if x.requires_grad or y.requires_grad:
+            gx, gy = _SinkhornLossGradFn.apply(x, y, a, b, log_a, log_b, grad_out, ctx.meta, x.requires_grad, y.requires_grad,
+                                               *(pots if ctx.meta.debias else pots[:4]))
+        debias = ctx.meta.debias
+        if a.requires_grad:
+            ga = grad_out.unsqueeze(-1) * (pots[0] - _half_sum(pots[4], pots[5]) if debias else pots[0])
+        if b.requires_grad:
+            gb = grad_out.unsqueeze(-1) * (pots[1] - _half_sum(pots[8], pots[9]) if debias else pots[1])
+        return (gx, gy, ga, gb) + (None,) * (3 + len(pots))
+
+
+def _half_sum(u, v):
+    return u if u.data_ptr() == v.data_ptr() else 0.5 * (u + v)
 
 
 class _SinkhornCostFn(torch.autograd.Function):

@@ -86,6 +86,7 @@ SIGNATURES = {
     ),
     "fs_symmetric_step_multi": (c_int, [_P, c_int, c_int, c_int, _P]),
     "fs_solve_symmetric_batched": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P]),
+    "fs_solve_symmetric_batched_labels": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P, _P]),
     "fs_grad_range": (
         c_int,
         [_P, _P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_float, c_float,
@@ -265,8 +266,10 @@ class LabelCost:
         if label_cost_matrix.shape[0] != label_cost_matrix.shape[1]:
             raise ValueError("label_cost_matrix must be square (V, V)")
         V = label_cost_matrix.shape[0]
-        for name, lab in (("label_x", label_x), ("label_y", label_y)):
-            lo, hi = int(lab.min()), int(lab.max())
+        # one read of the device for both ranges
+        ends = [lab.min().to(torch.int64) for lab in (label_x, label_y)] + [lab.max().to(torch.int64) for lab in (label_x, label_y)]
+        ends = torch.stack([e.to(ends[0].device) for e in ends]).tolist()
+        for name, lo, hi in (("label_x", ends[0], ends[2]), ("label_y", ends[1], ends[3])):
             if hi >= V or lo < 0:
                 raise ValueError(f"{name} values must be in [0, {V}), got range [{lo}, {hi}]")
         if not float(lambda_x) > 0.0:
@@ -275,6 +278,11 @@ class LabelCost:
                          label_y.to(dtype=torch.int32, device=device).contiguous(),
                          label_cost_matrix.to(dtype=torch.float32, device=device).contiguous(),
                          lambda_x, lambda_y)
+
+    def divergence_terms(self):
+        """Label costs of OT(x,y), OT(x,x) and OT(y,y) from that of OT(x,y), with labels of their own storage."""
+        lx, ly, lam_x, lam_y = self.label_x.clone(), self.label_y.clone(), self.struct.lambda_x, self.struct.lambda_y
+        return [LabelCost(u, v, self.table, lam_x, lam_y) for u, v in ((lx, ly), (lx, lx), (ly, ly))]
 
 
 class StepItem(ctypes.Structure):

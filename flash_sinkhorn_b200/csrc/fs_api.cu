@@ -1192,20 +1192,29 @@ int check_batch_item(const fs_batch_item& in, int i, int d, float cost_scale, in
 // Several symmetric solves in lockstep (batched inputs, or the three problems of a debiased loss): every step of
 // all problems that still have one goes out as fused multi-pass launches, so B small problems cost about one
 // solve's worth of launches instead of B. Schedules may differ in length; a finished problem drops out.
-extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
-                                          float cost_scale, double rho_x, double rho_y, int prec, void* stream) {
+static int solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
+                                   float cost_scale, double rho_x, double rho_y, int prec, void* stream,
+                                   const fs_label_cost* labels) {
   constexpr int kMaxBatch = 256;
   if (!items || n_items <= 0 || n_items > kMaxBatch)
     return fail(FS_ERR_BAD_ARG, "fs_solve_symmetric_batched takes 1..%d items", kMaxBatch);
   FS_TRY(check_device());
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   bool two_sided = true;
-  auto self_item = [&](const fs_batch_item& in) {
-    return in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y;
+  std::vector<LabelCost> lc(n_items);
+  float cs_kernel = cost_scale;
+  for (int i = 0; i < n_items && labels; ++i) {
+    if (!label_cost_from_abi(labels + i, cost_scale, lc[i], cs_kernel)) return fail(FS_ERR_BAD_ARG, "item %d: invalid label cost descriptor", i);
+    if (lc[i].V == 0 || lc[i].V != lc[0].V || labels[i].lambda_x != labels[0].lambda_x)
+      return fail(FS_ERR_BAD_ARG, "item %d: the items share the number of classes and lambda_x", i);
+  }
+  const int nlab = 3 * lc[0].V;
+  auto self_item = [&](const fs_batch_item& in) {  // a label table need not be symmetric
+    return in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y && !labels;
   };
   for (int i = 0; i < n_items && two_sided; ++i) {
     const bool sizes = items[i].n > 0 && items[i].m > 0;
-    const size_t need = sizes ? sym_workspace(items[i].n, items[i].m, d, prec, 0, self_item(items[i])) : 0;
+    const size_t need = sizes ? sym_workspace(items[i].n, items[i].m, d, prec, nlab, self_item(items[i])) : 0;
     two_sided = need > 0 && need <= items[i].ws_bytes && items[i].ws;
   }
   if (two_sided) {
@@ -1215,8 +1224,8 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
       std::vector<SymSolve> ss(cnt);
       for (int k = 0; k < cnt; ++k) {
         const fs_batch_item& in = items[i0 + k];
-        FS_TRY(sym_prepare(ss[k], in.x, in.y, in.n, in.m, d, in.log_a, in.log_b, nullptr, nullptr, self_item(in), cost_scale,
-                           cost_scale, LabelCost(), prec, in.ws));
+        FS_TRY(sym_prepare(ss[k], in.x, in.y, in.n, in.m, d, in.log_a, in.log_b, nullptr, nullptr, self_item(in), cs_kernel,
+                           cost_scale, lc[i0 + k], prec, in.ws));
         sym_schedule(ss[k], in.eps_list_host, in.n_eps, last_extrapolation);
         ss[k].pre[0] = in.f_pre; ss[k].pre[1] = in.g_pre; ss[k].out[0] = in.f; ss[k].out[1] = in.g;
       }
@@ -1224,6 +1233,7 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
     }
     return FS_OK;
   }
+  if (labels) return fail(FS_ERR_UNSUPPORTED, "several solves with a label cost need the scratch of two-sided steps");
   struct Item {
     Problem p;
     SolveBufs b;
@@ -1324,6 +1334,18 @@ extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_item
   }
   FS_CUDA(cudaGetLastError());
   return FS_OK;
+}
+
+extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
+                                          float cost_scale, double rho_x, double rho_y, int prec, void* stream) {
+  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, nullptr);
+}
+
+extern "C" int fs_solve_symmetric_batched_labels(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
+                                                 float cost_scale, double rho_x, double rho_y, int prec, void* stream,
+                                                 const fs_label_cost* labels) {
+  if (!labels) return fail(FS_ERR_BAD_ARG, "labels must be non-null");
+  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, labels);
 }
 
 extern "C" int fs_grad_range(const float* x, const float* y, int n, int m, int d, const float* a, const float* b,

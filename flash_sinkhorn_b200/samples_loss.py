@@ -18,13 +18,14 @@ from typing import Optional, Sequence, Tuple, Union
 import torch
 
 from flash_sinkhorn_b200 import _lib
-from flash_sinkhorn_b200._autograd import _SinkhornConfig, _SinkhornCostFn
-from flash_sinkhorn_b200.kernels._common import epsilon_schedule, max_diameter
+from flash_sinkhorn_b200._autograd import _LossTerms, _SinkhornConfig, _SinkhornCostFn, _SinkhornLossFn
+from flash_sinkhorn_b200.kernels._common import epsilon_schedule, log_weights, max_diameter
 from flash_sinkhorn_b200.sinkhorn_solvers import (
     sinkhorn_flashstyle_symmetric_batched,
     sinkhorn_flashstyle_alternating,
     sinkhorn_flashstyle_symmetric,
     sinkhorn_flashstyle_symmetric_many,
+    solve_loss_terms,
 )
 
 
@@ -290,29 +291,70 @@ class SamplesLoss(torch.nn.Module):
             threshold=self.threshold, check_every=self.inner_iterations, process_group=self.process_group,
         )
 
-    def _lockstep(self, x: torch.Tensor, y: torch.Tensor, labels_on: bool) -> bool:
-        """Whether the three solves of the divergence go to the library as one lockstep call. Early stopping, the
-        label cost and schedules fixed in the constructor keep the one-at-a-time solves."""
-        if (self.backend == "alternating" or self.threshold is not None or labels_on or self.eps_list is not None
-                or self.diameter is not None):
-            return False
-        prec = _lib.precision_id(self.allow_tf32)
-        (n, d), m = x.shape, y.shape[0]
-        return all(_lib.load().fs_two_sided(r, c, d, prec) for r, c in ((n, m), (n, n), (m, m)))
-
-    def _divergence_schedules(self, x: torch.Tensor, y: torch.Tensor):
-        """Schedules of OT(x,y), OT(x,x) and OT(y,y); with annealing the three diameters cost one host read."""
+    def _term_schedules(self, x: torch.Tensor, y: torch.Tensor):
+        """eps lists of OT(x,y), OT(x,x) and OT(y,y), one per item of ``[B, n, d]`` clouds; with annealing the diameters
+        of all of them cost one host read."""
+        B = x.shape[0]
         if not self.use_epsilon_scaling:
-            return [self._eps_list_for_inputs(x, y)] * 3
-        (lx, hx), (ly, hy) = ((t.float().amin(dim=0), t.float().amax(dim=0)) for t in (x, y))
-        diams = torch.stack([(torch.maximum(hx, hy) - torch.minimum(lx, ly)).norm(), (hx - lx).norm(),
-                             (hy - ly).norm()]).tolist()
-        out = [list(epsilon_schedule(diam, self.blur, self.scaling, p=2.0)) for diam in diams]
+            if self.eps is None or self.n_iters is None:
+                raise ValueError("When use_epsilon_scaling=False, provide eps and n_iters.")
+            sched = [self.eps] * self.n_iters
+            if not sched:
+                raise ValueError("eps_list is empty after applying n_iters.")
+            return [[sched] * B] * 3
+        (lx, hx), (ly, hy) = ((t.float().amin(dim=1), t.float().amax(dim=1)) for t in (x, y))
+        spans = [torch.maximum(hx, hy) - torch.minimum(lx, ly)] + ([hx - lx, hy - ly] if self.debias else [])
+        diams = torch.stack(spans).norm(dim=-1).tolist()
+        out = [[list(epsilon_schedule(diam, self.blur, self.scaling, p=2.0)) for diam in row] for row in diams]
         if self.n_iters is not None:
-            out = [sched[: int(self.n_iters)] for sched in out]
-        if not all(out):
+            out = [[sched[: self.n_iters] for sched in row] for row in out]
+        if not all(all(row) for row in out):
             raise ValueError("eps_list is empty after applying n_iters.")
         return out
+
+    def _one_node(self, x, y, a, b, config, label_x, label_y):
+        """The loss(es) as one autograd node whose terms are solved in one lockstep call, or None where they take the general
+        path: early stopping, schedules fixed in the constructor, terms that end at different eps, sizes without two-sided
+        steps."""
+        if self.eps_list is not None or self.diameter is not None:
+            return None
+        single = x.ndim == 2
+        (n, d), m = x.shape[-2:], y.shape[-2]
+        if not single and x.shape[0] == 0:
+            return None
+        dev = _lib.require_cuda(x=x, y=y, a=a, b=b)
+        prec = _lib.precision_id(self.allow_tf32)
+        sizes = ((n, m), (n, n), (m, m)) if self.debias else ((n, m),)
+        if not all(_lib.load().fs_two_sided(r, c, d, prec) for r, c in sizes):
+            return None
+        with torch.no_grad():
+            labels = _lib.LabelCost.make(label_x, label_y, self.label_cost_matrix, self.lambda_x, self.lambda_y, n, m, dev)
+            if labels is not None:
+                if any(_lib.symmetric_bytes(r, c, d, prec, labels.V) == _lib.symmetric_bytes(r, c, d, prec, labels.V, two_sided=False)
+                       for r, c in sizes):
+                    return None
+                labels = labels.divergence_terms()
+            xd, yd, wa, wb = (t.detach() for t in (x, y, a, b))
+            if single:
+                xd, yd, wa, wb = (t.unsqueeze(0) for t in (xd, yd, wa, wb))
+            schedules = self._term_schedules(xd, yd)
+            ends = {sched[-1] for row in schedules for sched in row}
+            if len(ends) != 1:
+                return None
+            log_a, log_b = log_weights(wa).contiguous(), log_weights(wb).contiguous()
+            try:
+                sols = solve_loss_terms(_lib.f32c(xd), _lib.f32c(yd), log_a, log_b, schedules, debias=self.debias, labels=labels,
+                                        prec=prec, cost_scale=self.cost_scale, rho_x=self.rho_x, rho_y=self.rho_y,
+                                        last_extrapolation=self.last_extrapolation)
+            except torch.cuda.OutOfMemoryError:
+                if labels is None:
+                    raise
+                return None
+            pots = [p[0] if single else p for sol in sols for p in sol]
+            if single:
+                log_a, log_b = log_a[0], log_b[0]
+        meta = _LossTerms(float(ends.pop()), config, self.debias, labels)
+        return _SinkhornLossFn.apply(x, y, a, b, log_a, log_b, meta, *pots)
 
     def forward(self, *args, label_x: Optional[torch.Tensor] = None, label_y: Optional[torch.Tensor] = None):
         parsed = _process_args(*args, normalize=self.normalize)
@@ -320,8 +362,8 @@ class SamplesLoss(torch.nn.Module):
             raise ValueError("flash_sinkhorn.SamplesLoss requires CUDA tensors.")
         config = self._make_config()
 
-        def ot(xs, ys, ws_a, ws_b, lx, ly, presolved=None, sched=None):
-            sched = tuple(self._eps_list_for_inputs(xs, ys)) if sched is None else tuple(sched)
+        def ot(xs, ys, ws_a, ws_b, lx, ly, presolved=None):
+            sched = tuple(self._eps_list_for_inputs(xs, ys))
             return _SinkhornCostFn.apply(xs, ys, ws_a, ws_b, sched, config, lx, ly, self.label_cost_matrix,
                                          presolved)
 
@@ -334,9 +376,13 @@ class SamplesLoss(torch.nn.Module):
         def divergence(xs, ys, ws_a, ws_b):
             if not self.debias:
                 return ot(xs, ys, ws_a, ws_b, label_x, label_y)
+            if self.backend != "alternating" and self.threshold is None and not multi_gpu:
+                val = self._one_node(xs, ys, ws_a, ws_b, config, label_x, label_y)
+                if val is not None:
+                    return val
             terms = [(xs, ys, ws_a, ws_b, label_x, label_y), (xs, xs, ws_a, ws_a, label_x, label_x),
                      (ys, ys, ws_b, ws_b, label_y, label_y)]
-            pre, scheds = [None, None, None], [None, None, None]
+            pre = [None, None, None]
             if multi_gpu and self.label_cost_matrix is not None and label_x is not None and self.lambda_y != 0.0:
                 raise NotImplementedError("The label cost is not available in the multi-GPU sharded solver.")
             if multi_gpu:
@@ -351,17 +397,7 @@ class SamplesLoss(torch.nn.Module):
                         rho_y=self.rho_y, last_extrapolation=self.last_extrapolation,
                         threshold=self.threshold, check_every=self.inner_iterations)
                 pre = [(f, g, f, g) if fp is None else (f, g, fp, gp) for (f, g, fp, gp, _) in sols]
-            elif self._lockstep(xs, ys, labels_on):
-                # One library call for the three solves: their steps share launches.
-                with torch.no_grad():
-                    scheds = self._divergence_schedules(xs.detach(), ys.detach())
-                    sols = sinkhorn_flashstyle_symmetric_batched(
-                        [tuple(u.detach() for u in t[:4]) for t in terms], schedules=scheds, blur=self.blur,
-                        scaling=self.scaling, use_epsilon_scaling=self.use_epsilon_scaling, eps=self.eps,
-                        n_iters=self.n_iters, allow_tf32=self.allow_tf32, cost_scale=self.cost_scale,
-                        rho_x=self.rho_x, rho_y=self.rho_y, last_extrapolation=self.last_extrapolation)
-                pre = [sol[:4] for sol in sols]
-            cross, self_x, self_y = (ot(*t, presolved=p, sched=e) for t, p, e in zip(terms, pre, scheds))
+            cross, self_x, self_y = (ot(*t, presolved=p) for t, p in zip(terms, pre))
             return cross - 0.5 * self_x - 0.5 * self_y
 
         # Batched inputs: the reference loops over the items (samples_loss.py:515-552). Here all symmetric solves of
@@ -370,6 +406,10 @@ class SamplesLoss(torch.nn.Module):
         # stopping, the label cost, the alternating backend and sharded runs keep the per-item loop.
         if (parsed.batched and self.backend != "alternating" and self.threshold is None and not labels_on
                 and not multi_gpu):
+            if not self.potentials:
+                vals = self._one_node(parsed.x, parsed.y, parsed.a, parsed.b, config, None, None)
+                if vals is not None:
+                    return vals
             items = list(zip(parsed.x, parsed.y, parsed.a, parsed.b))
             groups = []
             for xs, ys, wa, wb in items:

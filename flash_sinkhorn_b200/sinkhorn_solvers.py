@@ -11,7 +11,7 @@ is the optional read-back of the iteration counter (``return_n_iters=True``).
 from __future__ import annotations
 
 import ctypes
-from typing import Optional, Sequence, Tuple
+from typing import NamedTuple, Optional, Sequence, Tuple
 
 import torch
 
@@ -371,7 +371,7 @@ def sinkhorn_flashstyle_symmetric_batched(
     d = problems[0][0].shape[1]
     prec = _lib.precision_id(allow_tf32)
     dev = None
-    items, groups, group, taken = [], [], [], 0
+    items, keep = [], []
     for (x, y, a, b), given in zip(problems, schedules or [None] * len(problems)):
         if x.shape[1] != d or y.shape[1] != d:
             raise ValueError("all problems of a batched solve must share the feature dimension")
@@ -399,37 +399,66 @@ def sinkhorn_flashstyle_symmetric_batched(
         lb = la if _same_tensor(b, a) else log_weights(b).contiguous()
         same = x32 is y32 and la is lb and rho_x == rho_y
         out = tuple(torch.empty((k,), device=dev, dtype=torch.float32) for k in (n, m, n, m))
-        items.append((x32, y32, la, lb, _eps_array(sched), len(sched), same, out))
+        keep.append((x32, y32, la, lb, out))
+        items.append(_Solve(n, m, x32.data_ptr(), y32.data_ptr(), la.data_ptr(), lb.data_ptr(), _eps_array(sched), len(sched),
+                            same, tuple(t.data_ptr() for t in out)))
+    _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_x, rho_y)
+    return [k[4] + (item.n_eps + 1 + (1 if last_extrapolation else 0),) for k, item in zip(keep, items)]
 
+
+class _Solve(NamedTuple):
+    """One problem of a lockstep call, by address."""
+
+    n: int
+    m: int
+    x: int
+    y: int
+    log_a: int
+    log_b: int
+    eps: object  # ctypes array of n_eps doubles
+    n_eps: int
+    same: bool
+    out: Tuple[int, int, int, int]  # f, g, f_pre, g_pre
+    label: Optional[_lib.LabelCost] = None
+
+
+def _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_x, rho_y):
+    """Solves the items in as few library calls as their scratch allows. With label costs an OutOfMemoryError is the
+    caller's to handle (such solves have no form with linear scratch in one call)."""
+    n_classes = items[0].label.V if items[0].label else 0
     sizes = {}  # (n, m, same): bytes of the scratch, and of the per-tile sums in it
 
     def scratch(item):
-        n, m, same = item[0].shape[0], item[1].shape[0], item[6]
-        if (n, m, same) not in sizes:
-            full = _lib.symmetric_bytes(n, m, d, prec, same=same)
-            sizes[n, m, same] = (full, max(full - _lib.symmetric_bytes(n, m, d, prec, two_sided=False), 0))
-        return sizes[n, m, same]
+        key = item.n, item.m, item.same
+        if key not in sizes:
+            full = _lib.symmetric_bytes(item.n, item.m, d, prec, n_classes, item.same)
+            sizes[key] = (full, max(full - _lib.symmetric_bytes(item.n, item.m, d, prec, n_classes, two_sided=False), 0))
+        return sizes[key]
 
     def solve(group):
         arr = (_lib.BatchItem * len(group))()
-        keep = []
-        for slot, item in zip(arr, group):
-            x32, y32, la, lb, eps_arr, n_eps, same, out = item
-            n, m = x32.shape[0], y32.shape[0]
-            if len(group) == 1:
-                ws = _solver_scratch(n, m, d, prec, dev, same=same)
-            else:
-                ws = torch.empty(scratch(item)[0], dtype=torch.uint8, device=dev)
-            keep.append(ws)
-            slot.x, slot.y, slot.n, slot.m = x32.data_ptr(), y32.data_ptr(), n, m
-            slot.log_a, slot.log_b = la.data_ptr(), lb.data_ptr()
-            slot.eps_list_host, slot.n_eps = ctypes.cast(eps_arr, ctypes.c_void_p), n_eps
-            slot.f, slot.g, slot.f_pre, slot.g_pre = (t.data_ptr() for t in out)
-            slot.ws, slot.ws_bytes = ws.data_ptr(), ws.numel()
-        _lib.call("fs_solve_symmetric_batched", dev, ctypes.cast(arr, ctypes.c_void_p), len(group), d,
-                  1 if last_extrapolation else 0, float(cost_scale), _neg_if_none(rho_x), _neg_if_none(rho_y), prec,
-                  _lib.stream_ptr(dev))
+        if len(group) == 1 and not n_classes:
+            ws = _solver_scratch(group[0].n, group[0].m, d, prec, dev, same=group[0].same)
+            offsets, room = [0], [ws.numel()]
+        else:
+            room = [(scratch(item)[0] + 255) // 256 * 256 for item in group]
+            offsets = [sum(room[:k]) for k in range(len(group))]
+            ws = torch.empty(sum(room), dtype=torch.uint8, device=dev)
+        for slot, item, offset, size in zip(arr, group, offsets, room):
+            slot.x, slot.y, slot.n, slot.m = item.x, item.y, item.n, item.m
+            slot.log_a, slot.log_b = item.log_a, item.log_b
+            slot.eps_list_host, slot.n_eps = ctypes.cast(item.eps, ctypes.c_void_p), item.n_eps
+            slot.f, slot.g, slot.f_pre, slot.g_pre = item.out
+            slot.ws, slot.ws_bytes = ws.data_ptr() + offset, size
+        args = (ctypes.cast(arr, ctypes.c_void_p), len(group), d, 1 if last_extrapolation else 0, float(cost_scale),
+                _neg_if_none(rho_x), _neg_if_none(rho_y), prec, _lib.stream_ptr(dev))
+        if n_classes:
+            costs = (_lib.LabelCostStruct * len(group))(*[item.label.struct for item in group])
+            _lib.call("fs_solve_symmetric_batched_labels", dev, *args, ctypes.cast(costs, ctypes.c_void_p))
+        else:
+            _lib.call("fs_solve_symmetric_batched", dev, *args)
 
+    groups, group, taken = [], [], 0
     for item in items:
         sums = scratch(item)[1]
         if group and taken + sums > LOCKSTEP_SCRATCH_BYTES:
@@ -442,11 +471,41 @@ def sinkhorn_flashstyle_symmetric_batched(
         try:
             solve(group)
         except torch.cuda.OutOfMemoryError:
-            if len(group) == 1:
+            if len(group) == 1 or n_classes:
                 raise
             for item in group:
                 solve([item])
-    return [item[7] + (item[5] + 1 + (1 if last_extrapolation else 0),) for item in items]
+
+
+def solve_loss_terms(x, y, log_a, log_b, schedules, *, debias, labels, prec, cost_scale, rho_x, rho_y, last_extrapolation):
+    """Potentials of the terms of a batch of losses: OT(x,y) and, debiased, OT(x,x) and OT(y,y), of clouds ``x [B, n, d]``,
+    ``y [B, m, d]`` and log-weights ``[B, n]``, ``[B, m]`` (fp32, contiguous); ``schedules[term][item]``: eps lists. Returns
+    one ``(f, g, f_pre, g_pre)`` of ``[B, rows]`` tensors per term; a self term without labels has f for g."""
+    (B, n, d), m = x.shape, y.shape[1]
+    dev = x.device
+    new = lambda k: torch.empty((B, k), device=dev, dtype=torch.float32)  # noqa: E731
+    sides = [((x, log_a, n), (y, log_b, m)), ((x, log_a, n), (x, log_a, n)), ((y, log_b, m), (y, log_b, m))]
+    items, outs, arrays = [], [], {}
+    for term, ((u, lu, r), (v, lv, c)) in enumerate(sides[: 3 if debias else 1]):
+        same = term > 0 and labels is None and rho_x == rho_y
+        f, f_pre = new(r), new(r)
+        g, g_pre = (f, f_pre) if same else (new(c), new(c))
+        outs.append((f, g, f_pre, g_pre))
+        addr = [t.data_ptr() for t in (u, v, lu, lv, f, g, f_pre, g_pre)]
+        pitch = [4 * k for k in (r * d, c * d, r, c, r, c, r, c)]
+        for i in range(B):
+            sched = schedules[term][i]
+            key = tuple(sched)
+            if key not in arrays:
+                arrays[key] = _eps_array(sched)
+            at = [p + i * q for p, q in zip(addr, pitch)]
+            items.append(_Solve(r, c, at[0], at[1], at[2], at[3], arrays[key], len(sched), same, tuple(at[4:]),
+                                labels[term] if labels else None))
+    # item by item, its terms together: calls that are split keep the work of a divergence in one launch
+    terms = len(outs)
+    items = [items[t * B + i] for i in range(B) for t in range(terms)]
+    _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_x, rho_y)
+    return outs
 
 
 def sinkhorn_flashstyle_symmetric_many(problems, *, process_group, **kwargs):

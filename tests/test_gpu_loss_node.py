@@ -1,0 +1,121 @@
+"""Losses whose terms are one autograd node (debiased losses and batches) against the nodes of single terms, which
+``threshold=0`` (an early stop that never comes) keeps: values, gradients to clouds and weights, second order, refusals."""
+import pytest
+import torch
+
+from gpu_util import dev  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(B, n, m, d, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    x = torch.randn(B, n, d, generator=g)
+    y = 0.4 + torch.randn(B, m, d, generator=g)
+    a, b = (torch.softmax(torch.randn(B, k, generator=g), 1) for k in (n, m))
+    return [t.cuda() for t in (x, y, a, b)]
+
+
+def _err(u, v):
+    return float((u.double() - v.double()).norm() / v.double().norm().clamp(min=1e-30))
+
+
+CASES = [dict(eps=0.5, n_iters=12, use_epsilon_scaling=False),
+         dict(eps=0.5, n_iters=9, use_epsilon_scaling=False, last_extrapolation=False, reach=2.0, half_cost=True),
+         dict(eps=0.5, n_iters=9, use_epsilon_scaling=False, reach_x=1.5),
+         dict(eps=0.5, n_iters=9, use_epsilon_scaling=False, reach_x=1.5, reach_y=2.5),
+         dict(blur=0.4, scaling=0.6)]
+
+
+# fp32-exact products: values agree to 1e-5, gradients to 3e-4 (rounding of potentials over eps, as in the other tests of
+# this suite); the terms of one node are summed in another order
+@pytest.mark.parametrize("kw", CASES)
+@pytest.mark.parametrize("debias", [True, False])
+@pytest.mark.parametrize("B,n,m,d", [(3, 130, 97, 5), (1, 257, 300, 40), (2, 60, 1, 3)])
+def test_against_single_terms(B, n, m, d, debias, kw):
+    from flash_sinkhorn_b200 import SamplesLoss
+    if kw.get("blur") and m == 1:
+        kw = dict(kw, n_iters=3, eps=0.5, use_epsilon_scaling=False)  # one point has no diameter
+    x, y, a, b = _inputs(B, n, m, d)
+    one = SamplesLoss("sinkhorn", debias=debias, allow_tf32=False, normalize=False, **kw)
+    ref = SamplesLoss("sinkhorn", debias=debias, allow_tf32=False, normalize=False, threshold=0.0, **kw)
+    w = torch.linspace(0.5, 1.5, B, device="cuda")
+    outs = []
+    for loss in (one, ref):
+        args = [t.clone().requires_grad_(True) for t in (a, x, b, y)]
+        val = loss(*args)
+        outs.append((val, torch.autograd.grad((val * w).sum(), args)))
+    assert outs[0][0].shape == (B,)
+    scale = float(outs[1][0].abs().max()) + float((a * (x * x).sum(-1)).sum(-1).max())
+    assert float((outs[0][0] - outs[1][0]).abs().max()) < 1e-5 * scale
+    for u, v in zip(*(o[1] for o in outs)):
+        assert u.shape == v.shape and _err(u, v) < 3e-4
+    # the same loss, item by item
+    for i in range(B):
+        xi = x[i].clone().requires_grad_(True)
+        vi = one(a[i], xi, b[i], y[i])
+        assert vi.dim() == 0 and abs(float(vi) - float(outs[1][0][i])) < 1e-5 * scale
+        assert _err(w[i] * torch.autograd.grad(vi, xi)[0], outs[1][1][1][i]) < 3e-4
+
+
+def test_strided_half_and_shared_inputs():
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = _inputs(2, 150, 140, 6, seed=3)
+    kw = dict(eps=0.5, n_iters=8, use_epsilon_scaling=False, debias=True, allow_tf32=False)
+    one, ref = SamplesLoss("sinkhorn", **kw), SamplesLoss("sinkhorn", threshold=0.0, **kw)
+    wide = torch.randn(150, 2, 12, device="cuda").requires_grad_(True)
+    xs = wide.transpose(0, 1)[..., ::2]  # strides of its own in every axis
+    half = y.half().requires_grad_(True)
+    got, want = (torch.autograd.grad(f(xs, half).sum(), (wide, half)) for f in (one, ref))
+    assert got[1].dtype == torch.float16
+    assert _err(got[0], want[0]) < 3e-4 and _err(got[1], want[1]) < 2e-3
+    same = x.clone().requires_grad_(True)  # both clouds are one tensor
+    got, want = (torch.autograd.grad(f(same, same).sum(), same)[0] for f in (one, ref))
+    assert float((got - want).abs().max()) < 1e-6
+    big = x.double().requires_grad_(True)  # the value is computed in fp32, the gradient refused
+    val = one(big, y.double())
+    with pytest.raises(ValueError, match="Unsupported dtype"):
+        val.sum().backward()
+
+
+def test_second_order():
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = _inputs(2, 120, 110, 4, seed=5)
+    v = torch.randn_like(x)
+    kw = dict(eps=1.0, n_iters=30, use_epsilon_scaling=False, allow_tf32=False)
+    outs = []
+    for loss in (SamplesLoss("sinkhorn", **kw), SamplesLoss("sinkhorn", threshold=0.0, **kw)):
+        xs = x.clone().requires_grad_(True)
+        (gx,) = torch.autograd.grad((loss(xs, y) * torch.tensor([1.0, 2.0], device="cuda")).sum(), xs, create_graph=True)
+        outs.append(torch.autograd.grad((gx * v).sum(), xs)[0])
+    assert _err(*outs) < 1e-3  # each ends where its conjugate gradients meet rtol = 1e-6
+    xs = x.clone().requires_grad_(True)
+    (gx,) = torch.autograd.grad(SamplesLoss("sinkhorn", debias=True, **kw)(xs, y).sum(), xs, create_graph=True)
+    with pytest.raises(NotImplementedError):
+        torch.autograd.grad((gx * v).sum(), xs)
+
+
+@pytest.mark.parametrize("n,m,V", [(300, 260, 4), (900, 701, 7)])
+def test_labels_in_lockstep(n, m, V):
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = (t[0] for t in _inputs(1, n, m, 16, seed=7))
+    g = torch.Generator().manual_seed(1)
+    table = 3.0 * torch.rand(V, V, generator=g).cuda()  # not symmetric
+    lx, ly = torch.randint(0, V, (n,), generator=g).cuda(), torch.randint(0, V, (m,), generator=g).cuda()
+    kw = dict(eps=0.5, n_iters=10, use_epsilon_scaling=False, debias=True, allow_tf32=False, label_cost_matrix=table, lambda_x=0.7,
+              lambda_y=1.3)
+    outs = []
+    for extra in ({}, dict(threshold=0.0)):
+        args = [t.clone().requires_grad_(True) for t in (a, x, b, y)]
+        val = SamplesLoss("sinkhorn", **kw, **extra)(*args, label_x=lx, label_y=ly)
+        outs.append((val, torch.autograd.grad(val, args)))
+    assert abs(float(outs[0][0]) - float(outs[1][0])) < 1e-5 * (abs(float(outs[1][0])) + float((x * x).sum(1).max()))
+    for u, v in zip(outs[0][1], outs[1][1]):
+        assert _err(u, v) < 3e-4
+    with pytest.raises(ValueError, match="label_y values"):
+        SamplesLoss("sinkhorn", **kw)(a, x, b, y, label_x=lx, label_y=ly + V)
+    labels = lx.to(torch.int32)  # used as they were at the call
+    xs = x.clone().requires_grad_(True)
+    val = SamplesLoss("sinkhorn", **kw)(a, xs, b, y, label_x=labels, label_y=ly)
+    labels.fill_(1 << 20)
+    assert _err(torch.autograd.grad(val, xs)[0], outs[1][1][1]) < 3e-4
