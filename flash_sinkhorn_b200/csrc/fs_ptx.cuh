@@ -115,6 +115,11 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// Registers of a CTA of 128 + 512 threads, launched with 96 each: 32 for the service warps 0..3, 112 for the soft-max warps
+// (128 x 32 + 512 x 112 = 640 x 96). Executed by whole warpgroups.
+__device__ __forceinline__ void registers_down() { asm volatile("setmaxnreg.dec.sync.aligned.u32 32;"); }
+__device__ __forceinline__ void registers_up() { asm volatile("setmaxnreg.inc.sync.aligned.u32 112;"); }
+
 // D[tmem] (+)= A[smem desc] x B[smem desc]^T, M=128, N from idesc, K=8 (tf32)
 __device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {

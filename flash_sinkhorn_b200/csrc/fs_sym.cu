@@ -749,9 +749,9 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   int jt = 0, seg = 0, chunk = 0;
   unsigned met = 0;
   // The service warps and the soft-max warps go through the steps in loops of their own: the latter take registers from the
-  // former (512 x 112 + 128 x 32 = 640 x 96, what the CTA is launched with).
+  // former.
   if (warp < kFirst) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+  registers_down();
 #pragma unroll 1
   for (int t = P.t0;; ++t) {
   if (warp == 0) fence_proxy_async();  // the biases were written by ordinary stores, which the meeting has made visible
@@ -974,7 +974,7 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   }
   } else {
   // ===================== soft-max warpgroups =====================
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+  registers_up();
 #pragma unroll 1
   for (int t = P.t0;; ++t) {
     __syncthreads();

@@ -229,6 +229,10 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  // With four soft-max warpgroups these take registers from the four service warps (split_registers).
+  constexpr bool kSplitRegisters = NHALF * PARTS == 4;
+  if (warp < 4) {
+  if (kSplitRegisters) registers_down();
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (lane == 0) {
@@ -378,8 +382,10 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         mbar_wait_quiet(bar(DRAIN + h), 0);
       }
     }
-  } else if (warp >= 4) {
+  }
+  } else {
     // ===================== soft-max warpgroups =====================
+    if (kSplitRegisters) registers_up();
     // Twice the same code: points with scales of their own (wide_range) take registers that the ordinary form needs.
     auto soft_max = [&](auto wide_form) {
     constexpr bool WIDE = decltype(wide_form)::value;

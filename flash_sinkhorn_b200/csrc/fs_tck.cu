@@ -136,6 +136,9 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
+  constexpr bool kSplitRegisters = NHALF * kPartsK == 4;
+  if (warp < 4) {
+  if (kSplitRegisters) registers_down();
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (lane == 0) {
@@ -222,7 +225,9 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         mbar_wait_quiet(bar(DRAIN + h), 0);
       }
     }
-  } else if (warp >= 4) {
+  }
+  } else {
+    if (kSplitRegisters) registers_up();
     // ===================== epilogue warpgroups =====================
     // Twice the same code: points with scales of their own (wide_range) take registers that the ordinary form needs.
     auto epilogue = [&](auto wide_form) {
