@@ -117,6 +117,9 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int BM = 128 * NHALF;
+  // Score tiles in TMEM per half: all that fit. With one half a tile is 1024 clocks of ex2, and its sixteen warps would
+  // wait for one another at every tile with two.
+  constexpr int NBUF = NHALF == 1 && BN == 128 ? 4 : 2;
   // This CTA's items [w_begin, w_end) of the flattened (row block, column tile) list.
   static_assert(!CSR || (NHALF == 1 && BN == 128 && MODE == MODE_LSE), "tile lists are over 128 x 128 tiles");
   static_assert(NSUB == 1 || (!CSR && MODE == MODE_LSE), "multi-pass launches are dense soft-min passes");
@@ -192,8 +195,8 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   uint8_t* b_smem = a_smem + NHALF * a_half_bytes;
   uint64_t* bars = (uint64_t*)(b_smem + P.nstage * b_stage_bytes);
   // barrier indices
-  const int B_FULL = 0, B_EMPTY = P.nstage, S_FULL = 2 * P.nstage, S_EMPTY = S_FULL + 2 * NHALF,
-            A_FULL = S_EMPTY + 2 * NHALF, A_EMPTY = A_FULL + 1, DRAIN = A_EMPTY + 1, NBARS = DRAIN + 2;
+  const int B_FULL = 0, B_EMPTY = P.nstage, S_FULL = 2 * P.nstage, S_EMPTY = S_FULL + NBUF * NHALF,
+            A_FULL = S_EMPTY + NBUF * NHALF, A_EMPTY = A_FULL + 1, DRAIN = A_EMPTY + 1, NBARS = DRAIN + 2;
   uint32_t* tmem_slot = (uint32_t*)(bars + NBARS);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile int* last_flag = (volatile int*)(tmem_slot + 2);  // this CTA took the last ticket of its row block
@@ -201,14 +204,14 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   float* merge_sum = merge_off + (PARTS - 1) * NHALF * 128;
   auto bar = [&](int i) { return smem_u32(bars + i); };
 
-  constexpr uint32_t kTmemCols = (2 * NHALF * BN) < 32 ? 32 : (2 * NHALF * BN);
+  constexpr uint32_t kTmemCols = NBUF * NHALF * BN;
 
   if (tid == 0) {
     for (int s = 0; s < P.nstage; ++s) {
       mbar_init(bar(B_FULL + s), 1);
       mbar_init(bar(B_EMPTY + s), NHALF);  // one commit per MMA-issuing lane (one lane per 128-row half)
     }
-    for (int i = 0; i < 2 * NHALF; ++i) {
+    for (int i = 0; i < NBUF * NHALF; ++i) {
       mbar_init(bar(S_FULL + i), 1);
       mbar_init(bar(S_EMPTY + i), 4 * PARTS);  // one arrive per soft-max warp reading the buffer
     }
@@ -324,16 +327,16 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
           const int s = jt % P.nstage;
           const uint32_t ph = (jt / P.nstage) & 1;
           if (!vote(mbar_wait(bar(B_FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
-          const int buf = jt & 1;
-          const uint32_t sph = (jt >> 1) & 1;
-          if (!vote(mbar_wait(bar(S_EMPTY + h * 2 + buf), sph ^ 1, abort_flag, 2000))) {
+          const int buf = jt % NBUF;
+          const uint32_t sph = (jt / NBUF) & 1;
+          if (!vote(mbar_wait(bar(S_EMPTY + h * NBUF + buf), sph ^ 1, abort_flag, 2000))) {
             ok = false;
             break;
           }
           tc_fence_after();
           // Descriptors are advanced incrementally: the low word holds (address >> 4), the high word (stride,
           // version, swizzle) is a constant per block class.
-          const uint32_t d_tmem = tmem_base + (uint32_t)((h * 2 + buf) * BN);
+          const uint32_t d_tmem = tmem_base + (uint32_t)((h * NBUF + buf) * BN);
           uint32_t al = a_lo0, bl = desc_lo(smem_u32(b_smem + s * b_stage_bytes));
           // One election per tile where a tile has few MMAs (the 256-row plans: measured 1.3 % faster per pass,
           // 10 % for the arg-max pass), one per instruction in the 128-row plans with their long K (d = 128:
@@ -364,7 +367,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
               bl += (BN * 32) >> 4;
             }
             if (kTileElect || pick()) {
-              umma_commit(bar(S_FULL + h * 2 + buf));
+              umma_commit(bar(S_FULL + h * NBUF + buf));
               umma_commit(bar(B_EMPTY + s));
             }
           }
@@ -497,13 +500,13 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     // Issue the TMEM load of chunk g (first waits for its tile if g starts one). No wait for the data.
     auto issue = [&](int g, uint32_t (&r)[32]) -> bool {
       const int j = g / CH, c = g % CH;
-      const int buf = j & 1;
+      const int buf = j % NBUF;
       if (c == 0) {
-        if (!mbar_wait(bar(S_FULL + h * 2 + buf), (j >> 1) & 1, abort_flag)) return false;
+        if (!mbar_wait(bar(S_FULL + h * NBUF + buf), (j / NBUF) & 1, abort_flag)) return false;
         __syncwarp();  // lanes leave the poll loop at different times; tcgen05.ld is .sync.aligned
         tc_fence_after();
       }
-      tmem_ld32_nowait(lane_addr + (uint32_t)((h * 2 + buf) * BN) + (c_base + c) * 32, r);
+      tmem_ld32_nowait(lane_addr + (uint32_t)((h * NBUF + buf) * BN) + (c_base + c) * 32, r);
       return true;
     };
     // The load of chunk g has landed (tcgen05.wait::ld): if it was the last chunk of its tile,
@@ -514,7 +517,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         const int j = g / CH;
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar(S_EMPTY + h * 2 + (j & 1)));
+        if (lane == 0) mbar_arrive(bar(S_EMPTY + h * NBUF + j % NBUF));
       }
     };
     // Epilogue of a finished row: raw log2 normaliser and / or the damped, averaged potential update.
