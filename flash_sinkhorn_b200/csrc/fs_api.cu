@@ -862,6 +862,9 @@ int fs_solve_alternating(const float* x, const float* y, int n, int m, int d, co
   }
   FS_CUDA(cudaGetLastError());
 
+  // On the tensor cores the half-steps form a chain: each stages its potential as the column bias of the next.
+  const bool tiles_ok = !tile_row_ptr || tc::csr_supported(d, prec, p.nlab);
+  const bool chain = p.use_tc && tiles_ok && tc::chains(p.staged, tile_row_ptr != nullptr);
   int global_it = 0;
   for (int e = 0; e < n_eps; ++e) {
     const double eps = eps_list[e];
@@ -871,6 +874,22 @@ int fs_solve_alternating(const float* x, const float* y, int n, int m, int d, co
       ef.damping = df; ef.w = 1.f; ef.out = fh;
       eg.damping = dg; eg.w = 1.f; eg.out = gh;
       if (early) { ef.ctrl = b.ctrl; eg.ctrl = b.ctrl; }
+      // A pass behind the early-stop test is no dependent of the pass before: the test reads what that one wrote.
+      const bool tested = early && global_it > 0 && global_it % check_every == 0;
+      if (chain) {
+        LseEpilogue &one = ott_convention ? eg : ef, &two = ott_convention ? ef : eg;
+        const bool last = it + 1 == iters_per_eps && e + 1 == n_eps;
+        one.chain_bias = true;
+        one.next_logw = ott_convention ? b.zeros_m : log_a;
+        one.next_eps = (float)eps;
+        one.bias_ready = global_it > 0;
+        one.dependent = global_it > 0 && !tested;
+        two.chain_bias = !last;
+        two.next_logw = ott_convention ? b.zeros_n : log_b;
+        two.next_eps = (float)(it + 1 < iters_per_eps || last ? eps : eps_list[e + 1]);
+        two.bias_ready = two.dependent = true;
+        two.bump = &b.ctrl->iters_used;
+      }
       if (ott_convention) {
         // g first, log-marginals outside the LSE (sinkhorn_solvers.py:188-217)
         eg.addvec = log_b; eg.addcoef = (float)eps;
@@ -881,7 +900,7 @@ int fs_solve_alternating(const float* x, const float* y, int n, int m, int d, co
         FS_CUDA(p.lse(0, gh, log_b, (float)eps, ef));
         FS_CUDA(p.lse(1, fh, log_a, (float)eps, eg));
       }
-      bump_iters_kernel<<<1, 1, 0, st>>>(b.ctrl, early ? 1 : 0);
+      if (!chain) bump_iters_kernel<<<1, 1, 0, st>>>(b.ctrl, early ? 1 : 0);
       if (early && (global_it + 1) % check_every == 0) {
         delta_kernel<<<g1(n + m), 256, 0, st>>>(fh, b.pf, n, gh, b.pg, m, b.ctrl);
         decide_kernel<<<1, 1, 0, st>>>(b.ctrl, threshold);

@@ -76,6 +76,14 @@ struct LseEpilogue {
   float* out = nullptr;
   float* lse2 = nullptr;
   const Ctrl* ctrl = nullptr;
+  // Passes in a chain (tensor-core engine, operands resident): the epilogue stages the potential it writes as the column bias
+  // of the pass after it, whose rows are this one's columns; that pass then says bias_ready, and dependent where no other
+  // kernel is between the two. bump: counter of executed iterations, one more by this pass.
+  bool chain_bias = false;
+  const float* next_logw = nullptr;  // [nr]
+  float next_eps = 1.f;
+  bool bias_ready = false, dependent = false;
+  int* bump = nullptr;
 };
 
 // How the staged fp16 coordinates of a pair of clouds (0 = x, 1 = y) are scaled (fs_ptx.cuh, wide_range).

@@ -74,6 +74,10 @@ struct SubPass {
   // column-tile array (indexed with the values of csr_rp).
   const int* csr_rp;
   const int* csr_ci;
+  // LseEpilogue::chain_bias: the bias columns of the row cloud's column operand (null: not wanted)
+  float* next_bias;
+  int next_pitch;
+  float next_inv_eps, next_inv_scale2;
 };
 
 // A launch = up to NSUB passes over operands of the same shape class (same K blocks, tile shape and ring depth).
@@ -90,6 +94,15 @@ struct Launch {
   long long total;   // items of all passes (dense passes: sum of nblk * ntiles)
   SubPass sub[NSUB];
 };
+// The bias of a column (potential, log-weight) over the logit scale, times the scale of its products, as three TF32 pieces.
+__device__ __forceinline__ void write_column_bias(float* at, float pot, const float* logw, float inv_eps, float inv_scale2,
+                                                  float unit) {
+  // in log2 units, same association as the reference kernels
+  const float b2 = logw ? (pot * (inv_eps * kLog2e) + *logw * kLog2e) : pot * kLog2e;
+  const float b = b2 * inv_scale2 * unit;
+  const float hi = to_tf32(b), r1 = b - hi, mid = to_tf32(r1);
+  at[0] = hi; at[1] = mid; at[2] = to_tf32(r1 - mid);
+}
 constexpr int kMaxSub = 4;  // passes per multi-pass launch (keeps the kernel parameters under 4 KB)
 
 // Soft-max warpgroups per 128-row half of the plan-times-matrix kernel: each takes half of every tile's 32-column
@@ -138,6 +151,12 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
     if (cap < G) G = (int)cap;
   }
   const bool has_work = (int)blockIdx.x < G && total_items > 0;
+  if (MODE == MODE_LSE && NSUB == 1) {
+    // A pass in a chain starts while the last CTAs of the one before are still at work; what that one wrote is read below.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (p.ep.bump && blockIdx.x == 0 && tid == 0 && !(p.ep.ctrl && p.ep.ctrl->converged)) *p.ep.bump += 1;
+  }
   const int w_begin = has_work ? (int)((total_items * blockIdx.x) / G) : 0;
   const int w_end = has_work ? (int)((total_items * (blockIdx.x + 1)) / G) : 0;
   // Items of row block b are [row_start(b), row_end(b)); blk_of(w) = row block holding item w.
@@ -239,6 +258,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   if (warp == 0) {
     // ===================== TMA producer =====================
     if (lane == 0) {
+      asm volatile("fence.proxy.async;" ::: "memory");  // biases that the pass before wrote with ordinary stores
       int issued = 0, seg = 0;  // column tiles issued so far by this CTA (ring position), segment count
       bool ok = true;
       // Column tile `issued` (a CTA-wide running index) of the segment that starts at item w0.
@@ -531,6 +551,11 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
         if (ep.shift) o -= ep.shiftcoef * ep.shift[r];
         if (ep.addvec) o += ep.addcoef * ep.addvec[r];
         ep.out[r] = o;
+        if (MODE == MODE_LSE && NSUB == 1 && SP().next_bias) {
+          const float unit = bias_factor(SP().scales, WIDE && wide_range(SP().scales), SP().side, r);
+          write_column_bias(SP().next_bias + (size_t)r * SP().next_pitch, o, ep.next_logw + r, SP().next_inv_eps,
+                            SP().next_inv_scale2, unit);
+        }
       }
     };
     // A row block without any kept tile is visited by no item: its rows get the empty soft-min (log-sum of
@@ -1204,15 +1229,8 @@ __global__ void bias_kernel(float* __restrict__ opB, int rows, int kc, int kp, c
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= rows) return;
   const float pr = pot_shard > 0 ? pot[(size_t)(r / pot_shard) * pot_stride + r % pot_shard] : pot[r];
-  // bias in log2 units, same association as the reference kernels, then / scale2
-  float b2 = logw ? (pr * (inv_eps * kLog2e) + logw[r] * kLog2e) : pr * kLog2e;
-  float b = b2 * inv_scale2 * bias_factor(sc, wide_range(sc), cloud, r);
-  float hi = to_tf32(b);
-  float r1 = b - hi;
-  float mid = to_tf32(r1);
-  float lo = to_tf32(r1 - mid);
-  float* row = opB + (size_t)r * kp + kc;
-  row[0] = hi; row[1] = mid; row[2] = lo;
+  write_column_bias(opB + (size_t)r * kp + kc, pr, logw ? logw + r : nullptr, inv_eps, inv_scale2,
+                    bias_factor(sc, wide_range(sc), cloud, r));
 }
 
 // ------------------------------------------------------------------ host side
@@ -1291,13 +1309,26 @@ Shape plan_shape_csr(int d, int prec, int nlab) {
 }
 
 template <int NHALF, int BN, int MODE, bool CSR = false, int NSUB = 1>
-cudaError_t launch(const Launch<NSUB>& lp, dim3 grid, size_t smem, cudaStream_t st) {
+cudaError_t launch(const Launch<NSUB>& lp, dim3 grid, size_t smem, cudaStream_t st, bool chained = false) {
   auto kern = tc_lse_kernel<NHALF, BN, MODE, CSR, NSUB>;
   // Per device (context) attribute; cheap enough to set on every launch.
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   if (e != cudaSuccess) return e;
-  kern<<<grid, 128 + 128 * NHALF * lse_parts(NHALF, BN), smem, st>>>(lp);
-  return cudaGetLastError();
+  if (!chained) {
+    kern<<<grid, 128 + 128 * NHALF * lse_parts(NHALF, BN), smem, st>>>(lp);
+    return cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(128 + 128 * NHALF * lse_parts(NHALF, BN));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, lp);
 }
 
 // Bias columns of up to kMaxSub column operands in one launch (blockIdx.y = job).
@@ -1575,6 +1606,10 @@ bool fill_subpass(SubPass& kp, const Staged& s, int side, const StreamArgs& a, c
   kp.scale2 = scale2; kp.scales = s.scales; kp.side = side; kp.eps = a.eps; kp.ep = e;
   kp.part_m = s.part_m[side]; kp.part_s = s.part_s[side]; kp.part_stride = s.part_stride; kp.tickets = s.tickets[side];
   kp.out_idx = nullptr; kp.csr_rp = nullptr; kp.csr_ci = nullptr;
+  kp.next_bias = e.chain_bias ? rowc.opB + s.kc : nullptr;
+  kp.next_pitch = sh.kp;
+  kp.next_inv_eps = 1.0f / e.next_eps;
+  kp.next_inv_scale2 = 1.0f / ((2.0f * a.cost_scale) * (1.0f / e.next_eps) * kLog2e);
   return ok;
 }
 
@@ -1597,7 +1632,7 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   const float scale2 = am ? -2.0f * a.cost_scale : (2.0f * a.cost_scale) * (1.0f / a.eps) * kLog2e;
   if (am)
     detail::launch_bias(s, 1 - side, a.pot, nullptr, 1.0f, 1.0f / (scale2 * kLog2e), nullptr, st);
-  else
+  else if (!e.bias_ready)
     detail::launch_bias(s, 1 - side, a.pot, a.logw, 1.0f / a.eps, 1.0f / scale2, e.ctrl, st, a.pot_shard, a.pot_stride);
   Launch<1> lp{};
   lp.nsub = 1;
@@ -1610,16 +1645,22 @@ cudaError_t stream_pass(const Staged& s, int side, const StreamArgs& a, const Ls
   kp.csr_rp = csr ? a.tile_row_ptr + a.row_begin / 128 : nullptr;
   kp.csr_ci = a.tile_col_idx;
   dim3 grid(pick_ctas(kp.nblk, kp.ntiles));
-  if (csr) return launch<1, 128, MODE_LSE, true>(lp, grid, sh.smem, st);
+  const bool chained = e.dependent;
+  if (csr) return launch<1, 128, MODE_LSE, true>(lp, grid, sh.smem, st, chained);
   if (am) {
     if (sh.nhalf == 2) return launch<2, 128, MODE_MAX>(lp, grid, sh.smem, st);
     return launch<1, 128, MODE_MAX>(lp, grid, sh.smem, st);
   }
-  if (sh.nhalf == 2) return launch<2, 128, MODE_LSE>(lp, grid, sh.smem, st);
-  if (sh.bn == 128) return launch<1, 128, MODE_LSE>(lp, grid, sh.smem, st);
-  return launch<1, 64, MODE_LSE>(lp, grid, sh.smem, st);
+  if (sh.nhalf == 2) return launch<2, 128, MODE_LSE>(lp, grid, sh.smem, st, chained);
+  if (sh.bn == 128) return launch<1, 128, MODE_LSE>(lp, grid, sh.smem, st, chained);
+  return launch<1, 64, MODE_LSE>(lp, grid, sh.smem, st, chained);
 }
 }  // namespace
+
+bool chains(const Staged& s, bool tiles) {
+  const Shape sh = tiles ? plan_shape_csr(s.d, s.prec, s.nlab) : plan_shape(s.d, s.prec, s.nlab);
+  return sh.ok && !sh.streamed && !(sh.bn == 64 && !tiles && prefer_streamed());
+}
 
 cudaError_t lse(const Staged& s, int side, const StreamArgs& a, const LseEpilogue& e, cudaStream_t st) {
   return stream_pass(s, side, a, e, nullptr, st);

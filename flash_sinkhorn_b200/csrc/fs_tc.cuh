@@ -79,6 +79,8 @@ size_t staged_bytes(int n, int m, int d, int prec, int nlab = 0);
 cudaError_t stage(Staged& s, char* buf, const float* x, const float* y, int n, int m, int d, int prec,
                   cudaStream_t st, bool run_kernels = true, const LabelCost* lab = nullptr, float w_coef = 0.f);
 // One LSE pass: side 0 = rows of x against y, side 1 = rows of y against x.
+// Whether passes of these operands can stage the bias of the pass after them (LseEpilogue::chain_bias).
+bool chains(const Staged& s, bool tiles);
 cudaError_t lse(const Staged& s, int side, const StreamArgs& a, const LseEpilogue& e, cudaStream_t st);
 
 // Several dense LSE passes (of one or several staged problems with the same d, precision and label columns) as
