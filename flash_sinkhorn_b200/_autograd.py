@@ -13,6 +13,7 @@ Behaviour follows the reference's ``_autograd.py`` (``_SinkhornConfig`` :33-76,
 """
 from __future__ import annotations
 
+import ctypes
 from dataclasses import dataclass
 from typing import Optional, Tuple
 
@@ -137,8 +138,16 @@ def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
     prec = _lib.precision_id(cfg.allow_tf32)
     X, Y = (x32, a32, la, n), (y32, b32, lb, m)
 
+    waiting = []  # gradients of row clouds that share launches: (rows, columns, potential of the columns, scales, out)
+
     def term(k, u, v, scales, out_u, out_v):
         (pu, wu, lu, r), (pv, wv, lv, c) = u, v
+        if not meta.labels and all(_lib.load().fs_grad_many_bytes(p, q, d, prec) for p, q in ((r, c), (c, r))):
+            if out_u is not None:
+                waiting.append((u, v, pots[4 * k + 3], scales, out_u))
+            if out_v is not None:
+                waiting.append((v, u, pots[4 * k + 2], scales, out_v))
+            return
         f_pre, g_pre = pots[4 * k + 2], pots[4 * k + 3]
         label = meta.labels[k] if meta.labels else None
         ws = _lib.workspace(_lib.OP_GRAD, r, c, d, prec, dev, label.V if label else 0)
@@ -153,18 +162,49 @@ def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
     gx = torch.empty(x.shape, device=dev, dtype=torch.float32) if want_x else None
     gy = torch.empty(y.shape, device=dev, dtype=torch.float32) if want_y else None
     term(0, X, Y, gs, gx, gy)
+    added = []
     for k, side, out in ((1, X, gx), (2, Y, gy)):
         if not meta.debias or out is None:
             continue
         if pots[4 * k + 2].data_ptr() == pots[4 * k + 3].data_ptr():  # equal potentials: the two sides' gradients are equal
             own = torch.empty_like(out)
             term(k, side, side, -gs, own, None)
-            out += own
+            added.append((out, own))
         else:
             own, other = torch.empty_like(out), torch.empty_like(out)
             term(k, side, side, -0.5 * gs, own, other)
-            out += own + other
+            added += [(out, own), (out, other)]
+    _gradients_together(waiting, gs.numel(), d, meta.eps, float(cfg.cost_scale), prec, dev)
+    for out, own in added:
+        out += own
     return gx, gy
+
+
+# Scratch up to which gradients share launches. Beyond some tens of MB a launch fills the device by itself.
+SHARED_GRADIENT_BYTES = 1 << 27
+
+
+def _gradients_together(terms, B, d, eps, cost_scale, prec, dev):
+    """Runs the gradients of row clouds ``(rows, columns, column potential, scales, out)`` of B items each, 16 per call."""
+    lib = _lib.load()
+    items, sizes = [], []
+    for (pu, wu, _, r), (pv, _, lv, c), pot, scales, out in terms:
+        base = [_lib.ptr(t) for t in (pu, pv, wu, lv, pot, scales, out)]
+        pitch = [4 * q for q in (r * d, c * d, r, c, c, 1, r * d)]
+        nbytes = int(lib.fs_grad_many_bytes(r, c, d, prec))
+        for i in range(B):
+            x, y, weight, log_w, at_pot, scale, at_out = (p + i * q for p, q in zip(base, pitch))
+            items.append((x, y, r, c, weight, log_w, at_pot, scale, at_out))
+            sizes.append(nbytes)
+    while items:
+        k = 1
+        while k < min(len(items), 16) and sum(sizes[: k + 1]) <= SHARED_GRADIENT_BYTES:
+            k += 1
+        ws = torch.empty(sum(sizes[:k]), dtype=torch.uint8, device=dev)
+        arr = (_lib.GradItem * k)(*items[:k])
+        _lib.call("fs_grad_many", dev, ctypes.cast(arr, ctypes.c_void_p), k, d, float(eps), cost_scale, prec, _lib.ptr(ws),
+                  ws.numel(), _lib.stream_ptr(dev))
+        items, sizes = items[k:], sizes[k:]
 
 
 class _SinkhornLossGradFn(torch.autograd.Function):

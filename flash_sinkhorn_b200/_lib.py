@@ -87,6 +87,8 @@ SIGNATURES = {
     "fs_symmetric_step_multi": (c_int, [_P, c_int, c_int, c_int, _P]),
     "fs_solve_symmetric_batched": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P]),
     "fs_solve_symmetric_batched_labels": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P, _P]),
+    "fs_grad_many_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "fs_grad_many": (c_int, [_P, c_int, c_int, c_float, c_float, c_int, _P, c_size_t, _P]),
     "fs_grad_range": (
         c_int,
         [_P, _P, c_int, c_int, c_int, _P, _P, _P, _P, _P, _P, _P, _P, _P, c_float, c_float,
@@ -303,6 +305,13 @@ class BatchItem(ctypes.Structure):
     _fields_ = [("x", c_void_p), ("y", c_void_p), ("n", c_int), ("m", c_int), ("log_a", c_void_p), ("log_b", c_void_p),
                 ("eps_list_host", c_void_p), ("n_eps", c_int), ("f", c_void_p), ("g", c_void_p),
                 ("f_pre", c_void_p), ("g_pre", c_void_p), ("ws", c_void_p), ("ws_bytes", c_size_t)]
+
+
+class GradItem(ctypes.Structure):
+    """``fs_grad_item`` of the C header (gradient of the row cloud of one problem)."""
+
+    _fields_ = [("x", c_void_p), ("y", c_void_p), ("n", c_int), ("m", c_int), ("weight", c_void_p), ("log_w", c_void_p),
+                ("pot", c_void_p), ("scale", c_void_p), ("out", c_void_p)]
 
 
 def stream_ptr(device: torch.device) -> int:

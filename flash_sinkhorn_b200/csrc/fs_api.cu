@@ -1024,6 +1024,29 @@ int fs_grad(const float* x, const float* y, int n, int m, int d, const float* a,
   return FS_OK;
 }
 
+size_t fs_grad_many_bytes(int n, int m, int d, int prec) { return prec == FS_PREC_SIMT ? 0 : tc::grad_many_bytes(n, m, d, prec); }
+
+int fs_grad_many(const fs_grad_item* items, int n_items, int d, float eps, float cost_scale, int prec, void* wsp, size_t ws_bytes,
+                 void* stream) {
+  if (!items || n_items <= 0 || n_items > 16) return fail(FS_ERR_BAD_ARG, "fs_grad_many takes 1..16 items");
+  tc::GradJob jobs[16];
+  size_t need = 0;
+  for (int i = 0; i < n_items; ++i) {
+    const fs_grad_item& in = items[i];
+    FS_TRY(check_common(in.x, in.y, in.n, in.m, d, eps, cost_scale, prec));
+    if (!in.weight || !in.log_w || !in.pot || !in.out) return fail(FS_ERR_BAD_ARG, "item %d: null argument", i);
+    const size_t one = fs_grad_many_bytes(in.n, in.m, d, prec);
+    if (one == 0) return fail(FS_ERR_UNSUPPORTED, "item %d: sizes that gradients do not share launches at", i);
+    need += one;
+    jobs[i] = tc::GradJob{in.x, in.y, in.n, in.m, in.pot, in.log_w, in.weight, in.scale, in.out};
+  }
+  if (!wsp || ws_bytes < need) return fail(FS_ERR_WORKSPACE, "workspace too small: need %zu bytes", need);
+  FS_TRY(check_device());
+  g_launches.fetch_add(4, std::memory_order_relaxed);
+  FS_CUDA(tc::grad_many(jobs, n_items, d, prec, cost_scale, eps, static_cast<char*>(wsp), static_cast<cudaStream_t>(stream)));
+  return FS_OK;
+}
+
 int fs_mat5(const float* x, const float* y, int n, int m, int d, const float* f_ott, const float* g_ott,
             const float* A, float* out, float eps, float cost_scale, int prec, void* wsp, size_t ws_bytes,
             void* stream) {

@@ -103,6 +103,7 @@ __device__ __forceinline__ void write_column_bias(float* at, float pot, const fl
   const float hi = to_tf32(b), r1 = b - hi, mid = to_tf32(r1);
   at[0] = hi; at[1] = mid; at[2] = to_tf32(r1 - mid);
 }
+constexpr int kMaxGrads = 16;  // problems of a launch of gradients (grad_many)
 constexpr int kMaxSub = 4;  // passes per multi-pass launch (keeps the kernel parameters under 4 KB)
 
 // Soft-max warpgroups per 128-row half of the plan-times-matrix kernel: each takes half of every tile's 32-column
@@ -762,15 +763,25 @@ struct PvKernelParams {
 
 constexpr int kNSW = 3;  // S/W buffers of the plan-times-matrix kernel
 
+// A launch of several passes: CTAs [cta0, the next one's cta0) each.
+struct PvJob {
+  CUtensorMap mapA_full, mapA_tail, mapB_full, mapB_tail, mapV_hi, mapV_lo;
+  PvKernelParams p;
+  int cta0;
+};
+struct PvLaunch {
+  int njobs;
+  PvJob job[kMaxGrads];
+};
+
 template <int BN, bool SPLIT>
-__global__ void __launch_bounds__(128 + 128 * kParts, 1)
-tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constant__ CUtensorMap mapA_tail,
-             const __grid_constant__ CUtensorMap mapB_full, const __grid_constant__ CUtensorMap mapB_tail,
-             const __grid_constant__ CUtensorMap mapV_hi, const __grid_constant__ CUtensorMap mapV_lo,
-             const PvKernelParams p) {
+__device__ __forceinline__ void pv_pass(const CUtensorMap& mapA_full, const CUtensorMap& mapA_tail,
+                                        const CUtensorMap& mapB_full, const CUtensorMap& mapB_tail,
+                                        const CUtensorMap& mapV_hi, const CUtensorMap& mapV_lo, const PvKernelParams& p,
+                                        int cta) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int blk = (int)blockIdx.x / p.nsplit, share = (int)blockIdx.x % p.nsplit;
+  const int blk = cta / p.nsplit, share = cta % p.nsplit;
   const int row0 = p.row_begin + blk * 128;
   if (p.skip && *p.skip) return;  // uniform across the grid (set by an earlier kernel of the stream)
   constexpr int WCOLS = SPLIT ? 2 * BN : BN;  // TMEM columns per S/W buffer (Wl lives right after Wh)
@@ -1138,6 +1149,23 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
     tmem_dealloc(tmem_base, kTmemCols);
   }
   if (tid == 0 && *abort_flag) atomicExch(&g_tc_error, 1);
+}
+
+template <int BN, bool SPLIT>
+__global__ void __launch_bounds__(128 + 128 * kParts, 1)
+tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constant__ CUtensorMap mapA_tail,
+             const __grid_constant__ CUtensorMap mapB_full, const __grid_constant__ CUtensorMap mapB_tail,
+             const __grid_constant__ CUtensorMap mapV_hi, const __grid_constant__ CUtensorMap mapV_lo,
+             const PvKernelParams p) {
+  pv_pass<BN, SPLIT>(mapA_full, mapA_tail, mapB_full, mapB_tail, mapV_hi, mapV_lo, p, (int)blockIdx.x);
+}
+// (A kernel of its own: with its parameters found by the number of the pass the single one was 6 % slower.)
+template <int BN, bool SPLIT>
+__global__ void __launch_bounds__(128 + 128 * kParts, 1) tc_pv_many_kernel(const __grid_constant__ PvLaunch P) {
+  int nth = 0;
+  while (nth + 1 < P.njobs && P.job[nth + 1].cta0 <= (int)blockIdx.x) ++nth;
+  const PvJob& J = P.job[nth];
+  pv_pass<BN, SPLIT>(J.mapA_full, J.mapA_tail, J.mapB_full, J.mapB_tail, J.mapV_hi, J.mapV_lo, J.p, (int)blockIdx.x - J.cta0);
 }
 
 // V^T staging: vt[c][j] = tf32(V[j][c] * colscale_j) (hi) and the tf32 residual (lo), zero padded
@@ -1798,12 +1826,47 @@ PvShape plan_pv(int d, int prec, int dv, int nlab = 0) {
 }
 
 template <int BN, bool SPLIT>
-cudaError_t launch_pv(const CUtensorMap* maps, const PvKernelParams& kp, int grid, size_t smem, cudaStream_t st) {
+cudaError_t launch_pv(const PvJob& j, int grid, size_t smem, cudaStream_t st) {
   auto kern = tc_pv_kernel<BN, SPLIT>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   if (e != cudaSuccess) return e;
-  kern<<<grid, 128 + 128 * kParts, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[4], maps[5], kp);
+  kern<<<grid, 128 + 128 * kParts, smem, st>>>(j.mapA_full, j.mapA_tail, j.mapB_full, j.mapB_tail, j.mapV_hi, j.mapV_lo, j.p);
   return cudaGetLastError();
+}
+template <int BN, bool SPLIT>
+cudaError_t launch_pv_many(const PvLaunch& lp, int grid, size_t smem, cudaStream_t st) {
+  auto kern = tc_pv_many_kernel<BN, SPLIT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+  if (e != cudaSuccess) return e;
+  kern<<<grid, 128 + 128 * kParts, smem, st>>>(lp);
+  return cudaGetLastError();
+}
+// Maps and geometry of one pass; V^T at vt_hi, vt_lo [vrows, cols_pad].
+bool fill_pv(PvJob& J, const Staged& s, int side, const StreamArgs& a, const PvArgs& pa, const Shape& sh, const PvShape& ps,
+             const float* vt_hi, const float* vt_lo, float scale2) {
+  const CloudOps& rowc = s.cloud[side == 0 ? 0 : 1];
+  const CloudOps& colc = s.cloud[side == 0 ? 1 : 0];
+  const int vrows = ps.nslices * ps.dv_pad, vcols = colc.rows_pad;
+  const CUtensorMapSwizzle full = sh.nfull ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B;
+  bool ok = true;
+  ok &= encode_map(&J.mapA_full, rowc.opA, rowc.rows_pad, sh.kp, sh.nfull ? 32 : 8, 128, full);
+  ok &= encode_map(&J.mapA_tail, rowc.opA, rowc.rows_pad, sh.kp, 8, 128, CU_TENSOR_MAP_SWIZZLE_32B);
+  ok &= encode_map(&J.mapB_full, colc.opB, colc.rows_pad, sh.kp, sh.nfull ? 32 : 8, ps.bn, full);
+  ok &= encode_map(&J.mapB_tail, colc.opB, colc.rows_pad, sh.kp, 8, ps.bn, CU_TENSOR_MAP_SWIZZLE_32B);
+  ok &= encode_map(&J.mapV_hi, vt_hi, vrows, vcols, 32, ps.dv_pad, CU_TENSOR_MAP_SWIZZLE_128B);
+  ok &= encode_map(&J.mapV_lo, ps.split ? vt_lo : vt_hi, vrows, vcols, 32, ps.dv_pad, CU_TENSOR_MAP_SWIZZLE_128B);
+  PvKernelParams& kp = J.p;
+  kp.nr = a.nr; kp.nc = a.nc; kp.row_begin = a.row_begin;
+  kp.ntiles = (a.nc + ps.bn - 1) / ps.bn;
+  kp.hs = sh.lay.hs; kp.scales = s.scales; kp.side = side;
+  kp.nfull = sh.nfull; kp.ntail = sh.ntail; kp.nb = ps.nb; kp.nv = ps.nv;
+  kp.dv = pa.dv; kp.dv_pad = ps.dv_pad; kp.dv0 = 0; kp.ld_out = pa.dv;
+  kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;
+  kp.rowpot = pa.rowpot; kp.rowlogw = pa.rowlogw; kp.roww = pa.roww; kp.gs = pa.gs; kp.coef = pa.coef;
+  kp.rows_raw = a.rows; kp.ld_rows = a.d; kp.out = pa.out; kp.skip = pa.skip;
+  kp.tickets = s.tickets[side];
+  J.cta0 = 0;
+  return ok;
 }
 
 }  // namespace
@@ -1889,26 +1952,9 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   size_t total = (size_t)vrows * vcols;
   stage_vt_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(pa.V, a.nc, pa.dv, pa.colscale, vrows, vcols,
                                                                    vt_hi, vt_lo);
-  CUtensorMap maps[6];
-  bool ok = true;
-  ok &= encode_map(&maps[0], rowc.opA, rowc.rows_pad, sh.kp, sh.nfull ? 32 : 8, 128,
-                   sh.nfull ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
-  ok &= encode_map(&maps[1], rowc.opA, rowc.rows_pad, sh.kp, 8, 128, CU_TENSOR_MAP_SWIZZLE_32B);
-  ok &= encode_map(&maps[2], colc.opB, colc.rows_pad, sh.kp, sh.nfull ? 32 : 8, ps.bn,
-                   sh.nfull ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_32B);
-  ok &= encode_map(&maps[3], colc.opB, colc.rows_pad, sh.kp, 8, ps.bn, CU_TENSOR_MAP_SWIZZLE_32B);
-  ok &= encode_map(&maps[4], vt_hi, vrows, vcols, 32, ps.dv_pad, CU_TENSOR_MAP_SWIZZLE_128B);
-  ok &= encode_map(&maps[5], ps.split ? vt_lo : vt_hi, vrows, vcols, 32, ps.dv_pad, CU_TENSOR_MAP_SWIZZLE_128B);
-  if (!ok) return cudaErrorInvalidValue;
-  PvKernelParams kp;
-  kp.nr = a.nr; kp.nc = a.nc; kp.row_begin = a.row_begin;
-  kp.ntiles = (a.nc + ps.bn - 1) / ps.bn;
-  kp.hs = sh.lay.hs; kp.scales = s.scales; kp.side = side;
-  kp.nfull = sh.nfull; kp.ntail = sh.ntail; kp.nb = ps.nb; kp.nv = ps.nv;
-  kp.dv = pa.dv; kp.dv_pad = ps.dv_pad; kp.ld_out = pa.dv;
-  kp.scale2 = scale2; kp.eps = a.eps; kp.R = pa.R; kp.epilogue = pa.epilogue;
-  kp.rowpot = pa.rowpot; kp.rowlogw = pa.rowlogw; kp.roww = pa.roww; kp.gs = pa.gs; kp.coef = pa.coef;
-  kp.rows_raw = a.rows; kp.ld_rows = a.d; kp.out = pa.out; kp.skip = pa.skip;
+  PvJob job;
+  if (!fill_pv(job, s, side, a, pa, sh, ps, vt_hi, vt_lo, scale2)) return cudaErrorInvalidValue;
+  PvKernelParams& kp = job.p;
   const int nblk = (a.nr - a.row_begin + 127) / 128;
   if (nblk <= 0) return cudaSuccess;
   // Column shares per row block: as many as fill the SMs best, within the share slots the scratch was sized for.
@@ -1916,15 +1962,213 @@ cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& pa,
   kp.nsplit = pick_pv_split(nblk, kp.ntiles, pv_share_slots(nm, ps.bn),
                             detail::sm_count() - g_reserved_sms.load(std::memory_order_relaxed));
   kp.partial = reinterpret_cast<float*>(p + (ps.split ? 2 : 1) * one);
-  kp.tickets = s.tickets[side];
   const int grid = nblk * kp.nsplit;
   for (int sl = 0; sl < ps.nslices; ++sl) {
     kp.dv0 = sl * ps.dv_pad;
-    cudaError_t e = ps.split ? launch_pv<64, true>(maps, kp, grid, ps.smem, st)
-                             : launch_pv<128, false>(maps, kp, grid, ps.smem, st);
+    cudaError_t e = ps.split ? launch_pv<64, true>(job, grid, ps.smem, st) : launch_pv<128, false>(job, grid, ps.smem, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// ---- gradients of several problems in shared launches ----
+namespace {
+
+struct GradCloud {
+  const float* src;
+  int rows, rows_pad;
+  float* op;         // row role (cloud 0) or column role (cloud 1)
+  const float* pot;  // of the columns
+  const float* logw;
+  float* vt_hi;      // of the columns, transposed
+  float* vt_lo;
+};
+struct GradStage {
+  struct Job {
+    GradCloud cloud[2];
+    OperandScales scales;
+  } job[kMaxGrads];
+  int d, prec, dv_pad;
+  Layout lay;
+  float cs, inv_eps, inv_scale2;
+};
+__global__ void __launch_bounds__(256) grad_range_kernel(const __grid_constant__ GradStage P) {
+  const GradStage::Job& j = P.job[blockIdx.y];
+  const GradCloud& c = j.cloud[blockIdx.z];
+  row_ranges(c.src, c.rows, c.rows_pad, P.d, blockIdx.x, gridDim.x, const_cast<float*>(j.scales.inv[blockIdx.z]),
+             const_cast<unsigned*>(j.scales.range), blockIdx.z, 2 * gridDim.x, scale_octaves(P.prec));
+}
+// One warp per point: its operand row in the one role that the gradient of the rows needs, and for columns the bias
+// (potential less the squared norm, log-weight) and the column of V^T. One launch where a pass on its own takes five.
+__global__ void __launch_bounds__(256) grad_stage_kernel(const __grid_constant__ GradStage P) {
+  const GradStage::Job& j = P.job[blockIdx.y];
+  const int cloud = blockIdx.z, lane = threadIdx.x & 31;
+  const GradCloud& c = j.cloud[cloud];
+  const int r = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5);
+  if (r >= c.rows_pad) return;
+  const bool real = r < c.rows, wide = wide_range(j.scales);
+  const int d = P.d, kc = P.lay.kc, kp = P.lay.kp;
+  const float own = coord_factor(j.scales, wide, cloud, r);
+  const float* src = c.src + (size_t)r * d;
+  float* row = c.op + (size_t)r * kp;
+  for (int k = lane; k < kp; k += 32) {
+    if (cloud == 1 && k >= kc && k < kc + 3) continue;
+    float va = 0.f, vb = 0.f;
+    if (k < P.lay.kcoord && real) stage_coord(src, k, d, P.prec == 0 ? 1 : 3, P.lay.hs, own, va, vb);
+    if (k >= kc && k < kc + 3) va = ones_factor(j.scales, wide, cloud, r);
+    row[k] = cloud == 0 ? va : vb;
+  }
+  if (cloud == 0) return;
+  float nrm = 0.f;
+  if (real)
+    for (int k = lane; k < d; k += 32) { const float v = src[k]; nrm = fmaf(v, v, nrm); }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
+  for (int k = lane; k < P.dv_pad; k += 32) {
+    const float v = real && k < d ? src[k] : 0.f, hi = to_tf32(v);
+    c.vt_hi[(size_t)k * c.rows_pad + r] = hi;
+    if (c.vt_lo) c.vt_lo[(size_t)k * c.rows_pad + r] = to_tf32(v - hi);
+  }
+  if (lane == 0) {
+    if (real) {
+      write_column_bias(row + kc, c.pot[r] - P.cs * nrm, c.logw + r, P.inv_eps, P.inv_scale2, bias_factor(j.scales, wide, 1, r));
+    } else {
+      row[kc] = kMaskBias; row[kc + 1] = 0.f; row[kc + 2] = 0.f;
+    }
+  }
+}
+
+// Where the scratch of one job lies behind the control words of all of them.
+struct GradScratch {
+  size_t off = 0;
+  char* base = nullptr;
+  template <typename T>
+  T* take(size_t count) {
+    const size_t o = off;
+    off += (count * sizeof(T) + 1023) & ~size_t(1023);
+    return base ? reinterpret_cast<T*>(base + o) : nullptr;
+  }
+};
+constexpr size_t kGradControl = 64;  // bytes of range words per job
+int grad_tickets(int n, int m) { return detail::pad256(n > m ? n : m) / 128; }
+
+void carve_grad(GradScratch& c, Staged& s, GradCloud* cloud, float** R, float** partial, int n, int m, int d, int prec) {
+  const Shape sh = plan_shape(d, prec, 0);
+  const PvShape ps = plan_pv(d, prec, d, 0);
+  const int rows[2] = {n, m};
+  for (int k = 0; k < 2; ++k) {
+    s.cloud[k].rows = rows[k];
+    s.cloud[k].rows_pad = detail::pad256(rows[k]);
+    cloud[k].rows = rows[k];
+    cloud[k].rows_pad = s.cloud[k].rows_pad;
+    cloud[k].op = c.take<float>((size_t)s.cloud[k].rows_pad * sh.kp);
+    s.scales.inv[k] = c.take<float>(s.cloud[k].rows_pad);
+  }
+  s.cloud[0].opA = cloud[0].op;
+  s.cloud[1].opB = cloud[1].op;
+  s.part_stride = s.cloud[0].rows_pad;
+  s.part_m[0] = c.take<float>((size_t)kMaxChunks * s.part_stride);
+  s.part_s[0] = c.take<float>((size_t)kMaxChunks * s.part_stride);
+  *R = c.take<float>(s.cloud[0].rows_pad);
+  cloud[1].vt_hi = c.take<float>((size_t)ps.dv_pad * s.cloud[1].rows_pad);
+  cloud[1].vt_lo = ps.split ? c.take<float>((size_t)ps.dv_pad * s.cloud[1].rows_pad) : nullptr;
+  *partial = c.take<float>((size_t)pv_share_slots(n > m ? n : m, ps.bn) * 128 * ps.dv_pad);
+}
+}  // namespace
+
+size_t grad_many_bytes(int n, int m, int d, int prec) {
+  if (n <= 0 || m <= 0 || d <= 0 || !supported(n, m, d, prec, 0)) return 0;
+  const Shape sh = plan_shape(d, prec, 0);
+  const PvShape ps = plan_pv(d, prec, d, 0);
+  if (!sh.ok || sh.streamed || sh.bn != 128 || !ps.ok || ps.nslices != 1) return 0;
+  GradScratch c;
+  Staged s;
+  GradCloud cloud[2];
+  float *R, *partial;
+  carve_grad(c, s, cloud, &R, &partial, n, m, d, prec);
+  return c.off + kGradControl + (size_t)grad_tickets(n, m) * sizeof(int) + 3072;
+}
+
+cudaError_t grad_many(const GradJob* jobs, int cnt, int d, int prec, float cs, float eps, char* scratch, cudaStream_t st) {
+  if (cnt < 1 || cnt > kMaxGrads || !scratch) return cudaErrorInvalidValue;
+  const Shape sh = plan_shape(d, prec, 0);
+  const PvShape ps = plan_pv(d, prec, d, 0);
+  if (!sh.ok || sh.streamed || sh.bn != 128 || !ps.ok || ps.nslices != 1) return cudaErrorNotSupported;
+  GradScratch c;
+  c.base = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
+  char* control = c.take<char>(kGradControl * cnt);
+  size_t tickets = 0;
+  for (int i = 0; i < cnt; ++i) tickets += grad_tickets(jobs[i].n, jobs[i].m);
+  int* ticket = c.take<int>(tickets);
+  cudaError_t e = cudaMemsetAsync(control, 0, c.off, st);  // range words and tickets
+  if (e != cudaSuccess) return e;
+  const float scale2 = (2.0f * cs) * (1.0f / eps) * kLog2e;
+  GradStage stage;
+  Launch<kMaxGrads> lp{};
+  PvLaunch pv;
+  stage.d = d; stage.prec = prec; stage.dv_pad = ps.dv_pad; stage.lay = sh.lay;
+  stage.cs = cs; stage.inv_eps = 1.0f / eps; stage.inv_scale2 = 1.0f / scale2;
+  lp.nsub = pv.njobs = cnt;
+  lp.nfull = sh.nfull; lp.ntail = sh.ntail; lp.nstage = sh.nstage; lp.hs = sh.lay.hs;
+  long long total = 0, nblk = 0;
+  int pad = 0, max_tiles = 1, min_tiles = 1 << 30, slots_ok = 8;
+  Staged s[kMaxGrads];
+  float* partial[kMaxGrads];
+  for (int i = 0; i < cnt; ++i) {
+    const GradJob& g = jobs[i];
+    s[i].d = d; s[i].prec = prec; s[i].kc = sh.kc; s[i].kp = sh.kp; s[i].hs = sh.lay.hs;
+    GradCloud* cloud = stage.job[i].cloud;
+    float* R;
+    carve_grad(c, s[i], cloud, &R, &partial[i], g.n, g.m, d, prec);
+    s[i].tickets[0] = ticket;
+    ticket += grad_tickets(g.n, g.m);
+    cloud[0].src = g.x; cloud[1].src = g.y; cloud[1].pot = g.pot; cloud[1].logw = g.logw;
+    if (sh.lay.hs)
+      s[i].scales.range = reinterpret_cast<unsigned*>(control + kGradControl * i);
+    else
+      s[i].scales = OperandScales();
+    stage.job[i].scales = s[i].scales;
+    StreamArgs a;
+    a.rows = g.x; a.cols = g.y; a.nr = g.n; a.nc = g.m; a.d = d; a.eps = eps; a.cost_scale = cs;
+    LseEpilogue ep;
+    ep.lse2 = R;
+    if (!fill_subpass(lp.sub[i], s[i], 0, a, ep, sh, scale2)) return cudaErrorInvalidValue;
+    lp.sub[i].item0 = (int)total;
+    total += (long long)lp.sub[i].nblk * lp.sub[i].ntiles;
+    if (total >= (1ll << 31)) return cudaErrorNotSupported;
+    PvArgs pa;
+    pa.R = R; pa.V = g.y; pa.dv = d; pa.epilogue = PV_GRAD; pa.roww = g.weight; pa.gs = g.scale;
+    pa.coef = 2.f * cs; pa.out = g.out;
+    if (!fill_pv(pv.job[i], s[i], 0, a, pa, sh, ps, cloud[1].vt_hi, cloud[1].vt_lo, scale2)) return cudaErrorInvalidValue;
+    const int blocks = (g.n + 127) / 128, slots = pv_share_slots(g.n > g.m ? g.n : g.m, ps.bn);
+    nblk += blocks;
+    while (slots_ok > 1 && (long long)blocks * slots_ok > slots) --slots_ok;
+    min_tiles = pv.job[i].p.ntiles < min_tiles ? pv.job[i].p.ntiles : min_tiles;
+    max_tiles = lp.sub[i].ntiles > max_tiles ? lp.sub[i].ntiles : max_tiles;
+    for (int k = 0; k < 2; ++k) pad = cloud[k].rows_pad > pad ? cloud[k].rows_pad : pad;
+  }
+  lp.total = total;
+  if (sh.lay.hs) grad_range_kernel<<<dim3(detail::range_blocks(pad, d), cnt, 2), 256, 0, st>>>(stage);
+  grad_stage_kernel<<<dim3(pad / 8, cnt, 2), 256, 0, st>>>(stage);
+  // CTAs of the soft-min as in lse_multi
+  long long g = detail::free_ctas();
+  if (g > (total + 3) / 4) g = (total + 3) / 4;
+  if (g < 1) g = 1;
+  while (g > 1 && (long long)max_tiles * g / total + 2 > kMaxChunks) --g;
+  e = sh.nhalf == 2 ? launch<2, 128, MODE_LSE, false, kMaxGrads>(lp, dim3((unsigned)g), sh.smem, st)
+                    : launch<1, 128, MODE_LSE, false, kMaxGrads>(lp, dim3((unsigned)g), sh.smem, st);
+  if (e != cudaSuccess) return e;
+  // one count of column shares for all: the one that fills the SMs best with the row blocks of all of them
+  const int split = pick_pv_split((int)nblk, min_tiles, (int)nblk * slots_ok,
+                                  detail::sm_count() - g_reserved_sms.load(std::memory_order_relaxed));
+  int grid = 0;
+  for (int i = 0; i < cnt; ++i) {
+    pv.job[i].p.nsplit = split;
+    pv.job[i].p.partial = partial[i];
+    pv.job[i].cta0 = grid;
+    grid += (jobs[i].n + 127) / 128 * split;
+  }
+  return ps.split ? launch_pv_many<64, true>(pv, grid, ps.smem, st) : launch_pv_many<128, false>(pv, grid, ps.smem, st);
 }
 
 // ---- micro-benchmark: cycles per tcgen05.mma as issued by one lane ----

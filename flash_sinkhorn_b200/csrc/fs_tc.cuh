@@ -110,6 +110,20 @@ bool pv_supported(int d, int prec, int dv, int nlab = 0);
 size_t pv_scratch_bytes(int nc, int d, int prec, int dv, int nlab = 0);
 cudaError_t pv(const Staged& s, int side, const StreamArgs& a, const PvArgs& p, char* scratch, cudaStream_t st);
 
+// Gradient of the row cloud of one problem: out_i = 2 cs scale weight_i (x_i - barycentre of y under the soft-min of row i).
+struct GradJob {
+  const float *x, *y;
+  int n, m;
+  const float *pot, *logw;  // of the columns (potential in the standard convention)
+  const float* weight;      // of the rows
+  const float* scale;       // device scalar or null
+  float* out;
+};
+// Scratch that one job adds (0: sizes that go through lse() and pv() one by one).
+size_t grad_many_bytes(int n, int m, int d, int prec);
+// Up to 16 of them, of one dimension, in four launches.
+cudaError_t grad_many(const GradJob* jobs, int cnt, int d, int prec, float cs, float eps, char* scratch, cudaStream_t st);
+
 // ---- K-streamed passes (fs_tck.cu) --------------------------------------------------------------------
 // When the K-padded 128-row operand does not fit in shared memory (large d, or moderate d in the 3xTF32
 // mode) both operands stream through shared memory in 32-float K chunks and the score tile accumulates in

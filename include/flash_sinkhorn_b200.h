@@ -400,6 +400,21 @@ int fs_grad(const float* x, const float* y, int n, int m, int d,
             int prec, void* ws, size_t ws_bytes, void* stream,
             const fs_label_cost* labels);
 
+/* Gradients of the row clouds of 1..16 problems of one dimension in four launches (no reference counterpart):
+ *   out_i = 2 cs scale weight_i (x_i - sum_j w_ij y_j / sum_j w_ij), w_ij = exp((pot_j - C_ij)/eps + log_w_j),
+ * what fs_grad writes to grad_x with g = pot, a = weight, log_b = log_w. ws: the sum of fs_grad_many_bytes over the items
+ * (0 bytes: sizes that go through fs_grad). */
+typedef struct fs_grad_item {
+  const float* x; const float* y; int n, m;
+  const float* weight;                     /* [n] */
+  const float* log_w; const float* pot;    /* [m] */
+  const float* scale;                      /* device scalar or NULL */
+  float* out;                              /* [n, d] */
+} fs_grad_item;
+size_t fs_grad_many_bytes(int n, int m, int d, int prec);
+int fs_grad_many(const fs_grad_item* items, int n_items, int d, float eps, float cost_scale, int prec, void* ws,
+                 size_t ws_bytes, void* stream);
+
 /* out_i = (-4cs/eps) sum_j P_ij (A_i.y_j) y_j with P_ij = exp((f_i+g_j-C_ij)/eps)
  * (OTT-convention potentials, log-weights already inside f, g). Replaces
  * kernels/apply_ott.py:453-566 (mat5_sqeuclid). */

@@ -119,3 +119,35 @@ def test_labels_in_lockstep(n, m, V):
     val = SamplesLoss("sinkhorn", **kw)(a, xs, b, y, label_x=labels, label_y=ly)
     labels.fill_(1 << 20)
     assert _err(torch.autograd.grad(val, xs)[0], outs[1][1][1]) < 3e-4
+
+
+@pytest.mark.parametrize("mode", ["fp32", "tf32"])
+@pytest.mark.parametrize("B,n,m,d", [(9, 300, 200, 12), (17, 40, 50, 64), (1, 2300, 4100, 64), (2, 1, 1, 2), (3, 129, 257, 100),
+                                     (1, 700, 300, 128)])
+def test_gradients_that_share_launches(monkeypatch, mode, B, n, m, d):
+    """Against the same gradients one by one (more items than a call takes, column shares, one point, plans of one and two
+    128-row halves, one item with a far point). Same products and normalisers; sums in another order: 2e-5 of the
+    gradient's size in the exact mode, of TF32 weights up to 2^-11."""
+    from flash_sinkhorn_b200 import _autograd, _lib
+    monkeypatch.setenv("FLASH_SINKHORN_B200_PREC", mode)
+    lib = _lib.load()
+    prec = _lib.precision_id(True)
+    if not lib.fs_grad_many_bytes(n, m, d, prec):
+        pytest.skip("streamed operands")
+    x, y, a, b = _inputs(B, n, m, d, seed=11)
+    if B == 3:
+        x[1, 0] *= 1e9
+    la, lb, pot = a.log(), b.log(), torch.randn(B, m, device="cuda")
+    scales = torch.linspace(0.5, 2.0, B, device="cuda")
+    out, want = torch.empty_like(x), torch.empty_like(x)
+    _autograd._gradients_together([((x, a, la, n), (y, b, lb, m), pot, scales, out)], B, d, 0.3 * d, 0.5, prec, x.device)
+    ws = _lib.workspace(_lib.OP_GRAD, n, m, d, prec, x.device)
+    f = torch.zeros(n, device="cuda")
+    for i in range(B):
+        _lib.call("fs_grad", x.device, _lib.ptr(x[i]), _lib.ptr(y[i]), n, m, d, _lib.ptr(a[i]), _lib.ptr(b[i]), _lib.ptr(la[i]),
+                  _lib.ptr(lb[i]), _lib.ptr(f), _lib.ptr(pot[i]), _lib.ptr(scales[i]), _lib.ptr(want[i]), None, 0.3 * d, 0.5, prec,
+                  _lib.ptr(ws), ws.numel(), _lib.stream_ptr(x.device), None)
+    keep = x.abs().amax(dim=-1) < 1e6
+    assert _err(out[keep], want[keep]) < (2e-5 if mode == "fp32" else 5e-4)
+    assert _err(out[~keep], want[~keep]) < 1e-3 or bool(keep.all())
+    assert lib.fs_device_error() == 0
