@@ -86,7 +86,7 @@ SIGNATURES = {
     ),
     "fs_symmetric_step_multi": (c_int, [_P, c_int, c_int, c_int, _P]),
     "fs_solve_symmetric_batched": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P]),
-    "fs_solve_symmetric_batched_labels": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P, _P]),
+    "fs_solve_symmetric_batched_labels": (c_int, [_P, c_int, c_int, c_int, c_float, c_double, c_double, c_int, _P, _P, c_int]),
     "fs_grad_many_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "fs_grad_many": (c_int, [_P, c_int, c_int, c_float, c_float, c_int, _P, c_size_t, _P]),
     "fs_grad_range": (
@@ -245,8 +245,9 @@ class LabelCost:
     ``LabelCost.make`` returns None when the label cost is inactive (any of the four inputs missing, or
     ``lambda_y == 0``), exactly the reference's ``use_label_cost`` condition."""
 
-    def __init__(self, label_x, label_y, table, lambda_x, lambda_y):
+    def __init__(self, label_x, label_y, table, lambda_x, lambda_y, symmetric=False):
         self.label_x, self.label_y, self.table = label_x, label_y, table
+        self.symmetric = symmetric  # the table equals its transpose
         self.V = int(table.shape[0])
         self.struct = LabelCostStruct(label_x.data_ptr(), label_y.data_ptr(), table.data_ptr(), self.V,
                                       float(lambda_x), float(lambda_y))
@@ -268,8 +269,9 @@ class LabelCost:
         if label_cost_matrix.shape[0] != label_cost_matrix.shape[1]:
             raise ValueError("label_cost_matrix must be square (V, V)")
         V = label_cost_matrix.shape[0]
-        # one read of the device for both ranges
+        # one read of the device for both ranges and the symmetry of the table
         ends = [lab.min().to(torch.int64) for lab in (label_x, label_y)] + [lab.max().to(torch.int64) for lab in (label_x, label_y)]
+        ends.append((label_cost_matrix == label_cost_matrix.t()).all().to(torch.int64))
         ends = torch.stack([e.to(ends[0].device) for e in ends]).tolist()
         for name, lo, hi in (("label_x", ends[0], ends[2]), ("label_y", ends[1], ends[3])):
             if hi >= V or lo < 0:
@@ -279,12 +281,12 @@ class LabelCost:
         return LabelCost(label_x.to(dtype=torch.int32, device=device).contiguous(),
                          label_y.to(dtype=torch.int32, device=device).contiguous(),
                          label_cost_matrix.to(dtype=torch.float32, device=device).contiguous(),
-                         lambda_x, lambda_y)
+                         lambda_x, lambda_y, bool(ends[4]))
 
     def divergence_terms(self):
         """Label costs of OT(x,y), OT(x,x) and OT(y,y) from that of OT(x,y), with labels of their own storage."""
         lx, ly, lam_x, lam_y = self.label_x.clone(), self.label_y.clone(), self.struct.lambda_x, self.struct.lambda_y
-        return [LabelCost(u, v, self.table, lam_x, lam_y) for u, v in ((lx, ly), (lx, lx), (ly, ly))]
+        return [LabelCost(u, v, self.table, lam_x, lam_y, self.symmetric) for u, v in ((lx, ly), (lx, lx), (ly, ly))]
 
 
 class StepItem(ctypes.Structure):

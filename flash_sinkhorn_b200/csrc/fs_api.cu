@@ -1236,7 +1236,7 @@ int check_batch_item(const fs_batch_item& in, int i, int d, float cost_scale, in
 // solve's worth of launches instead of B. Schedules may differ in length; a finished problem drops out.
 static int solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
                                    float cost_scale, double rho_x, double rho_y, int prec, void* stream,
-                                   const fs_label_cost* labels) {
+                                   const fs_label_cost* labels, bool symmetric) {
   constexpr int kMaxBatch = 256;
   if (!items || n_items <= 0 || n_items > kMaxBatch)
     return fail(FS_ERR_BAD_ARG, "fs_solve_symmetric_batched takes 1..%d items", kMaxBatch);
@@ -1251,8 +1251,10 @@ static int solve_symmetric_batched(const fs_batch_item* items, int n_items, int 
       return fail(FS_ERR_BAD_ARG, "item %d: the items share the number of classes and lambda_x", i);
   }
   const int nlab = 3 * lc[0].V;
-  auto self_item = [&](const fs_batch_item& in) {  // a label table need not be symmetric
-    return in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y && !labels;
+  auto self_item = [&](const fs_batch_item& in) {
+    const fs_label_cost* l = labels ? labels + (&in - items) : nullptr;
+    return in.x == in.y && in.n == in.m && in.log_a == in.log_b && rho_x == rho_y &&
+           (!l || (symmetric && l->label_x == l->label_y));
   };
   for (int i = 0; i < n_items && two_sided; ++i) {
     const bool sizes = items[i].n > 0 && items[i].m > 0;
@@ -1380,14 +1382,14 @@ static int solve_symmetric_batched(const fs_batch_item* items, int n_items, int 
 
 extern "C" int fs_solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
                                           float cost_scale, double rho_x, double rho_y, int prec, void* stream) {
-  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, nullptr);
+  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, nullptr, false);
 }
 
 extern "C" int fs_solve_symmetric_batched_labels(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
                                                  float cost_scale, double rho_x, double rho_y, int prec, void* stream,
-                                                 const fs_label_cost* labels) {
+                                                 const fs_label_cost* labels, int symmetric) {
   if (!labels) return fail(FS_ERR_BAD_ARG, "labels must be non-null");
-  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, labels);
+  return solve_symmetric_batched(items, n_items, d, last_extrapolation, cost_scale, rho_x, rho_y, prec, stream, labels, symmetric != 0);
 }
 
 extern "C" int fs_grad_range(const float* x, const float* y, int n, int m, int d, const float* a, const float* b,

@@ -454,7 +454,8 @@ def _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_
                 _neg_if_none(rho_x), _neg_if_none(rho_y), prec, _lib.stream_ptr(dev))
         if n_classes:
             costs = (_lib.LabelCostStruct * len(group))(*[item.label.struct for item in group])
-            _lib.call("fs_solve_symmetric_batched_labels", dev, *args, ctypes.cast(costs, ctypes.c_void_p))
+            _lib.call("fs_solve_symmetric_batched_labels", dev, *args, ctypes.cast(costs, ctypes.c_void_p),
+                      int(items[0].label.symmetric))
         else:
             _lib.call("fs_solve_symmetric_batched", dev, *args)
 
@@ -480,14 +481,15 @@ def _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_
 def solve_loss_terms(x, y, log_a, log_b, schedules, *, debias, labels, prec, cost_scale, rho_x, rho_y, last_extrapolation):
     """Potentials of the terms of a batch of losses: OT(x,y) and, debiased, OT(x,x) and OT(y,y), of clouds ``x [B, n, d]``,
     ``y [B, m, d]`` and log-weights ``[B, n]``, ``[B, m]`` (fp32, contiguous); ``schedules[term][item]``: eps lists. Returns
-    one ``(f, g, f_pre, g_pre)`` of ``[B, rows]`` tensors per term; a self term without labels has f for g."""
+    one ``(f, g, f_pre, g_pre)`` of ``[B, rows]`` tensors per term; a self term (of a symmetric label table, if any) has f
+    for g."""
     (B, n, d), m = x.shape, y.shape[1]
     dev = x.device
     new = lambda k: torch.empty((B, k), device=dev, dtype=torch.float32)  # noqa: E731
     sides = [((x, log_a, n), (y, log_b, m)), ((x, log_a, n), (x, log_a, n)), ((y, log_b, m), (y, log_b, m))]
     items, outs, arrays = [], [], {}
     for term, ((u, lu, r), (v, lv, c)) in enumerate(sides[: 3 if debias else 1]):
-        same = term > 0 and labels is None and rho_x == rho_y
+        same = term > 0 and rho_x == rho_y and (labels is None or labels[0].symmetric)
         f, f_pre = new(r), new(r)
         g, g_pre = (f, f_pre) if same else (new(c), new(c))
         outs.append((f, g, f_pre, g_pre))

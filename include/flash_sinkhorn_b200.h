@@ -278,10 +278,12 @@ typedef struct fs_batch_item {
 int fs_solve_symmetric_batched(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
                                float cost_scale, double rho_x, double rho_y, int prec, void* stream);
 /* The same with a label cost per item (the number of classes and lambda_x are the same for all); every item's workspace
- * must be that of two-sided steps (fs_symmetric_workspace_bytes with n_classes), FS_ERR_UNSUPPORTED otherwise. */
+ * must be that of two-sided steps (fs_symmetric_workspace_bytes with n_classes), FS_ERR_UNSUPPORTED otherwise. symmetric
+ * != 0 says that every table equals its transpose: an item of one cloud, weights and labels against themselves is then a
+ * self-transport problem. */
 int fs_solve_symmetric_batched_labels(const fs_batch_item* items, int n_items, int d, int last_extrapolation,
                                       float cost_scale, double rho_x, double rho_y, int prec, void* stream,
-                                      const fs_label_cost* labels);
+                                      const fs_label_cost* labels, int symmetric);
 
 /* The same with a block-sparse list of kept 128 x 128 tiles (CSR over the 128-row blocks of x, and the
  * transposed list over the blocks of y, as fs_solve_alternating takes them; all four NULL = dense). No

@@ -95,12 +95,15 @@ def test_second_order():
         torch.autograd.grad((gx * v).sum(), xs)
 
 
-@pytest.mark.parametrize("n,m,V", [(300, 260, 4), (900, 701, 7)])
-def test_labels_in_lockstep(n, m, V):
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("n,m,V", [(300, 260, 4), (2900, 2701, 7)])
+def test_labels_in_lockstep(n, m, V, symmetric):
     from flash_sinkhorn_b200 import SamplesLoss
     x, y, a, b = (t[0] for t in _inputs(1, n, m, 16, seed=7))
     g = torch.Generator().manual_seed(1)
-    table = 3.0 * torch.rand(V, V, generator=g).cuda()  # not symmetric
+    table = 3.0 * torch.rand(V, V, generator=g).cuda()
+    if symmetric:
+        table = table + table.t()
     lx, ly = torch.randint(0, V, (n,), generator=g).cuda(), torch.randint(0, V, (m,), generator=g).cuda()
     kw = dict(eps=0.5, n_iters=10, use_epsilon_scaling=False, debias=True, allow_tf32=False, label_cost_matrix=table, lambda_x=0.7,
               lambda_y=1.3)
