@@ -588,11 +588,14 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
     if (v.sub < P.nsub)  // before rd is written again
       asm volatile("bar.sync %0, %1;" ::"r"(2 + team), "n"(kTeamWarps * 32) : "memory");
   }
-  const bool check = P.early && (recs[0].todo & kCheck);  // early stopping: one problem per launch
+  // Early stopping: one problem per launch. Read here: behind the second meeting warp 2 of this CTA may be writing the records
+  // of the next step (begin_step) while other warps still decide, and they all have to take this step's word.
+  const unsigned todo = recs[0].todo;
+  const bool check = P.early && (todo & kCheck);
   if (t + 1 == P.t1 && !check) return false;
   grid_arrive(meet, abort_flag);
   if (!grid_wait(meet, met, abort_flag)) return false;
-  const unsigned nth = recs[0].todo >> 8;
+  const unsigned nth = todo >> 8;
   if (check && nth > 0u && (double)__uint_as_float(__ldcg(&meet->delta[nth & 1u])) < P.threshold) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       P.sub[0].geo.ctrl->converged = 1;
