@@ -330,6 +330,8 @@ def _solver_scratch(n, m, d, prec, dev, n_classes=0, same=False) -> torch.Tensor
 # the other, beyond. Launches are what they share: the three solves of a divergence in 64 dimensions take 7.4 ms together
 # and 8.1 in turn at 20,000 points a side (20 steps), 37.8 and 38.3 at 50,000 (0.3 GB of sums), 54.6 and 54.8 at 80,000 (0.8).
 LOCKSTEP_SCRATCH_BYTES = 1 << 29
+# Problems of one call: the library takes up to 256, whole launches (24 problems) of whole divergences (3) are 240.
+LOCKSTEP_PROBLEMS = 240
 
 
 def sinkhorn_flashstyle_symmetric_batched(
@@ -357,7 +359,8 @@ def sinkhorn_flashstyle_symmetric_batched(
     samples_loss.py:515-552). ``problems`` is a sequence of ``(x, y, a, b)`` with one feature dimension; every
     problem gets the schedule :func:`sinkhorn_flashstyle_symmetric` would give it (its own diameter with
     ``use_epsilon_scaling``), and all of them advance in lockstep, up to 24 problems per kernel launch (four soft-min
-    passes where they step side by side), in several calls where their scratch passes ``LOCKSTEP_SCRATCH_BYTES``.
+    passes where they step side by side), in several calls where their scratch passes ``LOCKSTEP_SCRATCH_BYTES`` or
+    they are more than ``LOCKSTEP_PROBLEMS``.
     No early stopping, warm start or label cost. Returns one ``(f, g, f_prelast, g_prelast, n_steps)`` per problem
     (the pre-extrapolation pair equals ``(f, g)`` without ``last_extrapolation``); results equal the one-at-a-time
     solves up to the merge order of partial sums (rounding level). A problem given as ``(x, x, a, a)`` - the same
@@ -462,7 +465,7 @@ def _solve_in_lockstep(items, d, prec, dev, last_extrapolation, cost_scale, rho_
     groups, group, taken = [], [], 0
     for item in items:
         sums = scratch(item)[1]
-        if group and taken + sums > LOCKSTEP_SCRATCH_BYTES:
+        if group and (taken + sums > LOCKSTEP_SCRATCH_BYTES or len(group) == LOCKSTEP_PROBLEMS):
             groups.append(group)
             group, taken = [], 0
         group.append(item)

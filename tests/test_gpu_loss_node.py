@@ -154,3 +154,19 @@ def test_gradients_that_share_launches(monkeypatch, mode, B, n, m, d):
     assert _err(out[keep], want[keep]) < (2e-5 if mode == "fp32" else 5e-4)
     assert _err(out[~keep], want[~keep]) < 1e-3 or bool(keep.all())
     assert lib.fs_device_error() == 0
+
+
+@pytest.mark.parametrize("B,debias", [(90, True), (257, False)])
+def test_batches_beyond_one_library_call(B, debias):
+    """More problems (270, 257) than the library solves in one call (256): every item as on its own."""
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = _inputs(B, 20, 17, 3, seed=9)
+    loss = SamplesLoss("sinkhorn", eps=0.5, n_iters=6, use_epsilon_scaling=False, debias=debias, allow_tf32=False)
+    xs = x.clone().requires_grad_(True)
+    vals = loss(a, xs, b, y)
+    (gx,) = torch.autograd.grad(vals.sum(), xs)
+    for i in (0, 79, 80, B - 1):
+        xi = x[i].clone().requires_grad_(True)
+        vi = loss(a[i], xi, b[i], y[i])
+        assert abs(float(vi.detach()) - float(vals[i].detach())) < 1e-5 * float((x[i] * x[i]).sum(-1).max())
+        assert _err(gx[i], torch.autograd.grad(vi, xi)[0]) < 3e-4
