@@ -119,7 +119,7 @@ class _SinkhornGradFn(torch.autograd.Function):
 class _LossTerms:
     """What the node of a batch of losses knows beside its tensors."""
 
-    eps: float
+    eps: Tuple[Tuple[float, ...], ...]  # where the schedules end: [term][item]
     config: _SinkhornConfig
     debias: bool
     labels: Optional[list]  # label costs of the terms
@@ -138,15 +138,18 @@ def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
     prec = _lib.precision_id(cfg.allow_tf32)
     X, Y = (x32, a32, la, n), (y32, b32, lb, m)
 
-    waiting = []  # gradients of row clouds that share launches: (rows, columns, potential of the columns, scales, out)
+    # gradients of row clouds that share launches: (rows, columns, potential of the columns, scales, out), and their eps
+    waiting, waiting_eps = [], []
 
     def term(k, u, v, scales, out_u, out_v):
         (pu, wu, lu, r), (pv, wv, lv, c) = u, v
         if not meta.labels and all(_lib.load().fs_grad_many_bytes(p, q, d, prec) for p, q in ((r, c), (c, r))):
             if out_u is not None:
                 waiting.append((u, v, pots[4 * k + 3], scales, out_u))
+                waiting_eps.append(meta.eps[k])
             if out_v is not None:
                 waiting.append((v, u, pots[4 * k + 2], scales, out_v))
+                waiting_eps.append(meta.eps[k])
             return
         f_pre, g_pre = pots[4 * k + 2], pots[4 * k + 3]
         label = meta.labels[k] if meta.labels else None
@@ -156,7 +159,7 @@ def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
         addr = [_lib.ptr(t) for t in tensors]
         for i in range(gs.numel()):
             at = [None if p is None else p + i * q for p, q in zip(addr, pitch)]
-            _lib.call("fs_grad", dev, at[0], at[1], r, c, d, *at[2:], meta.eps, float(cfg.cost_scale), prec, _lib.ptr(ws),
+            _lib.call("fs_grad", dev, at[0], at[1], r, c, d, *at[2:], meta.eps[k][i], float(cfg.cost_scale), prec, _lib.ptr(ws),
                       ws.numel(), _lib.stream_ptr(dev), label.ref if label else None)
 
     gx = torch.empty(x.shape, device=dev, dtype=torch.float32) if want_x else None
@@ -174,7 +177,7 @@ def _loss_gradients(x, y, a, b, log_a, log_b, scale, meta, pots, want_x, want_y)
             own, other = torch.empty_like(out), torch.empty_like(out)
             term(k, side, side, -0.5 * gs, own, other)
             added += [(out, own), (out, other)]
-    _gradients_together(waiting, gs.numel(), d, meta.eps, float(cfg.cost_scale), prec, dev)
+    _gradients_together(waiting, gs.numel(), d, waiting_eps, float(cfg.cost_scale), prec, dev)
     for out, own in added:
         out += own
     return gx, gy
@@ -185,26 +188,29 @@ SHARED_GRADIENT_BYTES = 1 << 27
 
 
 def _gradients_together(terms, B, d, eps, cost_scale, prec, dev):
-    """Runs the gradients of row clouds ``(rows, columns, column potential, scales, out)`` of B items each, 16 per call."""
+    """Runs the gradients of row clouds ``(rows, columns, column potential, scales, out)`` of B items each, 16 of one eps per
+    call. ``eps``: a number, or one per term and item."""
     lib = _lib.load()
-    items, sizes = [], []
-    for (pu, wu, _, r), (pv, _, lv, c), pot, scales, out in terms:
+    by_eps = {}  # eps -> (items, sizes)
+    for t, ((pu, wu, _, r), (pv, _, lv, c), pot, scales, out) in enumerate(terms):
         base = [_lib.ptr(t) for t in (pu, pv, wu, lv, pot, scales, out)]
         pitch = [4 * q for q in (r * d, c * d, r, c, c, 1, r * d)]
         nbytes = int(lib.fs_grad_many_bytes(r, c, d, prec))
         for i in range(B):
             x, y, weight, log_w, at_pot, scale, at_out = (p + i * q for p, q in zip(base, pitch))
+            items, sizes = by_eps.setdefault(float(eps[t][i] if isinstance(eps, list) else eps), ([], []))
             items.append((x, y, r, c, weight, log_w, at_pot, scale, at_out))
             sizes.append(nbytes)
-    while items:
-        k = 1
-        while k < min(len(items), 16) and sum(sizes[: k + 1]) <= SHARED_GRADIENT_BYTES:
-            k += 1
-        ws = torch.empty(sum(sizes[:k]), dtype=torch.uint8, device=dev)
-        arr = (_lib.GradItem * k)(*items[:k])
-        _lib.call("fs_grad_many", dev, ctypes.cast(arr, ctypes.c_void_p), k, d, float(eps), cost_scale, prec, _lib.ptr(ws),
-                  ws.numel(), _lib.stream_ptr(dev))
-        items, sizes = items[k:], sizes[k:]
+    for at_eps, (items, sizes) in by_eps.items():
+        while items:
+            k = 1
+            while k < min(len(items), 16) and sum(sizes[: k + 1]) <= SHARED_GRADIENT_BYTES:
+                k += 1
+            ws = torch.empty(sum(sizes[:k]), dtype=torch.uint8, device=dev)
+            arr = (_lib.GradItem * k)(*items[:k])
+            _lib.call("fs_grad_many", dev, ctypes.cast(arr, ctypes.c_void_p), k, d, at_eps, cost_scale, prec, _lib.ptr(ws),
+                      ws.numel(), _lib.stream_ptr(dev))
+            items, sizes = items[k:], sizes[k:]
 
 
 class _SinkhornLossGradFn(torch.autograd.Function):
@@ -225,7 +231,8 @@ class _SinkhornLossGradFn(torch.autograd.Function):
         if v_x is not None:
             items = []
             for i in range(x.shape[0]):
-                sub = _HvpContext((x[i], y[i], a[i], b[i], f_pre[i], g_pre[i], scale[i]), ctx.meta.eps, ctx.meta.config)
+                sub = _HvpContext((x[i], y[i], a[i], b[i], f_pre[i], g_pre[i], scale[i]), ctx.meta.eps[0][i],
+                                  ctx.meta.config)
                 items.append(_SinkhornGradFn.backward(sub, v_x[i], None)[0])
             out = torch.stack(items, dim=0)
         return (out,) + (None,) * (9 + len(ctx.needs_input_grad) - 10)
@@ -253,19 +260,23 @@ class _SinkhornLossFn(torch.autograd.Function):
         ctx.meta = meta
         cfg = meta.config
 
-        def value(w, pot, rho):
+        def value(term, w, pot, rho):
             if cfg.rho_x is None or cfg.rho_y is None:  # balanced or semi-unbalanced
                 return w * pot
-            return (rho + meta.eps / 2) * (w * (1 - (-pot / rho).exp()))
+            eps = meta.eps[term]
+            mass = rho + eps[0] / 2
+            if len(set(eps)) > 1:
+                mass = torch.tensor([[rho + e / 2] for e in eps], device=pot.device, dtype=torch.float32)
+            return mass * (w * (1 - (-pot / rho).exp()))
 
         def side(k, w, rho, own, other):
-            # the potential of this side in OT(x,y), minus half of both potentials of the self term
+            # the potential of this side in OT(x,y), minus half of both potentials of the self term (number own // 4)
             if not meta.debias:
-                return value(w, pots[k], rho).sum(dim=-1)
+                return value(0, w, pots[k], rho).sum(dim=-1)
             if cfg.rho_x is None or cfg.rho_y is None:
                 return (w * (pots[k] - _half_sum(pots[own], pots[other]))).sum(dim=-1)
-            both = value(w, pots[own], cfg.rho_x) + value(w, pots[other], cfg.rho_y)
-            return (value(w, pots[k], rho) - 0.5 * both).sum(dim=-1)
+            both = value(own // 4, w, pots[own], cfg.rho_x) + value(own // 4, w, pots[other], cfg.rho_y)
+            return (value(0, w, pots[k], rho) - 0.5 * both).sum(dim=-1)
 
         return side(0, a, cfg.rho_x, 4, 5) + side(1, b, cfg.rho_y, 8, 9)
 

@@ -314,8 +314,7 @@ class SamplesLoss(torch.nn.Module):
 
     def _one_node(self, x, y, a, b, config, label_x, label_y):
         """The loss(es) as one autograd node whose terms are solved in one lockstep call, or None where they take the general
-        path: early stopping, schedules fixed in the constructor, terms that end at different eps, sizes without two-sided
-        steps."""
+        path: early stopping, schedules fixed in the constructor, sizes without two-sided steps."""
         if self.eps_list is not None or self.diameter is not None:
             return None
         single = x.ndim == 2
@@ -338,9 +337,6 @@ class SamplesLoss(torch.nn.Module):
             if single:
                 xd, yd, wa, wb = (t.unsqueeze(0) for t in (xd, yd, wa, wb))
             schedules = self._term_schedules(xd, yd)
-            ends = {sched[-1] for row in schedules for sched in row}
-            if len(ends) != 1:
-                return None
             log_a, log_b = log_weights(wa).contiguous(), log_weights(wb).contiguous()
             try:
                 sols = solve_loss_terms(_lib.f32c(xd), _lib.f32c(yd), log_a, log_b, schedules, debias=self.debias, labels=labels,
@@ -353,7 +349,7 @@ class SamplesLoss(torch.nn.Module):
             pots = [p[0] if single else p for sol in sols for p in sol]
             if single:
                 log_a, log_b = log_a[0], log_b[0]
-        meta = _LossTerms(float(ends.pop()), config, self.debias, labels)
+        meta = _LossTerms(tuple(tuple(float(sched[-1]) for sched in row) for row in schedules), config, self.debias, labels)
         return _SinkhornLossFn.apply(x, y, a, b, log_a, log_b, meta, *pots)
 
     def forward(self, *args, label_x: Optional[torch.Tensor] = None, label_y: Optional[torch.Tensor] = None):

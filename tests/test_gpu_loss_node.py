@@ -170,3 +170,33 @@ def test_batches_beyond_one_library_call(B, debias):
         vi = loss(a[i], xi, b[i], y[i])
         assert abs(float(vi.detach()) - float(vals[i].detach())) < 1e-5 * float((x[i] * x[i]).sum(-1).max())
         assert _err(gx[i], torch.autograd.grad(vi, xi)[0]) < 3e-4
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(reach=2.0), dict(label_cost_matrix=True, lambda_y=1.0)])
+@pytest.mark.parametrize("single,debias", [(True, True), (False, True), (False, False)])
+def test_terms_that_end_at_different_eps(single, debias, kw):
+    """``n_iters`` cuts annealed schedules that start at the diameters of their clouds: every term (and item) has an eps of its
+    own, and the loss stays one node. Tolerances as in test_against_single_terms."""
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = _inputs(3, 140, 150, 5, seed=13)
+    x = x * torch.tensor([1.0, 1.4, 0.6], device="cuda")[:, None, None]
+    if single:
+        x, y, a, b = (t[0] for t in (x, y, a, b))
+    labels = {}
+    if kw.get("label_cost_matrix"):
+        if not single:
+            pytest.skip("labels go item by item")
+        g = torch.Generator().manual_seed(2)
+        table = torch.rand(3, 3, generator=g).cuda()
+        kw = dict(kw, label_cost_matrix=table + table.t())
+        labels = {k: torch.randint(0, 3, (n,), generator=g).cuda() for k, n in (("label_x", 140), ("label_y", 150))}
+    kw = dict(blur=0.2, scaling=0.8, n_iters=5, debias=debias, allow_tf32=False, normalize=False, **kw)
+    outs = []
+    for extra in ({}, dict(threshold=0.0)):
+        args = [t.clone().requires_grad_(True) for t in (a, x, b, y)]
+        val = SamplesLoss("sinkhorn", **kw, **extra)(*args, **labels)
+        outs.append((val.detach(), torch.autograd.grad(val.sum(), args)))
+        assert (type(val.grad_fn).__name__ == "_SinkhornLossFnBackward") == (not extra)
+    assert float((outs[0][0] - outs[1][0]).abs().max()) < 1e-5 * float((x * x).sum(-1).max())
+    for u, v in zip(outs[0][1], outs[1][1]):
+        assert _err(u, v) < 3e-4
