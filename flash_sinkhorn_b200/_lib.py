@@ -284,9 +284,11 @@ class LabelCost:
                          lambda_x, lambda_y, bool(ends[4]))
 
     def divergence_terms(self):
-        """Label costs of OT(x,y), OT(x,x) and OT(y,y) from that of OT(x,y), with labels of their own storage."""
-        lx, ly, lam_x, lam_y = self.label_x.clone(), self.label_y.clone(), self.struct.lambda_x, self.struct.lambda_y
-        return [LabelCost(u, v, self.table, lam_x, lam_y, self.symmetric) for u, v in ((lx, ly), (lx, lx), (ly, ly))]
+        """Label costs of OT(x,y), OT(x,x) and OT(y,y) from that of OT(x,y), with labels and a table of their own storage: the
+        gradient reads them again, and has to find those that the potentials (and ``symmetric``) belong to."""
+        lx, ly, table = self.label_x.clone(), self.label_y.clone(), self.table.clone()
+        lam_x, lam_y = self.struct.lambda_x, self.struct.lambda_y
+        return [LabelCost(u, v, table, lam_x, lam_y, self.symmetric) for u, v in ((lx, ly), (lx, lx), (ly, ly))]
 
 
 class StepItem(ctypes.Structure):

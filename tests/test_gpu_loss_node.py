@@ -200,3 +200,24 @@ def test_terms_that_end_at_different_eps(single, debias, kw):
     assert float((outs[0][0] - outs[1][0]).abs().max()) < 1e-5 * float((x * x).sum(-1).max())
     for u, v in zip(outs[0][1], outs[1][1]):
         assert _err(u, v) < 3e-4
+
+
+def test_label_table_of_the_call():
+    """A table that is overwritten between the loss and its gradient, also by one that is not symmetric any more."""
+    from flash_sinkhorn_b200 import SamplesLoss
+    x, y, a, b = (t[0] for t in _inputs(1, 300, 260, 16, seed=7))
+    g = torch.Generator().manual_seed(1)
+    first = 3.0 * torch.rand(4, 4, generator=g).cuda()
+    first = first + first.t()
+    lx, ly = torch.randint(0, 4, (300,), generator=g).cuda(), torch.randint(0, 4, (260,), generator=g).cuda()
+    grads = []
+    for overwrite in (False, True):
+        table = first.clone()
+        loss = SamplesLoss("sinkhorn", eps=0.5, n_iters=10, use_epsilon_scaling=False, debias=True, label_cost_matrix=table,
+                           lambda_x=0.7, lambda_y=1.3)
+        xs = x.clone().requires_grad_(True)
+        val = loss(a, xs, b, y, label_x=lx, label_y=ly)
+        if overwrite:
+            table.copy_(torch.arange(16.0).reshape(4, 4))
+        grads.append(torch.autograd.grad(val, xs)[0])
+    assert _err(grads[1], grads[0]) < 1e-6  # the same numbers go in
