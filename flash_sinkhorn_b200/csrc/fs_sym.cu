@@ -689,6 +689,9 @@ __device__ __noinline__ float2 two_sided_run(uint32_t lane_addr, uint32_t bar0, 
       for (int k = 0; k < 32; ++k) acc[k] = 0ull;
     }
   }
+  // Where a wait gave up, the first scores of the next tile may still be on their way into registers that are used for other
+  // things from here on.
+  tmem_ld8_wait(ra);
   float v[64];
 #pragma unroll
   for (int k = 0; k < 32; ++k) upk(acc[k], v[2 * k], v[2 * k + 1]);
