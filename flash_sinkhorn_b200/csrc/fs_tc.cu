@@ -1159,7 +1159,7 @@ tc_pv_kernel(const __grid_constant__ CUtensorMap mapA_full, const __grid_constan
              const PvKernelParams p) {
   pv_pass<BN, SPLIT>(mapA_full, mapA_tail, mapB_full, mapB_tail, mapV_hi, mapV_lo, p, (int)blockIdx.x);
 }
-// (A kernel of its own: with its parameters found by the number of the pass the single one was 6 % slower.)
+// (A kernel of its own: the parameters of a pass are found by its number. Against the single one: grad_many.)
 template <int BN, bool SPLIT>
 __global__ void __launch_bounds__(128 + 128 * kParts, 1) tc_pv_many_kernel(const __grid_constant__ PvLaunch P) {
   int nth = 0;
@@ -2168,6 +2168,12 @@ cudaError_t grad_many(const GradJob* jobs, int cnt, int d, int prec, float cs, f
     pv.job[i].cta0 = grid;
     grid += (jobs[i].n + 127) / 128 * split;
   }
+  // A problem on its own takes the kernel that finds its parameters without a search where that one is the faster form of the
+  // same code (168 registers a thread against 126). Whole gradient of 20,000 x 20,000 points (us, single and shared form): TF32
+  // d = 16 361 and 367, 32 373 and 377, 64 420 and 422, 96 509 and 516, but 128 687 and 631; exact d = 64 754 and 797, 16 516 and
+  // 517, but 32 555 and 543. (The soft-min takes the same time in either form.)
+  if (cnt == 1 && (ps.split ? ps.dv_pad > 32 : ps.dv_pad < 128))
+    return ps.split ? launch_pv<64, true>(pv.job[0], grid, ps.smem, st) : launch_pv<128, false>(pv.job[0], grid, ps.smem, st);
   return ps.split ? launch_pv_many<64, true>(pv, grid, ps.smem, st) : launch_pv_many<128, false>(pv, grid, ps.smem, st);
 }
 
