@@ -61,6 +61,7 @@ SIGNATURES = {
     "fs_two_sided": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_two_sided_kernel": (c_int, [c_int, c_int, c_int, c_int]),
     "fs_two_sided_steps": (ctypes.c_longlong, []),
+    "fs_set_meeting_limit": (ctypes.c_longlong, [ctypes.c_longlong]),
     "fs_plan_ctas": (c_int, [c_int, c_int, c_int, c_int, c_int]),
     "fs_plan_pv_split": (c_int, [c_int, c_int, c_int, c_int, ctypes.POINTER(c_int)]),
     "fs_symmetric_workspace_bytes": (c_size_t, [c_int] * 7),

@@ -578,6 +578,7 @@ int fs_two_sided_kernel(int n, int m, int d, int prec) {
 }
 
 long long fs_two_sided_steps(void) { return sym::two_sided_steps(); }
+long long fs_set_meeting_limit(long long clocks) { return sym::set_meeting_limit(clocks); }
 
 int fs_two_sided(int n, int m, int d, int prec) { return sym_workspace(n, m, d, prec, 0, false) > 0 ? 1 : 0; }
 

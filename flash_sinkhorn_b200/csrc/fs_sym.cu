@@ -53,6 +53,7 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 namespace fs {
@@ -103,6 +104,7 @@ struct Launch {
   int t0, t1, t_table;  // steps of this launch, step of the first record
   int early;            // leave everything alone once the problem has converged
   double threshold;
+  long long meet_limit;  // clocks that a CTA waits for the others (grid_wait)
   Sub sub[NS];
 };
 
@@ -355,7 +357,7 @@ __device__ __forceinline__ bool own_inside(double pot, double own, double eps) {
 // The grid meets, twice per step: once all partial sums are in memory, and once the potentials and biases of the next step
 // are. Launches are cooperative, so every CTA is resident. False: some CTA has given up (one of its own waits, or here), and
 // all leave. `met` counts the meetings of this launch; leave_grid() puts the word back for the next one.
-constexpr long long kGridSpinLimit = 1ll << 33;  // ~4 s: the longest step of a solve takes milliseconds
+constexpr long long kMeetingLimit = 1ll << 33;  // clocks, ~4 s: the longest step of a solve takes milliseconds
 constexpr unsigned kGivenUp = 0x80000000u;
 __device__ __forceinline__ void grid_arrive(State* st, volatile int* abort_flag) {
   __syncthreads();
@@ -364,7 +366,7 @@ __device__ __forceinline__ void grid_arrive(State* st, volatile int* abort_flag)
     if (*abort_flag) atomicOr(&st->bar_count, kGivenUp); else atomicAdd(&st->bar_count, 1u);
   }
 }
-__device__ __forceinline__ bool grid_wait(State* st, unsigned& met, volatile int* abort_flag) {
+__device__ __forceinline__ bool grid_wait(State* st, unsigned& met, volatile int* abort_flag, long long limit) {
   ++met;
   if (threadIdx.x == 0) {
     const unsigned goal = met * gridDim.x;
@@ -373,7 +375,7 @@ __device__ __forceinline__ bool grid_wait(State* st, unsigned& met, volatile int
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&st->bar_count) : "memory");
       if (seen & kGivenUp) *abort_flag = 1;
       if (seen >= goal) break;
-      if (clock64() - t_begin > kGridSpinLimit) atomicOr(&st->bar_count, kGivenUp);
+      if (clock64() - t_begin > limit) atomicOr(&st->bar_count, kGivenUp);
     }
   }
   __syncthreads();
@@ -471,7 +473,7 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
   };
   grid_arrive(meet, abort_flag);
   if (WORK) look();
-  if (!grid_wait(meet, met, abort_flag)) return false;
+  if (!grid_wait(meet, met, abort_flag, P.meet_limit)) return false;
 #pragma unroll 1
   while (WORK && v.sub < P.nsub) {
     const Sub& u = P.sub[v.sub];
@@ -594,7 +596,7 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
   const bool check = P.early && (todo & kCheck);
   if (t + 1 == P.t1 && !check) return false;
   grid_arrive(meet, abort_flag);
-  if (!grid_wait(meet, met, abort_flag)) return false;
+  if (!grid_wait(meet, met, abort_flag, P.meet_limit)) return false;
   const unsigned nth = todo >> 8;
   if (check && nth > 0u && (double)__uint_as_float(__ldcg(&meet->delta[nth & 1u])) < P.threshold) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1524,6 +1526,7 @@ __global__ void sym_emit_kernel(const __grid_constant__ EmitJobs P) {
 }
 
 // ------------------------------------------------------------------ host side
+std::atomic<long long> g_meeting_limit{kMeetingLimit};
 enum Kind { RESIDENT = 0, STREAMED = 1, WIDE = 2, SMALL = 3 };
 struct Shape {
   int kind, bm, bn;
@@ -1656,6 +1659,7 @@ cudaError_t steps_n(Problem* const* p, int cnt, int t0, int t1, int t_table, boo
   lp.t0 = t0; lp.t1 = t1; lp.t_table = t_table;
   lp.early = early ? 1 : 0;
   lp.threshold = threshold;
+  lp.meet_limit = g_meeting_limit.load(std::memory_order_relaxed);
   long long most = 0;
   for (int i = 0; i < cnt; ++i) {
     const Problem& q = *p[i];
@@ -1887,6 +1891,10 @@ int kernel_of(int n, int m, int d, int prec, int nlab) {
 long long two_sided_steps() {
   unsigned long long v = 0;
   return cudaMemcpyFromSymbol(&v, g_sym_two_sided, sizeof(v)) == cudaSuccess ? (long long)v : -1;
+}
+
+long long set_meeting_limit(long long clocks) {
+  return g_meeting_limit.exchange(clocks < 0 ? kMeetingLimit : clocks, std::memory_order_relaxed);
 }
 
 int read_error_flag() {

@@ -144,6 +144,10 @@ int fs_two_sided_kernel(int n, int m, int d, int prec);
 /* Steps, counted per problem, that took one exponential for both potentials on the current device since the library was
  * loaded (first steps and problems whose range has no bound do not); waits for the device. -1 on an error. */
 long long fs_two_sided_steps(void);
+/* SM clocks that the thread blocks of a symmetric solve wait for one another at each end of a step before all of them give up
+ * and the solve ends with fs_device_error() set (its results are then void). Negative: the default, about four seconds.
+ * Returns the previous value. For tests of that path: with 0 a block gives up at the first look that finds others missing. */
+long long fs_set_meeting_limit(long long clocks);
 
 /* Host arithmetic only (no reference counterpart): the CTA count a streaming pass over n_row_blocks x
  * n_col_tiles work items gets on a device with `sms` SMs when `reserved` of them are left free and the CTA
