@@ -759,314 +759,314 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   // The service warps and the soft-max warps go through the steps in loops of their own: the latter take registers from the
   // former.
   if (warp < kFirst) {
-  registers_down();
+    registers_down();
 #pragma unroll 1
-  for (int t = P.t0;; ++t) {
-  if (warp == 0) fence_proxy_async();  // the biases were written by ordinary stores, which the meeting has made visible
-  if (warp == 2) begin_step(P, fixed, t, plan, runs, recs, lane);
-  __syncthreads();
-  const int w_begin = plan->w_begin, w_end = plan->w_end;
-  const bool has_work = w_begin < w_end;
-  if (warp == 0) {
-    // ===================== TMA producer =====================
-    if (KS && lane == 0 && has_work) {
-      int& issued = chunk;
-      bool ok = true;
+    for (int t = P.t0;; ++t) {
+      if (warp == 0) fence_proxy_async();  // the biases were written by ordinary stores, which the meeting has made visible
+      if (warp == 2) begin_step(P, fixed, t, plan, runs, recs, lane);
+      __syncthreads();
+      const int w_begin = plan->w_begin, w_end = plan->w_end;
+      const bool has_work = w_begin < w_end;
+      if (warp == 0) {
+        // ===================== TMA producer =====================
+        if (KS && lane == 0 && has_work) {
+          int& issued = chunk;
+          bool ok = true;
 #pragma unroll 1
-      for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
-        const Run s = run_at(P, *plan, runs, nth, w);
-        const Sub& u = P.sub[s.sub];
+          for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
+            const Run s = run_at(P, *plan, runs, nth, w);
+            const Sub& u = P.sub[s.sub];
 #pragma unroll 1
-        for (int t = 0; ok && t < s.len; ++t)
+            for (int t = 0; ok && t < s.len; ++t)
 #pragma unroll 1
-          for (int kc = 0; kc < P.nfull; ++kc) {
+              for (int kc = 0; kc < P.nfull; ++kc) {
+                const int st = issued % P.nstage;
+                if (!(ok = mbar_wait(bar(A_EMPTY + st), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000))) break;
+                mbar_expect_tx(bar(A_FULL + st), kChunk);
+                const uint32_t dst = smem_u32(a_smem + st * kChunk);
+                tma_load_2d(dst, &u.a_full[s.side], kc * 32, (s.rt + t) * 128, bar(A_FULL + st));
+                tma_load_2d(dst + 128 * 128, &u.b_full[s.side], kc * 32, s.ct * kBN, bar(A_FULL + st));
+                ++issued;
+              }
+            w += s.step;
+          }
+          if (*abort_flag)  // let every copy issued land before the CTA goes away
+            for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
+              mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
+        }
+        if (!KS && lane == 0 && has_work) {
+          int& issued = jt;
+          int pre = 0;
+          bool ok = true;
+          auto load_a = [&](const Run& s, int t) -> bool {
+            const Sub& u = P.sub[s.sub];
             const int st = issued % P.nstage;
-            if (!(ok = mbar_wait(bar(A_EMPTY + st), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000))) break;
-            mbar_expect_tx(bar(A_FULL + st), kChunk);
-            const uint32_t dst = smem_u32(a_smem + st * kChunk);
-            tma_load_2d(dst, &u.a_full[s.side], kc * 32, (s.rt + t) * 128, bar(A_FULL + st));
-            tma_load_2d(dst + 128 * 128, &u.b_full[s.side], kc * 32, s.ct * kBN, bar(A_FULL + st));
+            if (!mbar_wait(bar(A_EMPTY + st), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000)) return false;
+            mbar_expect_tx(bar(A_FULL + st), a_bytes);
+            const uint32_t dst = smem_u32(a_smem + st * a_bytes);
+            const int row0 = (s.rt + t) * 128;
+            for (int kb = 0; kb < P.nfull; ++kb)
+              tma_load_2d(dst + kb * (128 * 128), &u.a_full[s.side], kb * 32, row0, bar(A_FULL + st));
+            for (int k = 0; k < P.ntail; ++k)
+              tma_load_2d(dst + P.nfull * (128 * 128) + k * (128 * 32), &u.a_tail[s.side], P.nfull * 32 + k * 8, row0,
+                          bar(A_FULL + st));
             ++issued;
-          }
-        w += s.step;
-      }
-      if (*abort_flag)  // let every copy issued land before the CTA goes away
-        for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
-          mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
-    }
-    if (!KS && lane == 0 && has_work) {
-      int& issued = jt;
-      int pre = 0;
-      bool ok = true;
-      auto load_a = [&](const Run& s, int t) -> bool {
-        const Sub& u = P.sub[s.sub];
-        const int st = issued % P.nstage;
-        if (!mbar_wait(bar(A_EMPTY + st), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000)) return false;
-        mbar_expect_tx(bar(A_FULL + st), a_bytes);
-        const uint32_t dst = smem_u32(a_smem + st * a_bytes);
-        const int row0 = (s.rt + t) * 128;
-        for (int kb = 0; kb < P.nfull; ++kb)
-          tma_load_2d(dst + kb * (128 * 128), &u.a_full[s.side], kb * 32, row0, bar(A_FULL + st));
-        for (int k = 0; k < P.ntail; ++k)
-          tma_load_2d(dst + P.nfull * (128 * 128) + k * (128 * 32), &u.a_tail[s.side], P.nfull * 32 + k * 8, row0,
-                      bar(A_FULL + st));
-        ++issued;
-        return true;
-      };
-      auto load_b = [&](const Run& s) -> bool {  // column tile of run `seg`
-        const int sl = seg % P.nb;
-        // the column tile that was there must have been read by its last MMA
-        if (!mbar_wait(bar(B_EMPTY + sl), ((seg / P.nb) & 1) ^ 1, abort_flag, 2000)) return false;
-        mbar_expect_tx(bar(B_FULL + sl), b_bytes);
-        const Sub& u = P.sub[s.sub];
-        const uint32_t dst = smem_u32(b_smem + sl * b_bytes);
-        for (int kb = 0; kb < P.nfull; ++kb)
-          tma_load_2d(dst + kb * (kBN * 128), &u.b_full[s.side], kb * 32, s.ct * kBN, bar(B_FULL + sl));
-        for (int k = 0; k < P.ntail; ++k)
-          tma_load_2d(dst + P.nfull * (kBN * 128) + k * (kBN * 32), &u.b_tail[s.side], P.nfull * 32 + k * 8, s.ct * kBN,
-                      bar(B_FULL + sl));
-        ++seg;
-        return true;
-      };
-      Run s = runs[0];
-      ok = load_b(s);
-#pragma unroll 1
-      for (int w = w_begin, nth = 1; ok; ++nth) {
-#pragma unroll 1
-        for (int t = pre; ok && t < s.len; ++t) ok = load_a(s, t);
-        w += s.step;
-        if (!ok || w >= w_end) break;
-        s = run_at(P, *plan, runs, nth, w);
-        pre = 0;
-        if (P.nb > 1) {
+            return true;
+          };
+          auto load_b = [&](const Run& s) -> bool {  // column tile of run `seg`
+            const int sl = seg % P.nb;
+            // the column tile that was there must have been read by its last MMA
+            if (!mbar_wait(bar(B_EMPTY + sl), ((seg / P.nb) & 1) ^ 1, abort_flag, 2000)) return false;
+            mbar_expect_tx(bar(B_FULL + sl), b_bytes);
+            const Sub& u = P.sub[s.sub];
+            const uint32_t dst = smem_u32(b_smem + sl * b_bytes);
+            for (int kb = 0; kb < P.nfull; ++kb)
+              tma_load_2d(dst + kb * (kBN * 128), &u.b_full[s.side], kb * 32, s.ct * kBN, bar(B_FULL + sl));
+            for (int k = 0; k < P.ntail; ++k)
+              tma_load_2d(dst + P.nfull * (kBN * 128) + k * (kBN * 32), &u.b_tail[s.side], P.nfull * 32 + k * 8, s.ct * kBN,
+                          bar(B_FULL + sl));
+            ++seg;
+            return true;
+          };
+          Run s = runs[0];
           ok = load_b(s);
-        } else {
-          // The first row tiles of the next run do not need its column tile: they fill ring slots meanwhile (every
-          // slot waited for holds a tile that the MMA warp consumes without that column tile).
-          const int npre = s.len < P.nstage ? s.len : P.nstage;
 #pragma unroll 1
-          for (; ok && pre < npre; ++pre) ok = load_a(s, pre);
-          if (ok) ok = load_b(s);
+          for (int w = w_begin, nth = 1; ok; ++nth) {
+#pragma unroll 1
+            for (int t = pre; ok && t < s.len; ++t) ok = load_a(s, t);
+            w += s.step;
+            if (!ok || w >= w_end) break;
+            s = run_at(P, *plan, runs, nth, w);
+            pre = 0;
+            if (P.nb > 1) {
+              ok = load_b(s);
+            } else {
+              // The first row tiles of the next run do not need its column tile: they fill ring slots meanwhile (every
+              // slot waited for holds a tile that the MMA warp consumes without that column tile).
+              const int npre = s.len < P.nstage ? s.len : P.nstage;
+#pragma unroll 1
+              for (; ok && pre < npre; ++pre) ok = load_a(s, pre);
+              if (ok) ok = load_b(s);
+            }
+          }
+          if (*abort_flag) {  // let every copy issued land before the CTA goes away
+            for (int j = (seg > P.nb ? seg - P.nb : 0); j < seg; ++j) mbar_wait_quiet(bar(B_FULL + j % P.nb), (j / P.nb) & 1);
+            for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
+              mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
+          }
         }
-      }
-      if (*abort_flag) {  // let every copy issued land before the CTA goes away
-        for (int j = (seg > P.nb ? seg - P.nb : 0); j < seg; ++j) mbar_wait_quiet(bar(B_FULL + j % P.nb), (j / P.nb) & 1);
-        for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
-          mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
-      }
-    }
-  } else if (warp == 1) {
-    // ===================== MMA issuer (all lanes in the loop, one elected lane issues) =====================
-    constexpr uint32_t idesc = make_idesc(kBN), idesc_h = make_idesc_f16(kBN);
-    auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
-    bool ok = true;
-    if (KS) {
+      } else if (warp == 1) {
+        // ===================== MMA issuer (all lanes in the loop, one elected lane issues) =====================
+        constexpr uint32_t idesc = make_idesc(kBN), idesc_h = make_idesc_f16(kBN);
+        auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
+        bool ok = true;
+        if (KS) {
 #pragma unroll 1
-      for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
-      const Run s = run_at(P, *plan, runs, nth, w);
-      w += s.step;
+          for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
+            const Run s = run_at(P, *plan, runs, nth, w);
+            w += s.step;
 #pragma unroll 1
-      for (int i = 0; ok && i < s.len; ++i, ++jt) {
-        const int buf = jt & 1;
-        if (!vote(mbar_wait(bar(S_EMPTY + buf), ((jt >> 1) & 1) ^ 1, abort_flag, 2000))) break;
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
+            for (int i = 0; ok && i < s.len; ++i, ++jt) {
+              const int buf = jt & 1;
+              if (!vote(mbar_wait(bar(S_EMPTY + buf), ((jt >> 1) & 1) ^ 1, abort_flag, 2000))) break;
+              tc_fence_after();
+              const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
 #pragma unroll 1
-        for (int kc = 0; kc < P.nfull; ++kc, ++chunk) {
-          const int st = chunk % P.nstage;
-          if (!vote(mbar_wait(bar(A_FULL + st), (chunk / P.nstage) & 1, abort_flag, 2000))) { ok = false; break; }
+              for (int kc = 0; kc < P.nfull; ++kc, ++chunk) {
+                const int st = chunk % P.nstage;
+                if (!vote(mbar_wait(bar(A_FULL + st), (chunk / P.nstage) & 1, abort_flag, 2000))) { ok = false; break; }
+                tc_fence_after();
+                if (elect_one()) {
+                  const uint32_t at = smem_u32(a_smem + st * kChunk), al = desc_lo(at), bl = desc_lo(at + 128 * 128);
+                  const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
+#pragma unroll 1
+                  for (int ks = 0; ks < steps; ++ks)
+                    umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                              idesc, idesc_h, (kc | ks) != 0);
+                  umma_commit(bar(A_EMPTY + st));
+                  if (kc + 1 == P.nfull) umma_commit(bar(S_FULL + buf));
+                }
+                __syncwarp();
+              }
+            }
+          }
+        }
+#pragma unroll 1
+        for (int w = w_begin, nth = 0; !KS && ok && w < w_end; ++seg, ++nth) {
+          const Run s = run_at(P, *plan, runs, nth, w);
+          const int sl = seg % P.nb;
+          if (!vote(mbar_wait(bar(B_FULL + sl), (seg / P.nb) & 1, abort_flag, 2000))) break;
           tc_fence_after();
-          if (elect_one()) {
-            const uint32_t at = smem_u32(a_smem + st * kChunk), al = desc_lo(at), bl = desc_lo(at + 128 * 128);
-            const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
 #pragma unroll 1
-            for (int ks = 0; ks < steps; ++ks)
-              umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                        idesc, idesc_h, (kc | ks) != 0);
-            umma_commit(bar(A_EMPTY + st));
-            if (kc + 1 == P.nfull) umma_commit(bar(S_FULL + buf));
+          for (int i = 0; i < s.len; ++i, ++jt) {
+            const int st = jt % P.nstage, buf = jt & 1;
+            if (!vote(mbar_wait(bar(A_FULL + st), (jt / P.nstage) & 1, abort_flag, 2000)) ||
+                !vote(mbar_wait(bar(S_EMPTY + buf), ((jt >> 1) & 1) ^ 1, abort_flag, 2000))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            if (elect_one()) {
+              const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
+              int left = P.hs;  // fp16 K steps to go
+              uint32_t al = desc_lo(smem_u32(a_smem + st * a_bytes)), bl = desc_lo(smem_u32(b_smem + sl * b_bytes));
+              uint32_t acc = 0;
+#pragma unroll 1
+              for (int kb = 0; kb < P.nfull; ++kb) {
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) {
+                  umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc,
+                            idesc_h, acc);
+                  acc = 1;
+                }
+                left -= 4;
+                al += (128 * 128) >> 4;
+                bl += (kBN * 128) >> 4;
+              }
+#pragma unroll 1
+              for (int k = 0; k < P.ntail; ++k) {
+                umma_step(left > k, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
+                acc = 1;
+                al += (128 * 32) >> 4;
+                bl += (kBN * 32) >> 4;
+              }
+              umma_commit(bar(S_FULL + buf));
+              umma_commit(bar(A_EMPTY + st));
+            }
+            __syncwarp();
           }
+          if (elect_one()) umma_commit(bar(B_EMPTY + sl));  // the column tile may be replaced once these MMAs retired
           __syncwarp();
+          w += s.step;
         }
-      }
-      }
-    }
-#pragma unroll 1
-    for (int w = w_begin, nth = 0; !KS && ok && w < w_end; ++seg, ++nth) {
-      const Run s = run_at(P, *plan, runs, nth, w);
-      const int sl = seg % P.nb;
-      if (!vote(mbar_wait(bar(B_FULL + sl), (seg / P.nb) & 1, abort_flag, 2000))) break;
-      tc_fence_after();
-#pragma unroll 1
-      for (int i = 0; i < s.len; ++i, ++jt) {
-        const int st = jt % P.nstage, buf = jt & 1;
-        if (!vote(mbar_wait(bar(A_FULL + st), (jt / P.nstage) & 1, abort_flag, 2000)) ||
-            !vote(mbar_wait(bar(S_EMPTY + buf), ((jt >> 1) & 1) ^ 1, abort_flag, 2000))) {
-          ok = false;
-          break;
+        __syncwarp();
+        if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued before TMEM is freed
+          umma_commit(bar(DRAIN));
+          mbar_wait_quiet(bar(DRAIN), 0);
         }
-        tc_fence_after();
-        if (elect_one()) {
-          const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
-          int left = P.hs;  // fp16 K steps to go
-          uint32_t al = desc_lo(smem_u32(a_smem + st * a_bytes)), bl = desc_lo(smem_u32(b_smem + sl * b_bytes));
-          uint32_t acc = 0;
+      } else if (warp == 2) {
+        // ===================== row-sum collector: adds the warpgroups' parts, one value per row =====================
+        bool ok = true;
 #pragma unroll 1
-          for (int kb = 0; kb < P.nfull; ++kb) {
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128), idesc,
-                        idesc_h, acc);
-              acc = 1;
+        for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
+          const Run s = run_at(P, *plan, runs, nth, w);
+#pragma unroll 1
+          for (int i = 0; i < s.len; ++i, ++jt) {
+            const int slot = jt & 1;
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(R_FULL + slot), (jt >> 1) & 1, abort_flag, 1000))) {
+              ok = false;
+              break;
             }
-            left -= 4;
-            al += (128 * 128) >> 4;
-            bl += (kBN * 128) >> 4;
-          }
+            const float *pm = part + slot * 2 * kWG * 128 + lane, *ps = pm + kWG * 128;
 #pragma unroll 1
-          for (int k = 0; k < P.ntail; ++k) {
-            umma_step(left > k, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
-            acc = 1;
-            al += (128 * 32) >> 4;
-            bl += (kBN * 32) >> 4;
+            for (int r = 0; r < 128; r += 32) {  // one row per lane at a time: this warp has few registers
+              const size_t to = (size_t)i * 128 + r + lane;
+              const float s0 = ps[r], s1 = ps[128 + r], s2 = ps[256 + r], s3 = ps[384 + r];
+              if (s.two) {
+                s.row_s[to] = (s0 + s1) + (s2 + s3);
+              } else {
+                const float m0 = pm[r], m1 = pm[128 + r], m2 = pm[256 + r], m3 = pm[384 + r];
+                const float top = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+                s.row_m[to] = top;
+                s.row_s[to] = (s0 * ex2(m0 - top) + s1 * ex2(m1 - top)) + (s2 * ex2(m2 - top) + s3 * ex2(m3 - top));
+              }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(R_EMPTY + slot));
           }
-          umma_commit(bar(S_FULL + buf));
-          umma_commit(bar(A_EMPTY + st));
+          w += s.step;
         }
-        __syncwarp();
       }
-      if (elect_one()) umma_commit(bar(B_EMPTY + sl));  // the column tile may be replaced once these MMAs retired
       __syncwarp();
-      w += s.step;
+      if (!end_step<false>(P, *plan, fixed, recs, t, part, kFirst, met, abort_flag)) break;
     }
-    __syncwarp();
-    if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued before TMEM is freed
-      umma_commit(bar(DRAIN));
-      mbar_wait_quiet(bar(DRAIN), 0);
-    }
-  } else if (warp == 2) {
-    // ===================== row-sum collector: adds the warpgroups' parts, one value per row =====================
-    bool ok = true;
-#pragma unroll 1
-    for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
-      const Run s = run_at(P, *plan, runs, nth, w);
-#pragma unroll 1
-      for (int i = 0; i < s.len; ++i, ++jt) {
-        const int slot = jt & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(bar(R_FULL + slot), (jt >> 1) & 1, abort_flag, 1000))) {
-          ok = false;
-          break;
-        }
-        const float *pm = part + slot * 2 * kWG * 128 + lane, *ps = pm + kWG * 128;
-#pragma unroll 1
-        for (int r = 0; r < 128; r += 32) {  // one row per lane at a time: this warp has few registers
-          const size_t to = (size_t)i * 128 + r + lane;
-          const float s0 = ps[r], s1 = ps[128 + r], s2 = ps[256 + r], s3 = ps[384 + r];
-          if (s.two) {
-            s.row_s[to] = (s0 + s1) + (s2 + s3);
-          } else {
-            const float m0 = pm[r], m1 = pm[128 + r], m2 = pm[256 + r], m3 = pm[384 + r];
-            const float top = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-            s.row_m[to] = top;
-            s.row_s[to] = (s0 * ex2(m0 - top) + s1 * ex2(m1 - top)) + (s2 * ex2(m2 - top) + s3 * ex2(m3 - top));
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(R_EMPTY + slot));
-      }
-      w += s.step;
-    }
-  }
-  __syncwarp();
-  if (!end_step<false>(P, *plan, fixed, recs, t, part, kFirst, met, abort_flag)) break;
-  }
   } else {
-  // ===================== soft-max warpgroups =====================
-  registers_up();
+    // ===================== soft-max warpgroups =====================
+    registers_up();
 #pragma unroll 1
-  for (int t = P.t0;; ++t) {
-    __syncthreads();
-    const int w_begin = plan->w_begin, w_end = plan->w_end;
-    const bool has_work = w_begin < w_end;
-    const int wg = (warp - kFirst) >> 2, q = warp & 3;  // columns [64 wg, 64 wg + 64) of a tile; TMEM lane quarter
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + wg * 64;
-    const int trow = q * 32 + lane;
-    bool ok = true;
-    auto wait_tile = [&](int j) -> bool {
-      if (!mbar_wait(bar(S_FULL + (j & 1)), (j >> 1) & 1, abort_flag)) return false;
-      __syncwarp();
-      tc_fence_after();
-      return true;
-    };
-    auto release_tile = [&]() {  // every TMEM load of this warp from the buffer has landed
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(S_EMPTY + (jt & 1)));
-    };
-    auto post = [&](float m, float s) -> bool {  // this thread's part of the row sum goes to the collector
-      const int slot = jt & 1;
-      if (!mbar_wait(bar(R_EMPTY + slot), ((jt >> 1) & 1) ^ 1, abort_flag)) return false;
-      float* pp = part + slot * 2 * kWG * 128 + wg * 128 + trow;
-      pp[0] = m;
-      pp[kWG * 128] = s;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(R_FULL + slot));
-      return true;
-    };
+    for (int t = P.t0;; ++t) {
+      __syncthreads();
+      const int w_begin = plan->w_begin, w_end = plan->w_end;
+      const bool has_work = w_begin < w_end;
+      const int wg = (warp - kFirst) >> 2, q = warp & 3;  // columns [64 wg, 64 wg + 64) of a tile; TMEM lane quarter
+      const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + wg * 64;
+      const int trow = q * 32 + lane;
+      bool ok = true;
+      auto wait_tile = [&](int j) -> bool {
+        if (!mbar_wait(bar(S_FULL + (j & 1)), (j >> 1) & 1, abort_flag)) return false;
+        __syncwarp();
+        tc_fence_after();
+        return true;
+      };
+      auto release_tile = [&]() {  // every TMEM load of this warp from the buffer has landed
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(S_EMPTY + (jt & 1)));
+      };
+      auto post = [&](float m, float s) -> bool {  // this thread's part of the row sum goes to the collector
+        const int slot = jt & 1;
+        if (!mbar_wait(bar(R_EMPTY + slot), ((jt >> 1) & 1) ^ 1, abort_flag)) return false;
+        float* pp = part + slot * 2 * kWG * 128 + wg * 128 + trow;
+        pp[0] = m;
+        pp[kWG * 128] = s;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(R_FULL + slot));
+        return true;
+      };
 #pragma unroll 1
-    for (int w = w_begin, nth = 0; w < w_end; ++nth) {
-      const Run s = run_at(P, *plan, runs, nth, w);
-      const float pair = recs[s.sub].ratio;
-      if (s.two) {
-        float2 sums = make_float2(0.f, 0.f);
-        if (ok) sums = two_sided_run(lane_addr, bar0, smem_u32(part + kWG * 128 + wg * 128 + trow), pair, s.len, jt, s.diag);
-        jt += s.len;
-        ok = __all_sync(0xffffffffu, *abort_flag == 0) != 0;
-        if (ok) {  // one row of partials per warp (32 rows of each tile): no barrier at the end of a run
-          float* to = s.col + (size_t)(q * s.pitch + wg * 64 + 2 * lane);
-          *reinterpret_cast<float2*>(to) = sums;
-        }
-      } else {
-        const Geo& g = P.sub[s.sub].geo;
-        const bool wide = fixed[s.sub].unit < 0.f;
-#pragma unroll 1
-        for (int i = 0; ok && i < s.len; ++i, ++jt) {
-          if (!(ok = wait_tile(jt))) break;
-          const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
-          const float scale = wide ? recs[s.sub].scale2 * g.scales.inv[s.side][(s.rt + i) * 128 + trow] : pair;
-          uint32_t r[32];
-          float m_run = run_init(scale), off = __fmul_rn(scale, m_run), sum = 0.f;
-#pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
-            tmem_ld32_nowait(src + c * 32, r);
-            tmem_ld_wait(r);
-            if (wide) unscale_columns(r, g.scales.inv[1 - s.side] + s.ct * kBN + wg * 64 + c * 32);
-            float cm = __uint_as_float(r[0]);
-#pragma unroll
-            for (int k = 1; k < 31; k += 2) cm = max3(cm, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
-            m_run = fmaxf(m_run, fmaxf(cm, __uint_as_float(r[31])));
-            // the rounded product is the offset all terms are relative to (must not be contracted into an FMA)
-            const float off_new = __fmul_rn(scale, m_run);
-            float s0 = sum * ex2(off - off_new), s1 = 0.f, s2 = 0.f, s3 = 0.f;
-#pragma unroll
-            for (int k = 0; k < 32; k += 4) {
-              s0 += ex2(fmaf(__uint_as_float(r[k]), scale, -off_new));
-              s1 += ex2(fmaf(__uint_as_float(r[k + 1]), scale, -off_new));
-              s2 += ex2(fmaf(__uint_as_float(r[k + 2]), scale, -off_new));
-              s3 += ex2(fmaf(__uint_as_float(r[k + 3]), scale, -off_new));
-            }
-            sum = (s0 + s1) + (s2 + s3);
-            off = off_new;
+      for (int w = w_begin, nth = 0; w < w_end; ++nth) {
+        const Run s = run_at(P, *plan, runs, nth, w);
+        const float pair = recs[s.sub].ratio;
+        if (s.two) {
+          float2 sums = make_float2(0.f, 0.f);
+          if (ok) sums = two_sided_run(lane_addr, bar0, smem_u32(part + kWG * 128 + wg * 128 + trow), pair, s.len, jt, s.diag);
+          jt += s.len;
+          ok = __all_sync(0xffffffffu, *abort_flag == 0) != 0;
+          if (ok) {  // one row of partials per warp (32 rows of each tile): no barrier at the end of a run
+            float* to = s.col + (size_t)(q * s.pitch + wg * 64 + 2 * lane);
+            *reinterpret_cast<float2*>(to) = sums;
           }
-          release_tile();
-          if (!(ok = post(off, sum))) break;
+        } else {
+          const Geo& g = P.sub[s.sub].geo;
+          const bool wide = fixed[s.sub].unit < 0.f;
+#pragma unroll 1
+          for (int i = 0; ok && i < s.len; ++i, ++jt) {
+            if (!(ok = wait_tile(jt))) break;
+            const uint32_t src = lane_addr + (uint32_t)((jt & 1) * kBN);
+            const float scale = wide ? recs[s.sub].scale2 * g.scales.inv[s.side][(s.rt + i) * 128 + trow] : pair;
+            uint32_t r[32];
+            float m_run = run_init(scale), off = __fmul_rn(scale, m_run), sum = 0.f;
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+              tmem_ld32_nowait(src + c * 32, r);
+              tmem_ld_wait(r);
+              if (wide) unscale_columns(r, g.scales.inv[1 - s.side] + s.ct * kBN + wg * 64 + c * 32);
+              float cm = __uint_as_float(r[0]);
+#pragma unroll
+              for (int k = 1; k < 31; k += 2) cm = max3(cm, __uint_as_float(r[k]), __uint_as_float(r[k + 1]));
+              m_run = fmaxf(m_run, fmaxf(cm, __uint_as_float(r[31])));
+              // the rounded product is the offset all terms are relative to (must not be contracted into an FMA)
+              const float off_new = __fmul_rn(scale, m_run);
+              float s0 = sum * ex2(off - off_new), s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll
+              for (int k = 0; k < 32; k += 4) {
+                s0 += ex2(fmaf(__uint_as_float(r[k]), scale, -off_new));
+                s1 += ex2(fmaf(__uint_as_float(r[k + 1]), scale, -off_new));
+                s2 += ex2(fmaf(__uint_as_float(r[k + 2]), scale, -off_new));
+                s3 += ex2(fmaf(__uint_as_float(r[k + 3]), scale, -off_new));
+              }
+              sum = (s0 + s1) + (s2 + s3);
+              off = off_new;
+            }
+            release_tile();
+            if (!(ok = post(off, sum))) break;
+          }
         }
+        w += s.step;
       }
-      w += s.step;
+      __syncwarp();
+      if (!end_step<true>(P, *plan, fixed, recs, t, part, kFirst, met, abort_flag)) break;
     }
-    __syncwarp();
-    if (!end_step<true>(P, *plan, fixed, recs, t, part, kFirst, met, abort_flag)) break;
-  }
   }
 
   tc_fence_before();
@@ -1144,201 +1144,201 @@ __global__ void __launch_bounds__(128 + 128 * NHALF * PARTS, 1) sym_wide_kernel(
   unsigned met = 0;
 #pragma unroll 1
   for (int t = P.t0;; ++t) {
-  if (warp == 0) fence_proxy_async();  // the biases were written by ordinary stores, which the meeting has made visible
-  if (warp == 2) begin_step(P, fixed, t, plan, nullptr, recs, lane);
-  __syncthreads();
-  const int total = plan->item0[1];
-  const bool two = plan->two & 1u;
-  // Item k: (side, row tile, column tile).
-  auto locate_tile = [&](int k, int& side, int& rt, int& ct) {
-    side = 0;
-    if (two && g.self) {
-      const Run s = locate(P, *plan, k, k + 1);
-      rt = s.rt;
-      ct = s.ct;
-      return;
-    }
-    if (k >= g.nct[1] * g.nrt[0]) {
-      k -= g.nct[1] * g.nrt[0];
-      side = 1;
-    }
-    const int rows = g.nrt[side], cols = g.nct[1 - side], grp = k / (kGroup * rows), c0 = grp * kGroup;
-    const int width = cols - c0 < kGroup ? cols - c0 : kGroup, in = k - grp * kGroup * rows;
-    rt = in / width;
-    ct = c0 + in - rt * width;
-  };
+    if (warp == 0) fence_proxy_async();  // the biases were written by ordinary stores, which the meeting has made visible
+    if (warp == 2) begin_step(P, fixed, t, plan, nullptr, recs, lane);
+    __syncthreads();
+    const int total = plan->item0[1];
+    const bool two = plan->two & 1u;
+    // Item k: (side, row tile, column tile).
+    auto locate_tile = [&](int k, int& side, int& rt, int& ct) {
+      side = 0;
+      if (two && g.self) {
+        const Run s = locate(P, *plan, k, k + 1);
+        rt = s.rt;
+        ct = s.ct;
+        return;
+      }
+      if (k >= g.nct[1] * g.nrt[0]) {
+        k -= g.nct[1] * g.nrt[0];
+        side = 1;
+      }
+      const int rows = g.nrt[side], cols = g.nct[1 - side], grp = k / (kGroup * rows), c0 = grp * kGroup;
+      const int width = cols - c0 < kGroup ? cols - c0 : kGroup, in = k - grp * kGroup * rows;
+      rt = in / width;
+      ct = c0 + in - rt * width;
+    };
 
-  if (warp == 0) {
-    if (lane == 0) {
-      int& issued = chunk;
-      bool ok = true;
+    if (warp == 0) {
+      if (lane == 0) {
+        int& issued = chunk;
+        bool ok = true;
 #pragma unroll 1
-      for (int k = blockIdx.x; ok && k < total; k += gridDim.x) {
-        int side, rt, ct;
-        locate_tile(k, side, rt, ct);
+        for (int k = blockIdx.x; ok && k < total; k += gridDim.x) {
+          int side, rt, ct;
+          locate_tile(k, side, rt, ct);
+#pragma unroll 1
+          for (int kc = 0; kc < P.nfull; ++kc) {
+            const int s = issued % P.nstage;
+            if (!mbar_wait(bar(EMPTY + s), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000)) { ok = false; break; }
+            mbar_expect_tx(bar(FULL + s), kStage);
+            const uint32_t dst = smem_u32(base + (size_t)s * kStage);
+#pragma unroll
+            for (int h = 0; h < NHALF; ++h)
+              tma_load_2d(dst + h * kAHalf, &u.a_full[side], kc * 32, rt * BM + h * 128, bar(FULL + s));
+            tma_load_2d(dst + NHALF * kAHalf, &u.b_full[side], kc * 32, ct * BN, bar(FULL + s));
+            ++issued;
+          }
+        }
+        if (*abort_flag)  // let every copy issued land before the CTA goes away
+          for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
+            mbar_wait_quiet(bar(FULL + j % P.nstage), (j / P.nstage) & 1);
+      }
+    } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
+      const int h = warp == 1 ? 0 : 1;
+      constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
+      auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
+      bool ok = true;
+      int s = chunk % P.nstage;
+      uint32_t ph = (chunk / P.nstage) & 1;
+#pragma unroll 1
+      for (int k = blockIdx.x; ok && k < total; k += gridDim.x, ++jt) {
+        const int buf = h * NBUF + jt % NBUF;
+        if (!vote(mbar_wait(bar(S_EMPTY + buf), ((jt / NBUF) & 1) ^ 1, abort_flag, 2000))) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
 #pragma unroll 1
         for (int kc = 0; kc < P.nfull; ++kc) {
-          const int s = issued % P.nstage;
-          if (!mbar_wait(bar(EMPTY + s), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000)) { ok = false; break; }
-          mbar_expect_tx(bar(FULL + s), kStage);
-          const uint32_t dst = smem_u32(base + (size_t)s * kStage);
+          if (!vote(mbar_wait(bar(FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t at = smem_u32(base + (size_t)s * kStage);
+          const uint32_t al = desc_lo(at + h * kAHalf), bl = desc_lo(at + NHALF * kAHalf);
+          const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
 #pragma unroll
-          for (int h = 0; h < NHALF; ++h)
-            tma_load_2d(dst + h * kAHalf, &u.a_full[side], kc * 32, rt * BM + h * 128, bar(FULL + s));
-          tma_load_2d(dst + NHALF * kAHalf, &u.b_full[side], kc * 32, ct * BN, bar(FULL + s));
-          ++issued;
+          for (int ks = 0; ks < 4; ++ks)
+            if (ks < steps && elect_one())
+              umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                        idesc, idesc_h, (kc | ks) != 0);
+          if (elect_one()) umma_commit(bar(EMPTY + s));
+          __syncwarp();
+          if (++s == P.nstage) { s = 0; ph ^= 1; }
         }
-      }
-      if (*abort_flag)  // let every copy issued land before the CTA goes away
-        for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
-          mbar_wait_quiet(bar(FULL + j % P.nstage), (j / P.nstage) & 1);
-    }
-  } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
-    const int h = warp == 1 ? 0 : 1;
-    constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
-    auto vote = [&](bool v) { return __all_sync(0xffffffffu, v) != 0; };
-    bool ok = true;
-    int s = chunk % P.nstage;
-    uint32_t ph = (chunk / P.nstage) & 1;
-#pragma unroll 1
-    for (int k = blockIdx.x; ok && k < total; k += gridDim.x, ++jt) {
-      const int buf = h * NBUF + jt % NBUF;
-      if (!vote(mbar_wait(bar(S_EMPTY + buf), ((jt / NBUF) & 1) ^ 1, abort_flag, 2000))) break;
-      tc_fence_after();
-      const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
-#pragma unroll 1
-      for (int kc = 0; kc < P.nfull; ++kc) {
-        if (!vote(mbar_wait(bar(FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t at = smem_u32(base + (size_t)s * kStage);
-        const uint32_t al = desc_lo(at + h * kAHalf), bl = desc_lo(at + NHALF * kAHalf);
-        const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          if (ks < steps && elect_one())
-            umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                      idesc, idesc_h, (kc | ks) != 0);
-        if (elect_one()) umma_commit(bar(EMPTY + s));
+        chunk += P.nfull;
+        if (!ok) break;
+        if (elect_one()) umma_commit(bar(S_FULL + buf));
         __syncwarp();
-        if (++s == P.nstage) { s = 0; ph ^= 1; }
       }
-      chunk += P.nfull;
-      if (!ok) break;
-      if (elect_one()) umma_commit(bar(S_FULL + buf));
       __syncwarp();
-    }
-    __syncwarp();
-    if (*abort_flag && lane == 0) {
-      umma_commit(bar(DRAIN + h));
-      mbar_wait_quiet(bar(DRAIN + h), 0);
-    }
-  } else if (warp >= 4) {
-    const int wg = (warp - 4) >> 2, h = wg / PARTS, part = wg % PARTS, q = warp & 3;
-    const int trow = h * 128 + q * 32 + lane, et = tid - 128;  // row inside the tile, epilogue thread
-    const float pair = recs[0].ratio;
-    const bool wide = fixed->unit < 0.f;
-    bool ok = true;
+      if (*abort_flag && lane == 0) {
+        umma_commit(bar(DRAIN + h));
+        mbar_wait_quiet(bar(DRAIN + h), 0);
+      }
+    } else if (warp >= 4) {
+      const int wg = (warp - 4) >> 2, h = wg / PARTS, part = wg % PARTS, q = warp & 3;
+      const int trow = h * 128 + q * 32 + lane, et = tid - 128;  // row inside the tile, epilogue thread
+      const float pair = recs[0].ratio;
+      const bool wide = fixed->unit < 0.f;
+      bool ok = true;
 #pragma unroll 1
-    for (int k = blockIdx.x; k < total; k += gridDim.x, ++jt) {  // also after an abort: every warp takes every barrier
-      int side, rt, ct;
-      locate_tile(k, side, rt, ct);
-      const int buf = h * NBUF + jt % NBUF, sl = jt & 1;
-      if (ok) ok = mbar_wait(bar(S_FULL + buf), (jt / NBUF) & 1, abort_flag);
-      ok = __all_sync(0xffffffffu, ok) != 0;
-      const float scale = wide ? recs[0].scale2 * g.scales.inv[side][rt * BM + trow] : pair;
-      float m_run = run_init(scale), off = two ? 0.f : __fmul_rn(scale, m_run), sum = 0.f;
-      if (ok) {
-        tc_fence_after();
-        const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN) + part * CH * 32;
+      for (int k = blockIdx.x; k < total; k += gridDim.x, ++jt) {  // also after an abort: every warp takes every barrier
+        int side, rt, ct;
+        locate_tile(k, side, rt, ct);
+        const int buf = h * NBUF + jt % NBUF, sl = jt & 1;
+        if (ok) ok = mbar_wait(bar(S_FULL + buf), (jt / NBUF) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok) != 0;
+        const float scale = wide ? recs[0].scale2 * g.scales.inv[side][rt * BM + trow] : pair;
+        float m_run = run_init(scale), off = two ? 0.f : __fmul_rn(scale, m_run), sum = 0.f;
+        if (ok) {
+          tc_fence_after();
+          const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN) + part * CH * 32;
 #pragma unroll 1
-        for (int c = 0; c < CH; ++c) {
-          uint32_t r[32];
-          tmem_ld32_nowait(src + c * 32, r);
-          tmem_ld_wait(r);
-          if (c == CH - 1) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(S_EMPTY + buf));
-          }
-          if (wide) unscale_columns(r, g.scales.inv[1 - side] + ct * BN + (part * CH + c) * 32);
-          float v[32], s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-          if (two) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              s0 += v[i] = ex2(__uint_as_float(r[i]) * scale);
-              s1 += v[i + 1] = ex2(__uint_as_float(r[i + 1]) * scale);
-              s2 += v[i + 2] = ex2(__uint_as_float(r[i + 2]) * scale);
-              s3 += v[i + 3] = ex2(__uint_as_float(r[i + 3]) * scale);
+          for (int c = 0; c < CH; ++c) {
+            uint32_t r[32];
+            tmem_ld32_nowait(src + c * 32, r);
+            tmem_ld_wait(r);
+            if (c == CH - 1) {
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(bar(S_EMPTY + buf));
             }
-            sum += (s0 + s1) + (s2 + s3);
+            if (wide) unscale_columns(r, g.scales.inv[1 - side] + ct * BN + (part * CH + c) * 32);
+            float v[32], s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+            if (two) {
 #pragma unroll
-            for (int half = 16; half >= 1; half >>= 1) {  // over the warp's rows; lane l keeps column l
-              const bool up = (lane & half) != 0;
-#pragma unroll
-              for (int i = 0; i < half; ++i) {
-                const float keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
-                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+              for (int i = 0; i < 32; i += 4) {
+                s0 += v[i] = ex2(__uint_as_float(r[i]) * scale);
+                s1 += v[i + 1] = ex2(__uint_as_float(r[i + 1]) * scale);
+                s2 += v[i + 2] = ex2(__uint_as_float(r[i + 2]) * scale);
+                s3 += v[i + 3] = ex2(__uint_as_float(r[i + 3]) * scale);
               }
+              sum += (s0 + s1) + (s2 + s3);
+#pragma unroll
+              for (int half = 16; half >= 1; half >>= 1) {  // over the warp's rows; lane l keeps column l
+                const bool up = (lane & half) != 0;
+#pragma unroll
+                for (int i = 0; i < half; ++i) {
+                  const float keep = up ? v[i + half] : v[i], send = up ? v[i] : v[i + half];
+                  v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
+                }
+              }
+              colred[(sl * GROUPS + h * 4 + q) * BN + (part * CH + c) * 32 + lane] = v[0];
+            } else {
+              float cm = __uint_as_float(r[0]);
+#pragma unroll
+              for (int i = 1; i < 31; i += 2) cm = max3(cm, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+              m_run = fmaxf(m_run, fmaxf(cm, __uint_as_float(r[31])));
+              const float off_new = __fmul_rn(scale, m_run);
+              s0 = sum * ex2(off - off_new);
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                s0 += ex2(fmaf(__uint_as_float(r[i]), scale, -off_new));
+                s1 += ex2(fmaf(__uint_as_float(r[i + 1]), scale, -off_new));
+                s2 += ex2(fmaf(__uint_as_float(r[i + 2]), scale, -off_new));
+                s3 += ex2(fmaf(__uint_as_float(r[i + 3]), scale, -off_new));
+              }
+              sum = (s0 + s1) + (s2 + s3);
+              off = off_new;
             }
-            colred[(sl * GROUPS + h * 4 + q) * BN + (part * CH + c) * 32 + lane] = v[0];
-          } else {
-            float cm = __uint_as_float(r[0]);
+          }
+          float* rr = rowred + (sl * 2 * PARTS + part) * BM + trow;
+          rr[0] = off;
+          rr[PARTS * BM] = sum;
+        }
+        // one barrier per tile: the buffers alternate, and a thread reaches the barrier of tile j + 1 only after it
+        // has read those of tile j
+        asm volatile("bar.sync 1, %0;" ::"n"(NSYNC) : "memory");
+        if (ok) {
+          if (et < BM) {
+            const float* rm = rowred + sl * 2 * PARTS * BM + et;
+            const float* rs = rm + PARTS * BM;
+            const size_t at = (size_t)ct * g.pad[side] + (size_t)rt * BM + et;
+            float m = rm[0], s = 0.f;
+            if (two) {
 #pragma unroll
-            for (int i = 1; i < 31; i += 2) cm = max3(cm, __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-            m_run = fmaxf(m_run, fmaxf(cm, __uint_as_float(r[31])));
-            const float off_new = __fmul_rn(scale, m_run);
-            s0 = sum * ex2(off - off_new);
+              for (int i = 0; i < PARTS; ++i) s += rs[i * BM];
+              g.rp_s[0][at] = s;
+            } else {
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              s0 += ex2(fmaf(__uint_as_float(r[i]), scale, -off_new));
-              s1 += ex2(fmaf(__uint_as_float(r[i + 1]), scale, -off_new));
-              s2 += ex2(fmaf(__uint_as_float(r[i + 2]), scale, -off_new));
-              s3 += ex2(fmaf(__uint_as_float(r[i + 3]), scale, -off_new));
+              for (int i = 1; i < PARTS; ++i) m = fmaxf(m, rm[i * BM]);
+#pragma unroll
+              for (int i = 0; i < PARTS; ++i) s += rs[i * BM] * ex2(rm[i * BM] - m);
+              g.rp_m[side][at] = m;
+              g.rp_s[side][at] = s;
             }
-            sum = (s0 + s1) + (s2 + s3);
-            off = off_new;
           }
-        }
-        float* rr = rowred + (sl * 2 * PARTS + part) * BM + trow;
-        rr[0] = off;
-        rr[PARTS * BM] = sum;
-      }
-      // one barrier per tile: the buffers alternate, and a thread reaches the barrier of tile j + 1 only after it
-      // has read those of tile j
-      asm volatile("bar.sync 1, %0;" ::"n"(NSYNC) : "memory");
-      if (ok) {
-        if (et < BM) {
-          const float* rm = rowred + sl * 2 * PARTS * BM + et;
-          const float* rs = rm + PARTS * BM;
-          const size_t at = (size_t)ct * g.pad[side] + (size_t)rt * BM + et;
-          float m = rm[0], s = 0.f;
-          if (two) {
+          const int col = et - (NSYNC - BN);  // the other end of the threads
+          if (two && col >= 0) {
+            const float* cr = colred + sl * GROUPS * BN + col;
+            float s = 0.f;
 #pragma unroll
-            for (int i = 0; i < PARTS; ++i) s += rs[i * BM];
-            g.rp_s[0][at] = s;
-          } else {
-#pragma unroll
-            for (int i = 1; i < PARTS; ++i) m = fmaxf(m, rm[i * BM]);
-#pragma unroll
-            for (int i = 0; i < PARTS; ++i) s += rs[i * BM] * ex2(rm[i * BM] - m);
-            g.rp_m[side][at] = m;
-            g.rp_s[side][at] = s;
+            for (int i = 0; i < GROUPS; ++i) s += cr[i * BN];
+            g.cp[(size_t)rt * g.pad[1] + ct * BN + col] = s;
           }
-        }
-        const int col = et - (NSYNC - BN);  // the other end of the threads
-        if (two && col >= 0) {
-          const float* cr = colred + sl * GROUPS * BN + col;
-          float s = 0.f;
-#pragma unroll
-          for (int i = 0; i < GROUPS; ++i) s += cr[i * BN];
-          g.cp[(size_t)rt * g.pad[1] + ct * BN + col] = s;
         }
       }
     }
-  }
 
-  __syncwarp();
-  if (!end_step<true>(P, *plan, fixed, recs, t, rowred, 4, met, abort_flag)) break;
+    __syncwarp();
+    if (!end_step<true>(P, *plan, fixed, recs, t, rowred, 4, met, abort_flag)) break;
   }
 
   tc_fence_before();

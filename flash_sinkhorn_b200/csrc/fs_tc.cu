@@ -255,158 +255,158 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   // With four soft-max warpgroups these take registers from the four service warps (split_registers).
   constexpr bool kSplitRegisters = NHALF * PARTS == 4;
   if (warp < 4) {
-  if (kSplitRegisters) registers_down();
-  if (warp == 0) {
-    // ===================== TMA producer =====================
-    if (lane == 0) {
-      asm volatile("fence.proxy.async;" ::: "memory");  // biases that the pass before wrote with ordinary stores
-      int issued = 0, seg = 0;  // column tiles issued so far by this CTA (ring position), segment count
-      bool ok = true;
-      // Column tile `issued` (a CTA-wide running index) of the segment that starts at item w0.
-      auto load_b = [&](int j) -> bool {
-        const int s = issued % P.nstage;
-        const uint32_t ph = (issued / P.nstage) & 1;
-        if (!mbar_wait(bar(B_EMPTY + s), ph ^ 1, abort_flag, 2000)) return false;
-        mbar_expect_tx(bar(B_FULL + s), b_stage_bytes);
-        uint32_t dst = smem_u32(b_smem + s * b_stage_bytes);
-        const int col0 = j * BN;
-        for (int kb = 0; kb < P.nfull; ++kb)
-          tma_load_2d(dst + kb * (BN * 128), &SP().mapB_full, kb * 32, col0, bar(B_FULL + s));
-        for (int t = 0; t < P.ntail; ++t)
-          tma_load_2d(dst + P.nfull * (BN * 128) + t * (BN * 32), &SP().mapB_tail, P.nfull * 32 + t * 8, col0,
-                      bar(B_FULL + s));
-        ++issued;
-        return true;
-      };
-      int pre = 0;  // column tiles of the current segment that were already issued during the previous one
-#pragma unroll 1
-      int blk = has_work ? blk_of(w_begin) : 0;
-#pragma unroll 1
-      for (int w = w_begin; ok && w < w_end; ++seg) {
-        const int seg_end = row_end(blk) < w_end ? row_end(blk) : w_end;
-        const int row0 = SP().row_begin + blk * BM;
-        // The row operand of the previous segment must have been read by its last MMA.
-        if (!mbar_wait(bar(A_EMPTY), (seg & 1) ^ 1, abort_flag, 2000)) break;
-        mbar_expect_tx(bar(A_FULL), NHALF * a_half_bytes);
-#pragma unroll 1
-        for (int h = 0; h < NHALF; ++h) {
-          uint32_t dst = smem_u32(a_smem + h * a_half_bytes);
+    if (kSplitRegisters) registers_down();
+    if (warp == 0) {
+      // ===================== TMA producer =====================
+      if (lane == 0) {
+        asm volatile("fence.proxy.async;" ::: "memory");  // biases that the pass before wrote with ordinary stores
+        int issued = 0, seg = 0;  // column tiles issued so far by this CTA (ring position), segment count
+        bool ok = true;
+        // Column tile `issued` (a CTA-wide running index) of the segment that starts at item w0.
+        auto load_b = [&](int j) -> bool {
+          const int s = issued % P.nstage;
+          const uint32_t ph = (issued / P.nstage) & 1;
+          if (!mbar_wait(bar(B_EMPTY + s), ph ^ 1, abort_flag, 2000)) return false;
+          mbar_expect_tx(bar(B_FULL + s), b_stage_bytes);
+          uint32_t dst = smem_u32(b_smem + s * b_stage_bytes);
+          const int col0 = j * BN;
           for (int kb = 0; kb < P.nfull; ++kb)
-            tma_load_2d(dst + kb * (128 * 128), &SP().mapA_full, kb * 32, row0 + h * 128, bar(A_FULL));
+            tma_load_2d(dst + kb * (BN * 128), &SP().mapB_full, kb * 32, col0, bar(B_FULL + s));
           for (int t = 0; t < P.ntail; ++t)
-            tma_load_2d(dst + P.nfull * (128 * 128) + t * (128 * 32), &SP().mapA_tail, P.nfull * 32 + t * 8,
-                        row0 + h * 128, bar(A_FULL));
-        }
+            tma_load_2d(dst + P.nfull * (BN * 128) + t * (BN * 32), &SP().mapB_tail, P.nfull * 32 + t * 8, col0,
+                        bar(B_FULL + s));
+          ++issued;
+          return true;
+        };
+        int pre = 0;  // column tiles of the current segment that were already issued during the previous one
 #pragma unroll 1
-        for (int t = w + pre; ok && t < seg_end; ++t) ok = load_b(col_of(t, blk));
-        w = seg_end;
-        // Next segment (another row block, columns from 0): its first column tiles do not need the new row
-        // operand, so they go into ring slots as this segment's tiles retire - every slot waited for here
-        // holds a tile of this or an earlier segment, which the MMA lane consumes without the next A.
-        pre = 0;
-        if (ok && w < w_end) {
-          blk = next_blk(blk, w);
-          const int nnext = (row_end(blk) < w_end ? row_end(blk) : w_end) - w;
-          const int npre = nnext < P.nstage ? nnext : P.nstage;
+        int blk = has_work ? blk_of(w_begin) : 0;
 #pragma unroll 1
-          for (; ok && pre < npre; ++pre) ok = load_b(col_of(w + pre, blk));
-        }
-      }
-      if (*abort_flag) {  // let every copy we issued land before the CTA goes away
-        if (seg > 0) mbar_wait_quiet(bar(A_FULL), (seg - 1) & 1);
-        for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
-          mbar_wait_quiet(bar(B_FULL + j % P.nstage), (j / P.nstage) & 1);
-      }
-    }
-  } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
-    // ===================== MMA issuers: one warp per 128-row half =====================
-    // A stream that shares its scheduler with soft-max warps sustains one MMA per ~90 cycles, the tensor pipe
-    // one per 64: with one issuer per half (warps 1 and 3) the score tiles of the next column tile are ready
-    // well before the soft-max warps ask for them, instead of just in time. All 32 lanes run the loop and one
-    // elected lane issues: descriptor arithmetic is then warp-uniform (uniform registers, which is where
-    // tcgen05 instructions take their operands) instead of per-thread values moved over for every MMA. Every
-    // exit decision is a warp vote, since elect.sync needs all 32 lanes at the same instruction. Tile lists keep
-    // the loop on lane 0 alone (kWarpIssue false): with one MMA per tile (d = 3) and the list look-ups in the
-    // loop the converged form measured 15 % slower per pass there.
-    constexpr bool kWarpIssue = !CSR;
-    auto vote = [&](bool okl) { return kWarpIssue ? (__all_sync(0xffffffffu, okl) != 0) : okl; };
-    auto pick = [&]() { return kWarpIssue ? elect_one() : true; };
-    if (kWarpIssue || lane == 0) {
-      const int h = (warp == 1) ? 0 : 1;
-      constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
-      const uint32_t a_lo0 = desc_lo(smem_u32(a_smem + h * a_half_bytes));
-      bool ok = true;
-      int jt = 0, seg = 0;  // column tiles processed so far by this CTA (ring / buffer position), segment count
-      int blk = has_work ? blk_of(w_begin) : 0;
+        for (int w = w_begin; ok && w < w_end; ++seg) {
+          const int seg_end = row_end(blk) < w_end ? row_end(blk) : w_end;
+          const int row0 = SP().row_begin + blk * BM;
+          // The row operand of the previous segment must have been read by its last MMA.
+          if (!mbar_wait(bar(A_EMPTY), (seg & 1) ^ 1, abort_flag, 2000)) break;
+          mbar_expect_tx(bar(A_FULL), NHALF * a_half_bytes);
 #pragma unroll 1
-      for (int w = w_begin; ok && w < w_end; ++seg) {
-        const int nseg = (row_end(blk) < w_end ? row_end(blk) : w_end) - w;
-        if (!vote(mbar_wait(bar(A_FULL), seg & 1, abort_flag, 2000))) break;
-        tc_fence_after();
-#pragma unroll 1
-        for (int i = 0; i < nseg; ++i, ++jt) {
-          const int s = jt % P.nstage;
-          const uint32_t ph = (jt / P.nstage) & 1;
-          if (!vote(mbar_wait(bar(B_FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
-          const int buf = jt % NBUF;
-          const uint32_t sph = (jt / NBUF) & 1;
-          if (!vote(mbar_wait(bar(S_EMPTY + h * NBUF + buf), sph ^ 1, abort_flag, 2000))) {
-            ok = false;
-            break;
+          for (int h = 0; h < NHALF; ++h) {
+            uint32_t dst = smem_u32(a_smem + h * a_half_bytes);
+            for (int kb = 0; kb < P.nfull; ++kb)
+              tma_load_2d(dst + kb * (128 * 128), &SP().mapA_full, kb * 32, row0 + h * 128, bar(A_FULL));
+            for (int t = 0; t < P.ntail; ++t)
+              tma_load_2d(dst + P.nfull * (128 * 128) + t * (128 * 32), &SP().mapA_tail, P.nfull * 32 + t * 8,
+                          row0 + h * 128, bar(A_FULL));
           }
+#pragma unroll 1
+          for (int t = w + pre; ok && t < seg_end; ++t) ok = load_b(col_of(t, blk));
+          w = seg_end;
+          // Next segment (another row block, columns from 0): its first column tiles do not need the new row
+          // operand, so they go into ring slots as this segment's tiles retire - every slot waited for here
+          // holds a tile of this or an earlier segment, which the MMA lane consumes without the next A.
+          pre = 0;
+          if (ok && w < w_end) {
+            blk = next_blk(blk, w);
+            const int nnext = (row_end(blk) < w_end ? row_end(blk) : w_end) - w;
+            const int npre = nnext < P.nstage ? nnext : P.nstage;
+#pragma unroll 1
+            for (; ok && pre < npre; ++pre) ok = load_b(col_of(w + pre, blk));
+          }
+        }
+        if (*abort_flag) {  // let every copy we issued land before the CTA goes away
+          if (seg > 0) mbar_wait_quiet(bar(A_FULL), (seg - 1) & 1);
+          for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
+            mbar_wait_quiet(bar(B_FULL + j % P.nstage), (j / P.nstage) & 1);
+        }
+      }
+    } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
+      // ===================== MMA issuers: one warp per 128-row half =====================
+      // A stream that shares its scheduler with soft-max warps sustains one MMA per ~90 cycles, the tensor pipe
+      // one per 64: with one issuer per half (warps 1 and 3) the score tiles of the next column tile are ready
+      // well before the soft-max warps ask for them, instead of just in time. All 32 lanes run the loop and one
+      // elected lane issues: descriptor arithmetic is then warp-uniform (uniform registers, which is where
+      // tcgen05 instructions take their operands) instead of per-thread values moved over for every MMA. Every
+      // exit decision is a warp vote, since elect.sync needs all 32 lanes at the same instruction. Tile lists keep
+      // the loop on lane 0 alone (kWarpIssue false): with one MMA per tile (d = 3) and the list look-ups in the
+      // loop the converged form measured 15 % slower per pass there.
+      constexpr bool kWarpIssue = !CSR;
+      auto vote = [&](bool okl) { return kWarpIssue ? (__all_sync(0xffffffffu, okl) != 0) : okl; };
+      auto pick = [&]() { return kWarpIssue ? elect_one() : true; };
+      if (kWarpIssue || lane == 0) {
+        const int h = (warp == 1) ? 0 : 1;
+        constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
+        const uint32_t a_lo0 = desc_lo(smem_u32(a_smem + h * a_half_bytes));
+        bool ok = true;
+        int jt = 0, seg = 0;  // column tiles processed so far by this CTA (ring / buffer position), segment count
+        int blk = has_work ? blk_of(w_begin) : 0;
+#pragma unroll 1
+        for (int w = w_begin; ok && w < w_end; ++seg) {
+          const int nseg = (row_end(blk) < w_end ? row_end(blk) : w_end) - w;
+          if (!vote(mbar_wait(bar(A_FULL), seg & 1, abort_flag, 2000))) break;
           tc_fence_after();
-          // Descriptors are advanced incrementally: the low word holds (address >> 4), the high word (stride,
-          // version, swizzle) is a constant per block class.
-          const uint32_t d_tmem = tmem_base + (uint32_t)((h * NBUF + buf) * BN);
-          uint32_t al = a_lo0, bl = desc_lo(smem_u32(b_smem + s * b_stage_bytes));
-          // One election per tile where a tile has few MMAs (the 256-row plans: measured 1.3 % faster per pass,
-          // 10 % for the arg-max pass), one per instruction in the 128-row plans with their long K (d = 128:
-          // 1.3 % faster that way). kTileElect false: all lanes enter and every instruction is elected.
-          constexpr bool kTileElect = (NHALF == 2);
-          if (kTileElect ? pick() : true) {
-            uint32_t acc = 0;
-            int left = P.hs;  // fp16 K steps to go
 #pragma unroll 1
-            for (int kb = 0; kb < P.nfull; ++kb) {
+          for (int i = 0; i < nseg; ++i, ++jt) {
+            const int s = jt % P.nstage;
+            const uint32_t ph = (jt / P.nstage) & 1;
+            if (!vote(mbar_wait(bar(B_FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
+            const int buf = jt % NBUF;
+            const uint32_t sph = (jt / NBUF) & 1;
+            if (!vote(mbar_wait(bar(S_EMPTY + h * NBUF + buf), sph ^ 1, abort_flag, 2000))) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            // Descriptors are advanced incrementally: the low word holds (address >> 4), the high word (stride,
+            // version, swizzle) is a constant per block class.
+            const uint32_t d_tmem = tmem_base + (uint32_t)((h * NBUF + buf) * BN);
+            uint32_t al = a_lo0, bl = desc_lo(smem_u32(b_smem + s * b_stage_bytes));
+            // One election per tile where a tile has few MMAs (the 256-row plans: measured 1.3 % faster per pass,
+            // 10 % for the arg-max pass), one per instruction in the 128-row plans with their long K (d = 128:
+            // 1.3 % faster that way). kTileElect false: all lanes enter and every instruction is elected.
+            constexpr bool kTileElect = (NHALF == 2);
+            if (kTileElect ? pick() : true) {
+              uint32_t acc = 0;
+              int left = P.hs;  // fp16 K steps to go
+#pragma unroll 1
+              for (int kb = 0; kb < P.nfull; ++kb) {
 #pragma unroll
-              for (int ks = 0; ks < 4; ++ks) {
-                if (kTileElect || pick())
-                  umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                            idesc, idesc_h, acc);
-                acc = 1;
+                for (int ks = 0; ks < 4; ++ks) {
+                  if (kTileElect || pick())
+                    umma_step(left > ks, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                              idesc, idesc_h, acc);
+                  acc = 1;
+                }
+                left -= 4;
+                al += (128 * 128) >> 4;
+                bl += (BN * 128) >> 4;
               }
-              left -= 4;
-              al += (128 * 128) >> 4;
-              bl += (BN * 128) >> 4;
-            }
 #pragma unroll 1
-            for (int t = 0; t < P.ntail; ++t) {
-              if (kTileElect || pick())
-                umma_step(left > t, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
-              acc = 1;
-              al += (128 * 32) >> 4;
-              bl += (BN * 32) >> 4;
+              for (int t = 0; t < P.ntail; ++t) {
+                if (kTileElect || pick())
+                  umma_step(left > t, d_tmem, pack_desc(al, kDescHi32), pack_desc(bl, kDescHi32), idesc, idesc_h, acc);
+                acc = 1;
+                al += (128 * 32) >> 4;
+                bl += (BN * 32) >> 4;
+              }
+              if (kTileElect || pick()) {
+                umma_commit(bar(S_FULL + h * NBUF + buf));
+                umma_commit(bar(B_EMPTY + s));
+              }
             }
-            if (kTileElect || pick()) {
-              umma_commit(bar(S_FULL + h * NBUF + buf));
-              umma_commit(bar(B_EMPTY + s));
-            }
+            if (kWarpIssue) __syncwarp();
           }
+          // the row operand may be replaced once every MMA issued so far retired
+          if (pick()) umma_commit(bar(A_EMPTY));
           if (kWarpIssue) __syncwarp();
+          w += nseg;
+          if (w < w_end) blk = next_blk(blk, w);
         }
-        // the row operand may be replaced once every MMA issued so far retired
-        if (pick()) umma_commit(bar(A_EMPTY));
         if (kWarpIssue) __syncwarp();
-        w += nseg;
-        if (w < w_end) blk = next_blk(blk, w);
-      }
-      if (kWarpIssue) __syncwarp();
-      if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued by this warp before TMEM is freed
-        umma_commit(bar(DRAIN + h));
-        mbar_wait_quiet(bar(DRAIN + h), 0);
+        if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued by this warp before TMEM is freed
+          umma_commit(bar(DRAIN + h));
+          mbar_wait_quiet(bar(DRAIN + h), 0);
+        }
       }
     }
-  }
   } else {
     // ===================== soft-max warpgroups =====================
     if (kSplitRegisters) registers_up();

@@ -138,94 +138,94 @@ tck_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 
   constexpr bool kSplitRegisters = NHALF * kPartsK == 4;
   if (warp < 4) {
-  if (kSplitRegisters) registers_down();
-  if (warp == 0) {
-    // ===================== TMA producer =====================
-    if (lane == 0) {
-      int issued = 0;  // stages filled so far (ring position)
-      bool ok = true;
+    if (kSplitRegisters) registers_down();
+    if (warp == 0) {
+      // ===================== TMA producer =====================
+      if (lane == 0) {
+        int issued = 0;  // stages filled so far (ring position)
+        bool ok = true;
 #pragma unroll 1
-      for (int w = w_begin; ok && w < w_end; ++w) {
-        const int blk = w / p.ntiles, j = w - blk * p.ntiles;
-        const int row0 = p.row_begin + blk * BM, col0 = j * BN;
+        for (int w = w_begin; ok && w < w_end; ++w) {
+          const int blk = w / p.ntiles, j = w - blk * p.ntiles;
+          const int row0 = p.row_begin + blk * BM, col0 = j * BN;
 #pragma unroll 1
-        for (int kc = 0; kc < p.nk; ++kc) {
-          const int s = issued % p.nstage;
-          const uint32_t ph = (issued / p.nstage) & 1;
-          if (!mbar_wait(bar(EMPTY + s), ph ^ 1, abort_flag, 2000)) { ok = false; break; }
-          mbar_expect_tx(bar(FULL + s), kStage);
-          const uint32_t dst = smem_u32(ring + (size_t)s * kStage);
+          for (int kc = 0; kc < p.nk; ++kc) {
+            const int s = issued % p.nstage;
+            const uint32_t ph = (issued / p.nstage) & 1;
+            if (!mbar_wait(bar(EMPTY + s), ph ^ 1, abort_flag, 2000)) { ok = false; break; }
+            mbar_expect_tx(bar(FULL + s), kStage);
+            const uint32_t dst = smem_u32(ring + (size_t)s * kStage);
 #pragma unroll
-          for (int h = 0; h < NHALF; ++h) tma_load_2d(dst + h * kAHalf, &mapA, kc * 32, row0 + h * 128, bar(FULL + s));
-          tma_load_2d(dst + NHALF * kAHalf, &mapB, kc * 32, col0, bar(FULL + s));
-          ++issued;
-        }
-      }
-      if (*abort_flag) {  // let every copy we issued land before the CTA goes away
-        for (int j = (issued > p.nstage ? issued - p.nstage : 0); j < issued; ++j)
-          mbar_wait_quiet(bar(FULL + j % p.nstage), (j / p.nstage) & 1);
-      }
-    }
-  } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
-    // ===================== MMA issuers: one warp per 128-row half =====================
-    // All 32 lanes run the loop (warp-uniform descriptor arithmetic), one elected lane issues; every exit
-    // decision is a warp vote, since elect.sync needs all lanes at the same instruction.
-    {
-      const int h = (warp == 1) ? 0 : 1;
-      constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
-      bool ok = true;
-      int s = 0;
-      uint32_t ph = 0;
-      int jt = 0;  // items processed so far by this CTA (accumulator buffer position)
-#pragma unroll 1
-      for (int w = w_begin; ok && w < w_end; ++w, ++jt) {
-        const int buf = jt % NBUF;
-        const uint32_t sph = (jt / NBUF) & 1;
-        if (!__all_sync(0xffffffffu, mbar_wait(bar(S_EMPTY + h * NBUF + buf), sph ^ 1, abort_flag, 2000))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t d_tmem = tmem_base + (uint32_t)((h * NBUF + buf) * BN);
-        uint32_t acc = 0;
-#pragma unroll 1
-        for (int kc = 0; kc < p.nk; ++kc) {
-          if (!__all_sync(0xffffffffu, mbar_wait(bar(FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t stage_addr = smem_u32(ring + (size_t)s * kStage);
-          const uint32_t al = desc_lo(stage_addr + h * kAHalf), bl = desc_lo(stage_addr + NHALF * kAHalf);
-          if (kc + 1 < p.nk) {
-#pragma unroll
-            for (int ks = 0; ks < 4; ++ks) {
-              if (elect_one())
-                umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                          idesc, idesc_h, acc);
-              acc = 1;
-            }
-          } else {
-#pragma unroll 1
-            for (int ks = 0; ks < p.klast; ++ks) {
-              if (elect_one())
-                umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
-                          idesc, idesc_h, acc);
-              acc = 1;
-            }
+            for (int h = 0; h < NHALF; ++h) tma_load_2d(dst + h * kAHalf, &mapA, kc * 32, row0 + h * 128, bar(FULL + s));
+            tma_load_2d(dst + NHALF * kAHalf, &mapB, kc * 32, col0, bar(FULL + s));
+            ++issued;
           }
-          if (elect_one()) umma_commit(bar(EMPTY + s));
-          __syncwarp();
-          if (++s == p.nstage) { s = 0; ph ^= 1; }
         }
-        if (!ok) break;
-        if (elect_one()) umma_commit(bar(S_FULL + h * NBUF + buf));
-        __syncwarp();
+        if (*abort_flag) {  // let every copy we issued land before the CTA goes away
+          for (int j = (issued > p.nstage ? issued - p.nstage : 0); j < issued; ++j)
+            mbar_wait_quiet(bar(FULL + j % p.nstage), (j / p.nstage) & 1);
+        }
       }
-      __syncwarp();
-      if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued by this warp before TMEM is freed
-        umma_commit(bar(DRAIN + h));
-        mbar_wait_quiet(bar(DRAIN + h), 0);
+    } else if (warp == 1 || (warp == 3 && NHALF == 2)) {
+      // ===================== MMA issuers: one warp per 128-row half =====================
+      // All 32 lanes run the loop (warp-uniform descriptor arithmetic), one elected lane issues; every exit
+      // decision is a warp vote, since elect.sync needs all lanes at the same instruction.
+      {
+        const int h = (warp == 1) ? 0 : 1;
+        constexpr uint32_t idesc = make_idesc(BN), idesc_h = make_idesc_f16(BN);
+        bool ok = true;
+        int s = 0;
+        uint32_t ph = 0;
+        int jt = 0;  // items processed so far by this CTA (accumulator buffer position)
+#pragma unroll 1
+        for (int w = w_begin; ok && w < w_end; ++w, ++jt) {
+          const int buf = jt % NBUF;
+          const uint32_t sph = (jt / NBUF) & 1;
+          if (!__all_sync(0xffffffffu, mbar_wait(bar(S_EMPTY + h * NBUF + buf), sph ^ 1, abort_flag, 2000))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d_tmem = tmem_base + (uint32_t)((h * NBUF + buf) * BN);
+          uint32_t acc = 0;
+#pragma unroll 1
+          for (int kc = 0; kc < p.nk; ++kc) {
+            if (!__all_sync(0xffffffffu, mbar_wait(bar(FULL + s), ph, abort_flag, 2000))) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t stage_addr = smem_u32(ring + (size_t)s * kStage);
+            const uint32_t al = desc_lo(stage_addr + h * kAHalf), bl = desc_lo(stage_addr + NHALF * kAHalf);
+            if (kc + 1 < p.nk) {
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) {
+                if (elect_one())
+                  umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                            idesc, idesc_h, acc);
+                acc = 1;
+              }
+            } else {
+#pragma unroll 1
+              for (int ks = 0; ks < p.klast; ++ks) {
+                if (elect_one())
+                  umma_step(kc * 4 + ks < p.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
+                            idesc, idesc_h, acc);
+                acc = 1;
+              }
+            }
+            if (elect_one()) umma_commit(bar(EMPTY + s));
+            __syncwarp();
+            if (++s == p.nstage) { s = 0; ph ^= 1; }
+          }
+          if (!ok) break;
+          if (elect_one()) umma_commit(bar(S_FULL + h * NBUF + buf));
+          __syncwarp();
+        }
+        __syncwarp();
+        if (*abort_flag && lane == 0) {  // wait (bounded) for every MMA issued by this warp before TMEM is freed
+          umma_commit(bar(DRAIN + h));
+          mbar_wait_quiet(bar(DRAIN + h), 0);
+        }
       }
     }
-  }
   } else {
     if (kSplitRegisters) registers_up();
     // ===================== epilogue warpgroups =====================
