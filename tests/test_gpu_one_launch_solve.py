@@ -83,3 +83,23 @@ def test_capture_and_side_by_side():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("limit", [5, 0])
+def test_launch_that_ends_while_steps_are_one_sided(cta_limit, limit):  # noqa: F811
+    """At a small eps the first steps are one-sided; problems of the same call end among them, and the launch with them."""
+    from flash_sinkhorn_b200 import _lib
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric_batched
+    cta_limit(limit)
+    lib, eps, d = _lib.load(), 0.02, 8
+    sizes = [(300, 520), (1500, 1400), (2100, 1700)]
+    probs = [_problem(n, m, d, seed=k) for k, (n, m) in enumerate(sizes)]
+    kw = dict(use_epsilon_scaling=False, eps=eps, allow_tf32=False)
+    before = lib.fs_two_sided_steps()
+    sinkhorn_flashstyle_symmetric_batched([p[1] for p in probs], schedules=[[eps]] * 3, **kw)
+    assert lib.fs_two_sided_steps() == before  # three steps, all one-sided
+    lengths = (1, 30, 2)
+    got = sinkhorn_flashstyle_symmetric_batched([p[1] for p in probs], schedules=[[eps] * k for k in lengths], **kw)
+    assert lib.fs_two_sided_steps() > before
+    for g, p, k in zip(got, probs, lengths):
+        _close(g[:4], _dense(*p[0], eps, k), _size(p[0]))
