@@ -1043,7 +1043,7 @@ int fs_grad_many(const fs_grad_item* items, int n_items, int d, float eps, float
   }
   if (!wsp || ws_bytes < need) return fail(FS_ERR_WORKSPACE, "workspace too small: need %zu bytes", need);
   FS_TRY(check_device());
-  g_launches.fetch_add(4, std::memory_order_relaxed);
+  g_launches.fetch_add(tc::operand_layout(d, prec, 0, 3).hs ? 4 : 3, std::memory_order_relaxed);
   FS_CUDA(tc::grad_many(jobs, n_items, d, prec, cost_scale, eps, static_cast<char*>(wsp), static_cast<cudaStream_t>(stream)));
   return FS_OK;
 }

@@ -20,8 +20,8 @@
 // and column sum inside [2^-90, 2^120]; otherwise - the first steps of a solve from zero potentials at small eps,
 // weights of zero, any NaN, points with scales of their own (wide_range) - the same kernel runs it "one-sided": rows of
 // x, then rows of y, per-tile maxima, as (offset, sum) pairs. The decision is taken on the device from the same words by
-// every CTA; the host enqueues the same launches either way. Simulated over eps from 0.0002 d to annealed schedules: two-sided from the second to
-// the seventh step on, the row sums then within 2^+-30 of their weights.
+// every CTA; the host enqueues the same launches either way. Simulated over eps from 0.0002 d to annealed schedules: two-sided
+// from the second to the seventh step on, the row sums then within 2^+-30 of their weights.
 //
 // Launches. All steps of a solve (all that the same problems take) are ONE cooperative launch: per step the CTAs stream
 // their runs of tiles, meet, turn the partial sums of their share of the points into potentials and biases, and meet again
@@ -264,7 +264,9 @@ __device__ Run locate(const L& P, const Plan& pl, int w, int w_end) {
   s.col = g.cp + (size_t)piece * 4 * s.pitch + s.ct * g.bn;
   return s;
 }
-// The runs of a CTA, listed whenever the plan changes; the rest of a longer list is found again each time.
+// The runs of a CTA, listed whenever the plan changes; the rest of a longer list is found again each time. 24 problems of a few
+// column tiles each are about one run per CTA and problem at the most; longer lists are shares of many short column tiles (few
+// row tiles), whose items are found by a dozen instructions more. 64 bytes a run, in the service area beside 24 problems' words.
 constexpr int kRuns = 24;
 template <class L>
 __device__ __forceinline__ Run run_at(const L& P, const Plan& pl, const Run* runs, int nth, int w) {
@@ -549,7 +551,7 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
         write_bias(u.opA[c] + at + 3, inside_next ? ((double)now + own * eps_next) * to_unit : 0.0);
         write_bias(u.opB[c] + at, ((double)now + lw * eps_next) * to_unit);
         const float big_l = (float)((double)l2 - own * 1.4426950408889634);
-        const float dlt = (float)((double)now - old) * (kLog2e / rec.eps);
+        const float dlt = (float)((double)now - old) * (kLog2e / rec.eps);  // for the bounds alone, whose margins are octaves
         st_u = big_l + dlt;
         st_l = -st_u;
         st_dx = dlt;
@@ -609,7 +611,8 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
 }
 
 // ------------------------------------------------------------------ the streaming kernel
-// Bounded wait without a clock: one register. ~0.1 s of polls at the least.
+// Bounded wait without a clock: one register. The bound is a number of polls, each of which the hardware may suspend for a
+// while: 0.1 s at the least.
 __device__ __forceinline__ bool wait_polling(uint32_t bar, uint32_t parity, uint32_t abort_at) {
   if (mbar_try_wait(bar, parity)) return true;
   for (int polls = 1 << 22; polls; --polls) {
@@ -721,7 +724,8 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   Fixed* fixed = (Fixed*)(recs + NS);
   Plan* plan = (Plan*)(fixed + NS);
   Run* runs = (Run*)(((uintptr_t)(plan + 1) + 15) & ~(uintptr_t)15);
-  static_assert(sizeof(StepRec) % 16 == 0 && kWords + 16 + NS * (sizeof(StepRec) + sizeof(Fixed)) + sizeof(Plan) + 16 + kRuns * sizeof(Run) <= kOperands, "service area");
+  static_assert(sizeof(StepRec) % 16 == 0 && kWords + 16 + NS * (sizeof(StepRec) + sizeof(Fixed)) + sizeof(Plan) + 16 +
+                                                     kRuns * sizeof(Run) <= kOperands, "service area");
   const uint32_t bar0 = smem_u32(base + kBars);
   auto bar = [&](int i) { return bar0 + 8u * (uint32_t)i; };
   if (P.early && P.sub[0].geo.ctrl->converged) return;
@@ -1585,17 +1589,6 @@ int max_pieces(int n, int m) {
   const long long share = 2ll * kMaxCtas / tiles(m, kBN) + 2;
   return (int)(share < tiles(n, 128) ? share : tiles(n, 128));
 }
-
-struct Carve {
-  char* base;
-  size_t off = 0;
-  template <typename T>
-  T* take(size_t count) {
-    const size_t o = off;
-    off += (count * sizeof(T) + 1023) & ~size_t(1023);
-    return base ? reinterpret_cast<T*>(base + o) : nullptr;
-  }
-};
 
 // The scratch of the per-tile row sums grows with n*m (16 bytes per 256 entries and side): up to this much.
 constexpr size_t kMaxPartialBytes = size_t(2) << 30;

@@ -28,7 +28,9 @@ struct alignas(16) StepRec {
   unsigned todo;                       // kEmitPre | kEmitOut | kCheck | ordinal of the check << 8
 };
 constexpr unsigned kEmitPre = 1, kEmitOut = 2, kCheck = 4;  // write the potentials after this step to pre / out; early-stop test
-constexpr int kTableSteps = 256;                            // records that a problem's table holds
+// Records that a problem's table holds: 8 KB of its scratch, more steps than solves usually take. A longer solve goes on with a
+// second launch behind an upload of the next 256.
+constexpr int kTableSteps = 256;
 
 // What every kernel of a step needs to know about a problem. Cloud 0 = x, cloud 1 = y.
 struct Geo {

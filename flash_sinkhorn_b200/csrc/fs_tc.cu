@@ -103,7 +103,9 @@ __device__ __forceinline__ void write_column_bias(float* at, float pot, const fl
   const float hi = to_tf32(b), r1 = b - hi, mid = to_tf32(r1);
   at[0] = hi; at[1] = mid; at[2] = to_tf32(r1 - mid);
 }
-constexpr int kMaxGrads = 16;  // problems of a launch of gradients (grad_many)
+// Problems of a launch of gradients (grad_many): those of eight debiased items. The parameters of a launch (32 KB) would hold
+// about thirty; a gradient of 300 x 300 points takes 33 us when two share launches, 17 of four, 8.5 of eight and 4.8 of sixteen.
+constexpr int kMaxGrads = 16;
 constexpr int kMaxSub = 4;  // passes per multi-pass launch (keeps the kernel parameters under 4 KB)
 
 // Soft-max warpgroups per 128-row half of the plan-times-matrix kernel: each takes half of every tile's 32-column
@@ -252,7 +254,7 @@ tc_lse_kernel(const __grid_constant__ Launch<NSUB> P) {
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  // With four soft-max warpgroups these take registers from the four service warps (split_registers).
+  // With four soft-max warpgroups these take registers from the four service warps (registers_up).
   constexpr bool kSplitRegisters = NHALF * PARTS == 4;
   if (warp < 4) {
     if (kSplitRegisters) registers_down();
@@ -2038,21 +2040,10 @@ __global__ void __launch_bounds__(256) grad_stage_kernel(const __grid_constant__
   }
 }
 
-// Where the scratch of one job lies behind the control words of all of them.
-struct GradScratch {
-  size_t off = 0;
-  char* base = nullptr;
-  template <typename T>
-  T* take(size_t count) {
-    const size_t o = off;
-    off += (count * sizeof(T) + 1023) & ~size_t(1023);
-    return base ? reinterpret_cast<T*>(base + o) : nullptr;
-  }
-};
 constexpr size_t kGradControl = 64;  // bytes of range words per job
 int grad_tickets(int n, int m) { return detail::pad256(n > m ? n : m) / 128; }
 
-void carve_grad(GradScratch& c, Staged& s, GradCloud* cloud, float** R, float** partial, int n, int m, int d, int prec) {
+void carve_grad(Carve& c, Staged& s, GradCloud* cloud, float** R, float** partial, int n, int m, int d, int prec) {
   const Shape sh = plan_shape(d, prec, 0);
   const PvShape ps = plan_pv(d, prec, d, 0);
   const int rows[2] = {n, m};
@@ -2081,7 +2072,7 @@ size_t grad_many_bytes(int n, int m, int d, int prec) {
   const Shape sh = plan_shape(d, prec, 0);
   const PvShape ps = plan_pv(d, prec, d, 0);
   if (!sh.ok || sh.streamed || sh.bn != 128 || !ps.ok || ps.nslices != 1) return 0;
-  GradScratch c;
+  Carve c;
   Staged s;
   GradCloud cloud[2];
   float *R, *partial;
@@ -2094,7 +2085,7 @@ cudaError_t grad_many(const GradJob* jobs, int cnt, int d, int prec, float cs, f
   const Shape sh = plan_shape(d, prec, 0);
   const PvShape ps = plan_pv(d, prec, d, 0);
   if (!sh.ok || sh.streamed || sh.bn != 128 || !ps.ok || ps.nslices != 1) return cudaErrorNotSupported;
-  GradScratch c;
+  Carve c;
   c.base = (char*)(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
   char* control = c.take<char>(kGradControl * cnt);
   size_t tickets = 0;

@@ -33,6 +33,18 @@ inline Layout operand_layout(int d, int prec, int nlab, int aug) {
   return l;
 }
 
+// Takes arrays from a buffer one after the other, 1024-byte aligned; without a buffer it only counts.
+struct Carve {
+  char* base = nullptr;
+  size_t off = 0;
+  template <typename T>
+  T* take(size_t count) {
+    const size_t o = off;
+    off += (count * sizeof(T) + 1023) & ~size_t(1023);
+    return base ? reinterpret_cast<T*>(base + o) : nullptr;
+  }
+};
+
 struct CloudOps {
   float* opA = nullptr;  // [rows_pad, kp] row-operand form (ones in the bias columns)
   float* opB = nullptr;  // [rows_pad, kp] column-operand form (bias columns rewritten per pass)

@@ -406,7 +406,7 @@ int fs_grad(const float* x, const float* y, int n, int m, int d,
             int prec, void* ws, size_t ws_bytes, void* stream,
             const fs_label_cost* labels);
 
-/* Gradients of the row clouds of 1..16 problems of one dimension in four launches (no reference counterpart):
+/* Gradients of the row clouds of 1..16 problems of one dimension in at most four launches (no reference counterpart):
  *   out_i = 2 cs scale weight_i (x_i - sum_j w_ij y_j / sum_j w_ij), w_ij = exp((pot_j - C_ij)/eps + log_w_j),
  * what fs_grad writes to grad_x with g = pot, a = weight, log_b = log_w. ws: the sum of fs_grad_many_bytes over the items
  * (0 bytes: sizes that go through fs_grad). */
