@@ -757,8 +757,14 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Counts that every role keeps over the steps: tiles, runs, K chunks, meetings of the grid.
-  int jt = 0, seg = 0, chunk = 0;
+  // Counts that every role keeps over the steps: tiles, runs, K chunks (with the ring slot of the next one and its phase: a
+  // division per chunk by the length of the ring cost the streamed kernel a tenth of its rate), meetings of the grid.
+  int jt = 0, seg = 0, chunk = 0, ring = 0;
+  uint32_t ring_phase = 0;
+  auto ring_next = [&]() {
+    ++chunk;
+    if (++ring == P.nstage) { ring = 0; ring_phase ^= 1; }
+  };
   unsigned met = 0;
   // The service warps and the soft-max warps go through the steps in loops of their own: the latter take registers from the
   // former.
@@ -774,7 +780,6 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
       if (warp == 0) {
         // ===================== TMA producer =====================
         if (KS && lane == 0 && has_work) {
-          int& issued = chunk;
           bool ok = true;
 #pragma unroll 1
           for (int w = w_begin, nth = 0; ok && w < w_end; ++nth) {
@@ -784,18 +789,18 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
             for (int t = 0; ok && t < s.len; ++t)
 #pragma unroll 1
               for (int kc = 0; kc < P.nfull; ++kc) {
-                const int st = issued % P.nstage;
-                if (!(ok = mbar_wait(bar(A_EMPTY + st), ((issued / P.nstage) & 1) ^ 1, abort_flag, 2000))) break;
-                mbar_expect_tx(bar(A_FULL + st), kChunk);
-                const uint32_t dst = smem_u32(a_smem + st * kChunk);
-                tma_load_2d(dst, &u.a_full[s.side], kc * 32, (s.rt + t) * 128, bar(A_FULL + st));
-                tma_load_2d(dst + 128 * 128, &u.b_full[s.side], kc * 32, s.ct * kBN, bar(A_FULL + st));
-                ++issued;
+                const uint32_t full = bar(A_FULL + ring);
+                if (!(ok = mbar_wait(bar(A_EMPTY + ring), ring_phase ^ 1, abort_flag, 2000))) break;
+                mbar_expect_tx(full, kChunk);
+                const uint32_t dst = smem_u32(a_smem + ring * kChunk);
+                tma_load_2d(dst, &u.a_full[s.side], kc * 32, (s.rt + t) * 128, full);
+                tma_load_2d(dst + 128 * 128, &u.b_full[s.side], kc * 32, s.ct * kBN, full);
+                ring_next();
               }
             w += s.step;
           }
           if (*abort_flag)  // let every copy issued land before the CTA goes away
-            for (int j = (issued > P.nstage ? issued - P.nstage : 0); j < issued; ++j)
+            for (int j = (chunk > P.nstage ? chunk - P.nstage : 0); j < chunk; ++j)
               mbar_wait_quiet(bar(A_FULL + j % P.nstage), (j / P.nstage) & 1);
         }
         if (!KS && lane == 0 && has_work) {
@@ -876,21 +881,21 @@ __global__ void __launch_bounds__(kThreads, 1) sym_kernel(const __grid_constant_
               tc_fence_after();
               const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kBN);
 #pragma unroll 1
-              for (int kc = 0; kc < P.nfull; ++kc, ++chunk) {
-                const int st = chunk % P.nstage;
-                if (!vote(mbar_wait(bar(A_FULL + st), (chunk / P.nstage) & 1, abort_flag, 2000))) { ok = false; break; }
+              for (int kc = 0; kc < P.nfull; ++kc) {
+                if (!vote(mbar_wait(bar(A_FULL + ring), ring_phase, abort_flag, 2000))) { ok = false; break; }
                 tc_fence_after();
                 if (elect_one()) {
-                  const uint32_t at = smem_u32(a_smem + st * kChunk), al = desc_lo(at), bl = desc_lo(at + 128 * 128);
+                  const uint32_t at = smem_u32(a_smem + ring * kChunk), al = desc_lo(at), bl = desc_lo(at + 128 * 128);
                   const int steps = kc + 1 < P.nfull ? 4 : P.ntail;
 #pragma unroll 1
                   for (int ks = 0; ks < steps; ++ks)
                     umma_step(kc * 4 + ks < P.hs, d_tmem, pack_desc(al + 2 * ks, kDescHi128), pack_desc(bl + 2 * ks, kDescHi128),
                               idesc, idesc_h, (kc | ks) != 0);
-                  umma_commit(bar(A_EMPTY + st));
+                  umma_commit(bar(A_EMPTY + ring));
                   if (kc + 1 == P.nfull) umma_commit(bar(S_FULL + buf));
                 }
                 __syncwarp();
+                ring_next();
               }
             }
           }
