@@ -2026,10 +2026,15 @@ __global__ void __launch_bounds__(256) grad_stage_kernel(const __grid_constant__
     for (int k = lane; k < d; k += 32) { const float v = src[k]; nrm = fmaf(v, v, nrm); }
 #pragma unroll
   for (int o = 16; o; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-  for (int k = lane; k < P.dv_pad; k += 32) {
-    const float v = real && k < d ? src[k] : 0.f, hi = to_tf32(v);
-    c.vt_hi[(size_t)k * c.rows_pad + r] = hi;
-    if (c.vt_lo) c.vt_lo[(size_t)k * c.rows_pad + r] = to_tf32(v - hi);
+  // V^T along the points: the eight of this block are one 32-byte sector of each of its rows. (A warp that stored its own
+  // point's coordinates wrote a sector per word. Whole gradient, us, so and now: 6,000 points exact d = 64 143.0 and 141.0, TF32
+  // d = 128 152.0 and 148.3; 20,000 points exact d = 64 760.6 and 758.3, TF32 d = 128 641 and 636; d = 3 the same.)
+  const int p = (int)blockIdx.x * 8 + (int)(threadIdx.x & 7);
+  for (int k = (int)threadIdx.x >> 3; k < P.dv_pad; k += 32) {
+    const float v = p < c.rows && k < d ? c.src[(size_t)p * d + k] : 0.f, hi = to_tf32(v);
+    const size_t at = (size_t)k * c.rows_pad + p;
+    c.vt_hi[at] = hi;
+    if (c.vt_lo) c.vt_lo[at] = to_tf32(v - hi);
   }
   if (lane == 0) {
     if (real) {
