@@ -103,3 +103,20 @@ def test_launch_that_ends_while_steps_are_one_sided(cta_limit, limit):  # noqa: 
     assert lib.fs_two_sided_steps() > before
     for g, p, k in zip(got, probs, lengths):
         _close(g[:4], _dense(*p[0], eps, k), _size(p[0]))
+
+
+# column tiles of y = pairs per point of x that the end of a one-sided step adds: eight warps with eight offsets and four pairs in
+# flight each (64 and 32 pairs a round), at the edges of a round; x has two pairs per point of y
+@pytest.mark.parametrize("zeros", [False, True])
+@pytest.mark.parametrize("tiles", [1, 8, 9, 31, 33, 64, 65, 97])
+def test_pairs_of_one_sided_steps(tiles, zeros):
+    from flash_sinkhorn_b200 import _lib
+    from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric
+    x, y, a, b = _clouds(130, 128 * (tiles - 1) + 5, 8, seed=tiles)
+    if zeros and tiles > 1:  # a tile of columns that add nothing
+        b[:128] = 0.0
+    args = [torch.as_tensor(v, dtype=torch.float32).cuda() for v in (x, y, a, b)]
+    before = _lib.load().fs_two_sided_steps()
+    got = sinkhorn_flashstyle_symmetric(*args, use_epsilon_scaling=False, eps=0.02, n_iters=1, allow_tf32=False, return_prelast=True)
+    assert _lib.load().fs_two_sided_steps() == before  # three steps, all one-sided
+    _close(got, _dense(x, y, a, b, 0.02, 1), _size((x, y, a, b)))
