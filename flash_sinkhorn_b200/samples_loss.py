@@ -21,6 +21,7 @@ from flash_sinkhorn_b200 import _lib
 from flash_sinkhorn_b200._autograd import _LossTerms, _SinkhornConfig, _SinkhornCostFn, _SinkhornLossFn
 from flash_sinkhorn_b200.kernels._common import epsilon_schedule, log_weights, max_diameter
 from flash_sinkhorn_b200.sinkhorn_solvers import (
+    _same_tensor,
     sinkhorn_flashstyle_symmetric_batched,
     sinkhorn_flashstyle_alternating,
     sinkhorn_flashstyle_symmetric,
@@ -337,10 +338,13 @@ class SamplesLoss(torch.nn.Module):
             if single:
                 xd, yd, wa, wb = (t.unsqueeze(0) for t in (xd, yd, wa, wb))
             schedules = self._term_schedules(xd, yd)
-            log_a, log_b = log_weights(wa).contiguous(), log_weights(wb).contiguous()
+            x32, log_a = _lib.f32c(xd), log_weights(wa).contiguous()
+            # a cloud against itself is a self-transport problem
+            y32 = x32 if _same_tensor(yd, xd) else _lib.f32c(yd)
+            log_b = log_a if _same_tensor(wb, wa) else log_weights(wb).contiguous()
             try:
-                sols = solve_loss_terms(_lib.f32c(xd), _lib.f32c(yd), log_a, log_b, schedules, debias=self.debias, labels=labels,
-                                        prec=prec, cost_scale=self.cost_scale, rho_x=self.rho_x, rho_y=self.rho_y,
+                sols = solve_loss_terms(x32, y32, log_a, log_b, schedules, debias=self.debias, labels=labels, prec=prec,
+                                        cost_scale=self.cost_scale, rho_x=self.rho_x, rho_y=self.rho_y,
                                         last_extrapolation=self.last_extrapolation)
             except torch.cuda.OutOfMemoryError:
                 if labels is None:

@@ -485,14 +485,14 @@ def solve_loss_terms(x, y, log_a, log_b, schedules, *, debias, labels, prec, cos
     """Potentials of the terms of a batch of losses: OT(x,y) and, debiased, OT(x,x) and OT(y,y), of clouds ``x [B, n, d]``,
     ``y [B, m, d]`` and log-weights ``[B, n]``, ``[B, m]`` (fp32, contiguous); ``schedules[term][item]``: eps lists. Returns
     one ``(f, g, f_pre, g_pre)`` of ``[B, rows]`` tensors per term; a self term (of a symmetric label table, if any) has f
-    for g."""
+    for g, and so has OT(x,y) where ``y`` is ``x`` and ``log_b`` is ``log_a``."""
     (B, n, d), m = x.shape, y.shape[1]
     dev = x.device
     new = lambda k: torch.empty((B, k), device=dev, dtype=torch.float32)  # noqa: E731
     sides = [((x, log_a, n), (y, log_b, m)), ((x, log_a, n), (x, log_a, n)), ((y, log_b, m), (y, log_b, m))]
     items, outs, arrays = [], [], {}
     for term, ((u, lu, r), (v, lv, c)) in enumerate(sides[: 3 if debias else 1]):
-        same = term > 0 and rho_x == rho_y and (labels is None or labels[0].symmetric)
+        same = u is v and lu is lv and rho_x == rho_y and (labels is None or (term > 0 and labels[0].symmetric))
         f, f_pre = new(r), new(r)
         g, g_pre = (f, f_pre) if same else (new(c), new(c))
         outs.append((f, g, f_pre, g_pre))

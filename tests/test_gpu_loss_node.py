@@ -221,3 +221,29 @@ def test_label_table_of_the_call():
             table.copy_(torch.arange(16.0).reshape(4, 4))
         grads.append(torch.autograd.grad(val, xs)[0])
     assert _err(grads[1], grads[0]) < 1e-6  # the same numbers go in
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(reach=2.0), dict(reach_x=2.0)])
+@pytest.mark.parametrize("single,debias", [(True, True), (False, True), (False, False)])
+def test_cloud_against_itself(monkeypatch, single, debias, kw):
+    """The same cloud and weights on both sides: OT(x,y) is a self-transport problem too (of equal relaxations), with the values and
+    gradients of a copy of the cloud."""
+    from flash_sinkhorn_b200 import SamplesLoss, samples_loss
+    x, _, a, _ = _inputs(2, 300, 1, 20, seed=5)
+    if single:
+        x, a = x[0], a[0]
+    outs, solves, solve = [], [], samples_loss.solve_loss_terms
+    monkeypatch.setattr(samples_loss, "solve_loss_terms", lambda *args, **kws: solves.append(solve(*args, **kws)) or solves[-1])
+    loss = SamplesLoss("sinkhorn", eps=3.0, n_iters=12, use_epsilon_scaling=False, debias=debias, normalize=False, allow_tf32=False, **kw)
+    for copy in (False, True):
+        u, w = x.clone().requires_grad_(True), a.clone().requires_grad_(True)
+        val = loss(w, u, w.clone() if copy else w, u.clone() if copy else u)
+        outs.append((val.detach(), torch.autograd.grad(val.sum(), (u, w))))
+        f, g = solves[-1][0][:2]
+        assert (f is g) == (not copy and "reach_x" not in kw)
+    size = float((x * x).sum(-1).max())
+    assert float((outs[0][0] - outs[1][0]).abs().max()) < 1e-5 * size
+    (gx, ga), (want_gx, want_ga) = outs[0][1], outs[1][1]
+    # a debiased loss is at its minimum: what the terms' gradients leave is rounding of 4 w |x|, in weights that of a potential
+    assert float((gx - want_gx).abs().max()) < 3e-4 * 4 * float(a.max()) * size ** 0.5
+    assert float((ga - want_ga).abs().max()) < 2e-5 * size
