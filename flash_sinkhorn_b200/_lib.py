@@ -258,7 +258,7 @@ class LabelCost:
         return ctypes.cast(ctypes.pointer(self.struct), c_void_p)
 
     @staticmethod
-    def make(label_x, label_y, label_cost_matrix, lambda_x, lambda_y, n, m, device):
+    def make(label_x, label_y, label_cost_matrix, lambda_x, lambda_y, n, m, device, of_divergence=False):
         if label_x is None or label_y is None or label_cost_matrix is None or float(lambda_y) == 0.0:
             return None
         if label_x.shape[0] != n:
@@ -270,9 +270,10 @@ class LabelCost:
         if label_cost_matrix.shape[0] != label_cost_matrix.shape[1]:
             raise ValueError("label_cost_matrix must be square (V, V)")
         V = label_cost_matrix.shape[0]
-        # one read of the device for both ranges and the symmetry of the table
+        # one read of the device for both ranges and, where self terms ask for it, the symmetry of the table
         ends = [lab.min().to(torch.int64) for lab in (label_x, label_y)] + [lab.max().to(torch.int64) for lab in (label_x, label_y)]
-        ends.append((label_cost_matrix == label_cost_matrix.t()).all().to(torch.int64))
+        if of_divergence:
+            ends.append((label_cost_matrix == label_cost_matrix.t()).all().to(torch.int64))
         ends = torch.stack([e.to(ends[0].device) for e in ends]).tolist()
         for name, lo, hi in (("label_x", ends[0], ends[2]), ("label_y", ends[1], ends[3])):
             if hi >= V or lo < 0:
@@ -282,7 +283,7 @@ class LabelCost:
         return LabelCost(label_x.to(dtype=torch.int32, device=device).contiguous(),
                          label_y.to(dtype=torch.int32, device=device).contiguous(),
                          label_cost_matrix.to(dtype=torch.float32, device=device).contiguous(),
-                         lambda_x, lambda_y, bool(ends[4]))
+                         lambda_x, lambda_y, of_divergence and bool(ends[4]))
 
     def divergence_terms(self):
         """Label costs of OT(x,y), OT(x,x) and OT(y,y) from that of OT(x,y), with labels and a table of their own storage: the

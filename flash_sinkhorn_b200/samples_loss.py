@@ -328,7 +328,8 @@ class SamplesLoss(torch.nn.Module):
         if not all(_lib.load().fs_two_sided(r, c, d, prec) for r, c in sizes):
             return None
         with torch.no_grad():
-            labels = _lib.LabelCost.make(label_x, label_y, self.label_cost_matrix, self.lambda_x, self.lambda_y, n, m, dev)
+            labels = _lib.LabelCost.make(label_x, label_y, self.label_cost_matrix, self.lambda_x, self.lambda_y, n, m, dev,
+                                         of_divergence=True)
             if labels is not None:
                 if any(_lib.symmetric_bytes(r, c, d, prec, labels.V) == _lib.symmetric_bytes(r, c, d, prec, labels.V, two_sided=False)
                        for r, c in sizes):

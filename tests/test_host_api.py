@@ -121,3 +121,21 @@ def test_epsilon_schedule_argument_checks():
             epsilon_schedule(*bad)
     sched = epsilon_schedule(4.0, 0.5, 0.5)
     assert sched[0] == 16.0 and sched[-1] == 0.25 and all(a >= b for a, b in zip(sched, sched[1:]))
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+def test_symmetry_of_label_tables(symmetric):
+    """Only divergences, whose self terms ask for it, look at the table: transposes compared once, NaN is not symmetric."""
+    from flash_sinkhorn_b200 import _lib
+    table = torch.arange(9.0).reshape(3, 3)
+    table = table + table.t() if symmetric else table
+    args = (1.0, 2.0, 3, 2, torch.device("cpu"))
+    labels = torch.tensor([0, 2, 1]), torch.tensor([1, 1])
+    assert not _lib.LabelCost.make(*labels, table, *args).symmetric
+    made = _lib.LabelCost.make(*labels, table, *args, of_divergence=True)
+    assert made.symmetric == symmetric
+    terms = made.divergence_terms()
+    assert [t.symmetric for t in terms] == [symmetric] * 3
+    assert terms[0].table.data_ptr() != made.table.data_ptr() and torch.equal(terms[0].table, table)
+    table[1, 2] = table[2, 1] = float("nan")
+    assert not _lib.LabelCost.make(*labels, table, *args, of_divergence=True).symmetric
