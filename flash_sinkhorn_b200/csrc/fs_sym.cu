@@ -53,7 +53,6 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstring>
 
 namespace fs {
@@ -1556,7 +1555,7 @@ __global__ void sym_emit_kernel(const __grid_constant__ EmitJobs P) {
 }
 
 // ------------------------------------------------------------------ host side
-std::atomic<long long> g_meeting_limit{kMeetingLimit};
+thread_local long long t_meeting_limit = kMeetingLimit;  // of the solves that this thread launches, no other's
 enum Kind { RESIDENT = 0, STREAMED = 1, WIDE = 2, SMALL = 3 };
 struct Shape {
   int kind, bm, bn;
@@ -1678,7 +1677,7 @@ cudaError_t steps_n(Problem* const* p, int cnt, int t0, int t1, int t_table, boo
   lp.t0 = t0; lp.t1 = t1; lp.t_table = t_table;
   lp.early = early ? 1 : 0;
   lp.threshold = threshold;
-  lp.meet_limit = g_meeting_limit.load(std::memory_order_relaxed);
+  lp.meet_limit = t_meeting_limit;
   long long most = 0;
   for (int i = 0; i < cnt; ++i) {
     const Problem& q = *p[i];
@@ -1913,7 +1912,9 @@ long long two_sided_steps() {
 }
 
 long long set_meeting_limit(long long clocks) {
-  return g_meeting_limit.exchange(clocks < 0 ? kMeetingLimit : clocks, std::memory_order_relaxed);
+  const long long was = t_meeting_limit;
+  t_meeting_limit = clocks < 0 ? kMeetingLimit : clocks;
+  return was;
 }
 
 int read_error_flag() {

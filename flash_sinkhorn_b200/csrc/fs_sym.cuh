@@ -96,7 +96,8 @@ int kernel_of(int n, int m, int d, int prec, int nlab);
 // Two-sided steps that problems have taken on the current device (-1: error).
 long long two_sided_steps();
 
-// Clocks that the CTAs of a solve wait for one another before they give up; returns what it was. Negative: the usual ~4 s.
+// Clocks that the CTAs of a solve wait for one another before they give up, for solves that the calling
+// thread launches; returns what it was. Negative: the usual ~4 s.
 long long set_meeting_limit(long long clocks);
 int read_error_flag();
 int clear_error_flag();

@@ -146,7 +146,8 @@ int fs_two_sided_kernel(int n, int m, int d, int prec);
 long long fs_two_sided_steps(void);
 /* SM clocks that the thread blocks of a symmetric solve wait for one another at each end of a step before all of them give up
  * and the solve ends with fs_device_error() set (its results are then void). Negative: the default, about four seconds.
- * Returns the previous value. For tests of that path: with 0 a block gives up at the first look that finds others missing. */
+ * Holds for the solves that the calling thread launches. Returns the previous value. For tests of that path: with 0 a block
+ * gives up at the first look that finds others missing. */
 long long fs_set_meeting_limit(long long clocks);
 
 /* Host arithmetic only (no reference counterpart): the CTA count a streaming pass over n_row_blocks x

@@ -139,3 +139,22 @@ def test_symmetry_of_label_tables(symmetric):
     assert terms[0].table.data_ptr() != made.table.data_ptr() and torch.equal(terms[0].table, table)
     table[1, 2] = table[2, 1] = float("nan")
     assert not _lib.LabelCost.make(*labels, table, *args, of_divergence=True).symmetric
+
+
+def test_meeting_limit_is_of_one_thread():
+    import threading
+    from flash_sinkhorn_b200 import _lib
+    lib = _lib.load()
+    usual = lib.fs_set_meeting_limit(-1)
+    seen = []
+
+    def other():
+        seen.append(lib.fs_set_meeting_limit(0))
+        seen.append(lib.fs_set_meeting_limit(-1))
+
+    lib.fs_set_meeting_limit(7)
+    worker = threading.Thread(target=other)
+    worker.start()
+    worker.join()
+    assert seen == [usual, 0]  # another thread starts from the usual limit,
+    assert lib.fs_set_meeting_limit(-1) == 7  # and what it sets stays with it
