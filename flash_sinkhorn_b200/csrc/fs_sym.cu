@@ -483,7 +483,6 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
     const StepRec& rec = recs[v.sub];
     const int c = v.c, i = v.i0 + warp * 32 + lane;
     auto fetch = [&](const float* at) { return __ldcg(reinterpret_cast<const float4*>(at + 4 * lane)); };
-    float m_i = -INFINITY;
     if (v.two) {
       const size_t row_pitch = g.pad[0], col_pitch = g.pad[1];
       float4 s0 = make_float4(0.f, 0.f, 0.f, 0.f), s1 = s0;
@@ -503,7 +502,8 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
       }
       *reinterpret_cast<float4*>(rd + warp * 128 + 4 * lane) = make_float4(s0.x + s1.x, s0.y + s1.y, s0.z + s1.z, s0.w + s1.w);
     } else {
-      // (offset, sum) pairs: the largest offset of each point over the whole team first, then the sums against it
+      // (offset, sum) pairs. Warp w and warp w + 4 find the largest offset of the pairs k = w mod 4, warp w adds them in their
+      // order, so that potentials do not depend on how many warps load.
       const size_t pitch = g.pad[c];
       float4 m = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY), s = make_float4(0.f, 0.f, 0.f, 0.f);
       auto larger = [](const float4& p, const float4& q) {
@@ -519,39 +519,47 @@ __device__ __forceinline__ bool end_step(const L& P, const Plan& plan, const Fix
 #pragma unroll
         for (int e = 0; e < 8; ++e) m = larger(m, x[e]);
       }
-      *reinterpret_cast<float4*>(rd + warp * 128 + 4 * lane) = m;
+      float4* own = reinterpret_cast<float4*>(rd + warp * 128 + 4 * lane);
+      *own = m;
       team_sync();
+      if (warp < 4) {
+        float4* sum = own + 128;  // of warp w + 4: read here by the thread that writes its sum there
+        m = larger(m, *sum);
+        *own = m;
+        for (int k = warp; k < v.count; k += 16) {
+          float4 x[4], o[4];
 #pragma unroll
-      for (int k = 0; k < kTeamWarps; ++k) {
-        m = larger(m, *reinterpret_cast<const float4*>(rd + k * 128 + 4 * lane));
-        if (warp < 4) m_i = fmaxf(m_i, rd[k * 128 + warp * 32 + lane]);
-      }
-      for (int k = warp; k < v.count; k += 4 * kTeamWarps) {
-        float4 x[4], o[4];
+          for (int e = 0; e < 4; ++e) {
+            const int at = k + 4 * e;
+            x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+            o[e] = m;
+            if (at < v.count) {
+              x[e] = fetch(v.cols + at * pitch);
+              o[e] = fetch(v.rows + at * pitch);
+            }
+          }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int at = k + kTeamWarps * e;
-          x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-          o[e] = m;
-          if (at < v.count) {
-            x[e] = fetch(v.cols + at * pitch);
-            o[e] = fetch(v.rows + at * pitch);
+          for (int e = 0; e < 4; ++e) {
+            s.x += x[e].x * ex2(o[e].x - m.x); s.y += x[e].y * ex2(o[e].y - m.y);
+            s.z += x[e].z * ex2(o[e].z - m.z); s.w += x[e].w * ex2(o[e].w - m.w);
           }
         }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s.x += x[e].x * ex2(o[e].x - m.x); s.y += x[e].y * ex2(o[e].y - m.y);
-          s.z += x[e].z * ex2(o[e].z - m.z); s.w += x[e].w * ex2(o[e].w - m.w);
-        }
+        *sum = s;
       }
-      team_sync();  // everyone has read the offsets
-      *reinterpret_cast<float4*>(rd + warp * 128 + 4 * lane) = s;
     }
     team_sync();
     if (warp < 4) {
-      const float* at_s = rd + warp * 32 + lane;
-      const float m = v.two ? 0.f : m_i;
-      const float s = ((at_s[0] + at_s[128]) + (at_s[256] + at_s[384])) + ((at_s[512] + at_s[640]) + (at_s[768] + at_s[896]));
+      const float* at_m = rd + warp * 32 + lane;
+      const float* at_s = at_m + 512;
+      float m = 0.f, s = 0.f;
+      if (v.two) {
+        s = ((at_m[0] + at_m[128]) + (at_m[256] + at_m[384])) + ((at_s[0] + at_s[128]) + (at_s[256] + at_s[384]));
+      } else {
+        m = fmaxf(fmaxf(at_m[0], at_m[128]), fmaxf(at_m[256], at_m[384]));
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (at_s[k * 128] != 0.f) s += at_s[k * 128] * ex2(at_m[k * 128] - m);
+      }
       float st_u = -INFINITY, st_l = -INFINITY, st_dx = -INFINITY, st_dn = -INFINITY, move = 0.f;
       if (i < g.n[c]) {
         // log2 of the weighted sum with the point's own bias inside; the candidate takes that bias out again
