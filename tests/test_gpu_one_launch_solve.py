@@ -105,10 +105,10 @@ def test_launch_that_ends_while_steps_are_one_sided(cta_limit, limit):  # noqa: 
         _close(g[:4], _dense(*p[0], eps, k), _size(p[0]))
 
 
-# column tiles of y = pairs per point of x that the end of a one-sided step adds: eight warps with eight offsets and four pairs in
-# flight each (64 and 32 pairs a round), at the edges of a round; x has two pairs per point of y
+# column tiles of y = pairs per point of x that the end of a one-sided step adds: eight warps with eight offsets, four with four pairs
+# in flight each (64 and 16 pairs a round), at the edges of a round; x has two pairs per point of y
 @pytest.mark.parametrize("zeros", [False, True])
-@pytest.mark.parametrize("tiles", [1, 8, 9, 31, 33, 64, 65, 97])
+@pytest.mark.parametrize("tiles", [1, 8, 9, 16, 17, 31, 33, 64, 65, 97])
 def test_pairs_of_one_sided_steps(tiles, zeros):
     from flash_sinkhorn_b200 import _lib
     from flash_sinkhorn_b200.sinkhorn_solvers import sinkhorn_flashstyle_symmetric
